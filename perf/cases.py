@@ -216,9 +216,8 @@ def prepare(case, seed):
         layer.prepare_int8(scale, state["bias"])
         state["layer"] = layer
         return state
-    x = normal(t.n_in, C).half()
+    x, w, extra = _values(case, seed, t.n_in, t.n_out)
     if case["kind"] == "pairs":
-        w = (normal(kv, C, K) / math.sqrt(kv * C)).half()
         out = torch.zeros((t.n_out, K), dtype=torch.float16, device="cuda")
         state.update(x=x, w=w, out=out, calls=[])
         for f in range(kv):
@@ -228,12 +227,11 @@ def prepare(case, seed):
         if case["api"] == "sequence":
             state["sequence"] = prepare_gemm_sequence([_gemm_params(state, *c) for c in state["calls"]])
         return state
-    w = (normal(K, kv, C) / math.sqrt(kv * C)).half()
     state.update(x=x, w=w, out=torch.zeros((t.n_out, K), dtype=torch.float16, device="cuda"))
     if case["kind"] == "infer":
-        state["bias"] = normal(K).half()
+        state["bias"] = extra
         return state
-    state["dout"] = normal(t.n_out, K).half()
+    state["dout"] = extra
     state["din"] = torch.zeros((t.n_in, C), dtype=torch.float16, device="cuda")
     state["dw"] = torch.zeros((K, kv, C), dtype=torch.float32 if case.get("dw") == "f32" else torch.float16, device="cuda")
     if case["api"] == "prepared":
@@ -241,7 +239,22 @@ def prepare(case, seed):
     return state
 
 
-def _prepare_dense(case, seed):
+def _values(case, seed, n_in, n_out):
+    """fp16 rows, weights and the third operand (bias, or the output's gradient) of a sparse case."""
+    gen = _generator(seed + 1)
+    C, K, kv = case["C"], case["K"], case["ksize"] ** 3
+
+    def normal(*shape):
+        return torch.randn(shape, generator=gen, device="cuda")
+
+    x = normal(n_in, C).half()
+    w = (normal(*((kv, C, K) if case["kind"] == "pairs" else (K, kv, C))) / math.sqrt(kv * C)).half()
+    if case["kind"] == "pairs":
+        return x, w, None
+    return x, w, (normal(K) if case["kind"] == "infer" else normal(n_out, K)).half()
+
+
+def _dense_values(case, seed):
     gen = _generator(seed)
     B, H, W, C, K, k, s = (case[q] for q in ("batch", "height", "width", "C", "K", "ksize", "stride"))
 
@@ -250,6 +263,11 @@ def _prepare_dense(case, seed):
 
     x, w = half(B, H, W, C), half(K, k, k, C, scale=1 / math.sqrt(k * k * C))
     dout = half(B, (H + 2 * (k // 2) - k) // s + 1, (W + 2 * (k // 2) - k) // s + 1, K)
+    return x, w, dout
+
+
+def _prepare_dense(case, seed):
+    x, w, dout = _dense_values(case, seed)
     return {"case": case, "x": x, "w": w, "dout": dout, "out": torch.zeros_like(dout), "din": torch.zeros_like(x),
             "dw": torch.zeros_like(w)}
 
@@ -380,3 +398,76 @@ def tolerance(case):
     if case["kind"] == "pairs":
         return {"rel": 1.6e-3, "max": 1.5e-2}
     return {"rel": 8.4e-4, "max": 2e-3}
+
+
+# ---------------------------------------------------------------- the same in 64 bits
+def _keys(c, grid):
+    return ((c[:, 0] * grid[0] + c[:, 1]) * grid[1] + c[:, 2]) * grid[2] + c[:, 3]
+
+
+def _neighbours(case, coords):
+    """(number of output rows, [(input rows, output rows) per filter offset])."""
+    k, s, grid = case["ksize"], case["stride"], _grid(case)
+    offsets = [(z, y, x) for z in range(k) for y in range(k) for x in range(k)]
+    coords = coords.long()
+    shift = lambda r: torch.tensor((0,) + r, device="cuda") - torch.tensor([0] + 3 * [k // 2], device="cuda")
+    out = coords
+    if s != 1:  # every position that reads some input row, in row-major order
+        ogrid = [(g + 2 * (k // 2) - k) // s + 1 for g in grid]
+        limit = torch.tensor(ogrid, device="cuda")
+        found = []
+        for r in offsets:
+            at = (coords - shift(r))[:, 1:]
+            ok = ((at >= 0) & (at % s == 0) & (at // s < limit)).all(1)
+            found.append(_keys(torch.cat([coords[ok, :1], at[ok] // s], 1), ogrid))
+        key = torch.unique(torch.cat(found))
+        out = torch.stack([key // (ogrid[0] * ogrid[1] * ogrid[2]), key // (ogrid[1] * ogrid[2]) % ogrid[0],
+                           key // ogrid[2] % ogrid[1], key % ogrid[2]], 1)
+    keys, order = torch.sort(_keys(coords, grid))
+    limit = torch.tensor(grid, device="cuda")
+    pairs = []
+    for r in offsets:
+        at = torch.cat([out[:, :1], out[:, 1:] * s], 1) + shift(r)
+        inside = ((at[:, 1:] >= 0) & (at[:, 1:] < limit)).all(1)
+        want = _keys(at, grid)
+        place = torch.searchsorted(keys, want).clamp(max=len(keys) - 1)
+        rows = torch.nonzero(inside & (keys[place] == want)).flatten()
+        pairs.append((order[place[rows]], rows))
+    return len(out), pairs
+
+
+def exact(case, seed):
+    """Results of floating point in 64 bits; tables and int8 rows are compared bit for bit instead."""
+    if case["kind"] in ("tables", "infer8"):
+        return None
+    if case["kind"] == "dense":
+        x, w, dout = (v.double() for v in _dense_values(case, seed))
+        k, s, half = case["ksize"], case["stride"], case["ksize"] // 2
+        H, W = dout.shape[1:3]
+        x = torch.nn.functional.pad(x, (0, 0, half, half, half, half))
+        out, din, dw = torch.zeros_like(dout), torch.zeros_like(x), torch.zeros_like(w)
+        for y in range(k):
+            for z in range(k):
+                rows = (slice(None), slice(y, y + s * (H - 1) + 1, s), slice(z, z + s * (W - 1) + 1, s))
+                out += x[rows] @ w[:, y, z].T
+                din[rows] += dout @ w[:, y, z]
+                dw[:, y, z] = dout.flatten(0, 2).T @ x[rows].flatten(0, 2)
+        return {"out": out, "din": din[:, half:-half, half:-half], "dw": dw}
+    coords = _coords(case, seed)
+    n_out, pairs = _neighbours(case, coords)
+    x, w, extra = _values(case, seed, len(coords), n_out)
+    x, w = x.double(), w.double()
+    if case["kind"] == "pairs":
+        w = w.permute(2, 0, 1)
+    out = torch.zeros((n_out, case["K"]), dtype=torch.float64, device="cuda")
+    for f, (i, o) in enumerate(pairs):
+        out[o] += x[i] @ w[:, f].T
+    if case["kind"] == "pairs":
+        return out
+    if case["kind"] == "infer":
+        return (out + extra.double()).clamp(min=0)
+    dout, din, dw = extra.double(), torch.zeros_like(x), torch.zeros_like(w)
+    for f, (i, o) in enumerate(pairs):
+        din[i] += dout[o] @ w[:, f]
+        dw[:, f] = dout[o].T @ x[i]
+    return {"out": out, "din": din, "dw": dw}
