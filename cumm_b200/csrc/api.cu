@@ -507,13 +507,19 @@ namespace {
 
 struct PairgenLayout {
   cb2pg::Geometry g;
-  uint32_t cap_in, cap_set;  // hash capacities (powers of two)
+  cb2pg::SortShape shape;
+  uint32_t cap_in, cap_set;  // hash capacities (powers of two); 0 = not used
+  bool exact;                // a voxel's linear index fits the hash table's 32-bit tag
+  bool mirror;               // the backward table is the forward one with the offsets reversed
+  bool bitmap;               // active outputs of a strided conv through a bitmap of the output grid
+  long long bitmap_words;    // whole blocks
   long long list_cap;        // active outputs a strided conv can have at most
   long long nmax;            // rows the mask sorts may have to hold
   int key_bits;
-  int words;                 // mask words per row
-  size_t off_in_keys, off_in_vals, off_set_keys, off_list_a, off_list_b, off_m, off_v, off_hist, off_counters, total;
-  size_t off_rows, off_k;    // several mask words per row: the unsorted rows, and the key array of a word's sort
+  size_t hist_ints;          // of one side
+  size_t off_counters, off_hash, off_bits, off_word_first, off_block_first, off_set_keys, off_list_a, off_list_b,
+      off_key_hist, off_hist, total;
+  size_t off_rows[2], off_m[2], off_v[2];  // per side: unsorted masks (several words), mask and row scratch
 };
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -548,9 +554,16 @@ int pairgen_layout(const cb2_pairgen_args *a, PairgenLayout *L) {
     for (int i = 0; i < 3; ++i)
       CB2_CHECK_ARG(a->stride[i] == 1, "a submanifold convolution has stride 1");
   L->g.kv = static_cast<int>(kv);
-  L->words = static_cast<int>((kv + 31) / 32);
+  L->shape = cb2pg::sort_shape(L->g.kv);
   L->g.batch_size = a->batch_size;
-  L->cap_in = pow2_at_least(2ull * static_cast<unsigned long long>(a->n_in));
+  const long long n_in = a->n_in;
+  unsigned __int128 in_cells = a->batch_size;
+  L->mirror = a->subm;
+  for (int i = 0; i < 3; ++i) {
+    in_cells *= static_cast<unsigned>(a->grid[i]);
+    L->mirror = L->mirror && a->ksize[i] % 2 == 1 && 2ll * a->pad[i] == static_cast<long long>(a->ksize[i] - 1) * a->dil[i];
+  }
+  L->exact = in_cells < 0xffffffffull;
   // outputs an input can feed: per axis, the offsets r with (in + pad - r * dil) divisible by the stride
   long long per_input = 1;
   for (int i = 0; i < 3; ++i) {
@@ -563,10 +576,17 @@ int pairgen_layout(const cb2_pairgen_args *a, PairgenLayout *L) {
     const int period = a->stride[i] / gcd;  // r takes every period-th value
     per_input *= std::min(a->ksize[i], (a->ksize[i] + period - 1) / period);
   }
-  L->list_cap = a->subm ? 0 : std::min<long long>(static_cast<long long>(a->n_in) * per_input, cells);
+  L->list_cap = a->subm ? 0 : std::min<long long>(n_in * per_input, cells);
   CB2_CHECK_RT(L->list_cap < (1ll << 30), "too many candidate outputs (%lld)", L->list_cap);
-  L->cap_set = a->subm ? 0 : pow2_at_least(2ull * static_cast<unsigned long long>(L->list_cap));
-  L->nmax = std::max<long long>(a->subm ? a->n_in : L->list_cap, a->n_in);
+  // The bitmap is cleared, counted and read once each whatever the scene, so it has to be small
+  // beside the scene or small altogether: up to 64 bytes per input voxel, or 4 MiB.
+  L->bitmap = !a->subm && cells < (1ll << 31) - 64 && cells / 8 <= std::max<long long>(4 << 20, 64 * n_in);
+  const long long block_words = cb2pg::kBitmapBlockWords;
+  L->bitmap_words = L->bitmap ? ((cells + 31) / 32 + block_words - 1) / block_words * block_words : 0;
+  L->cap_in = L->bitmap ? 0 : pow2_at_least(2ull * static_cast<unsigned long long>(n_in));
+  L->cap_set = (a->subm || L->bitmap) ? 0 : pow2_at_least(2ull * static_cast<unsigned long long>(L->list_cap));
+  const long long keys_cap = L->cap_set ? L->list_cap : 0;
+  L->nmax = std::max<long long>(a->subm ? n_in : L->list_cap, n_in);
   L->key_bits = 1;
   while (L->key_bits < 63 && (1ll << L->key_bits) < cells)
     ++L->key_bits;
@@ -577,75 +597,141 @@ int pairgen_layout(const cb2_pairgen_args *a, PairgenLayout *L) {
     return at;
   };
   L->off_counters = take(256);
-  L->off_in_keys = take(static_cast<size_t>(L->cap_in) * 8);
-  L->off_in_vals = take(static_cast<size_t>(L->cap_in) * 4);
+  L->off_hash = take(static_cast<size_t>(L->cap_in) * 8);
+  L->off_bits = take(static_cast<size_t>(L->bitmap_words) * 4);
+  L->off_word_first = take(static_cast<size_t>(L->bitmap_words) * 4);
+  L->off_block_first = take(static_cast<size_t>(L->bitmap_words / block_words) * 4);
   L->off_set_keys = take(static_cast<size_t>(L->cap_set) * 8);
-  L->off_list_a = take(static_cast<size_t>(L->list_cap) * 8);
-  L->off_list_b = take(static_cast<size_t>(L->list_cap) * 8);
-  L->off_m = take(static_cast<size_t>(L->nmax) * 4);
-  L->off_v = take(static_cast<size_t>(L->nmax) * 4);
-  const long long sort_n = std::max<long long>(L->nmax, L->list_cap);
-  L->off_hist = take(static_cast<size_t>(256) * ((sort_n + cb2pg::kSortTile - 1) / cb2pg::kSortTile + 1) * 4);
-  L->off_rows = L->off_k = 0;
-  if (L->words > 1) {
-    L->off_rows = take(static_cast<size_t>(L->nmax) * L->words * 4);
-    L->off_k = take(static_cast<size_t>(L->nmax) * 4);
+  L->off_list_a = take(static_cast<size_t>(keys_cap) * 8);
+  L->off_list_b = take(static_cast<size_t>(keys_cap) * 8);
+  L->off_key_hist = take(keys_cap ? static_cast<size_t>(256) * ((keys_cap + cb2pg::kKeySortTile - 1) / cb2pg::kKeySortTile + 1) * 4 : 0);
+  L->hist_ints = cb2pg::sort_hist_ints(L->shape, L->nmax);
+  L->off_hist = take(2 * L->hist_ints * 4);
+  for (int side = 0; side < 2; ++side) {
+    const size_t n = static_cast<size_t>(side == 0 ? L->nmax : n_in);
+    L->off_rows[side] = take(L->shape.words > 1 ? n * L->shape.words * 4 : 0);
+    L->off_m[side] = take(L->shape.words > 1 ? 0 : n * 4);
+    L->off_v[side] = take(n * 4);
   }
   L->total = off;
   return CB2_OK;
 }
 
-// Stable ascending sort of n keys (and values) on `bits` low bits, 8 per pass, ping-ponging
-// between the result buffers and the scratch buffers.  The unsorted input has to be where
-// sort_source() says -- the scratch pair for an odd number of passes, the result pair for an
-// even number -- so that the last pass lands in the result buffers.
-inline int sort_passes(int bits) { return bits <= 8 ? 1 : (bits + 7) / 8; }
-template <typename T> T *sort_source(T *result, T *scratch, int bits) {
-  return sort_passes(bits) % 2 ? scratch : result;
+// Ascending sort of n output keys on `bits` low bits, 8 per pass, ping-ponging between the result
+// buffer and the scratch buffer.  The unsorted input has to be where key_sort_source() says -- the
+// scratch buffer for an odd number of passes, the result buffer for an even number.
+inline int key_sort_passes(int bits) { return bits <= 8 ? 1 : (bits + 7) / 8; }
+unsigned long long *key_sort_source(unsigned long long *result, unsigned long long *scratch, int bits) {
+  return key_sort_passes(bits) % 2 ? scratch : result;
 }
-template <typename K, bool HAS_VAL>
-int radix_sort(K *k_result, int *v_result, K *k_scratch, int *v_scratch, int n, int bits, int *hist, cudaStream_t s) {
+int key_sort(unsigned long long *result, unsigned long long *scratch, int n, int bits, int *hist, cudaStream_t s) {
   if (n <= 0)
     return CB2_OK;
-  const int passes = sort_passes(bits);
-  const int ntiles = (n + cb2pg::kSortTile - 1) / cb2pg::kSortTile;
-  K *ks = sort_source(k_result, k_scratch, bits), *kd = (ks == k_result) ? k_scratch : k_result;
-  int *vs = sort_source(v_result, v_scratch, bits), *vd = (vs == v_result) ? v_scratch : v_result;
-  for (int p = 0; p < passes; ++p) {
-    cb2pg::sort_hist_kernel<K><<<ntiles, cb2pg::kSortThreads, 0, s>>>(ks, n, 8 * p, hist, ntiles);
-    cb2pg::sort_scan_kernel<<<1, 1024, 0, s>>>(reinterpret_cast<int4 *>(hist), (256 * ntiles + 3) / 4);
-    cb2pg::sort_scatter_kernel<K, HAS_VAL><<<ntiles, cb2pg::kSortThreads, 0, s>>>(ks, vs, kd, vd, n, 8 * p, hist, ntiles);
+  const int ntiles = (n + cb2pg::kKeySortTile - 1) / cb2pg::kKeySortTile;
+  unsigned long long *ks = key_sort_source(result, scratch, bits), *kd = (ks == result) ? scratch : result;
+  for (int p = 0; p < key_sort_passes(bits); ++p) {
+    cb2pg::key_hist_kernel<<<ntiles, cb2pg::kKeySortThreads, 0, s>>>(ks, n, 8 * p, hist, ntiles);
+    cb2pg::key_scan_kernel<<<1, 1024, 0, s>>>(reinterpret_cast<int4 *>(hist), (256 * ntiles + 3) / 4);
+    cb2pg::key_scatter_kernel<<<ntiles, cb2pg::kKeySortThreads, 0, s>>>(ks, kd, n, 8 * p, hist, ntiles);
     CB2_CUDA(cudaGetLastError());
     g_launches.fetch_add(3);
     std::swap(ks, kd);
-    std::swap(vs, vd);
   }
   return CB2_OK;
 }
 
-// Masks of `words` words per row from a finished table, sorted (see mask_words_from_table_kernel):
-// writes mask [n, words] and mask_argsort [n].
-int sort_mask_words(const int32_t *table, int n, int kv, int words, uint32_t *rows, uint32_t *k_result,
-                    uint32_t *k_scratch, int *v_scratch, uint32_t *mask, int *argsort, int *hist, cudaStream_t s) {
-  const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
-  cb2pg::mask_words_from_table_kernel<<<blocks, 256, 0, s>>>(table, n, kv, words, rows);
-  g_launches.fetch_add(1);
-  for (int w = 0; w < words; ++w) {
-    const int bits = std::min(32, kv - 32 * w);
-    cb2pg::gather_word_kernel<<<blocks, 256, 0, s>>>(rows, w == 0 ? nullptr : argsort, n, words, w,
-                                                     sort_source(k_result, k_scratch, bits),
-                                                     sort_source(argsort, v_scratch, bits));
+// One side's masks on their way to being sorted: where the unsorted masks are built, and what the
+// sort needs and leaves.
+struct MaskSort {
+  cb2pg::MaskSide side;
+  uint32_t *m_tmp;
+  int *v_tmp;
+  uint32_t *mask;  // results
+  int *argsort;
+  uint32_t *tile_masks;
+};
+// `rows`: room for unsorted masks of several words; one-word masks are sorted between `mask` and `m_tmp`
+// and start in whichever lets the last pass end in `mask`.
+MaskSort make_mask_sort(const cb2pg::SortShape &shape, int32_t *indices, int n, uint32_t *rows, uint32_t *m_tmp,
+                        int *v_tmp, int *hist, uint32_t *mask, int *argsort, uint32_t *tile_masks) {
+  MaskSort j;
+  j.side.indices = indices;
+  j.side.rows = shape.words > 1 ? rows : (shape.passes % 2 ? m_tmp : mask);
+  j.side.hist = hist;
+  j.side.n = n;
+  j.side.chunk = cb2pg::sort_chunk(n);
+  j.m_tmp = m_tmp;
+  j.v_tmp = v_tmp;
+  j.mask = mask;
+  j.argsort = argsort;
+  j.tile_masks = tile_masks;
+  return j;
+}
+
+// All passes, both sides of a table set in the same launches.  Counts of the first pass and the
+// unsorted masks are there, the other counts and the tile masks are zero.
+int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, cudaStream_t s) {
+  int max_chunks = 1;
+  for (int p = 0; p < shape.passes; ++p) {
+    cb2pg::SortSides sides;
+    memset(&sides, 0, sizeof(sides));
+    const int to_go = shape.passes - 1 - p;
+    for (int q = 0; q < count; ++q) {
+      const MaskSort &j = jobs[q];
+      cb2pg::SortSide &o = sides.side[q];
+      o.n = j.side.n;
+      o.chunk = j.side.chunk;
+      o.n_chunks = (j.side.n + j.side.chunk - 1) / j.side.chunk;
+      max_chunks = std::max(max_chunks, o.n_chunks);
+      const size_t hist_pass = static_cast<size_t>(o.n_chunks) * cb2pg::kSortBins;
+      o.hist = j.side.hist + p * hist_pass;
+      o.hist_next = to_go ? j.side.hist + (p + 1) * hist_pass : nullptr;
+      o.rows = j.side.rows;
+      // results of the last pass in the result arrays, of the one before it in scratch, and so on
+      o.vout = to_go % 2 ? j.v_tmp : j.argsort;
+      o.vin = p == 0 ? nullptr : (to_go % 2 ? j.argsort : j.v_tmp);
+      o.kout = shape.words > 1 ? j.mask : (to_go % 2 ? j.m_tmp : j.mask);
+      o.kin = shape.words > 1 ? nullptr : (to_go % 2 ? j.mask : j.m_tmp);
+      o.tile_masks = to_go ? nullptr : j.tile_masks;
+    }
+    const dim3 grid(max_chunks, count);
+    if (shape.words > 1)
+      cb2pg::sort_pass_kernel<true><<<grid, cb2pg::kSortThreads, 0, s>>>(sides, p, shape);
+    else
+      cb2pg::sort_pass_kernel<false><<<grid, cb2pg::kSortThreads, 0, s>>>(sides, p, shape);
     CB2_CUDA(cudaGetLastError());
     g_launches.fetch_add(1);
-    const int rc = radix_sort<uint32_t, true>(k_result, argsort, k_scratch, v_scratch, n, bits, hist, s);
-    if (rc)
-      return rc;
   }
-  const long long total = static_cast<long long>(n) * words;
-  cb2pg::gather_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(rows, argsort, n, words, mask);
-  CB2_CUDA(cudaGetLastError());
-  g_launches.fetch_add(1);
   return CB2_OK;
+}
+
+struct Fill {
+  cb2pg::FillRanges r;
+  long long most = 0;
+  Fill() { r.count = 0; }
+  void add(void *ptr, size_t bytes, uint32_t value) {
+    if (!ptr || !bytes)
+      return;
+    r.ptr[r.count] = reinterpret_cast<uint32_t *>(ptr);
+    r.words[r.count] = static_cast<long long>(bytes / 4);
+    r.value[r.count++] = value;
+    most = std::max<long long>(most, static_cast<long long>(bytes / 4));
+  }
+  void run(const DeviceState *dev, cudaStream_t s) const {
+    const long long blocks = std::min<long long>((most / 4 + 255) / 256 + 1, 8ll * dev->num_sms);
+    cb2pg::fill_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(r);
+    g_launches.fetch_add(1);
+  }
+};
+
+cb2pg::Bitmap pairgen_bitmap(const PairgenLayout &L, uint8_t *ws) {
+  cb2pg::Bitmap bm;
+  bm.words = reinterpret_cast<uint32_t *>(ws + L.off_bits);
+  bm.word_first = reinterpret_cast<int *>(ws + L.off_word_first);
+  bm.block_first = reinterpret_cast<int *>(ws + L.off_block_first);
+  bm.n_words = static_cast<int>(L.bitmap_words);
+  bm.n_blocks = static_cast<int>(L.bitmap_words / cb2pg::kBitmapBlockWords);
+  return bm;
 }
 
 int pairgen_common(const cb2_pairgen_args *a, PairgenLayout *L, DeviceState **dev) {
@@ -687,24 +773,38 @@ int cb2_pairgen_count_outputs(const cb2_pairgen_args *a, int *n_out, void *strea
   }
   uint8_t *ws = reinterpret_cast<uint8_t *>(a->workspace);
   int *counter = reinterpret_cast<int *>(ws + L.off_counters);
+  Fill fill;
+  fill.add(counter, 256, 0u);
   unsigned long long *set_keys = reinterpret_cast<unsigned long long *>(ws + L.off_set_keys);
   unsigned long long *list_a = reinterpret_cast<unsigned long long *>(ws + L.off_list_a);
   unsigned long long *list_b = reinterpret_cast<unsigned long long *>(ws + L.off_list_b);
-  CB2_CUDA(cudaMemsetAsync(counter, 0, 256, stream));
-  CB2_CUDA(cudaMemsetAsync(set_keys, 0xFF, static_cast<size_t>(L.cap_set) * 8, stream));
-  cb2pg::out_candidates_kernel<<<(a->n_in + 255) / 256, 256, 0, stream>>>(
-      a->in_coords, a->n_in, L.g, set_keys, L.cap_set - 1, sort_source(list_a, list_b, L.key_bits),
-      static_cast<int>(L.list_cap), counter, dev->status);
+  if (L.bitmap) {
+    const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
+    fill.add(bm.words, static_cast<size_t>(L.bitmap_words) * 4, 0u);
+    fill.run(dev, stream);
+    const long long threads = static_cast<long long>(a->n_in) * L.g.ksize[0] * L.g.ksize[1];
+    cb2pg::bitmap_mark_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(a->in_coords, a->n_in, L.g,
+                                                                                              bm.words);
+    cb2pg::bitmap_rank_kernel<<<bm.n_blocks, cb2pg::kBitmapThreads, 0, stream>>>(bm, counter);
+    g_launches.fetch_add(2);
+  } else {
+    fill.add(set_keys, static_cast<size_t>(L.cap_set) * 8, 0xffffffffu);
+    fill.run(dev, stream);
+    cb2pg::out_candidates_kernel<<<(a->n_in + 255) / 256, 256, 0, stream>>>(
+        a->in_coords, a->n_in, L.g, set_keys, L.cap_set - 1, key_sort_source(list_a, list_b, L.key_bits),
+        static_cast<int>(L.list_cap), counter, dev->status);
+    g_launches.fetch_add(1);
+  }
   CB2_CUDA(cudaGetLastError());
-  g_launches.fetch_add(1);
   int count = 0;
   CB2_CUDA(cudaMemcpyAsync(&count, counter, sizeof(int), cudaMemcpyDeviceToHost, stream));
   CB2_CUDA(cudaStreamSynchronize(stream));
   CB2_CHECK_RT(count >= 0 && count <= L.list_cap, "active-output count %d out of range", count);
-  rc = radix_sort<unsigned long long, false>(list_a, nullptr, list_b, nullptr, count, L.key_bits,
-                                             reinterpret_cast<int *>(ws + L.off_hist), stream);
-  if (rc)
-    return rc;
+  if (!L.bitmap) {
+    rc = key_sort(list_a, list_b, count, L.key_bits, reinterpret_cast<int *>(ws + L.off_key_hist), stream);
+    if (rc)
+      return rc;
+  }
   *n_out = count;
   return CB2_OK;
 }
@@ -727,69 +827,68 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
   const bool bwd = a->indices_bwd != nullptr;
   CB2_CHECK_RT(!bwd || (a->mask_bwd && a->mask_argsort_bwd), "error: backward mask or mask_argsort empty");
   uint8_t *ws = reinterpret_cast<uint8_t *>(a->workspace);
-  unsigned long long *in_keys = reinterpret_cast<unsigned long long *>(ws + L.off_in_keys);
-  int *in_vals = reinterpret_cast<int *>(ws + L.off_in_vals);
-  uint32_t *m_tmp = reinterpret_cast<uint32_t *>(ws + L.off_m);
-  int *v_tmp = reinterpret_cast<int *>(ws + L.off_v);
-  int *hist = reinterpret_cast<int *>(ws + L.off_hist);
-  CB2_CUDA(cudaMemsetAsync(in_keys, 0xFF, static_cast<size_t>(L.cap_in) * 8, stream));
-  CB2_CUDA(cudaMemsetAsync(in_vals, 0x7F, static_cast<size_t>(L.cap_in) * 4, stream));
-  cb2pg::hash_insert_kernel<<<(n_in + 255) / 256, 256, 0, stream>>>(a->in_coords, n_in, L.g, in_keys, in_vals,
-                                                                     L.cap_in - 1, dev->status);
-  const int32_t *out_coords = a->in_coords;
-  if (!a->subm) {
-    cb2pg::decode_out_coords_kernel<<<(n_out + 255) / 256, 256, 0, stream>>>(
-        reinterpret_cast<const unsigned long long *>(ws + L.off_list_a), n_out, L.g, a->out_coords);
-    out_coords = a->out_coords;
-    g_launches.fetch_add(1);
-  }
-  const bool wide = L.words > 1;
-  uint32_t *rows = reinterpret_cast<uint32_t *>(ws + L.off_rows), *k_res = reinterpret_cast<uint32_t *>(ws + L.off_k);
-  // several mask words per row: the probe's one-word mask and row numbers go to scratch, the masks
-  // are built from the finished table instead
-  cb2pg::probe_kernel<<<(n_out + 255) / 256, 256, 0, stream>>>(
-      out_coords, n_out, L.g, in_keys, in_vals, L.cap_in - 1, a->indices,
-      wide ? m_tmp : sort_source(a->mask, m_tmp, L.g.kv), wide ? v_tmp : sort_source(a->mask_argsort, v_tmp, L.g.kv));
-  CB2_CUDA(cudaGetLastError());
-  g_launches.fetch_add(2);
-  if (wide)
-    rc = sort_mask_words(a->indices, n_out, L.g.kv, L.words, rows, k_res, m_tmp, v_tmp, a->mask, a->mask_argsort, hist,
-                         stream);
-  else
-    rc = radix_sort<uint32_t, true>(a->mask, a->mask_argsort, m_tmp, v_tmp, n_out, L.g.kv, hist, stream);
-  if (rc)
-    return rc;
-  if (a->tile_masks) {
-    if (wide)
-      cb2pg::tile_masks_words_kernel<<<((n_out + 127) / 128 + 7) / 8, 256, 0, stream>>>(a->mask, n_out, L.words,
-                                                                                       a->tile_masks);
-    else
-      cb2pg::tile_masks_kernel<<<((n_out + 127) / 128 + 7) / 8, 256, 0, stream>>>(a->mask, n_out, a->tile_masks);
+  const cb2pg::SortShape &shape = L.shape;
+  const int words = shape.words;
+  auto at32 = [&](size_t off) { return reinterpret_cast<uint32_t *>(ws + off); };
+  auto at_int = [&](size_t off) { return reinterpret_cast<int *>(ws + off); };
+  MaskSort jobs[2];
+  jobs[0] = make_mask_sort(shape, a->indices, n_out, at32(L.off_rows[0]), at32(L.off_m[0]), at_int(L.off_v[0]),
+                           at_int(L.off_hist), a->mask, a->mask_argsort, a->tile_masks);
+  jobs[1] = make_mask_sort(shape, a->indices_bwd, n_in, at32(L.off_rows[1]), at32(L.off_m[1]), at_int(L.off_v[1]),
+                           at_int(L.off_hist) + L.hist_ints, a->mask_bwd, a->mask_argsort_bwd, nullptr);
+  const cb2pg::MaskSide none = {nullptr, nullptr, nullptr, 0, 1};
+  const auto blocks = [](long long n) { return static_cast<unsigned>((n + 255) / 256); };
+  Fill fill;
+  fill.add(at_int(L.off_hist), 2 * L.hist_ints * 4, 0u);
+  fill.add(a->tile_masks, static_cast<size_t>((n_out + 127) / 128) * words * 4, 0u);
+  if (L.bitmap) {
+    const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
+    fill.add(a->indices, static_cast<size_t>(L.g.kv) * n_out * 4, 0xffffffffu);
+    fill.add(jobs[0].side.rows, static_cast<size_t>(n_out) * words * 4, 0u);
+    fill.run(dev, stream);
+    cb2pg::bitmap_coords_kernel<<<blocks(bm.n_words), 256, 0, stream>>>(bm, n_out, L.g, a->out_coords);
+    const long long threads = static_cast<long long>(n_in) * L.g.ksize[0] * L.g.ksize[1];
+    cb2pg::bitmap_scatter_kernel<<<blocks(threads), 256, 0, stream>>>(a->in_coords, n_in, L.g, bm, jobs[0].side, words,
+                                                                      dev->status);
+    const int bwd_blocks = bwd ? static_cast<int>(blocks(n_in)) : 0;
+    auto kern = words > 1 ? cb2pg::bitmap_backward_kernel<4> : cb2pg::bitmap_backward_kernel<1>;
+    kern<<<bwd_blocks + blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(a->in_coords, L.g, bm, jobs[0].side, jobs[1].side,
+                                                                         bwd_blocks, words, shape.width);
     CB2_CUDA(cudaGetLastError());
-    g_launches.fetch_add(1);
-  }
-  if (bwd) {
-    CB2_CUDA(cudaMemsetAsync(a->indices_bwd, 0xFF, static_cast<size_t>(L.g.kv) * n_in * 4, stream));
-    const long long threads = static_cast<long long>(n_out) * L.g.kv;
-    cb2pg::invert_table_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-        a->indices, n_out, L.g.kv, n_in, a->indices_bwd);
-    CB2_CUDA(cudaGetLastError());
-    g_launches.fetch_add(1);
-    if (wide) {
-      rc = sort_mask_words(a->indices_bwd, n_in, L.g.kv, L.words, rows, k_res, m_tmp, v_tmp, a->mask_bwd,
-                           a->mask_argsort_bwd, hist, stream);
-    } else {
-      cb2pg::mask_from_table_kernel<<<(n_in + 255) / 256, 256, 0, stream>>>(
-          a->indices_bwd, n_in, L.g.kv, sort_source(a->mask_bwd, m_tmp, L.g.kv),
-          sort_source(a->mask_argsort_bwd, v_tmp, L.g.kv));
-      CB2_CUDA(cudaGetLastError());
+    g_launches.fetch_add(3);
+  } else {
+    cb2pg::HashView h;
+    h.slots = reinterpret_cast<unsigned long long *>(ws + L.off_hash);
+    h.cap_mask = L.cap_in - 1;
+    h.exact = L.exact;
+    h.coords = a->in_coords;
+    const bool mirror = bwd && L.mirror;
+    fill.add(h.slots, static_cast<size_t>(L.cap_in) * 8, 0xffffffffu);
+    if (bwd && !mirror)
+      fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
+    fill.run(dev, stream);
+    cb2pg::hash_insert_kernel<<<blocks(n_in), 256, 0, stream>>>(a->in_coords, n_in, L.g, h, dev->status);
+    const int32_t *out_coords = a->in_coords;
+    if (!a->subm) {
+      cb2pg::decode_out_coords_kernel<<<blocks(n_out), 256, 0, stream>>>(
+          reinterpret_cast<const unsigned long long *>(ws + L.off_list_a), n_out, L.g, a->out_coords);
+      out_coords = a->out_coords;
       g_launches.fetch_add(1);
-      rc = radix_sort<uint32_t, true>(a->mask_bwd, a->mask_argsort_bwd, m_tmp, v_tmp, n_in, L.g.kv, hist, stream);
     }
-    if (rc)
-      return rc;
+    auto kern = words > 1 ? cb2pg::probe_kernel<4> : cb2pg::probe_kernel<1>;
+    kern<<<blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(out_coords, L.g, h, jobs[0].side, mirror ? jobs[1].side : none,
+                                                            words, shape.width);
+    g_launches.fetch_add(2);
+    if (bwd && !mirror) {
+      cb2pg::invert_table_kernel<<<blocks(static_cast<long long>(n_out) * L.g.kv), 256, 0, stream>>>(
+          a->indices, n_out, L.g.kv, n_in, a->indices_bwd);
+      cb2pg::masks_from_table_kernel<<<blocks(n_in), cb2pg::kProbeThreads, 0, stream>>>(jobs[1].side, L.g.kv, words,
+                                                                                       shape.width);
+      g_launches.fetch_add(2);
+    }
+    CB2_CUDA(cudaGetLastError());
   }
-  return CB2_OK;
+  return sort_masks(jobs, bwd ? 2 : 1, shape, stream);
 }
 
 // ---------------------------------------------------------------- a layer's ShuffleAC calls in one launch
@@ -797,6 +896,7 @@ struct SeqLayout {
   size_t off_table, off_mask, off_argsort, off_m, off_v, off_hist, off_tickets, total;
 };
 static void seq_layout(int count, long long n, SeqLayout *L) {
+  const cb2pg::SortShape shape = cb2pg::sort_shape(count);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -809,7 +909,7 @@ static void seq_layout(int count, long long n, SeqLayout *L) {
   L->off_argsort = take(static_cast<size_t>(n) * 4);
   L->off_m = take(static_cast<size_t>(n) * 4);
   L->off_v = take(static_cast<size_t>(n) * 4);
-  L->off_hist = take(static_cast<size_t>(256) * ((n + cb2pg::kSortTile - 1) / cb2pg::kSortTile + 1) * 4);
+  L->off_hist = take(cb2pg::sort_hist_ints(shape, n) * 4);
   L->total = off;
 }
 
@@ -874,19 +974,26 @@ int cb2_gemm_sequence_run(const cb2_gemm_sequence_args *a, void *stream_v) {
   uint32_t *mask = reinterpret_cast<uint32_t *>(ws + L.off_mask);
   int32_t *argsort = reinterpret_cast<int32_t *>(ws + L.off_argsort);
   if (!a->reuse_tables) {
-    uint32_t *m_tmp = reinterpret_cast<uint32_t *>(ws + L.off_m);
-    int *v_tmp = reinterpret_cast<int *>(ws + L.off_v);
-    CB2_CUDA(cudaMemsetAsync(ws + L.off_tickets, 0, 256, stream));
-    CB2_CUDA(cudaMemsetAsync(table, 0xFF, static_cast<size_t>(a->count) * n * 4, stream));
+    const cb2pg::SortShape shape = cb2pg::sort_shape(a->count);
+    const MaskSort job = make_mask_sort(shape, table, n, nullptr, reinterpret_cast<uint32_t *>(ws + L.off_m),
+                                        reinterpret_cast<int *>(ws + L.off_v), reinterpret_cast<int *>(ws + L.off_hist), mask,
+                                        argsort, nullptr);
+    Fill fill;
+    fill.add(ws + L.off_tickets, 256, 0u);
+    fill.add(table, static_cast<size_t>(a->count) * n * 4, 0xffffffffu);
+    fill.add(ws + L.off_hist, cb2pg::sort_hist_ints(shape, n) * 4, 0u);
+    fill.run(dev, stream);
     const long long pairs = lists.first[a->count];
-    if (pairs > 0)
+    if (pairs > 0) {
       cb2pg::seq_scatter_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, stream>>>(lists, n, c0.rows_A, table,
                                                                                               dev->status);
-    cb2pg::mask_from_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(table, n, a->count, sort_source(mask, m_tmp, a->count),
-                                                                        sort_source(argsort, v_tmp, a->count));
+      g_launches.fetch_add(1);
+    }
+    cb2pg::masks_from_table_kernel<<<(n + cb2pg::kProbeThreads - 1) / cb2pg::kProbeThreads, cb2pg::kProbeThreads, 0, stream>>>(
+        job.side, a->count, 1, shape.width);
     CB2_CUDA(cudaGetLastError());
-    g_launches.fetch_add(2);
-    rc = radix_sort<uint32_t, true>(mask, argsort, m_tmp, v_tmp, n, a->count, reinterpret_cast<int *>(ws + L.off_hist), stream);
+    g_launches.fetch_add(1);
+    rc = sort_masks(&job, 1, shape, stream);
     if (rc)
       return rc;
   }

@@ -90,6 +90,40 @@ def test_kernel_volumes_above_32(torch, ksize, subm, stride):
     compare(torch, t, oc, ref, subm)
 
 
+@pytest.mark.parametrize("n,shift,grid,kw", [
+    # rows around the sort's chunk of 2048 and past 74 of them (the chunks grow)
+    (2048, 0, (8, 24, 24), {}), (2049, 0, (8, 24, 24), {}), (151553, 0, (41, 200, 176), {}),
+    # offsets that are not symmetric: the backward table is inverted, not mirrored
+    (3000, 0, (8, 24, 24), dict(ksize=(2, 3, 3))), (3000, 0, (8, 24, 24), dict(pad=(0, 1, 1))),
+    # grids of more than 2^32 cells: the hash table's tag is not the voxel itself
+    (3000, 1990, (2000, 2050, 2050), {}), (3000, 1990, (2000, 2050, 2050), dict(ksize=(5, 5, 5))),
+    # output grids too large for the bitmap, just small enough for it, and one cell more than a block
+    (3000, 1990, (2000, 2050, 2050), dict(stride=(2, 2, 2), subm=False)),
+    (2000, 300, (400, 400, 209), dict(subm=False)), (2000, 300, (400, 400, 210), dict(subm=False)),
+    (4000, 0, (8, 128, 128), dict(subm=False)), (4000, 0, (9, 128, 128), dict(subm=False)),
+])
+def test_every_route_of_the_builder(torch, n, shift, grid, kw):
+    small = tuple(min(a, g - min(shift, g - a)) for a, g in zip((8, 24, 24) if shift else grid, grid))
+    coords = W.sample_coords(n, 11, small)
+    coords[:, 1:] += np.array([g - a for g, a in zip(grid, small)], np.int32) if shift else 0
+    t, oc = gpu_tables(torch, coords, 1, grid, **kw)
+    compare(torch, t, oc, W.build_tables(coords, grid=grid, **kw), kw.get("subm", True))
+
+
+@pytest.mark.parametrize("kw", [{}, dict(stride=(2, 2, 2), subm=False)])
+def test_repeated_voxels_resolve_to_the_first_row(torch, kw):
+    grid = (8, 24, 24)
+    coords = W.sample_coords(2000, 12, grid)
+    twice = np.concatenate([coords, coords[:700]])
+    one, _ = gpu_tables(torch, coords, 1, grid, **kw)
+    t, _ = gpu_tables(torch, twice, 1, grid, **kw)
+    assert t.n_out == (one.n_out if kw else 2700)
+    assert (t.indices[:, :one.n_out] == one.indices).all()
+    # nothing points at a repeated row
+    assert (t.indices_bwd[:, 2000:] == -1).all()
+    assert int((t.mask_bwd == 0).sum()) >= 700
+
+
 def test_benchmark_scene_full_size(torch):
     """The 150 000-voxel scene of the benchmark configurations, submanifold and stride 2."""
     coords = W.sample_coords(150000, 1)
