@@ -45,15 +45,19 @@ def itemsize(code: int) -> int:
     return _ITEMSIZE[int(code)]
 
 
+_TORCH_CODES = {}
+
+
 def _torch_dtype_code(dt) -> int:
-    import torch
-    table = {torch.float32: float32, torch.int32: int32, torch.int16: int16, torch.int8: int8,
-             torch.float64: float64, torch.bool: bool_, torch.uint8: uint8, torch.float16: float16,
-             torch.int64: int64, torch.bfloat16: bfloat16}
-    for name, code in (("uint16", uint16), ("uint32", uint32), ("uint64", uint64)):
-        if hasattr(torch, name):
-            table[getattr(torch, name)] = code
-    return table[dt]
+    if not _TORCH_CODES:
+        import torch
+        for name, code in (("float32", float32), ("int32", int32), ("int16", int16), ("int8", int8),
+                           ("float64", float64), ("bool", bool_), ("uint8", uint8), ("float16", float16),
+                           ("int64", int64), ("bfloat16", bfloat16), ("uint16", uint16), ("uint32", uint32),
+                           ("uint64", uint64)):
+            if hasattr(torch, name):
+                _TORCH_CODES[getattr(torch, name)] = code
+    return _TORCH_CODES[dt]
 
 
 class Tensor:
@@ -129,13 +133,34 @@ def as_view(t) -> Optional[Tensor]:
         return None
     if isinstance(t, Tensor):
         return None if t._ptr == 0 else t
-    # torch tensor
+    # torch tensor (fields set directly: this runs a dozen times per call)
     if t.numel() == 0 and t.dim() <= 1:
         return None
     if not t.is_cuda:
         raise RuntimeError("tensors must live on a CUDA device (there is no CPU path)")
-    return Tensor(t.data_ptr(), list(t.shape), _torch_dtype_code(t.dtype), t.device.index or 0,
-                  list(t.stride()), keepalive=t)
+    v = Tensor.__new__(Tensor)
+    v._ptr = t.data_ptr()
+    v.shape = list(t.shape)
+    v.dtype = _TORCH_CODES.get(t.dtype)
+    if v.dtype is None:
+        v.dtype = _torch_dtype_code(t.dtype)
+    v.device = t.get_device()
+    v.stride_ = list(t.stride())
+    v._keepalive = t
+    return v
+
+
+def dtype_of(t) -> Optional[int]:
+    """``as_view(t).dtype``, None when empty."""
+    if t is None:
+        return None
+    if isinstance(t, Tensor):
+        return None if t._ptr == 0 else t.dtype
+    if t.numel() == 0 and t.dim() <= 1:
+        return None
+    if not t.is_cuda:
+        raise RuntimeError("tensors must live on a CUDA device (there is no CPU path)")
+    return _torch_dtype_code(t.dtype)
 
 
 class CUDAKernelTimer:

@@ -20,7 +20,7 @@ import ctypes
 import enum
 from typing import List, Optional, Tuple
 
-from . import as_view, dtype_short_str, itemsize, unknown
+from . import CUDAKernelTimer, _TimerGuard, as_view, dtype_of, dtype_short_str, itemsize, unknown
 from .. import _lib
 
 
@@ -398,9 +398,9 @@ class GemmParams:
     @a.setter
     def a(self, v):
         self._a = v
-        t = as_view(v)
-        if t is not None:
-            self.algo_desp.dtype_a = t.dtype
+        code = dtype_of(v)
+        if code is not None:
+            self.algo_desp.dtype_a = code
 
     @property
     def b(self):
@@ -409,9 +409,9 @@ class GemmParams:
     @b.setter
     def b(self, v):
         self._b = v
-        t = as_view(v)
-        if t is not None:
-            self.algo_desp.dtype_b = t.dtype
+        code = dtype_of(v)
+        if code is not None:
+            self.algo_desp.dtype_b = code
 
     @property
     def c(self):
@@ -420,9 +420,9 @@ class GemmParams:
     @c.setter
     def c(self, v):
         self._c = v
-        t = as_view(v)
-        if t is not None:
-            self.algo_desp.dtype_c = t.dtype
+        code = dtype_of(v)
+        if code is not None:
+            self.algo_desp.dtype_c = code
 
     @property
     def d(self):
@@ -430,22 +430,32 @@ class GemmParams:
 
     @d.setter
     def d(self, v):
-        tc, td = as_view(self._c), as_view(v)
-        if tc is not None and td is not None and tc.dtype != td.dtype:
+        code_c, code_d = dtype_of(self._c), dtype_of(v)
+        if code_c is not None and code_d is not None and code_c != code_d:
             raise RuntimeError("d dtype must equal to c")
         self._d = v
 
     def check_valid(self) -> None:
         """params.h:353-365."""
+        self._checked_views()
+
+    def _checked_views(self):
+        """The checks of :meth:`check_valid`; returns the views they made: (a, b, c, a_inds, b_inds, c_inds),
+        the row lists only as far as the shuffle type requires them."""
         self.algo_desp.check_valid()
-        if as_view(self.a) is None or as_view(self.b) is None or as_view(self.c) is None:
+        a, b, c = as_view(self._a), as_view(self._b), as_view(self._c)
+        if a is None or b is None or c is None:
             raise RuntimeError("a,b,c must not empty")
+        a_inds = b_inds = c_inds = None
         if self.algo_desp.shuffle_type == ShuffleStrideType.ShuffleAC:
-            if as_view(self.c_inds) is None:
+            c_inds = as_view(self.c_inds)
+            if c_inds is None:
                 raise RuntimeError("a_inds,c_inds tensor must not empty")
         elif self.algo_desp.shuffle_type == ShuffleStrideType.ShuffleAB:
-            if as_view(self.a_inds) is None or as_view(self.b_inds) is None:
+            a_inds, b_inds = as_view(self.a_inds), as_view(self.b_inds)
+            if a_inds is None or b_inds is None:
                 raise RuntimeError("a_inds,b_inds tensor must not empty")
+        return a, b, c, a_inds, b_inds, c_inds
 
 
 class ConvParams:
@@ -514,15 +524,26 @@ def _workspace_for(device: int, stream: int, nbytes: int, user_ws):
     return buf.data_ptr(), buf.numel()
 
 
+def _call_on(device: int, fn, args, stream: int) -> None:
+    """One call of the C ABI with ``device`` current."""
+    import torch
+    if torch.cuda.current_device() == device:
+        rc = fn(ctypes.byref(args), stream)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(ctypes.byref(args), stream)
+    if rc:
+        _lib.raise_for(rc)
+
+
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t._ptr
 
 
 def _gemm_args(params: GemmParams) -> _lib.GemmArgs:
     """Shape extraction of the reference's GEMM prologue (cumm/gemm/nvrtc_code.py:34-146)."""
-    params.check_valid()
+    a, b, c, a_inds, b_inds, c_inds = params._checked_views()
     desp = params.algo_desp
-    a, b, c = as_view(params.a), as_view(params.b), as_view(params.c)
     d = as_view(params.d)
     for t in (a, b, c):
         if t.ndim != 2:
@@ -533,7 +554,9 @@ def _gemm_args(params: GemmParams) -> _lib.GemmArgs:
     if tc:
         ta, tb = (not tb), (not ta)
         a, b = b, a
-    a_inds, b_inds, c_inds = as_view(params.a_inds), as_view(params.b_inds), as_view(params.c_inds)
+    a_inds = a_inds or as_view(params.a_inds)
+    b_inds = b_inds or as_view(params.b_inds)
+    c_inds = c_inds or as_view(params.c_inds)
     if not (desp.split_k_serial or desp.split_k_parallel) and params.split_k_slices > 1:
         raise RuntimeError("algo don't support splitk but you provide split_k_slices > 1.")
     args = _lib.GemmArgs()
@@ -603,14 +626,17 @@ def run_gemm(params: GemmParams) -> None:
     pick a kernel for the descriptor, launch on ``params.stream``."""
     L = _lib.load()
     args = _gemm_args(params)
-    need = L.cb2_gemm_workspace_size(ctypes.byref(args))
-    if need:
-        ptr, nbytes = _workspace_for(args._device, int(params.stream), need, params.workspace)
-        args.workspace, args.workspace_bytes = ptr, nbytes
-    import torch
-    from . import _TimerGuard
-    with torch.cuda.device(args._device), _TimerGuard(params.algo_desp.__repr__(), params.timer, int(params.stream)):
-        _lib.raise_for(L.cb2_gemm_run(ctypes.byref(args), ctypes.c_void_p(int(params.stream))))
+    stream = int(params.stream)
+    if args.shuffle_type == ShuffleStrideType.ShuffleAB:  # the only kind that needs scratch
+        need = L.cb2_gemm_workspace_size(ctypes.byref(args))
+        if need:
+            args.workspace, args.workspace_bytes = _workspace_for(args._device, stream, need, params.workspace)
+    timer = params.timer
+    if timer is not None and getattr(timer, "enable", False):
+        with _TimerGuard(repr(params.algo_desp), timer, stream):
+            _call_on(args._device, L.cb2_gemm_run, args, stream)
+    else:
+        _call_on(args._device, L.cb2_gemm_run, args, stream)
 
 
 def _conv_args(params: ConvParams) -> _lib.ConvArgs:
@@ -744,20 +770,23 @@ def run_conv(params: ConvParams) -> None:
         return run_dense_conv(params)
     L = _lib.load()
     args = _conv_args(params)
-    need = L.cb2_conv_workspace_size(ctypes.byref(args))
-    if need:
-        ptr, nbytes = _workspace_for(args._device, int(params.stream), need, params.workspace)
-        args.workspace, args.workspace_bytes = ptr, nbytes
-    import torch
-    from . import CUDAKernelTimer, _TimerGuard
-    name = params.conv_algo_desp.__repr__()
+    stream = int(params.stream)
+    if args.op_type == ConvOpType.BackwardWeight:  # the only operator that needs scratch
+        need = L.cb2_conv_workspace_size(ctypes.byref(args))
+        if need:
+            args.workspace, args.workspace_bytes = _workspace_for(args._device, stream, need, params.workspace)
     # verbose: registers of the kernel and the time of this launch (cumm/conv/main.py:723-729)
     timer = params.timer
+    enabled = timer is not None and getattr(timer, "enable", False)
+    if not (enabled or params.verbose):
+        _call_on(args._device, L.cb2_conv_run, args, stream)
+        return
+    name = repr(params.conv_algo_desp)
     own = None
-    if params.verbose and not (timer is not None and getattr(timer, "enable", False)):
+    if not enabled:
         timer = own = CUDAKernelTimer(True)
-    with torch.cuda.device(args._device), _TimerGuard(name, timer, int(params.stream)):
-        _lib.raise_for(L.cb2_conv_run(ctypes.byref(args), ctypes.c_void_p(int(params.stream))))
+    with _TimerGuard(name, timer, stream):
+        _call_on(args._device, L.cb2_conv_run, args, stream)
     if params.verbose:
         info = _lib.last_launch_info()
         t = (own or timer).get_pair_duration(name)
