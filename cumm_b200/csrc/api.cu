@@ -186,8 +186,8 @@ cudaError_t launch_after(int level, Kern kern, dim3 grid, dim3 block, size_t sme
 }
 
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MW = 1>
-int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const RowConvParams &p, int grid_x,
-                        int grid_y, cudaStream_t stream) {
+int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const RowConvParams &p, int gx, int gy,
+                        cudaStream_t stream) {
   using Cfg = RowConvCfg<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW>;
   auto kern = rowconv_kernel<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW>;
   static std::atomic<uint64_t> configured{0};  // bit per device
@@ -207,7 +207,7 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   // convolutions it measured +4 % for the int8 kernels (long epilogue tail) and neutral to
   // slightly worse for fp16, so only the former take part by default.
   const int pdl_level = p.mode != kModeMaskConv ? 1 : (KIND == 1 ? 1 : 2);
-  CB2_CUDA(launch_after(pdl_level, kern, dim3(grid_x, grid_y), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, map,
+  CB2_CUDA(launch_after(pdl_level, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, map,
                         map_a, p));
   g_launches.fetch_add(1);
   return CB2_OK;
@@ -319,13 +319,13 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
               : sched_scratch ? reinterpret_cast<int *>(sched_scratch)
                               : dev->status + 16 + 2 * (next_slot.fetch_add(1) % kTicketSlots);
   const int ntiles = (p.n_rows + 127) / 128;
-  const int gy = (p.nn + pl.block_n - 1) / pl.block_n;
+  const int parts = (p.nn + pl.block_n - 1) / pl.block_n;
+  const int gy = kind == 0 ? 1 : parts;  // RowConvCfg::PARTS
+  p.n_parts = kind == 0 ? parts : 1;
+  const long long items = static_cast<long long>(ntiles) * p.n_parts;
+  CB2_CHECK_RT(items < (1ll << 30), "too many output tiles (%lld)", items);
   const int sms = (max_ctas > 0 && max_ctas < dev->num_sms) ? max_ctas : dev->num_sms;
-  int gx = sms / gy;
-  if (gx < 1)
-    gx = 1;
-  if (gx > ntiles)
-    gx = ntiles;
+  const int gx = static_cast<int>(std::min<long long>(std::max(sms / gy, 1), items));
   return launch_rowconv(pl, map, map_a, tma_gather, p, gx, gy, stream);
 }
 

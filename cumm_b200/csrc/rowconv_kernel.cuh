@@ -46,6 +46,7 @@ struct RowConvParams {
   int red;                 // reduction width per filter offset
   int nn;                  // output width
   int kv;
+  int n_parts;             // column parts of BLOCK_N that a row tile is computed in, each an item of its own
   int mask_words;          // 32-bit words per row mask: ceil(kv / 32), word w covers offsets 32w .. 32w+31
   int mode;
   int src_mode;
@@ -69,6 +70,9 @@ struct RowConvParams {
 #ifndef CB2_ROWCONV_TICKET_BATCH
 #define CB2_ROWCONV_TICKET_BATCH 4
 #endif
+#ifndef CB2_ROWCONV_NARROW_STAGES
+#define CB2_ROWCONV_NARROW_STAGES 6
+#endif
 #ifndef CB2_ROWCONV_EPI_PARTS
 #define CB2_ROWCONV_EPI_PARTS 4
 #endif
@@ -85,18 +89,28 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int UMMA_K = 32 / ES;
   static constexpr int KRED = NATOM_K * ATOM_ELEMS;       // reduction elements per stage
   static constexpr int TILE_M = 128;
-  static constexpr int SA = 3;                            // A stages == producer groups
+  // A stages == producer groups.  The kernel with sixteen epilogue warps keeps to 24 warps: six per
+  // SM sub-partition leave 80 registers per thread, seven would leave 72 and spill.
+  static constexpr int SA =
+      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES) : 3;
   static constexpr int A_STAGE_BYTES = TILE_M * 128 * NATOM_K;
   static constexpr int B_SLOT_BYTES = BLOCK_N * 128 * NATOM_K;
   static constexpr int OUT_ROW_BYTES = BLOCK_N * OES;
   static constexpr int STAGING_BYTES = TILE_M * OUT_ROW_BYTES;
   static constexpr int MW = MASK_WORDS;
+  // Outputs wider than BLOCK_N: column parts drawn with the tiles (fp16), or one grid row per part
+  // (int8, whose sixteen epilogue warps have no register to spare for a part that changes).
+  static constexpr bool PARTS = KIND == 0;
   static constexpr int RING = MASK_WORDS == 1 ? CB2_ROWCONV_RING : CB2_ROWCONV_RING / 2;  // tile ring slots
   static constexpr int RING_SLOT_INTS = 136 + 128 * MASK_WORDS;  // header; 128 gather rows; 128 output rows / row masks
+  // mbarriers: operand stages, accumulators, the final one, weight slots, tile ring
+  static constexpr int BAR_EMPTY_A = SA, BAR_ACC_FULL = 2 * SA, BAR_ACC_EMPTY = BAR_ACC_FULL + 2,
+                       BAR_FINAL = BAR_ACC_EMPTY + 2, BAR_FULL_B = BAR_FINAL + 1, BAR_EMPTY_B = BAR_FULL_B + 6,
+                       BAR_RING = (BAR_EMPTY_B + 6 + 1) / 2 * 2;
   // Weight slots: as many as fit (2 to 6).  A tile whose mask carries many offsets needs a new
   // weight tile every step, and with two slots the L2 latency of that load bounds the step.
   static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + STAGING_BYTES + SA * 2 * 128 * 4 + 128 * 4 +
-                                     2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (32 + 3 * RING) * 8 + 64 + 1024;
+                                     2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (BAR_RING + 3 * RING) * 8 + 64 + 1024;
   static constexpr int SB_FIT = (232448 - FIXED_BYTES) / B_SLOT_BYTES;
   static constexpr int SB = SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
   static constexpr int NUM_ACC = 2;                       // TMEM accumulators: one fills while one drains
@@ -122,11 +136,12 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int OFF_OUTROW = OFF_ROWIDX + SA * 2 * 128 * 4;   // 128 ints
   static constexpr int OFF_SCALE = OFF_OUTROW + 128 * 4;             // 2 * BLOCK_N floats
   static constexpr int OFF_RING = OFF_SCALE + 2 * BLOCK_N * 4;       // RING slots
-  static constexpr int OFF_BARS = OFF_RING + RING * RING_SLOT_INTS * 4;  // 32 + 3 * RING mbarriers
-  static constexpr int OFF_MISC = OFF_BARS + (32 + 3 * RING) * 8;                 // tmem ptr, abort, flags
+  static constexpr int OFF_BARS = OFF_RING + RING * RING_SLOT_INTS * 4;  // BAR_RING + 3 * RING mbarriers
+  static constexpr int OFF_MISC = OFF_BARS + (BAR_RING + 3 * RING) * 8;  // tmem ptr, abort, flags
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;            // + alignment slack
   static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
-  static_assert(SB <= 8, "barrier table holds eight weight slots");
+  static_assert(SB <= 6, "the barrier table holds six weight slots");
+  static_assert(NUM_ACC == 2, "the barrier table holds two accumulators");
 };
 
 __device__ __forceinline__ float apply_act(float x, int act_type, float act_alpha) {
@@ -161,8 +176,10 @@ __device__ __forceinline__ uint32_t cvt_pack4_s8(float a, float b, float c, floa
 }
 
 // Tiles are handed out by one scheduler warp per CTA through a small shared-memory ring.
-// A slot holds {tile, OR-ed neighbour mask of the tile, the 128 rows the gather starts from,
-// the 128 destination rows}.  With `tickets` the scheduler draws tiles from a global counter
+// A slot holds {tile, OR-ed neighbour mask of the tile, first output column, the 128 rows the
+// gather starts from, the 128 destination rows}.  Outputs wider than BLOCK_N are cut into column
+// parts; an item is one part of one tile, and the parts of a tile are drawn one after the other, by
+// different CTAs at about the same time, so that the operand rows are fetched from memory once.  With `tickets` the scheduler draws tiles from a global counter
 // (dynamic scheduling: a tile whose mask carries many offsets costs many steps, and a static
 // split leaves the CTAs that own such tiles running long after the others), last tiles of
 // the sorted order first because those carry the most offsets.
@@ -211,116 +228,91 @@ __device__ __forceinline__ int ring_tile_masks(const RowConvParams &p, const int
   return count;
 }
 
-// Walks the tiles the scheduler publishes and, inside each, the (filter offset, reduction
-// pass) steps.  on_tile(tile, slot, kmask_for_store, has_work) -> bool; on_step(tile, f, kp,
-// first, last) -> bool; a false return aborts the walk.  Every consumer warp of the CTA runs
-// the identical walk, so their step counters agree.  All 32 lanes take part.
-// SINGLE: the walk is run by one thread on its own (no warp-collective operation inside), which
-// is what the roles that issue from a single thread anyway use: their time per step is pure
-// instruction latency, and the collectives would only add to it.
-template <bool SINGLE, int MW, class TileFn, class StepFn>
-__device__ __forceinline__ bool walk_steps_impl(const RowConvParams &p, const RingView &rv, int kpasses,
-                                                TileFn on_tile, StepFn on_step, long long *prof_c = nullptr,
-                                                long long *prof_prev_p = nullptr) {
-#ifdef CB2_TRACE
-#define CB2_WALK_MARK(i)                                                                                  \
-  do {                                                                                                    \
-    if (prof_c && (SINGLE || lane_id() == 0)) {                                                           \
-      long long t = clock64();                                                                            \
-      prof_c[i] += t - *prof_prev_p;                                                                      \
-      *prof_prev_p = t;                                                                                   \
-    }                                                                                                     \
-  } while (0)
-#else
-#define CB2_WALK_MARK(i) ((void)0)
-#endif
-  for (int seq = 0;; ++seq) {
-    const int si = seq % rv.ring;
-    CB2_WALK_MARK(8);  // previous slot released
-    if (!(SINGLE ? mbar_wait(rv.full0 + 8u * si, (seq / rv.ring) & 1, rv.abort_flag)
-                 : mbar_wait_warp(rv.full0 + 8u * si, (seq / rv.ring) & 1, rv.abort_flag)))
-      return false;
-    CB2_WALK_MARK(9);  // slot published
-    const int *sl = rv.slot(si);
-    const int tile = sl[0];
-    uint32_t kmask = static_cast<uint32_t>(sl[1]);  // MW == 1: the tile's mask; else: OR of its words
-    const uint32_t kmask_store = kmask;
-    bool cont = true;
-    if (tile >= 0 && !(p.skip_empty_tiles && kmask == 0)) {
-      if constexpr (MW == 1) {
-        if (p.reverse_mask)
-          kmask = __brev(kmask) >> (32 - p.kv);
-        cont = on_tile(tile, sl, kmask_store, kmask != 0);
-        uint32_t bits = kmask;
-        bool first = true;
-        while (cont && bits) {
-          int f = __ffs(bits) - 1;
-          bits &= bits - 1;
-          for (int kp = 0; cont && kp < kpasses; ++kp) {
-            bool last = (bits == 0) && (kp == kpasses - 1);
-            cont = on_step(tile, f, kp, first, last);
-            first = false;
-          }
-        }
-      } else {
-        // several mask words: offsets in ascending order word by word; with reverse_mask step
-        // `pos` (weight offset pos) is taken iff the bit of offset kv - 1 - pos is set, so the
-        // words are walked from the last bit down
-        uint32_t km[MW];
-        int remaining = 0;
-#pragma unroll
-        for (int w = 0; w < MW; ++w) {
-          km[w] = static_cast<uint32_t>(sl[4 + w]);
-          remaining += __popc(km[w]);
-        }
-        cont = on_tile(tile, sl, kmask_store, remaining != 0);
-        bool first = true;
-        for (int ww = 0; cont && ww < MW; ++ww) {
-          const int w = p.reverse_mask ? MW - 1 - ww : ww;
-          uint32_t bits = km[w];
-          while (cont && bits) {
-            const int b = p.reverse_mask ? 31 - __clz(bits) : __ffs(bits) - 1;
-            bits &= ~(1u << b);
-            const int f = p.reverse_mask ? p.kv - 1 - (32 * w + b) : 32 * w + b;
-            --remaining;
-            for (int kp = 0; cont && kp < kpasses; ++kp) {
-              bool last = (remaining == 0) && (kp == kpasses - 1);
-              cont = on_step(tile, f, kp, first, last);
-              first = false;
-            }
-          }
-        }
+// Walks the tiles the scheduler publishes; every consumer warp of the CTA has one and runs the
+// identical walk, so their step counters agree.  next() reads a tile's header into registers, the same
+// in every lane, lets the role read its rows and gives the slot back at once; the role loops over the
+// tile's (filter offset, reduction pass) steps itself.  A walk that called a function per step, run by one
+// thread, had the MMA issuer at 1500 cycles per step (walk 360, waits 500, four MMAs 260, commits 130),
+// which paced every tile with several offsets.
+template <int MW> struct TileCursor {
+  static_assert(MW == 1 || MW == 4, "one mask word, or four");
+  int slot = 0;
+  uint32_t phase = 0;
+  int tile, n0;
+  int offsets;  // filter offsets present
+  // the offsets still to be taken, bit i = weight offset i (reverse_mask has been applied)
+  uint32_t m;
+  unsigned long long lo, hi;  // four words
+  // Returns 1 on a tile, 0 at the end, -1 when the wait gave up.  read(slot) runs before the slot is
+  // given back.
+  template <class ReadFn>
+  __device__ __forceinline__ int next(const RowConvParams &p, const RingView &rv, ReadFn read) {
+    const bool ok = mbar_wait(rv.full0 + 8u * slot, phase, rv.abort_flag);
+    if (!__all_sync(0xffffffffu, ok))
+      return -1;
+    const int *sl = rv.slot(slot);
+    const int4 head = *reinterpret_cast<const int4 *>(sl);
+    tile = __shfl_sync(0xffffffffu, head.x, 0);
+    n0 = __shfl_sync(0xffffffffu, head.w, 0);
+    if constexpr (MW == 1) {
+      m = __shfl_sync(0xffffffffu, static_cast<uint32_t>(head.y), 0);
+      if (p.reverse_mask)
+        m = __brev(m) >> (32 - p.kv);
+      offsets = __popc(m);
+    } else {
+      const int4 w = *reinterpret_cast<const int4 *>(sl + 4);
+      auto join = [](int a, int b) {
+        return (static_cast<unsigned long long>(static_cast<uint32_t>(b)) << 32) | static_cast<uint32_t>(a);
+      };
+      lo = __shfl_sync(0xffffffffu, join(w.x, w.y), 0);
+      hi = __shfl_sync(0xffffffffu, join(w.z, w.w), 0);
+      if (p.reverse_mask) {  // 128 bits reversed, then shifted down by 128 - kv
+        const unsigned long long rl = __brevll(hi), rh = __brevll(lo);
+        const int s = 128 - p.kv;
+        lo = s >= 64 ? rh >> (s - 64) : (s == 0 ? rl : (rl >> s) | (rh << (64 - s)));
+        hi = s >= 64 ? 0ull : rh >> s;
       }
+      offsets = __popcll(lo) + __popcll(hi);
     }
-    CB2_WALK_MARK(10);  // steps done
-    if (!SINGLE)
-      __syncwarp();
-    if (SINGLE || lane_id() == 0)
-      mbar_arrive(rv.empty0 + 8u * si);
-    if (!cont)
-      return false;
-    if (tile < 0)
-      return true;  // end marker
+    read(sl);
+    __syncwarp();
+    if (lane_id() == 0)
+      mbar_arrive(rv.empty0 + 8u * slot);
+    if (++slot == rv.ring) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    return tile >= 0 ? 1 : 0;
   }
-}
-
-template <int MW, class TileFn, class StepFn>
-__device__ __forceinline__ bool walk_steps(const RowConvParams &p, const RingView &rv, int kpasses, TileFn on_tile,
-                                           StepFn on_step) {
-  return walk_steps_impl<false, MW>(p, rv, kpasses, on_tile, on_step);
-}
-template <int MW, class TileFn, class StepFn>
-__device__ __forceinline__ bool walk_steps_single(const RowConvParams &p, const RingView &rv, int kpasses,
-                                                  TileFn on_tile, StepFn on_step, long long *prof_c = nullptr,
-                                                  long long *prof_prev_p = nullptr) {
-  return walk_steps_impl<true, MW>(p, rv, kpasses, on_tile, on_step, prof_c, prof_prev_p);
-}
+  __device__ __forceinline__ int first_offset() const {
+    if constexpr (MW == 1)
+      return __ffs(m) - 1;
+    else
+      return lo ? __ffsll(lo) - 1 : 63 + __ffsll(hi);
+  }
+  __device__ __forceinline__ int last_offset() const {
+    if constexpr (MW == 1)
+      return 31 - __clz(m);
+    else
+      return hi ? 127 - __clzll(hi) : 63 - __clzll(lo);
+  }
+  __device__ __forceinline__ int take() {
+    const int f = first_offset();
+    if constexpr (MW == 1)
+      m &= m - 1;
+    else if (lo)
+      lo &= lo - 1;
+    else
+      hi &= hi - 1;
+    return f;
+  }
+};
 
 // The scheduler warp: draws tiles and fetches their mask words and row numbers straight into
 // a ring slot with 4-byte cp.async.  The slot's "landed" barrier is completed by the copies
 // themselves (one asynchronous arrival per lane), so any number of tiles can be in flight and
 // each is published -- its OR-ed mask computed once, here -- as soon as ITS words are there.
-// Slot layout (ints): [0] tile (-1 = no more tiles), [1] OR-ed mask (with several mask words per
+// Slot layout (ints): [0] tile (-1 = no more tiles), [3] first output column, [1] OR-ed mask (with several mask words per
 // row: the OR of all of them, and the OR-ed words themselves at [4, 4 + MW)), [2] steps charged
 // for the tile (scheduler only), [8,136) rows the gather starts from, from 136 on the destination
 // rows in gather-GEMM mode / the rows' raw mask words (MW per row) in conv mode (in conv mode the
@@ -332,14 +324,10 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // The first batch of tickets is requested at kernel entry (first_ticket_request), long before the
 // scheduler can use it: the counter's round trip, and an L2 prefetch of the first tile's words,
 // run while the CTA sets up its barriers and tensor memory.
-__device__ __forceinline__ int first_ticket_count(int ntiles) {
-  const int b = ntiles / ((int)gridDim.x * 4);
-  return b < 1 ? 1 : (b > CB2_ROWCONV_TICKET_BATCH ? CB2_ROWCONV_TICKET_BATCH : b);
-}
-
 template <int MW>
-__device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int kpasses,
-                                              int first_base, int first_cnt) {
+__device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int block_n,
+                                              int kpasses, int first_base, int first_cnt) {
+  const int nitems = ntiles * p.n_parts;
   constexpr int STEP_BUDGET = CB2_ROWCONV_STEP_BUDGET;  // steps a CTA may hold (drawn, not finished)
   const int lane = (int)lane_id();
   const bool dynamic = p.tickets != nullptr && gridDim.y == 1;
@@ -350,8 +338,9 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // one ticket as the counter nears the end so the tail stays balanced.
   constexpr int MAX_BATCH = CB2_ROWCONV_TICKET_BATCH;
   int cur_base = 0, cur_left = 0, next_base = 0, next_cnt = 0;
-  auto request = [&](int seen) {
-    int b = (ntiles - seen) / ((int)gridDim.x * 4);
+  auto request = [&](int seen, int last_steps) {
+    // (the first tiles carry the most offsets: four of those in one hand set the length of a launch)
+    int b = last_steps > 2 ? 1 : (nitems - seen) / ((int)gridDim.x * 4);
     next_cnt = b < 1 ? 1 : (b > MAX_BATCH ? MAX_BATCH : b);
     if (lane == 0)
       next_base = atomicAdd(p.tickets, next_cnt);
@@ -360,15 +349,15 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
     next_base = first_base;  // requested at kernel entry (lane 0 holds the counter's answer)
     next_cnt = first_cnt;
   }
-  auto draw = [&]() -> int {
+  auto draw = [&](int last_steps) -> int {
     int t;
     if (dynamic) {
       if (cur_left == 0) {
         cur_base = __shfl_sync(0xffffffffu, next_base, 0);
         cur_left = next_cnt;
         next_cnt = 0;
-        if (cur_base < ntiles)
-          request(cur_base);
+        if (cur_base < nitems)
+          request(cur_base, last_steps);
       }
       t = cur_base++;
       --cur_left;
@@ -445,20 +434,28 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
       continue;
     }
     const int si = issued % rv.ring;
-    const int ticket = draw();
+    const int ticket = draw(guess);
 #ifndef CB2_TRACE_TICKET
 #define CB2_TRACE_TICKET 0  // 0: follow the CTA that got the heaviest tile
 #endif
     if (ticket == CB2_TRACE_TICKET && lane == 0)
       CB2_TRACE_SELECT(1);
-    int tile = -1;
-    if (ticket < ntiles)
-      tile = conv ? (ntiles - 1 - ticket) : ticket;  // the last tiles of the sorted order carry the most offsets
+    int tile = -1, part = 0;
+    if (ticket < nitems) {
+      tile = ticket;
+      if (p.n_parts > 1) {
+        tile = ticket / p.n_parts;
+        part = ticket - tile * p.n_parts;
+      }
+      if (conv)
+        tile = ntiles - 1 - tile;  // the last tiles of the sorted order carry the most offsets
+    }
     int *sl = rv.slot(si);
     const uint32_t sa = slots_addr + static_cast<uint32_t>(si * rv.slot_ints) * 4u;
     if (lane == 0) {
       sl[0] = tile;
       sl[2] = guess;
+      sl[3] = part * block_n;
     }
     held_steps += guess;
     if (wide_copies && tile >= 0 && (tile + 1) * 128 <= p.n_rows) {
@@ -550,17 +547,17 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
 
   const uint32_t bars = sbase + Cfg::OFF_BARS;
   auto full_a = [&](int s) { return bars + 8u * s; };
-  auto empty_a = [&](int s) { return bars + 8u * (3 + s); };
-  auto acc_full = [&](int s) { return bars + 8u * (6 + s); };
-  auto acc_empty = [&](int s) { return bars + 8u * (10 + s); };
-  const uint32_t final_bar = bars + 8u * 14;
-  auto full_b = [&](int s) { return bars + 8u * (16 + s); };
-  auto empty_b = [&](int s) { return bars + 8u * (24 + s); };
+  auto empty_a = [&](int s) { return bars + 8u * (Cfg::BAR_EMPTY_A + s); };
+  auto acc_full = [&](int s) { return bars + 8u * (Cfg::BAR_ACC_FULL + s); };
+  auto acc_empty = [&](int s) { return bars + 8u * (Cfg::BAR_ACC_EMPTY + s); };
+  const uint32_t final_bar = bars + 8u * Cfg::BAR_FINAL;
+  auto full_b = [&](int s) { return bars + 8u * (Cfg::BAR_FULL_B + s); };
+  auto empty_b = [&](int s) { return bars + 8u * (Cfg::BAR_EMPTY_B + s); };
   RingView rv;
   rv.slots = reinterpret_cast<int *>(smem + Cfg::OFF_RING);
-  rv.full0 = bars + 8u * 32;
-  rv.empty0 = bars + 8u * (32 + Cfg::RING);
-  rv.landed0 = bars + 8u * (32 + 2 * Cfg::RING);
+  rv.full0 = bars + 8u * Cfg::BAR_RING;
+  rv.empty0 = rv.full0 + 8u * Cfg::RING;
+  rv.landed0 = rv.empty0 + 8u * Cfg::RING;
   rv.ring = Cfg::RING;
   rv.slot_ints = Cfg::RING_SLOT_INTS;
   rv.abort_flag = abort_flag;
@@ -569,12 +566,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   const int lane = threadIdx.x & 31;
   const int ntiles = (p.n_rows + 127) / 128;
   const int kpasses = (p.red + Cfg::KRED - 1) / Cfg::KRED;
-  const int n0 = blockIdx.y * BLOCK_N;
 
   // Scheduler warp: ask for the first tickets now; their round trip overlaps the set-up below.
   int early_base = 0, early_cnt = 0;
   if (warp == Cfg::SCHED_WARP && p.tickets != nullptr && gridDim.y == 1) {
-    early_cnt = first_ticket_count(ntiles);
+    early_cnt = 1;
     if (lane == 0)
       early_base = atomicAdd(p.tickets, early_cnt);
   }
@@ -605,7 +601,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   }
   if (KIND == 1) {
     for (int i = threadIdx.x; i < BLOCK_N; i += blockDim.x) {
-      int n = n0 + i;
+      int n = blockIdx.y * BLOCK_N + i;
       s_scale[i] = (n < p.nn && p.scale) ? p.scale[n] : 0.f;
       s_bias[i] = (n < p.nn && p.bias) ? p.bias[n] : 0.f;
     }
@@ -617,7 +613,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   if (warp == Cfg::SCHED_WARP && early_cnt > 0 && p.mode == kModeMaskConv) {
     // the first tile's sort order and masks: 128 ints each, four 128-byte lines each
     const int first = __shfl_sync(0xffffffffu, early_base, 0);
-    const int tile = ntiles - 1 - first;
+    const int tile = ntiles - 1 - first / p.n_parts;
     if (tile >= 0 && lane < 8) {
       const int r = tile * 128 + (lane & 3) * 32;
       if (r < p.n_rows) {
@@ -652,22 +648,30 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     int acc_use = 0;
     bool dep_waited = false;
     CB2_PROF_BEGIN();
-    walk_steps<MW>(
-        p, rv, kpasses,
-        [&](int tile, const int *sl, uint32_t kmask_store, bool has_work) -> bool {
+    TileCursor<MW> tc;
+    int o = -1;  // destination row of this thread's tile row
+    for (int more; (more = tc.next(p, rv, [&](const int *sl) {
+                      o = (p.mode == kModeMaskConv) ? sl[8 + erow] : sl[136 + erow];
+                    })) > 0;) {
+          const int tile = tc.tile;
+          const bool has_work = tc.offsets != 0;
+          if (!has_work && p.skip_empty_tiles)
+            continue;
+          const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
           if (et == 0)
             CB2_PROF_MARK(0);  // walk
           if (!dep_waited) {
             grid_dep_wait();
             dep_waited = true;
           }
-          const int o = (p.mode == kModeMaskConv) ? sl[8 + erow] : sl[136 + erow];  // destination row of this thread's tile row
-          if (et == 0 && p.mask_out && blockIdx.y == 0) {
+          if (et == 0 && p.mask_out && n0 == 0) {
             if constexpr (MW == 1) {
-              p.mask_out[tile] = kmask_store;
+              p.mask_out[tile] = tc.m;  // forward: not reversed
             } else {
-              for (int w = 0; w < p.mask_words; ++w)
-                p.mask_out[(long long)tile * p.mask_words + w] = static_cast<uint32_t>(sl[4 + w]);
+#pragma unroll
+              for (int w = 0; w < MW; ++w)
+                if (w < p.mask_words)
+                  p.mask_out[(long long)tile * p.mask_words + w] = static_cast<uint32_t>((w < 2 ? tc.lo : tc.hi) >> (32 * (w & 1)));
             }
           }
           const int buf = acc_use % Cfg::NUM_ACC;
@@ -686,7 +690,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           if (et == 0)
             CB2_PROF_MARK(2);  // barrier
           if (has_work && misc[2] == 0)
-            return false;
+            break;
           if (half == 0)
             outrow[erow] = o;
           tc_fence_after();
@@ -865,107 +869,112 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             CB2_TRACE_EVENT(4, 9, tile);  // rows stored
             CB2_PROF_MARK(5);  // staging -> global
           }
-          return true;
-        },
-        [&](int, int, int, bool, bool) -> bool { return true; });
+    }
     if (et == 0)
       CB2_PROF_END2();
   } else if (warp == Cfg::MMA_WARP) {
-    // ======================= MMA issuer (one thread walks and issues)
+    // ======================= MMA issuer: the warp walks together (its state is the same in every
+    // lane), lane 0 issues
     constexpr uint32_t idesc = make_idesc(KIND, false, B_MN, 128, BLOCK_N);
-    int step = 0, acc_use = 0, bcount = 0, last_key = -1, cur_slot = 0;
-    bool ok_all = true;
+    constexpr int KSTEPS_FULL = NATOM_K * 4;
     const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_A, 16, 1024);
     const uint64_t bdesc_base = B_MN ? make_smem_desc(sbase + Cfg::OFF_B, p.b_lbo, p.b_sbo)
                                      : make_smem_desc(sbase + Cfg::OFF_B, 16, 1024);
+    const int ksteps_last = (p.red - (kpasses - 1) * Cfg::KRED + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
+    TileCursor<MW> tc;
+    int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
+    uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
+    bool ok = true;
     CB2_PROF_BEGIN();
-    if (lane == 0) {
-    walk_steps_single<MW>(
-        p, rv, kpasses,
-        [&](int, const int *, uint32_t, bool) -> bool {
-          CB2_PROF_MARK(7);  // previous slot released, this tile's slot read
-          return true;
-        },
-        [&](int tile, int f, int kp, bool first, bool last) -> bool {
-          const int buf = acc_use % Cfg::NUM_ACC;
-          int ok = 1;
-          {
-            CB2_PROF_MARK(0);  // the walk between steps
-            if (first)
-              ok = mbar_wait(acc_empty(buf), ((acc_use / Cfg::NUM_ACC) & 1) ^ 1, abort_flag);
-            CB2_PROF_MARK(1);  // accumulator free
-            const int key = f * kpasses + kp;
-            if (ok && key != last_key) {
-              if (bcount > 0)
-                tc_commit(empty_b(cur_slot));
-              cur_slot = bcount % Cfg::SB;
-              ok = mbar_wait(full_b(cur_slot), (bcount / Cfg::SB) & 1, abort_flag);
-              ++bcount;
-              last_key = key;
-            }
-            const int stage = step % Cfg::SA;
-            CB2_PROF_MARK(2);  // weight tile present
-            CB2_TRACE_EVENT(3, 4, step);  // waiting for rows
-            if (ok)
-              ok = mbar_wait(full_a(stage), (step / Cfg::SA) & 1, abort_flag);
-            CB2_TRACE_EVENT(3, 5, step);  // rows landed
-            CB2_PROF_MARK(3);  // rows present
-            if (ok) {
-              if constexpr (!TMA_GATHER)
-                fence_proxy_async_smem();  // gathered rows were written through the generic proxy
-              tc_fence_after();
-              CB2_PROF_MARK(4);  // fences
-              // Descriptors differ from the stage's / slot's base descriptor only in the start
-              // address field (bits 0-13, units of 16 bytes), so each one is an add.  This loop is
-              // issued by a single thread: every instruction saved here shortens each step.
-              const uint64_t adesc0 = adesc_base + static_cast<uint64_t>((stage * Cfg::A_STAGE_BYTES) >> 4);
-              const uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((cur_slot * Cfg::B_SLOT_BYTES) >> 4);
-              const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
-              const int red_left = p.red - kp * Cfg::KRED;
-              constexpr int KSTEPS_FULL = NATOM_K * 4;
-              auto issue = [&](int ks, uint32_t acc) {
-                const int ka = ks >> 2, kk = ks & 3;
-                const uint64_t adesc = adesc0 + static_cast<uint64_t>((ka * (Cfg::TILE_M * 128) + kk * 32) >> 4);
-                const uint64_t bdesc =
-                    bdesc0 + static_cast<uint64_t>(B_MN ? (((ka * 4 + kk) * (Cfg::UMMA_K * 128)) >> 4)
-                                                        : ((ka * (BLOCK_N * 128) + kk * 32) >> 4));
-                tc_mma<KIND>(d_tmem, adesc, bdesc, idesc, acc);
-              };
-              if (red_left >= Cfg::KRED) {
-#pragma unroll
-                for (int ks = 0; ks < KSTEPS_FULL; ++ks)
-                  issue(ks, (first && ks == 0) ? 0u : 1u);
-              } else {
-                const int ksteps_total = (red_left + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
-                for (int ks = 0; ks < ksteps_total; ++ks)
-                  issue(ks, (first && ks == 0) ? 0u : 1u);
-              }
-              CB2_PROF_MARK(5);  // MMAs issued
-              tc_commit(empty_a(stage));
-              CB2_TRACE_EVENT(3, 6, step);  // MMAs issued
-              if (last)
-                tc_commit(acc_full(buf));
-              CB2_PROF_MARK(6);  // commits
-            }
+    for (int more; ok && (more = tc.next(p, rv, [](const int *) {})) != 0;) {
+      CB2_PROF_MARK(0);  // next tile
+      if (more < 0) {
+        ok = false;
+        break;
+      }
+      if (tc.offsets == 0)
+        continue;
+      // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
+      // are in the key: weights have as many columns)
+      bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
+      ok = mbar_wait(acc_empty(buf), acc_phase, abort_flag);
+      CB2_PROF_MARK(1);  // accumulator free
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
+      const int total = tc.offsets * kpasses;
+      int kp = 0;
+      for (int s = 0; s < total; ++s) {
+        if (new_b) {
+          if (last_key >= 0 && lane == 0)
+            tc_commit(empty_b(bslot));
+          last_key = 0;
+          if (++bslot == Cfg::SB) {
+            bslot = 0;
+            b_phase ^= 1u;
           }
-          ++step;
-          if (last)
-            ++acc_use;
-          if (!ok) {
-            fail(kStatusWaitTimeout);
-            ok_all = false;
-            return false;
-          }
-          return true;
         }
-#ifdef CB2_TRACE
-        , prof_c, &prof_prev
-#endif
-        );
-      CB2_TRACE_CTA(2, (unsigned long long)step);
+        const bool b_there = mbar_test(full_b(bslot), b_phase), a_there = mbar_test(full_a(stage), a_phase);
+        if (!b_there)
+          ok = ok && mbar_wait(full_b(bslot), b_phase, abort_flag);
+        CB2_PROF_MARK(2);  // weight tile present
+        if (!a_there)
+          ok = ok && mbar_wait(full_a(stage), a_phase, abort_flag);
+        CB2_PROF_MARK(3);  // rows present
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok)
+          break;
+        if constexpr (!TMA_GATHER)
+          fence_proxy_async_smem();  // gathered rows were written through the generic proxy
+        tc_fence_after();
+        // descriptors differ from the stage's / slot's base descriptor only in the start address field
+        // (bits 0-13, units of 16 bytes)
+        const uint64_t adesc0 = adesc_base + static_cast<uint64_t>((stage * Cfg::A_STAGE_BYTES) >> 4);
+        const uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((bslot * Cfg::B_SLOT_BYTES) >> 4);
+        auto issue = [&](int ks, uint32_t acc) {
+          const int ka = ks >> 2, kk = ks & 3;
+          const uint64_t adesc = adesc0 + static_cast<uint64_t>((ka * (Cfg::TILE_M * 128) + kk * 32) >> 4);
+          const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(B_MN ? (((ka * 4 + kk) * (Cfg::UMMA_K * 128)) >> 4)
+                                                                     : ((ka * (BLOCK_N * 128) + kk * 32) >> 4));
+          tc_mma<KIND>(d_tmem, adesc, bdesc, idesc, acc);
+        };
+        const bool last_pass = ++kp == kpasses;
+        if (lane == 0) {
+          if (!last_pass || ksteps_last == KSTEPS_FULL) {
+#pragma unroll
+            for (int ks = 0; ks < KSTEPS_FULL; ++ks)
+              issue(ks, (s == 0 && ks == 0) ? 0u : 1u);
+          } else {
+            for (int ks = 0; ks < ksteps_last; ++ks)
+              issue(ks, (s == 0 && ks == 0) ? 0u : 1u);
+          }
+          CB2_PROF_MARK(5);  // MMAs issued
+          tc_commit(empty_a(stage));
+          if (s == total - 1)
+            tc_commit(acc_full(buf));
+        }
+        __syncwarp();
+        CB2_PROF_MARK(6);  // commits
+        if (last_pass)
+          kp = 0;
+        if (++stage == Cfg::SA) {
+          stage = 0;
+          a_phase ^= 1u;
+        }
+        new_b = true;
+        ++steps;
+      }
+      last_key = (tc.last_offset() * kpasses + kpasses - 1) * p.nn + tc.n0;
+      if (++buf == Cfg::NUM_ACC) {
+        buf = 0;
+        acc_phase ^= 1u;
+      }
+    }
+    if (lane == 0) {
+      CB2_TRACE_CTA(2, (unsigned long long)steps);
       CB2_PROF_END();
-      // make sure every MMA has retired before TMEM is released
-      if (ok_all) {
+      if (!ok) {
+        fail(kStatusWaitTimeout);
+      } else {
+        // make sure every MMA has retired before TMEM is released
         tc_commit(final_bar);
         if (!mbar_wait(final_bar, 0, abort_flag))
           fail(kStatusWaitTimeout);
@@ -974,51 +983,53 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     __syncwarp();
   } else if (warp == Cfg::TMA_WARP) {
     // ======================= weight tiles by TMA (lane 0 issues)
-    int bcount = 0, last_key = -1;
-    if (lane == 0) {
-    tma_prefetch_desc(&tmap_b);
+    TileCursor<MW> tc;
+    int bslot = 0, last_key = -1;
+    uint32_t b_phase = 1;
+    bool ok = true;
+    if (lane == 0)
+      tma_prefetch_desc(&tmap_b);
     grid_dep_wait();
-    walk_steps_single<MW>(
-        p, rv, kpasses, [&](int, const int *, uint32_t, bool) -> bool { return true; },
-        [&](int tile, int f, int kp, bool, bool) -> bool {
-          int ok = 1;
-          const int key = f * kpasses + kp;
-          if (key != last_key) {
-            {
-              const int slot = bcount % Cfg::SB;
-              ok = mbar_wait(empty_b(slot), ((bcount / Cfg::SB) & 1) ^ 1, abort_flag);
-              if (ok) {
-                const uint32_t dst = sbase + Cfg::OFF_B + slot * Cfg::B_SLOT_BYTES;
-                mbar_arrive_expect_tx(full_b(slot), Cfg::B_SLOT_BYTES);
-                if constexpr (!B_MN) {
-                  // [BLOCK_N rows x 128 B] per reduction atom; rows = output channels
+    for (int more; ok && (more = tc.next(p, rv, [](const int *) {})) != 0;) {
+      ok = more > 0;
+      for (int left = ok ? tc.offsets : 0; ok && left > 0; --left) {
+        const int f = tc.take();
+        for (int kp = 0; ok && kp < kpasses; ++kp) {
+          const int key = (f * kpasses + kp) * p.nn + tc.n0;
+          if (key == last_key)
+            continue;
+          last_key = key;
+          ok = __all_sync(0xffffffffu, mbar_wait(empty_b(bslot), b_phase, abort_flag));
+          if (ok && lane == 0) {
+            const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
+            const uint32_t dst = sbase + Cfg::OFF_B + bslot * Cfg::B_SLOT_BYTES;
+            mbar_arrive_expect_tx(full_b(bslot), Cfg::B_SLOT_BYTES);
+            if constexpr (!B_MN) {
+              // [BLOCK_N rows x 128 B] per reduction atom; rows = output channels
 #pragma unroll
-                  for (int ka = 0; ka < NATOM_K; ++ka)
-                    tma_load_3d(dst + ka * (BLOCK_N * 128), &tmap_b, full_b(slot),
-                                kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS, f, n0);
-                } else {
-                  // [KRED rows x 128 B] per block of ATOM_ELEMS output channels; rows = reduction
+              for (int ka = 0; ka < NATOM_K; ++ka)
+                tma_load_3d(dst + ka * (BLOCK_N * 128), &tmap_b, full_b(bslot), kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS, f, n0);
+            } else {
+              // [KRED rows x 128 B] per block of ATOM_ELEMS output channels; rows = reduction
 #pragma unroll
-                  for (int na = 0; na < BLOCK_N / Cfg::ATOM_ELEMS; ++na)
-                    tma_load_3d(dst + na * (Cfg::KRED * 128), &tmap_b, full_b(slot),
-                                n0 + na * Cfg::ATOM_ELEMS, f, kp * Cfg::KRED);
-                }
-              }
+              for (int na = 0; na < BLOCK_N / Cfg::ATOM_ELEMS; ++na)
+                tma_load_3d(dst + na * (Cfg::KRED * 128), &tmap_b, full_b(bslot), n0 + na * Cfg::ATOM_ELEMS, f, kp * Cfg::KRED);
             }
-            ++bcount;
-            last_key = key;
           }
-          if (!ok) {
-            fail(kStatusWaitTimeout);
-            return false;
+          __syncwarp();
+          if (++bslot == Cfg::SB) {
+            bslot = 0;
+            b_phase ^= 1u;
           }
-          return true;
-        });
+        }
+      }
     }
+    if (!ok && lane == 0)
+      fail(kStatusWaitTimeout);
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
-    scheduler_run<MW>(p, rv, ntiles, kpasses, early_base, early_cnt);
+    scheduler_run<MW>(p, rv, ntiles, BLOCK_N, kpasses, early_base, early_cnt);
   } else {
     // ======================= operand-row gather: group g owns stage g
     if constexpr (TMA_GATHER) {
@@ -1031,43 +1042,49 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       const int g = warp - Cfg::FIRST_GATHER_WARP;
       if (lane == 0)
         tma_prefetch_desc(&tmap_a);
-      const uint32_t my_quad = sbase + Cfg::OFF_A + g * Cfg::A_STAGE_BYTES + lane * (4 * 128);
-      auto clear_quad = [&]() {
+      const uint32_t first_quad = sbase + Cfg::OFF_A + g * Cfg::A_STAGE_BYTES;
+      const uint32_t my_quad = first_quad + lane * (4 * 128);
+      // The warp clears one quad at a time, every lane 16 of its 512 bytes: with a quad per lane the
+      // lanes' addresses are 512 bytes apart and all meet in the same banks.
+      auto clear_quads = [&](uint32_t quads) {
+        for (; quads; quads &= quads - 1) {
+          const uint32_t at = first_quad + (__ffs(quads) - 1) * (4 * 128) + lane * 16;
 #pragma unroll
-        for (int ka = 0; ka < NATOM_K; ++ka)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            st_shared_zero16(my_quad + ka * (Cfg::TILE_M * 128) + i * 16);
+          for (int ka = 0; ka < NATOM_K; ++ka)
+            st_shared_zero16(at + ka * (Cfg::TILE_M * 128));
+        }
+        fence_proxy_async_smem();  // generic-proxy stores, read by the tensor core
       };
-      clear_quad();
-      fence_proxy_async_smem();
+      clear_quads(0xffffffffu);
       __syncwarp();
       uint32_t dirty = 0;  // quads of this stage that hold gathered rows
-      bool dep_waited = false;
-      int step = 0;
-      int o[4] = {-1, -1, -1, -1};
-      walk_steps<MW>(
-          p, rv, kpasses,
-          [&](int tile, const int *sl, uint32_t, bool) -> bool {
-            const int4 v = *reinterpret_cast<const int4 *>(sl + 8 + lane * 4);
-            o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
-            return true;
-          },
-          [&](int tile, int f, int kp, bool, bool) -> bool {
-            const bool mine = (step % Cfg::SA) == g;
-            const int use = step / Cfg::SA;
-            ++step;
+      bool dep_waited = false, ok = true;
+      int stage = 0;         // stage of the CTA's next step
+      uint32_t phase = 1;    // of this warp's own stage
+      TileCursor<MW> tc;
+      int4 o = make_int4(-1, -1, -1, -1);
+      for (int more; ok && (more = tc.next(p, rv, [&](const int *sl) {
+                             o = *reinterpret_cast<const int4 *>(sl + 8 + lane * 4);
+                           })) != 0;) {
+        ok = more > 0;
+        for (int left = ok ? tc.offsets : 0; ok && left > 0; --left) {
+          const int f = tc.take();
+          for (int kp = 0; kp < kpasses; ++kp) {
+            const bool mine = stage == g;
+            if (++stage == Cfg::SA)
+              stage = 0;
             if (!mine)
-              return true;
+              continue;
+            const int row[4] = {o.x, o.y, o.z, o.w};
             int idx[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
               idx[r] = -1;
-              if (o[r] >= 0) {
+              if (row[r] >= 0) {
                 if (p.mode == kModeMaskConv)
-                  idx[r] = __ldg(p.indices + (long long)f * p.n_rows + o[r]);
+                  idx[r] = __ldg(p.indices + (long long)f * p.n_rows + row[r]);
                 else
-                  idx[r] = p.a_inds ? __ldg(p.a_inds + o[r]) : o[r];
+                  idx[r] = p.a_inds ? __ldg(p.a_inds + row[r]) : row[r];
               }
             }
 #pragma unroll
@@ -1077,25 +1094,22 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                 idx[r] = -1;
               }
             if (lane == 0)
-              CB2_TRACE_EVENT(g, 1, step - 1 + (idx[0] == 0x7fffffff));  // index loaded
-            if (!mbar_wait_warp(empty_a(g), (use & 1) ^ 1, abort_flag)) {
-              if (lane == 0)
-                fail(kStatusWaitTimeout);
-              return false;
-            }
+              CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
+            ok = mbar_wait_warp(empty_a(g), phase, abort_flag);
+            if (!ok)
+              break;
+            phase ^= 1u;
             if (!dep_waited) {
               grid_dep_wait();
               dep_waited = true;
             }
             const bool wanted = (idx[0] & idx[1] & idx[2] & idx[3]) >= 0;  // some row index is not -1
             const uint32_t need = __ballot_sync(0xffffffffu, wanted);
-            if (((dirty >> lane) & 1u) && !wanted) {
-              clear_quad();
-              fence_proxy_async_smem();  // generic-proxy stores, read by the tensor core
-            }
+            if (dirty & ~need)
+              clear_quads(dirty & ~need);
             __syncwarp();
             if (lane == 0) {
-              CB2_TRACE_EVENT(g, 2, step - 1);  // stage free
+              CB2_TRACE_EVENT(g, 2, f);  // stage free
               mbar_arrive_expect_tx(full_a(g), static_cast<uint32_t>(__popc(need)) * (NATOM_K * 512));
             }
             __syncwarp();
@@ -1107,9 +1121,12 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             }
             dirty = need;
             if (lane == 0)
-              CB2_TRACE_EVENT(g, 3, step - 1);  // copies issued
-            return true;
-          });
+              CB2_TRACE_EVENT(g, 3, f);  // copies issued
+          }
+        }
+      }
+      if (!ok && lane == 0)
+        fail(kStatusWaitTimeout);
     } else {
       constexpr int GT = Cfg::GROUP_THREADS;
       constexpr int RPT = (128 + GT - 1) / GT;                  // tile rows whose index each thread fetches
@@ -1121,28 +1138,29 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       const int row0 = gt / CPR;
       int *group_rowidx = rowidx + g * 256;  // two buffers, alternating per use of the stage
       volatile int *my_flag = misc + 3 + g;
-      bool dep_waited = false;
-      int step = 0;
+      bool dep_waited = false, ok = true;
+      int stage = 0;       // stage of the CTA's next step
+      uint32_t use = 0;    // of this group's own stage
       int o[RPT];
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
         o[r] = -1;
       const uint8_t *a_bytes = reinterpret_cast<const uint8_t *>(p.a);
-      walk_steps<MW>(
-          p, rv, kpasses,
-          [&](int tile, const int *sl, uint32_t, bool) -> bool {
-            // the rows this thread's gathers start from (sort index, or the row itself)
+      TileCursor<MW> tc;
+      for (int more; ok && (more = tc.next(p, rv, [&](const int *sl) {
+                             // the rows this thread's gathers start from (sort index, or the row itself)
 #pragma unroll
-            for (int r = 0; r < RPT; ++r)
-              o[r] = (gt + r * GT < 128) ? sl[8 + gt + r * GT] : -1;
-            return true;
-          },
-          [&](int tile, int f, int kp, bool, bool) -> bool {
-            const bool mine = (step % Cfg::SA) == g;
-            const int use = step / Cfg::SA;
-            ++step;
+                             for (int r = 0; r < RPT; ++r)
+                               o[r] = (gt + r * GT < 128) ? sl[8 + gt + r * GT] : -1;
+                           })) > 0;) {
+        for (int left = tc.offsets; ok && left > 0; --left) {
+          const int f = tc.take();
+          for (int kp = 0; ok && kp < kpasses; ++kp) {
+            const bool mine = stage == g;
+            if (++stage == Cfg::SA)
+              stage = 0;
             if (!mine)
-              return true;
+              continue;
             int idx[RPT];
 #pragma unroll
             for (int r = 0; r < RPT; ++r) {
@@ -1161,11 +1179,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                 idx[r] = -1;
               }
             if (gt == 0) {
-              CB2_TRACE_EVENT(g, 1, step - 1 + (idx[0] == 0x7fffffff));  // index loaded
-              bool ok = mbar_wait(empty_a(g), (use & 1) ^ 1, abort_flag);
-              CB2_TRACE_EVENT(g, 2, step - 1);  // stage free
-              *my_flag = ok ? 1 : 0;
-              if (!ok)
+              CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
+              const bool free = mbar_wait(empty_a(g), (use & 1) ^ 1, abort_flag);
+              CB2_TRACE_EVENT(g, 2, f);  // stage free
+              *my_flag = free ? 1 : 0;
+              if (!free)
                 fail(kStatusWaitTimeout);
             }
             // Double-buffered: a thread that runs ahead writes the other buffer than the one
@@ -1176,8 +1194,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
               if (gt + r * GT < 128)
                 my_rowidx[gt + r * GT] = idx[r];
             named_bar_sync(2 + g, Cfg::GROUP_THREADS);
-            if (*my_flag == 0)
-              return false;
+            ++use;
+            if (*my_flag == 0) {
+              ok = false;
+              break;
+            }
             if (!dep_waited) {
               grid_dep_wait();
               dep_waited = true;
@@ -1202,9 +1223,10 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             // to the tensor core with a proxy fence after its wait.
             cp_async_mbar_arrive_noinc(full_a(g));
             if (gt == 0)
-              CB2_TRACE_EVENT(g, 3, step - 1);  // copies issued
-            return true;
-          });
+              CB2_TRACE_EVENT(g, 3, f);  // copies issued
+          }
+        }
+      }
       cp_async_wait_all();
     }
   }
