@@ -358,11 +358,11 @@ void wgrad_layout(int num_sms, int max_ctas, int m_total, int n_total, long long
   L->total = L->off_lists + (size_t)kvs * L->list_stride * 4;
 }
 
-template <int BLOCK_N, int GATHER>
+template <int BLOCK_N, int A_ATOMS, int GATHER>
 int launch_wgrad_inst(const CUtensorMap &ma, const CUtensorMap &mb, const WgradParams &p, int gx, int gy,
                       cudaStream_t stream) {
-  using Cfg = WgradCfg<BLOCK_N, GATHER>;
-  auto kern = wgrad_kernel<BLOCK_N, GATHER>;
+  using Cfg = WgradCfg<BLOCK_N, A_ATOMS, GATHER>;
+  auto kern = wgrad_kernel<BLOCK_N, A_ATOMS, GATHER>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> regs{0};
   int dev = 0;
@@ -418,11 +418,16 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int re
   if (rc)
     return rc;
   const bool tma = gather_mode() != 0;
-  if (L.block_n == 64)
-    return tma ? launch_wgrad_inst<64, kGatherTma4>(ma, mb, p, L.G, L.gy, stream)
-               : launch_wgrad_inst<64, kGatherCpAsync>(ma, mb, p, L.G, L.gy, stream);
-  return tma ? launch_wgrad_inst<128, kGatherTma4>(ma, mb, p, L.G, L.gy, stream)
-             : launch_wgrad_inst<128, kGatherCpAsync>(ma, mb, p, L.G, L.gy, stream);
+#define CB2_INST(N, A)                                                                              \
+  if (tma && L.block_n == N && (p.m_total <= 64 ? 1 : 2) == A)                                      \
+    return launch_wgrad_inst<N, A, kGatherTma4>(ma, mb, p, L.G, L.gy, stream);
+  CB2_INST(64, 1)
+  CB2_INST(64, 2)
+  CB2_INST(128, 1)
+  CB2_INST(128, 2)
+#undef CB2_INST
+  return L.block_n == 64 ? launch_wgrad_inst<64, 2, kGatherCpAsync>(ma, mb, p, L.G, L.gy, stream)
+                         : launch_wgrad_inst<128, 2, kGatherCpAsync>(ma, mb, p, L.G, L.gy, stream);
 }
 
 // ---------------------------------------------------------------- allocation-free variant

@@ -67,22 +67,34 @@ struct WgradParams {
   int mode;
 };
 
-template <int BLOCK_N, int GATHER> struct WgradCfg {
-  static constexpr int SA = 3;
-  static constexpr int A_BYTES = 128 * 256;                 // 128 rows x (2 x 128 B): M = 128 channels
+// A_ATOMS: 64-channel column blocks of dout a tile loads.  With up to 64 output channels one is
+// enough: the MMA still has 128 rows, the upper 64 read whatever follows the stage's first block and
+// their sums are never stored.  The stages are as many as 192 KB hold, so that narrow layers have as
+// many bytes in flight as wide ones.
+template <int BLOCK_N, int A_ATOMS, int GATHER> struct WgradCfg {
+  static constexpr int A_BYTES = 128 * 128 * A_ATOMS;       // 128 rows x 64 channels per block
   static constexpr int B_BYTES = 128 * 2 * BLOCK_N;         // 128 rows x BLOCK_N fp16
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int SA = GATHER == kGatherCpAsync ? 3 : 192 * 1024 / STAGE_BYTES;  // 3, 4 or 6
+  static constexpr int M_ROWS = 64 * A_ATOMS;               // rows of a partial sum that are kept
   static constexpr int TMEM_COLS = 2 * BLOCK_N;
-  static constexpr int THREADS = 128 + 32 + SA * 128;       // epilogue, mma, 3 gather groups
+  // Epilogue (4 warps), MMA issuer, twelve warps that gather: four per stage, or two where there are
+  // more than three stages (issuing a stage's requests takes a warp longer than an MMA step: with one
+  // warp per stage the 128-channel layer took 45 instead of 35 us).
+  static constexpr int GW = SA == 3 ? 4 : 2;
+  static constexpr int THREADS = 544;
   static constexpr int FULL_COUNT = GATHER == kGatherCpAsync ? 128 : 1;
   static constexpr int OFF_STAGES = 0;
-  static constexpr int OFF_ROWIDX = SA * STAGE_BYTES;       // SA x 2 buffers x 2 operands x 128 ints
-  static constexpr int OFF_SCHED = OFF_ROWIDX + SA * 2 * 2 * 128 * 4;  // this CTA's units, then units per offset
+  static constexpr int OFF_ROWIDX = SA * STAGE_BYTES;       // 3 x 2 buffers x 2 operands x 128 ints
+  static constexpr int OFF_SCHED = OFF_ROWIDX + 3 * 2 * 2 * 128 * 4;  // this CTA's units, then units per offset
   static constexpr int TILE_CAP = 2048;                      // tiles of one CTA staged in shared memory
   static constexpr int OFF_TILES = OFF_SCHED + 1024 * 4;
   static constexpr int OFF_BARS = OFF_TILES + TILE_CAP * 4;
-  static constexpr int OFF_MISC = OFF_BARS + 16 * 8;
+  static constexpr int BAR_ACC_FULL = 2 * SA, BAR_ACC_EMPTY = BAR_ACC_FULL + 2, BAR_FINAL = BAR_ACC_EMPTY + 2;
+  static constexpr int OFF_MISC = OFF_BARS + (BAR_FINAL + 2) / 2 * 2 * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;
+  static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
+  static_assert(A_ATOMS == 2 || GATHER == kGatherTma4, "the cp.async path loads both column blocks");
 };
 
 // Does row tile `tile` (sorted rows [128*tile, 128*tile + 128)) carry filter offset f?  OR of the
@@ -314,11 +326,11 @@ __device__ __forceinline__ void wgrad_walk(const int *lists, int list_stride, co
   }
 }
 
-template <int BLOCK_N, int GATHER>
-__global__ void __launch_bounds__(WgradCfg<BLOCK_N, GATHER>::THREADS, 1)
+template <int BLOCK_N, int A_ATOMS, int GATHER>
+__global__ void __launch_bounds__(WgradCfg<BLOCK_N, A_ATOMS, GATHER>::THREADS, 1)
 wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constant__ CUtensorMap tmap_x,
              const WgradParams p) {
-  using Cfg = WgradCfg<BLOCK_N, GATHER>;
+  using Cfg = WgradCfg<BLOCK_N, A_ATOMS, GATHER>;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0)
     CB2_TRACE_CTA(0, 0);
@@ -333,10 +345,10 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
   volatile int *abort_flag = misc + 1;
   const uint32_t bars = sbase + Cfg::OFF_BARS;
   auto full_s = [&](int s) { return bars + 8u * s; };
-  auto empty_s = [&](int s) { return bars + 8u * (3 + s); };
-  auto acc_full = [&](int s) { return bars + 8u * (6 + s); };
-  auto acc_empty = [&](int s) { return bars + 8u * (8 + s); };
-  const uint32_t final_bar = bars + 8u * 10;
+  auto empty_s = [&](int s) { return bars + 8u * (Cfg::SA + s); };
+  auto acc_full = [&](int s) { return bars + 8u * (Cfg::BAR_ACC_FULL + s); };
+  auto acc_empty = [&](int s) { return bars + 8u * (Cfg::BAR_ACC_EMPTY + s); };
+  const uint32_t final_bar = bars + 8u * Cfg::BAR_FINAL;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -388,8 +400,9 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
   // ---- shared by the epilogue warps and the summing phase at the end
   const int *s_units = s_plan + kWgradPlanUnits;
   const int *s_first = s_plan + kWgradPlanFirst;
-  constexpr int kTileF4 = 32 * BLOCK_N;  // float4 per [128 x BLOCK_N] tile
-  // partial layout: float4 (col/4, row) at index (col/4) * 128 + row, so that the 32 rows of a
+  constexpr int ROWS = Cfg::M_ROWS;
+  constexpr int kTileF4 = ROWS * BLOCK_N / 4;  // float4 per [ROWS x BLOCK_N] tile
+  // partial layout: float4 (col/4, row) at index (col/4) * ROWS + row, so that the 32 rows of a
   // warp touch 512 contiguous bytes
   auto partial_of = [&](int u) {
     return reinterpret_cast<float4 *>(p.partials) + ((long long)u * gy + blockIdx.y) * kTileF4;
@@ -430,7 +443,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     for (int f = blockIdx.x; f < p.kv; f += gridDim.x)
       if ((p.mode != kWgradMaskConv || ((p.mask_filter >> (f & 31)) & 1u)) && s_units[f] == 0)
         for (int q = 0; q < BLOCK_N / 4; ++q)
-          write_out(f, et, q, make_float4(0.f, 0.f, 0.f, 0.f));
+          write_out(f, et, q, make_float4(0.f, 0.f, 0.f, 0.f));  // rows past m_total are left out there
     int acc_use = 0;
     wgrad_walk(
         p.lists, p.list_stride, s_plan, s_tiles, [&](int, int) -> bool { return true; },
@@ -439,8 +452,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           float4 *dst = partial_of(u) + et;
           if (active == 0) {
             // a unit without tiles (fewer steps than CTAs) still owns a partial: all zeros
-            for (int q = 0; q < BLOCK_N / 4; ++q)
-              dst[q * 128] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < BLOCK_N / 4 && et < ROWS; ++q)
+              dst[q * ROWS] = make_float4(0.f, 0.f, 0.f, 0.f);
           } else {
             const int buf = acc_use & 1;
             if (et == 0) {
@@ -458,13 +471,13 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
             const uint32_t trow = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) +
                                   static_cast<uint32_t>(buf * BLOCK_N);
 #pragma unroll 1
-            for (int round = 0; round < BLOCK_N / 32; ++round) {
+            for (int round = 0; round < BLOCK_N / 32 && warp * 32 < ROWS; ++round) {
               uint32_t v[32];
               tmem_ld32(trow + round * 32, v);
               tmem_ld_wait();
 #pragma unroll
               for (int q = 0; q < 8; ++q)
-                reinterpret_cast<uint4 *>(dst)[(round * 8 + q) * 128] = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                reinterpret_cast<uint4 *>(dst)[(round * 8 + q) * ROWS] = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
             }
             tc_fence_before();
             mbar_arrive(acc_empty(buf));
@@ -485,48 +498,50 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
   } else if (warp == 4) {
     // ======================= MMA issuer
     constexpr uint32_t idesc = make_idesc(0, true, true, 128, BLOCK_N);
-    int step = 0, acc_use = 0;
+    int stage = 0, acc_use = 0;
+    uint32_t phase = 0;
     bool ok_all = true;
+    const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES, 128 * 128, 1024);
+    const uint64_t bdesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES + Cfg::A_BYTES, 128 * 128, 1024);
     wgrad_walk(
         p.lists, p.list_stride, s_plan, s_tiles, [&](int, int) -> bool { return true; },
-        [&](int tile, int f, bool first) -> bool {
+        [&](int tile, int, bool first) -> bool {
           const int buf = acc_use & 1;
-          int ok = 1;
-          if (lane == 0) {
-            if (first)
-              ok = mbar_wait(acc_empty(buf), ((acc_use >> 1) & 1) ^ 1, abort_flag);
-            const int stage = step % Cfg::SA;
-            CB2_TRACE_EVENT(3, 4, step);  // waiting for data
-            if (ok)
-              ok = mbar_wait(full_s(stage), (step / Cfg::SA) & 1, abort_flag);
-            CB2_TRACE_EVENT(3, 5, step);  // data landed
-            if (ok) {
-              if constexpr (GATHER == kGatherCpAsync)
-                fence_proxy_async_smem();
-              tc_fence_after();
-              const uint32_t a_base = sbase + Cfg::OFF_STAGES + stage * Cfg::STAGE_BYTES;
-              const uint32_t b_base = a_base + Cfg::A_BYTES;
-              const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
-              int rows = p.n_rows - tile * 128;
-              if (rows > 128)
-                rows = 128;
-              const int ksteps = (rows + 15) / 16;
-              for (int ks = 0; ks < ksteps; ++ks) {
-                const uint64_t adesc = make_smem_desc(a_base + ks * 2048, 128 * 128, 1024);
-                const uint64_t bdesc = make_smem_desc(b_base + ks * 2048, 128 * 128, 1024);
-                tc_mma<0>(d_tmem, adesc, bdesc, idesc, (first && ks == 0) ? 0u : 1u);
-              }
-              tc_commit(empty_s(stage));
-              CB2_TRACE_EVENT(3, 6, step);  // MMAs issued
-            }
-          }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          ++step;
-          if (!ok) {
+          // the warp walks together, its state the same in every lane; lane 0 issues
+          bool ok = true;
+          if (first)
+            ok = mbar_wait(acc_empty(buf), ((acc_use >> 1) & 1) ^ 1, abort_flag);
+          ok = ok && mbar_wait(full_s(stage), phase, abort_flag);
+          if (!__all_sync(0xffffffffu, ok)) {
             if (lane == 0)
               fail(kStatusWaitTimeout);
             ok_all = false;
             return false;
+          }
+          if constexpr (GATHER == kGatherCpAsync)
+            fence_proxy_async_smem();
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
+          // descriptors differ from the first stage's only in the start address (units of 16 bytes)
+          const uint64_t adesc = adesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
+          const uint64_t bdesc = bdesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
+          const int rows = p.n_rows - __shfl_sync(0xffffffffu, tile, 0) * 128;
+          if (lane == 0) {
+            if (rows >= 128) {
+#pragma unroll
+              for (int ks = 0; ks < 8; ++ks)
+                tc_mma<0>(d_tmem, adesc + ks * (2048 >> 4), bdesc + ks * (2048 >> 4), idesc, (first && ks == 0) ? 0u : 1u);
+            } else {
+              for (int ks = 0; ks < (rows + 15) / 16; ++ks)
+                tc_mma<0>(d_tmem, adesc + ks * (2048 >> 4), bdesc + ks * (2048 >> 4), idesc, (first && ks == 0) ? 0u : 1u);
+            }
+            tc_commit(empty_s(stage));
+            CB2_TRACE_EVENT(3, 6, tile);  // MMAs issued
+          }
+          __syncwarp();
+          if (++stage == Cfg::SA) {
+            stage = 0;
+            phase ^= 1u;
           }
           return true;
         },
@@ -545,8 +560,127 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
         fail(kStatusWaitTimeout);
     }
     __syncwarp();
+  } else if constexpr (GATHER == kGatherTma4) {
+    // ======================= gather both operands: the GW warps of group g own stage g, steps g,
+    // g + SA, ... of this CTA.  A lane fetches a quad of four tile rows, one request per column block and
+    // operand; a row of -1 is out of bounds and reads as zeros.  The row numbers run ahead of the copies:
+    // while the group waits for its stage, the neighbour indices of its next step and the sort order of
+    // the one after are on their way.
+    const int g = (warp - 5) / Cfg::GW;
+    const int quad = (warp - 5) % Cfg::GW * (32 / Cfg::GW) + lane;
+    const bool has_quad = lane < 32 / Cfg::GW;
+    const bool first_lane = quad == 0;
+    if (g < Cfg::SA) {
+      const int n_units = s_plan[0];
+      const bool staged = s_plan[1] != 0;
+      struct Step {
+        int tile, f;
+      };
+      int unit = 0, seen = 0;  // the unit `next_step` stands in, and the CTA's steps before it
+      int at = g;              // the step `next_step` returns next
+      auto next_step = [&]() -> Step {
+        Step r = {-1, 0};
+        while (unit < n_units) {
+          const int *e = s_plan + 8 + 5 * unit;
+          const int len = e[2] - e[1];
+          if (at < seen + len) {
+            const int k = at - seen;
+            r.f = e[0];
+            r.tile = staged ? s_tiles[e[4] + k] : __ldg(p.lists + (long long)e[0] * p.list_stride + e[1] + k);
+            break;
+          }
+          seen += len;
+          ++unit;
+        }
+        at += Cfg::SA;
+        return r;
+      };
+      struct Rows {
+        int v[4];
+      };
+      const bool wide_order = (reinterpret_cast<uintptr_t>(p.argsort) & 15u) == 0;
+      // rows of dout (pair lists: of both operands) that lane's tile rows stand for
+      auto load_order = [&](const Step &st, Rows &a) {
+        const int r0 = st.tile * 128 + 4 * quad;
+        if (p.mode == kWgradMaskConv && st.tile >= 0 && has_quad && wide_order && r0 + 4 <= p.n_rows) {
+          const int4 o = __ldg(reinterpret_cast<const int4 *>(p.argsort + r0));
+          a.v[0] = o.x, a.v[1] = o.y, a.v[2] = o.z, a.v[3] = o.w;
+          return;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a.v[j] = -1;
+          if (st.tile >= 0 && has_quad && r0 + j < p.n_rows)
+            a.v[j] = __ldg((p.mode == kWgradMaskConv ? p.argsort : p.a_inds) + r0 + j);
+        }
+      };
+      auto load_rows = [&](const Step &st, const Rows &a, Rows &b) {
+        const int r0 = st.tile * 128 + 4 * quad;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          b.v[j] = -1;
+          if (st.tile >= 0 && has_quad && r0 + j < p.n_rows) {
+            if (p.mode == kWgradMaskConv) {
+              // a chunk of at least a tile carries the offset, or the tile would not be in the list
+              const bool on = p.mask_width >= 128 ||
+                              ((__ldg(p.rmask + (long long)((r0 + j) / p.mask_width) * p.words + (st.f >> 5)) >> (st.f & 31)) & 1u);
+              if (on && a.v[j] >= 0)
+                b.v[j] = __ldg(p.indices + (long long)st.f * p.n_rows + a.v[j]);
+            } else {
+              b.v[j] = __ldg(p.b_inds + r0 + j);
+            }
+          }
+        }
+      };
+      const uint32_t a_quad = sbase + Cfg::OFF_STAGES + g * Cfg::STAGE_BYTES + quad * (4 * 128);
+      const uint32_t b_quad = a_quad + Cfg::A_BYTES;
+      Step cur = next_step(), nxt = next_step();
+      Rows ca, cb, na, nb;
+      load_order(cur, ca);
+      load_order(nxt, na);
+      load_rows(cur, ca, cb);
+      for (uint32_t phase = 1; cur.tile >= 0; phase ^= 1u) {
+        const Step after = next_step();
+        Rows fa;
+        load_rows(nxt, na, nb);
+        load_order(after, fa);
+        int ia[4], ib[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          ib[j] = cb.v[j];
+          ia[j] = (p.mode != kWgradMaskConv || ib[j] >= 0) ? ca.v[j] : -1;  // a zero B row makes the A row irrelevant
+          if (ia[j] >= p.a_rows || ib[j] >= p.b_rows) {
+            fail(kStatusBadIndex);
+            ia[j] = ib[j] = -1;
+          }
+        }
+        if (first_lane)
+          CB2_TRACE_EVENT(g, 1, cur.tile + (ib[0] == 0x7fffffff));  // indices loaded
+        if (!mbar_wait_warp(empty_s(g), phase, abort_flag)) {
+          if (lane == 0)
+            fail(kStatusWaitTimeout);
+          break;
+        }
+        if (first_lane) {
+          CB2_TRACE_EVENT(g, 2, cur.tile);  // stage free
+          mbar_arrive_expect_tx(full_s(g), Cfg::STAGE_BYTES);
+        }
+        if (has_quad) {
+#pragma unroll
+          for (int ka = 0; ka < A_ATOMS; ++ka)
+            tma_gather4(a_quad + ka * (128 * 128), &tmap_dout, full_s(g), m0 + ka * 64, ia[0], ia[1], ia[2], ia[3]);
+#pragma unroll
+          for (int kb = 0; kb < BLOCK_N / 64; ++kb)
+            tma_gather4(b_quad + kb * (128 * 128), &tmap_x, full_s(g), n0 + kb * 64, ib[0], ib[1], ib[2], ib[3]);
+        }
+        if (first_lane)
+          CB2_TRACE_EVENT(g, 3, cur.tile);  // copies issued
+        cur = nxt, nxt = after;
+        ca = na, cb = nb, na = fa;
+      }
+    }
   } else {
-    // ======================= gather both operands: group g owns stage g
+    // ======================= the same with 16-byte cp.async: group g of 128 threads owns stage g
     const int g = (warp - 5) >> 2;
     const int gt = threadIdx.x - (5 * 32 + g * 128);
     int *group_rowidx = rowidx + g * 512;
@@ -584,89 +718,59 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           }
           const uint32_t a_stage = sbase + Cfg::OFF_STAGES + g * Cfg::STAGE_BYTES;
           const uint32_t b_stage = a_stage + Cfg::A_BYTES;
-          if constexpr (GATHER == kGatherCpAsync) {
-            if (gt == 0) {
-              CB2_TRACE_EVENT(g, 1, step - 1 + (ib == 0x7fffffff));  // indices loaded
-              bool ok = mbar_wait(empty_s(g), (use & 1) ^ 1, abort_flag);
-              CB2_TRACE_EVENT(g, 2, step - 1);             // stage free
-              *my_flag = ok ? 1 : 0;
-              if (!ok)
-                fail(kStatusWaitTimeout);
-            }
-            int *ridx_a = group_rowidx + (use & 1) * 256;
-            int *ridx_b = ridx_a + 128;
-            ridx_a[gt] = ia;
-            ridx_b[gt] = ib;
-            named_bar_sync(2 + g, 128);
-            if (*my_flag == 0)
-              return false;
-            {
-              // A rows: 256 B (128 channels of dout starting at m0), 16 chunks per row
-              const int c = gt & 15, row0 = gt >> 4;
-              const bool col_ok = (m0 + c * 8) < p.m_total;
-              const uint32_t dst_c = a_stage + (c >> 3) * (128 * 128);
+          if (gt == 0) {
+            CB2_TRACE_EVENT(g, 1, step - 1 + (ib == 0x7fffffff));  // indices loaded
+            bool ok = mbar_wait(empty_s(g), (use & 1) ^ 1, abort_flag);
+            CB2_TRACE_EVENT(g, 2, step - 1);             // stage free
+            *my_flag = ok ? 1 : 0;
+            if (!ok)
+              fail(kStatusWaitTimeout);
+          }
+          int *ridx_a = group_rowidx + (use & 1) * 256;
+          int *ridx_b = ridx_a + 128;
+          ridx_a[gt] = ia;
+          ridx_b[gt] = ib;
+          named_bar_sync(2 + g, 128);
+          if (*my_flag == 0)
+            return false;
+          {
+            // A rows: 256 B (128 channels of dout starting at m0), 16 chunks per row
+            const int c = gt & 15, row0 = gt >> 4;
+            const bool col_ok = (m0 + c * 8) < p.m_total;
+            const uint32_t dst_c = a_stage + (c >> 3) * (128 * 128);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const int row = row0 + i * 8;
-                const int ridx = ridx_a[row];
-                const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
-                const bool valid = col_ok && ridx >= 0;
-                const uint8_t *srcp = valid ? a_bytes + ((long long)ridx * p.ld_dout + m0 + c * 8) * 2 : a_bytes;
-                cp_async_16(dst, srcp, valid ? 16u : 0u);
-              }
-            }
-            {
-              const int c = gt % CPR_B, row0 = gt / CPR_B;
-              constexpr int RSTEP = 128 / CPR_B;
-              const bool col_ok = (n0 + c * 8) < p.n_total;
-              const uint32_t dst_c = b_stage + (c >> 3) * (128 * 128);
-#pragma unroll
-              for (int i = 0; i < CPR_B; ++i) {
-                const int row = row0 + i * RSTEP;
-                const int ridx = ridx_b[row];
-                const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
-                const bool valid = col_ok && ridx >= 0;
-                const uint8_t *srcp = valid ? b_bytes + ((long long)ridx * p.ld_x + n0 + c * 8) * 2 : b_bytes;
-                cp_async_16(dst, srcp, valid ? 16u : 0u);
-              }
-            }
-            // async arrive when this thread's copies land; the consumer fences (see rowconv kernel)
-            cp_async_mbar_arrive_noinc(full_s(g));
-          } else {
-            if (gt == 0)
-              CB2_TRACE_EVENT(g, 1, step - 1 + (ib == 0x7fffffff));  // indices loaded
-            if (!mbar_wait_warp(empty_s(g), (use & 1) ^ 1, abort_flag)) {
-              if (lane == 0)
-                fail(kStatusWaitTimeout);
-              return false;
-            }
-            if (gt == 0) {
-              CB2_TRACE_EVENT(g, 2, step - 1);  // stage free
-              mbar_arrive_expect_tx(full_s(g), Cfg::STAGE_BYTES);
-            }
-            // four rows per request and column block; row -1 reads as zeros
-            {
-              const int a1 = __shfl_down_sync(0xffffffffu, ia, 1), a2 = __shfl_down_sync(0xffffffffu, ia, 2),
-                        a3 = __shfl_down_sync(0xffffffffu, ia, 3);
-              const int b1 = __shfl_down_sync(0xffffffffu, ib, 1), b2 = __shfl_down_sync(0xffffffffu, ib, 2),
-                        b3 = __shfl_down_sync(0xffffffffu, ib, 3);
-              if ((lane & 3) == 0) {
-#pragma unroll
-                for (int ka = 0; ka < 2; ++ka)
-                  tma_gather4(a_stage + ka * (128 * 128) + gt * 128, &tmap_dout, full_s(g), m0 + ka * 64, ia, a1, a2, a3);
-#pragma unroll
-                for (int kb = 0; kb < BLOCK_N / 64; ++kb)
-                  tma_gather4(b_stage + kb * (128 * 128) + gt * 128, &tmap_x, full_s(g), n0 + kb * 64, ib, b1, b2, b3);
-              }
+            for (int i = 0; i < 16; ++i) {
+              const int row = row0 + i * 8;
+              const int ridx = ridx_a[row];
+              const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
+              const bool valid = col_ok && ridx >= 0;
+              const uint8_t *srcp = valid ? a_bytes + ((long long)ridx * p.ld_dout + m0 + c * 8) * 2 : a_bytes;
+              cp_async_16(dst, srcp, valid ? 16u : 0u);
             }
           }
+          {
+            const int c = gt % CPR_B, row0 = gt / CPR_B;
+            constexpr int RSTEP = 128 / CPR_B;
+            const bool col_ok = (n0 + c * 8) < p.n_total;
+            const uint32_t dst_c = b_stage + (c >> 3) * (128 * 128);
+#pragma unroll
+            for (int i = 0; i < CPR_B; ++i) {
+              const int row = row0 + i * RSTEP;
+              const int ridx = ridx_b[row];
+              const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
+              const bool valid = col_ok && ridx >= 0;
+              const uint8_t *srcp = valid ? b_bytes + ((long long)ridx * p.ld_x + n0 + c * 8) * 2 : b_bytes;
+              cp_async_16(dst, srcp, valid ? 16u : 0u);
+            }
+          }
+          // async arrive when this thread's copies land; the consumer fences (see rowconv kernel)
+          cp_async_mbar_arrive_noinc(full_s(g));
           if (gt == 0)
             CB2_TRACE_EVENT(g, 3, step - 1);  // copies issued
           return true;
         },
         [&](int, int, int) -> bool { return true; });
-    if constexpr (GATHER == kGatherCpAsync)
-      cp_async_wait_all();
+    cp_async_wait_all();
   }
 
   // ---------------------------------------------------------------- summing
@@ -778,7 +882,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           }
 #pragma unroll
           for (int g = 0; g < 2; ++g)
-            write_out(f, (q0 + g) & 127, (q0 + g) >> 7, acc[g]);
+            write_out(f, (q0 + g) % ROWS, (q0 + g) / ROWS, acc[g]);
         }
       } else {
         for (int q0 = lo; q0 < hi; q0 += 32) {
@@ -807,7 +911,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
               acc.w += v.w;
             }
             const int q = q0 + lane;
-            write_out(f, q & 127, q >> 7, acc);
+            write_out(f, q % ROWS, q / ROWS, acc);
           }
           __syncthreads();
         }
