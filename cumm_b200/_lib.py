@@ -18,12 +18,14 @@ CB2_ERR_INVALID_ARG = -1
 CB2_ERR_RUNTIME = -2
 CB2_ERR_UNSUPPORTED = -3
 CB2_ERR_CUDA = -4
+CB2_PLAN_ROW_LISTS = 2
 
 EXPORTED_SYMBOLS = (
     "cb2_gemm_run",
     "cb2_conv_run",
     "cb2_gemm_workspace_size",
     "cb2_conv_workspace_size",
+    "cb2_conv_workspace_size_lists",
     "cb2_tile_m",
     "cb2_last_error",
     "cb2_device_status",
@@ -204,6 +206,8 @@ def load() -> ctypes.CDLL:
     L.cb2_gemm_workspace_size.argtypes = [ctypes.POINTER(GemmArgs)]
     L.cb2_conv_workspace_size.restype = ctypes.c_size_t
     L.cb2_conv_workspace_size.argtypes = [ctypes.POINTER(ConvArgs)]
+    L.cb2_conv_workspace_size_lists.restype = ctypes.c_size_t
+    L.cb2_conv_workspace_size_lists.argtypes = [ctypes.POINTER(ConvArgs)]
     L.cb2_tile_m.restype = ctypes.c_int
     L.cb2_last_error.restype = ctypes.c_char_p
     L.cb2_device_status.restype = ctypes.c_int

@@ -333,6 +333,10 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
 struct WgradLayout {
   int block_n, gy, G, slots, list_stride, n_ctl;
   size_t off_ctl, off_partials, off_lists, total;
+  // with row lists (see wgrad_mark_rows_kernel): their part comes after `total`
+  int n_chunks;
+  long long row_capacity;
+  size_t off_head, off_counts, off_bits, off_rows, total_lists;
 };
 
 // Workspace of the weight gradient: 512-byte header (tile counts per offset), the control words,
@@ -356,6 +360,17 @@ void wgrad_layout(int num_sms, int max_ctas, int m_total, int n_total, long long
   const long long ntiles = (n_rows + 127) / 128;
   L->list_stride = (int)((ntiles + 63) / 64 * 64);
   L->total = L->off_lists + (size_t)kvs * L->list_stride * 4;
+  // Room for 8 + kv / 8 listed rows per row (11 of 27 offsets, 23 of 125): scanned scenes have five and
+  // thirteen neighbours per row, the centre, which every row has, is not listed.
+  const int per = wgrad_chunk_tiles((int)ntiles);
+  L->n_chunks = per > 0 ? (int)((ntiles + per - 1) / per) : 0;
+  L->row_capacity = (n_rows * std::min(kvs, 8 + kvs / 8) + 127) / 128 * 128;
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  L->off_head = up(L->total);
+  L->off_counts = L->off_head + 2 * kWgradMaxOffsets * 4;
+  L->off_bits = up(L->off_counts + (size_t)kvs * L->n_chunks * 8);
+  L->off_rows = L->off_bits + (size_t)kvs * L->list_stride * 16;
+  L->total_lists = L->off_rows + (size_t)L->row_capacity * 4;
 }
 
 template <int BLOCK_N, int A_ATOMS, int GATHER>
@@ -380,8 +395,9 @@ int launch_wgrad_inst(const CUtensorMap &ma, const CUtensorMap &mb, const WgradP
   return CB2_OK;
 }
 
-int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int reuse_plan, void *workspace,
+int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int plan_flags, void *workspace,
               size_t workspace_bytes, cudaStream_t stream) {
+  const bool reuse_plan = (plan_flags & ~CB2_PLAN_ROW_LISTS) != 0;
   CB2_CHECK_RT(tile_n == 0 || tile_n == 64 || tile_n == 128,
                "can't find any suitable algo: tile_shape[1] = %d (kernels exist for 64 and 128)", tile_n);
   CB2_CHECK_ARG(max_ctas >= 0, "max_ctas must not be negative");
@@ -404,7 +420,23 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int re
   p.lists = reinterpret_cast<const int *>(ws + L.off_lists);
   p.list_stride = L.list_stride;
   p.status = dev->status;
-  if (!reuse_plan) {
+  // Row lists where the caller allows them and the workspace has room, tiles otherwise.
+  const bool row_lists = (plan_flags & CB2_PLAN_ROW_LISTS) && p.mode == kWgradMaskConv && p.n_rows > 0 && workspace_bytes >= L.total_lists &&
+                         L.row_capacity < (1ll << 31);
+  if (row_lists) {
+    p.row_head = reinterpret_cast<int *>(ws + L.off_head);
+    p.rows = reinterpret_cast<const int *>(ws + L.off_rows);
+  }
+  if (!reuse_plan && row_lists) {
+    const dim3 grid(L.n_chunks, p.kv);
+    uint4 *bits = reinterpret_cast<uint4 *>(ws + L.off_bits);
+    int2 *counts = reinterpret_cast<int2 *>(ws + L.off_counts);
+    wgrad_mark_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, L.n_ctl);
+    wgrad_list_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, reinterpret_cast<int *>(ws + L.off_lists),
+                                                                   reinterpret_cast<int *>(ws + L.off_rows), L.row_capacity);
+    CB2_CUDA(cudaGetLastError());
+    g_launches.fetch_add(2);
+  } else if (!reuse_plan) {
     // counts and lists of the row tiles per offset; control words to zero
     wgrad_plan_kernel<<<p.kv, 1024, 0, stream>>>(p, reinterpret_cast<int *>(ws + L.off_lists), L.list_stride, L.n_ctl);
     CB2_CUDA(cudaGetLastError());
@@ -1278,6 +1310,17 @@ size_t cb2_conv_workspace_size(const cb2_conv_args *a) {
   WgradLayout L;
   wgrad_layout(dev->num_sms, a->max_ctas, a->K, a->C, a->N, a->kernel_volume, a->tile_n, &L);
   return L.total;
+}
+
+size_t cb2_conv_workspace_size_lists(const cb2_conv_args *a) {
+  if (!a || a->op_type != CB2_CONV_BACKWARD_WEIGHT)
+    return 0;
+  DeviceState *dev;
+  if (get_device(&dev))
+    return 0;
+  WgradLayout L;
+  wgrad_layout(dev->num_sms, a->max_ctas, a->K, a->C, a->N, a->kernel_volume, a->tile_n, &L);
+  return L.total_lists;
 }
 
 size_t cb2_static_scratch_bytes(void) { return kStaticScratchBytes; }

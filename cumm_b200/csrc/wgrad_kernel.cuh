@@ -48,6 +48,9 @@ struct WgradParams {
   int *sched;              // workspace header: [0,128) number of row tiles carrying offset f
   const int *lists;        // workspace: per offset, the ordered list of those tiles
   int list_stride;         // ints between two offsets' lists
+  int *row_head;           // workspace or null: [0,128) first entry of offset f's row list, -1 = walked by tiles;
+                           // [128,256) its entries
+  const int *rows;         // workspace: the row lists
   int *status;
   void *out;               // dW
   const void *src;         // source for beta (dW itself unless the caller gave another)
@@ -88,7 +91,7 @@ template <int BLOCK_N, int A_ATOMS, int GATHER> struct WgradCfg {
   static constexpr int OFF_ROWIDX = SA * STAGE_BYTES;       // 3 x 2 buffers x 2 operands x 128 ints
   static constexpr int OFF_SCHED = OFF_ROWIDX + 3 * 2 * 2 * 128 * 4;  // this CTA's units, then units per offset
   static constexpr int TILE_CAP = 2048;                      // tiles of one CTA staged in shared memory
-  static constexpr int OFF_TILES = OFF_SCHED + 1024 * 4;
+  static constexpr int OFF_TILES = OFF_SCHED + 1280 * 4;
   static constexpr int OFF_BARS = OFF_TILES + TILE_CAP * 4;
   static constexpr int BAR_ACC_FULL = 2 * SA, BAR_ACC_EMPTY = BAR_ACC_FULL + 2, BAR_FINAL = BAR_ACC_EMPTY + 2;
   static constexpr int OFF_MISC = OFF_BARS + (BAR_FINAL + 2) / 2 * 2 * 8;
@@ -230,15 +233,166 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
     p.sched[f] = running;
 }
 
-// Per CTA, in shared memory: s_plan[0] = number of units of this CTA, then five ints per unit
-// {f, first list index, one past the last, unit number, offset of its tiles in s_tiles};
-// s_tiles = the CTA's tiles in step order (when they fit; otherwise the walk reads the lists).
+// ---------------------------------------------------------------- plan with row lists
+// A tile of 128 sorted rows carries every offset that any of its rows has, so away from the centre
+// most of a tile's rows are empty for most of its offsets: on a scanned scene every second row, with
+// 125 offsets four of five.  Where that is so the reduction does not run over tiles but over the rows
+// themselves: a step takes the next 128 rows that have a neighbour at the offset, and an offset has
+// ceil(pairs / 128) steps.  Two kernels make the lists: one marks, per (offset, tile), the rows that take
+// part (a 128-bit word) and counts them per chunk of tiles, the other turns counts into places and
+// writes the lists in sorted order, so the sums have one fixed order.  Offsets whose tiles are at least
+// four fifths full, and lists that find no room, are walked by tiles.
+constexpr int kWgradPlanThreads = 256;
+constexpr int kWgradMaxChunks = 64;
+// tiles per chunk: whole groups of 32
+__host__ __device__ inline int wgrad_chunk_tiles(int ntiles) {
+  return 32 * ((ntiles + 32 * kWgradMaxChunks - 1) / (32 * kWgradMaxChunks));
+}
+
+// grid (chunks, offsets); bits[f][tile][4], counts[f][chunk] = {rows, tiles with any}
+__global__ void __launch_bounds__(kWgradPlanThreads) wgrad_mark_rows_kernel(const WgradParams p, uint4 *bits, int2 *counts,
+                                                                            int n_ctl) {
+  __shared__ int2 s_sum[kWgradPlanThreads / 32];
+  const int f = blockIdx.y, chunk = blockIdx.x;
+  for (int i = (f * gridDim.x + chunk) * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * gridDim.y * blockDim.x)
+    p.ctl[i] = 0;
+  const int ntiles = (p.n_rows + 127) / 128;
+  const int per = wgrad_chunk_tiles(ntiles);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int rows = 0, tiles = 0;
+  for (int t = chunk * per + wid; t < min((chunk + 1) * per, ntiles); t += kWgradPlanThreads / 32) {
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (wgrad_tile_has(p, t, f)) {
+      int o[4];
+      bool on[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = t * 128 + q * 32 + lane;
+        o[q] = r < p.n_rows ? __ldg(p.argsort + r) : -1;
+        on[q] = o[q] >= 0;
+        if (p.mask_width < 128 && on[q])
+          on[q] = (__ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5)) >> (f & 31)) & 1u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        w[q] = __ballot_sync(0xffffffffu, on[q] && __ldg(p.indices + (long long)f * p.n_rows + o[q]) >= 0);
+    }
+    const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
+    rows += n;
+    tiles += n > 0;
+    if (lane == 0)
+      bits[(long long)f * p.list_stride + t] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  if (lane == 0)
+    s_sum[wid] = make_int2(rows, tiles);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int2 all = make_int2(0, 0);
+    for (int w = 0; w < kWgradPlanThreads / 32; ++w)
+      all.x += s_sum[w].x, all.y += s_sum[w].y;
+    counts[f * gridDim.x + chunk] = all;
+  }
+}
+
+__global__ void __launch_bounds__(kWgradPlanThreads) wgrad_list_rows_kernel(const WgradParams p, const uint4 *bits,
+                                                                            const int2 *counts, int *lists, int *rows,
+                                                                            long long capacity) {
+  __shared__ int s_rows[kWgradMaxOffsets], s_tiles[kWgradMaxOffsets], s_base[kWgradMaxOffsets];
+  __shared__ int s_before[2];
+  __shared__ int s_place[32], s_count[2];
+  const int f = blockIdx.y, chunk = blockIdx.x, n_chunks = gridDim.x;
+  grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the plan
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x < kWgradMaxOffsets) {
+    int r = 0, t = 0;
+    if ((int)threadIdx.x < p.kv) {
+#pragma unroll 8
+      for (int c = 0; c < n_chunks; ++c) {
+        if ((int)threadIdx.x == f && c == chunk)
+          s_before[0] = r, s_before[1] = t;
+        const int2 v = __ldg(counts + threadIdx.x * n_chunks + c);
+        r += v.x, t += v.y;
+      }
+    }
+    s_rows[threadIdx.x] = r;
+    s_tiles[threadIdx.x] = t;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    int size[4], first[4], total;
+    bool listed[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int g = 4 * lane + j;
+      listed[j] = 512ll * s_tiles[g] > 5ll * s_rows[g];  // tiles less than four fifths full
+      size[j] = listed[j] ? (s_rows[g] + 127) / 128 : 0;  // in steps
+    }
+    wgrad_scan4(size, first, total);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      s_base[4 * lane + j] = listed[j] && 128ll * (first[j] + size[j]) <= capacity ? 128 * first[j] : -1;
+  }
+  __syncthreads();
+  const int base = s_base[f];
+  if (chunk == 0 && threadIdx.x == 0) {
+    p.sched[f] = base >= 0 ? (s_rows[f] + 127) / 128 : s_tiles[f];
+    p.row_head[f] = base;
+    p.row_head[kWgradMaxOffsets + f] = s_rows[f];
+  }
+  const int ntiles = (p.n_rows + 127) / 128;
+  const int per = wgrad_chunk_tiles(ntiles);
+  const int end = min((chunk + 1) * per, ntiles);
+  int before_rows = s_before[0], before_tiles = s_before[1];
+  const uint4 *mine = bits + (long long)f * p.list_stride;
+  for (int t0 = chunk * per; t0 < end; t0 += 32) {
+    if (wid == 0) {
+      const int t = t0 + lane;
+      const uint4 w = t < end ? __ldg(mine + t) : make_uint4(0u, 0u, 0u, 0u);
+      const int n = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+      int incl = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d)
+          incl += v;
+      }
+      s_place[lane] = incl - n;
+      const unsigned any = __ballot_sync(0xffffffffu, n > 0);
+      if (base < 0 && n > 0)
+        lists[(long long)f * p.list_stride + before_tiles + __popc(any & ((1u << lane) - 1u))] = t;
+      if (lane == 31)
+        s_count[0] = incl, s_count[1] = __popc(any);
+    }
+    __syncthreads();
+    if (base >= 0)
+      for (int l = wid; l < 32 && t0 + l < end; l += kWgradPlanThreads / 32) {
+        const uint4 v = __ldg(mine + t0 + l);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        int at = base + before_rows + s_place[l];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if ((w[q] >> lane) & 1u)
+            rows[at + __popc(w[q] & ((1u << lane) - 1u))] = __ldg(p.argsort + (t0 + l) * 128 + q * 32 + lane);
+          at += __popc(w[q]);
+        }
+      }
+    before_rows += s_count[0], before_tiles += s_count[1];
+    __syncthreads();
+  }
+}
+
+// Per CTA, in shared memory: s_plan[0] = number of units of this CTA, then seven ints per unit
+// {f, first step of the offset, one past the last, unit number, offset of its tiles in s_tiles, first
+// entry of the offset's row list or -1, its entries};
+// s_tiles = the CTA's tiles in step order (when they fit; otherwise the walk reads the lists); a step
+// of a row list stands there as its own number.
 // The unit number is global: the units of an offset are consecutive.  After the unit records:
 // s_plan[kWgradPlanUnits + f] = units of offset f over all CTAs, s_plan[kWgradPlanFirst + f] = the
 // first of them.
-constexpr int kWgradPlanUnits = 8 + 5 * kWgradMaxOffsets;
+constexpr int kWgradPlanUnits = 8 + 7 * kWgradMaxOffsets;
 constexpr int kWgradPlanFirst = kWgradPlanUnits + kWgradMaxOffsets;
-constexpr int kWgradPlanInts = kWgradPlanFirst + kWgradMaxOffsets;  // 904 <= the 1024 reserved
+constexpr int kWgradPlanInts = kWgradPlanFirst + kWgradMaxOffsets;
+static_assert(kWgradPlanInts <= 1280, "room reserved in shared memory");
 constexpr int kWgradMaxOutTiles = 128; // (m, n) tiles of the weight gradient a launch can have
 constexpr int kWgradCtlBase = 8 + 8 * kWgradMaxOutTiles;  // first per-(offset, tile) control word
 constexpr int kWgradSharedSumUnits = 16;  // offsets with more units than this are summed by all CTAs together
@@ -278,8 +432,10 @@ __device__ __forceinline__ void wgrad_load_plan(const WgradParams &p, const int 
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (has[j]) {
-        int *e = s_plan + 8 + 5 * slot[j];
+        int *e = s_plan + 8 + 7 * slot[j];
         e[0] = 4 * lane + j;
+        e[5] = p.row_head ? __ldg(p.row_head + 4 * lane + j) : -1;
+        e[6] = p.row_head ? __ldg(p.row_head + kWgradMaxOffsets + 4 * lane + j) : 0;
         e[1] = k0[j];
         e[2] = k1[j];
         e[3] = U[j] + (c - c_first[j]);
@@ -294,31 +450,34 @@ __device__ __forceinline__ void wgrad_load_plan(const WgradParams &p, const int 
   if (s_plan[1]) {
     const int n = s_plan[0];
     for (int j = 0; j < n; ++j) {
-      const int *e = s_plan + 8 + 5 * j;
+      const int *e = s_plan + 8 + 7 * j;
       const int *src = lists + (long long)e[0] * list_stride + e[1];
       for (int i = threadIdx.x; i < e[2] - e[1]; i += blockDim.x)
-        s_tiles[e[4] + i] = __ldg(src + i);
+        s_tiles[e[4] + i] = e[5] >= 0 ? e[1] + i : __ldg(src + i);
     }
   }
   __syncthreads();
 }
 
-// Walk this CTA's units.  on_unit(u, f) at unit start, on_tile(tile, f, first_of_unit) for each
-// of its tiles, on_unit_end(u, f, n_tiles).  Every role runs the identical walk.
-template <class UnitFn, class TileFn, class EndFn>
+// Rows of step `tile` of the unit e.
+__device__ __forceinline__ int wgrad_step_rows(const WgradParams &p, const int *e, int tile) {
+  return (e[5] >= 0 ? e[6] : p.n_rows) - tile * 128;
+}
+
+// Walk this CTA's units.  on_tile(tile, e, first_of_unit) for each step of the unit with record e,
+// on_unit_end(u, f, n_tiles).  Every role runs the identical walk.
+template <class TileFn, class EndFn>
 __device__ __forceinline__ void wgrad_walk(const int *lists, int list_stride, const int *s_plan, const int *s_tiles,
-                                           UnitFn on_unit, TileFn on_tile, EndFn on_unit_end) {
+                                           TileFn on_tile, EndFn on_unit_end) {
   const int n = s_plan[0];
   const bool staged = s_plan[1] != 0;
   for (int j = 0; j < n; ++j) {
-    const int *e = s_plan + 8 + 5 * j;
+    const int *e = s_plan + 8 + 7 * j;
     const int f = e[0], k0 = e[1], k1 = e[2], u = e[3], toff = e[4];
-    if (!on_unit(u, f))
-      return;
     const int *src = lists + (long long)f * list_stride + k0;
     for (int i = 0; i < k1 - k0; ++i) {
-      const int tile = staged ? s_tiles[toff + i] : __ldg(src + i);
-      if (!on_tile(tile, f, i == 0))
+      const int tile = staged ? s_tiles[toff + i] : e[5] >= 0 ? k0 + i : __ldg(src + i);
+      if (!on_tile(tile, e, i == 0))
         return;
     }
     if (!on_unit_end(u, f, k1 - k0))
@@ -446,8 +605,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           write_out(f, et, q, make_float4(0.f, 0.f, 0.f, 0.f));  // rows past m_total are left out there
     int acc_use = 0;
     wgrad_walk(
-        p.lists, p.list_stride, s_plan, s_tiles, [&](int, int) -> bool { return true; },
-        [&](int, int, bool) -> bool { return true; },
+        p.lists, p.list_stride, s_plan, s_tiles,
+        [&](int, const int *, bool) -> bool { return true; },
         [&](int u, int f, int active) -> bool {
           float4 *dst = partial_of(u) + et;
           if (active == 0) {
@@ -504,8 +663,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES, 128 * 128, 1024);
     const uint64_t bdesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES + Cfg::A_BYTES, 128 * 128, 1024);
     wgrad_walk(
-        p.lists, p.list_stride, s_plan, s_tiles, [&](int, int) -> bool { return true; },
-        [&](int tile, int, bool first) -> bool {
+        p.lists, p.list_stride, s_plan, s_tiles,
+        [&](int tile, const int *e, bool first) -> bool {
           const int buf = acc_use & 1;
           // the warp walks together, its state the same in every lane; lane 0 issues
           bool ok = true;
@@ -525,7 +684,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           // descriptors differ from the first stage's only in the start address (units of 16 bytes)
           const uint64_t adesc = adesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
           const uint64_t bdesc = bdesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
-          const int rows = p.n_rows - __shfl_sync(0xffffffffu, tile, 0) * 128;
+          const int rows = __shfl_sync(0xffffffffu, wgrad_step_rows(p, e, tile), 0);
           if (lane == 0) {
             if (rows >= 128) {
 #pragma unroll
@@ -574,19 +733,21 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
       const int n_units = s_plan[0];
       const bool staged = s_plan[1] != 0;
       struct Step {
-        int tile, f;
+        int tile, f, list, rows;
       };
       int unit = 0, seen = 0;  // the unit `next_step` stands in, and the CTA's steps before it
       int at = g;              // the step `next_step` returns next
       auto next_step = [&]() -> Step {
-        Step r = {-1, 0};
+        Step r = {-1, 0, -1, 0};
         while (unit < n_units) {
-          const int *e = s_plan + 8 + 5 * unit;
+          const int *e = s_plan + 8 + 7 * unit;
           const int len = e[2] - e[1];
           if (at < seen + len) {
             const int k = at - seen;
             r.f = e[0];
-            r.tile = staged ? s_tiles[e[4] + k] : __ldg(p.lists + (long long)e[0] * p.list_stride + e[1] + k);
+            r.list = e[5];
+            r.rows = e[6];
+            r.tile = staged ? s_tiles[e[4] + k] : e[5] >= 0 ? e[1] + k : __ldg(p.lists + (long long)e[0] * p.list_stride + e[1] + k);
             break;
           }
           seen += len;
@@ -598,20 +759,22 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
       struct Rows {
         int v[4];
       };
-      const bool wide_order = (reinterpret_cast<uintptr_t>(p.argsort) & 15u) == 0;
+      const bool wide_order = (reinterpret_cast<uintptr_t>(p.mode == kWgradMaskConv ? p.argsort : p.a_inds) & 15u) == 0;
       // rows of dout (pair lists: of both operands) that lane's tile rows stand for
       auto load_order = [&](const Step &st, Rows &a) {
         const int r0 = st.tile * 128 + 4 * quad;
-        if (p.mode == kWgradMaskConv && st.tile >= 0 && has_quad && wide_order && r0 + 4 <= p.n_rows) {
-          const int4 o = __ldg(reinterpret_cast<const int4 *>(p.argsort + r0));
+        const int *order = p.mode != kWgradMaskConv ? p.a_inds : st.list >= 0 ? p.rows + st.list : p.argsort;
+        const int n = st.list >= 0 ? st.rows : p.n_rows;
+        if (st.tile >= 0 && has_quad && (wide_order || st.list >= 0) && r0 + 4 <= n) {
+          const int4 o = __ldg(reinterpret_cast<const int4 *>(order + r0));
           a.v[0] = o.x, a.v[1] = o.y, a.v[2] = o.z, a.v[3] = o.w;
           return;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           a.v[j] = -1;
-          if (st.tile >= 0 && has_quad && r0 + j < p.n_rows)
-            a.v[j] = __ldg((p.mode == kWgradMaskConv ? p.argsort : p.a_inds) + r0 + j);
+          if (st.tile >= 0 && has_quad && r0 + j < n)
+            a.v[j] = __ldg(order + r0 + j);
         }
       };
       auto load_rows = [&](const Step &st, const Rows &a, Rows &b) {
@@ -619,10 +782,10 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           b.v[j] = -1;
-          if (st.tile >= 0 && has_quad && r0 + j < p.n_rows) {
+          if (st.tile >= 0 && has_quad && r0 + j < (st.list >= 0 ? st.rows : p.n_rows)) {
             if (p.mode == kWgradMaskConv) {
               // a chunk of at least a tile carries the offset, or the tile would not be in the list
-              const bool on = p.mask_width >= 128 ||
+              const bool on = st.list >= 0 || p.mask_width >= 128 ||
                               ((__ldg(p.rmask + (long long)((r0 + j) / p.mask_width) * p.words + (st.f >> 5)) >> (st.f & 31)) & 1u);
               if (on && a.v[j] >= 0)
                 b.v[j] = __ldg(p.indices + (long long)st.f * p.n_rows + a.v[j]);
@@ -690,8 +853,9 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     const uint8_t *b_bytes = reinterpret_cast<const uint8_t *>(p.x);
     constexpr int CPR_B = BLOCK_N / 8;  // 16-byte chunks per B row (fp16)
     wgrad_walk(
-        p.lists, p.list_stride, s_plan, s_tiles, [&](int, int) -> bool { return true; },
-        [&](int tile, int f, bool) -> bool {
+        p.lists, p.list_stride, s_plan, s_tiles,
+        [&](int tile, const int *e, bool) -> bool {
+          const int f = e[0];
           const bool mine = (step % Cfg::SA) == g;
           const int use = step / Cfg::SA;
           ++step;
@@ -699,7 +863,12 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
             return true;
           const int r = tile * 128 + gt;
           int ia = -1, ib = -1;
-          if (r < p.n_rows) {
+          if (e[5] >= 0) {
+            if (r < e[6]) {
+              ia = __ldg(p.rows + e[5] + r);
+              ib = __ldg(p.indices + (long long)f * p.n_rows + ia);
+            }
+          } else if (r < p.n_rows) {
             if (p.mode == kWgradMaskConv) {
               const uint32_t word = __ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5));
               const int o = __ldg(p.argsort + r);  // independent of `word`: both loads are in flight together
@@ -711,10 +880,10 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
               ia = __ldg(p.a_inds + r);
               ib = __ldg(p.b_inds + r);
             }
-            if (ia >= p.a_rows || ib >= p.b_rows) {
-              fail(kStatusBadIndex);
-              ia = ib = -1;
-            }
+          }
+          if (ia >= p.a_rows || ib >= p.b_rows) {
+            fail(kStatusBadIndex);
+            ia = ib = -1;
           }
           const uint32_t a_stage = sbase + Cfg::OFF_STAGES + g * Cfg::STAGE_BYTES;
           const uint32_t b_stage = a_stage + Cfg::A_BYTES;

@@ -140,7 +140,7 @@ class SparseConvLayer:
             r.split_k_slices = 32
             r.stream = stream
             r.max_ctas = int(shares.get(ConvOpType.BackwardWeight, 0))
-            self.wgrad = prepare_conv(r, static_tables=True)
+            self.wgrad = prepare_conv(r, static_tables=True, static_rows=True)
 
     def prepare_int8(self, scale, bias) -> None:
         self.fwd_params.scale, self.fwd_params.bias = scale, bias

@@ -502,20 +502,22 @@ class ConvParams:
 _WORKSPACES = {}
 
 
-def _workspace_for(device: int, stream: int, nbytes: int, user_ws):
+def _workspace_for(device: int, stream: int, nbytes: int, user_ws, best: int = 0):
     """The reference's callee allocates scratch when the caller passes none
     (cumm/gemm/nvrtc_code.py:137-140).  Here a per-(device, stream) buffer is cached so no
     allocation happens on the steady-state path.  Calls on one stream that rely on it share
     the buffer; they are ordered by the stream, and the weight-gradient kernel waits for its
     predecessor before it touches the workspace, so they do not race.  Callers that run weight
     gradients on several streams at once pass their own ``workspace`` (or use
-    :func:`prepare_conv`, which gives every call its own)."""
+    :func:`prepare_conv`, which gives every call its own).  ``best``: bytes with which the call runs
+    fastest, if those are more than it needs; a buffer of the caller's only has to hold ``nbytes``."""
     t = as_view(user_ws)
     if t is not None and t.nbytes() >= nbytes and t.data_ptr() % 256 == 0:
         return t.data_ptr(), t.nbytes()
     if t is not None and t.nbytes() < nbytes:
         raise RuntimeError(f"workspace at least {nbytes} bytes.")
     import torch
+    nbytes = max(nbytes, best)
     key = (device, stream)
     buf = _WORKSPACES.get(key)
     if buf is None or buf.numel() < nbytes:
@@ -774,7 +776,9 @@ def run_conv(params: ConvParams) -> None:
     if args.op_type == ConvOpType.BackwardWeight:  # the only operator that needs scratch
         need = L.cb2_conv_workspace_size(ctypes.byref(args))
         if need:
-            args.workspace, args.workspace_bytes = _workspace_for(args._device, stream, need, params.workspace)
+            args.workspace, args.workspace_bytes = _workspace_for(
+                args._device, stream, need, params.workspace, L.cb2_conv_workspace_size_lists(ctypes.byref(args)))
+            args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS  # this call's tables, planned for this call
     # verbose: registers of the kernel and the time of this launch (cumm/conv/main.py:723-729)
     timer = params.timer
     enabled = timer is not None and getattr(timer, "enable", False)
@@ -858,15 +862,17 @@ class PreparedCall:
         if rc:
             _lib.raise_for(rc)
         if self._plan_once:
-            self._args.reuse_plan = 1
+            self._args.reuse_plan |= 1
 
 
-def _attach_workspace(L, args, params, keep, size_fn) -> None:
+def _attach_workspace(L, args, params, keep, size_fn, best_fn=None) -> None:
     need = size_fn(ctypes.byref(args))
     if need:
         t = as_view(params.workspace)
         if t is None or t.nbytes() < need:
             import torch
+            if best_fn is not None:
+                need = max(need, best_fn(ctypes.byref(args)))
             ws = torch.empty(need, dtype=torch.uint8, device=f"cuda:{args._device}")
             keep.append(ws)
             args.workspace, args.workspace_bytes = ws.data_ptr(), need
@@ -875,15 +881,21 @@ def _attach_workspace(L, args, params, keep, size_fn) -> None:
             args.workspace, args.workspace_bytes = t.data_ptr(), t.nbytes()
 
 
-def prepare_conv(params: ConvParams, static_tables: bool = False) -> PreparedCall:
+def prepare_conv(params: ConvParams, static_tables: bool = False, static_rows: bool = False) -> PreparedCall:
     """Validate ``params`` like :func:`run_conv` and return a replayable call.  The tensors
     in ``params`` must stay alive and in place while the call is in use.  Every prepared call
-    has a workspace of its own (two prepared weight gradients may overlap on the GPU)."""
+    has a workspace of its own (two prepared weight gradients may overlap on the GPU).
+    ``static_rows``, beside ``static_tables``: ``indices`` and ``mask_argsort`` keep their contents too, so
+    that the weight gradient's plan may list rows (without ``static_tables`` it plans, and lists, on
+    every launch)."""
     L = _lib.load()
     args = _conv_args(params)
     keep = [params.input, params.weight, params.output, params.indices, params.mask, params.mask_argsort,
             params.mask_output, params.bias, params.scale, params.output_add]
-    _attach_workspace(L, args, params, keep, L.cb2_conv_workspace_size)
+    if static_rows or not static_tables:
+        args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS
+    _attach_workspace(L, args, params, keep, L.cb2_conv_workspace_size,
+                      L.cb2_conv_workspace_size_lists if args.reuse_plan else None)
     return PreparedCall("conv", args, args._device, params.stream, keep, static_tables)
 
 

@@ -176,7 +176,10 @@ typedef struct cb2_conv_args {
    * reuse_plan (backward weight only): the workspace still holds the plan of an earlier, stream-ordered
    *   call on the same workspace with the same reduced masks (contents, not just address), row count,
    *   mask_width, mask_filter, tile_n and max_ctas -- skip the planning kernel.  The plan depends on
-   *   the neighbour tables only, so a training loop plans once per scene. */
+   *   the neighbour tables only, so a training loop plans once per scene.  Bit 0 says so; bit 1
+   *   (CB2_PLAN_ROW_LISTS, with or without bit 0) lets the plan list rows where the workspace has
+   *   cb2_conv_workspace_size_lists() bytes: such a plan may be reused only while indices and
+   *   mask_argsort are as they were, too. */
   void *sched_scratch;
   int max_ctas;
   int reuse_plan;
@@ -223,6 +226,11 @@ int cb2_gemm_sequence_run(const cb2_gemm_sequence_args *args, void *stream);
  * callee never allocates. */
 size_t cb2_gemm_workspace_size(const cb2_gemm_args *args);
 size_t cb2_conv_workspace_size(const cb2_conv_args *args);
+/* Bytes with which backward weight runs fastest (0 for the other operators): room for per-offset lists
+ * of the rows that have a neighbour, which a call with CB2_PLAN_ROW_LISTS in reuse_plan walks instead
+ * of whole row tiles. */
+#define CB2_PLAN_ROW_LISTS 2
+size_t cb2_conv_workspace_size_lists(const cb2_conv_args *args);
 
 /*
  * Weight gradient without any allocation.  (No counterpart in the reference: its callee
