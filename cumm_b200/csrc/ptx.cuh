@@ -183,6 +183,13 @@ __device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// 32 bytes to a 32-byte boundary in one store
+__device__ __forceinline__ void st_global_32(void *dst, const uint32_t *v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
 __device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
 }

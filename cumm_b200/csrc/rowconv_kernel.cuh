@@ -7,8 +7,8 @@
 // to 128 bytes, 16-byte cp.async for wider ones; missing neighbours read as zeros), brings the
 // matching weight slice in by TMA, and one thread issues tcgen05.mma into a TMEM accumulator.
 // Eight (fp16) or sixteen (int8) epilogue warps read the accumulator back, apply
-// alpha/beta/bias/activation (or the int8 requantisation), stage the tile through shared
-// memory and write whole rows to their scattered destinations.  No atomics on data: every
+// alpha/beta/bias/activation (or the int8 requantisation) and write the rows to their scattered
+// destinations, whole 32-byte sectors per thread.  No atomics on data: every
 // output row is owned by exactly one tile.
 //
 // What it computes follows the reference kernel's control flow
@@ -73,6 +73,9 @@ struct RowConvParams {
 #ifndef CB2_ROWCONV_NARROW_STAGES
 #define CB2_ROWCONV_NARROW_STAGES 6
 #endif
+#ifndef CB2_ROWCONV_WIDE_STAGES
+#define CB2_ROWCONV_WIDE_STAGES 3
+#endif
 #ifndef CB2_ROWCONV_EPI_PARTS
 #define CB2_ROWCONV_EPI_PARTS 4
 #endif
@@ -92,11 +95,9 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // A stages == producer groups.  The kernel with sixteen epilogue warps keeps to 24 warps: six per
   // SM sub-partition leave 80 registers per thread, seven would leave 72 and spill.
   static constexpr int SA =
-      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES) : 3;
+      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES) : CB2_ROWCONV_WIDE_STAGES;
   static constexpr int A_STAGE_BYTES = TILE_M * 128 * NATOM_K;
   static constexpr int B_SLOT_BYTES = BLOCK_N * 128 * NATOM_K;
-  static constexpr int OUT_ROW_BYTES = BLOCK_N * OES;
-  static constexpr int STAGING_BYTES = TILE_M * OUT_ROW_BYTES;
   static constexpr int MW = MASK_WORDS;
   // Outputs wider than BLOCK_N: column parts drawn with the tiles (fp16), or one grid row per part
   // (int8, whose sixteen epilogue warps have no register to spare for a part that changes).
@@ -109,7 +110,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
                        BAR_RING = (BAR_EMPTY_B + 6 + 1) / 2 * 2;
   // Weight slots: as many as fit (2 to 6).  A tile whose mask carries many offsets needs a new
   // weight tile every step, and with two slots the L2 latency of that load bounds the step.
-  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + STAGING_BYTES + SA * 2 * 128 * 4 + 128 * 4 +
+  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + SA * 2 * 128 * 4 +
                                      2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (BAR_RING + 3 * RING) * 8 + 64 + 1024;
   static constexpr int SB_FIT = (232448 - FIXED_BYTES) / B_SLOT_BYTES;
   static constexpr int SB = SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
@@ -131,10 +132,8 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // shared memory map (offsets from a 1024-byte aligned base)
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + SA * A_STAGE_BYTES;
-  static constexpr int OFF_STAGING = OFF_B + SB * B_SLOT_BYTES;
-  static constexpr int OFF_ROWIDX = OFF_STAGING + STAGING_BYTES;     // SA * 2 * 128 ints
-  static constexpr int OFF_OUTROW = OFF_ROWIDX + SA * 2 * 128 * 4;   // 128 ints
-  static constexpr int OFF_SCALE = OFF_OUTROW + 128 * 4;             // 2 * BLOCK_N floats
+  static constexpr int OFF_ROWIDX = OFF_B + SB * B_SLOT_BYTES;       // SA * 2 * 128 ints
+  static constexpr int OFF_SCALE = OFF_ROWIDX + SA * 2 * 128 * 4;    // 2 * BLOCK_N floats
   static constexpr int OFF_RING = OFF_SCALE + 2 * BLOCK_N * 4;       // RING slots
   static constexpr int OFF_BARS = OFF_RING + RING * RING_SLOT_INTS * 4;  // BAR_RING + 3 * RING mbarriers
   static constexpr int OFF_MISC = OFF_BARS + (BAR_RING + 3 * RING) * 8;  // tmem ptr, abort, flags
@@ -538,7 +537,6 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   const uint32_t sbase = raw_addr + pad;
 
   int *rowidx = reinterpret_cast<int *>(smem + Cfg::OFF_ROWIDX);
-  int *outrow = reinterpret_cast<int *>(smem + Cfg::OFF_OUTROW);
   float *s_scale = reinterpret_cast<float *>(smem + Cfg::OFF_SCALE);
   float *s_bias = s_scale + BLOCK_N;
   volatile int *misc = reinterpret_cast<volatile int *>(smem + Cfg::OFF_MISC);
@@ -586,7 +584,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     }
     for (int s = 0; s < Cfg::NUM_ACC; ++s) {
       mbar_init(acc_full(s), 1);
-      mbar_init(acc_empty(s), Cfg::EPI_THREADS);
+      mbar_init(acc_empty(s), Cfg::EPI_THREADS / 32);
     }
     mbar_init(final_bar, 1);
     for (int s = 0; s < Cfg::RING; ++s) {
@@ -636,16 +634,18 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   };
 
   if (warp < Cfg::MMA_WARP) {
-    // ======================= epilogue: TMEM -> registers -> staging -> scattered rows
+    // ======================= epilogue: TMEM -> registers -> scattered rows.  A thread holds 32
+    // consecutive columns of one row and stores them itself, 32 bytes at a time (whole sectors); nothing
+    // is staged, so every warp runs at its own pace and the accumulator is free again as soon as the
+    // last column has been read.  (Staging a tile in shared memory to store whole rows put two barriers
+    // of all epilogue warps into every tile.)
     const int et = threadIdx.x;
     const int erow = et & 127;   // the tile row this thread reads from TMEM (lane quarter = warp & 3)
     const int half = et >> 7;    // which share of the columns
     constexpr int COLS_PER_HALF = BLOCK_N / Cfg::EPI_HALVES;
-    uint8_t *staging = smem + Cfg::OFF_STAGING;
-    constexpr int CPR = Cfg::OUT_ROW_BYTES / 16;       // 16-byte chunks per output row
-    constexpr int SWZ = (CPR >= 8 ? 8 : CPR) - 1;
-    constexpr int CH_PER_ROUND = 32 * Cfg::OES / 16;   // chunks produced per 32 columns
-    int acc_use = 0;
+    const bool sectors = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(p.ldo * Cfg::OES)) & 31u) == 0;
+    int buf = 0;
+    uint32_t acc_phase = 0;
     bool dep_waited = false;
     CB2_PROF_BEGIN();
     TileCursor<MW> tc;
@@ -658,8 +658,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           if (!has_work && p.skip_empty_tiles)
             continue;
           const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
-          if (et == 0)
-            CB2_PROF_MARK(0);  // walk
+          CB2_PROF_MARK(0);  // walk
           if (!dep_waited) {
             grid_dep_wait();
             dep_waited = true;
@@ -674,32 +673,44 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                   p.mask_out[(long long)tile * p.mask_words + w] = static_cast<uint32_t>((w < 2 ? tc.lo : tc.hi) >> (32 * (w & 1)));
             }
           }
-          const int buf = acc_use % Cfg::NUM_ACC;
           if (has_work) {
-            if (et == 0) {
+            if (et == 0)
               CB2_TRACE_EVENT(4, 7, tile);
-              bool ok = mbar_wait(acc_full(buf), (acc_use / Cfg::NUM_ACC) & 1, abort_flag);
+            const bool ok = mbar_wait(acc_full(buf), acc_phase, abort_flag);
+            if (et == 0)
               CB2_TRACE_EVENT(4, 8, tile);  // accumulator complete
-              misc[2] = ok ? 1 : 0;
-              if (!ok)
+            if (!__all_sync(0xffffffffu, ok)) {
+              if (lane == 0)
                 fail(kStatusWaitTimeout);
-              CB2_PROF_MARK(1);  // accumulator complete
+              break;
             }
+            tc_fence_after();
           }
-          named_bar_sync(1, Cfg::EPI_THREADS);  // wait result visible; staging free again
-          if (et == 0)
-            CB2_PROF_MARK(2);  // barrier
-          if (has_work && misc[2] == 0)
-            break;
-          if (half == 0)
-            outrow[erow] = o;
-          tc_fence_after();
+          CB2_PROF_MARK(1);  // accumulator complete
           const uint32_t trow = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) +
                                 static_cast<uint32_t>(buf * BLOCK_N);
           const bool use_src = (p.src_mode != kSrcNone) && (p.beta != 0.f);
           // fast path: out = cvt(acc); everything else goes through the general epilogue
           const bool plain = !use_src && p.act_type == 0 && p.alpha == 1.f;
           constexpr int ROUNDS = COLS_PER_HALF / 32;
+          // 16-byte pieces of this thread's row; the columns past nn are not stored
+          auto store = [&](int ncol, const auto &packed) {
+            constexpr int N = sizeof(packed) / 16, PIECE = 16 / Cfg::OES;
+            if (o < 0)
+              return;
+            uint8_t *dst = reinterpret_cast<uint8_t *>(p.out) + ((long long)o * p.ldo + ncol) * Cfg::OES;
+            if (sectors && ncol + N * PIECE <= p.nn) {
+#pragma unroll
+              for (int q = 0; q < N; q += 2)
+                st_global_32(dst + 16 * q, &packed[4 * q]);
+            } else {
+#pragma unroll
+              for (int q = 0; q < N; ++q)
+                if (ncol + q * PIECE < p.nn)
+                  *reinterpret_cast<uint4 *>(dst + 16 * q) =
+                      make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+            }
+          };
 #pragma unroll 1
           for (int round = 0; round < ROUNDS; ++round) {
             uint32_t v[32];
@@ -707,6 +718,12 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             if (has_work) {
               tmem_ld32(trow + col0, v);
               tmem_ld_wait();
+              if (round == ROUNDS - 1) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                  mbar_arrive(acc_empty(buf));
+              }
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
@@ -771,13 +788,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                   packed[i / 2] = *reinterpret_cast<uint32_t *>(&h2);
                 }
               }
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const int c = (col0 / 32) * CH_PER_ROUND + q;
-                const int pc = (c & ~SWZ) | ((c ^ erow) & SWZ);
-                *reinterpret_cast<uint4 *>(staging + erow * Cfg::OUT_ROW_BYTES + pc * 16) =
-                    make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]);
-              }
+              store(ncol0, packed);
             } else {
               uint32_t packed[8];
               float t[32];
@@ -823,52 +834,16 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 32; i += 4)
                 packed[i / 4] = cvt_pack4_s8(t[i], t[i + 1], t[i + 2], t[i + 3]);
-#pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                const int c = (col0 / 32) * CH_PER_ROUND + q;
-                const int pc = (c & ~SWZ) | ((c ^ erow) & SWZ);
-                *reinterpret_cast<uint4 *>(staging + erow * Cfg::OUT_ROW_BYTES + pc * 16) =
-                    make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]);
-              }
+              store(ncol0, packed);
             }
           }
-          if (has_work) {
-            tc_fence_before();
-            mbar_arrive(acc_empty(buf));
-            ++acc_use;
+          CB2_PROF_MARK(3);  // TMEM -> rows
+          if (has_work && ++buf == Cfg::NUM_ACC) {
+            buf = 0;
+            acc_phase ^= 1u;
           }
-          if (et == 0) {
-            CB2_TRACE_EVENT(4, 12, tile);  // staged
-            CB2_PROF_MARK(3);  // TMEM -> staging
-          }
-          named_bar_sync(1, Cfg::EPI_THREADS);  // staging complete
           if (et == 0)
-            CB2_PROF_MARK(4);  // barrier
-          // phase 2: CPR threads per row write whole rows
-          {
-            const int c = et % CPR;
-            const int row0 = et / CPR;
-            constexpr int RSTEP = Cfg::EPI_THREADS / CPR;
-            const int ncol = n0 + c * (16 / Cfg::OES);
-            if (ncol < p.nn) {
-#pragma unroll 4
-              for (int i = 0; i < 128 / RSTEP; ++i) {
-                const int row = row0 + i * RSTEP;
-                const int orow = outrow[row];
-                if (orow >= 0) {
-                  const int pc = (c & ~SWZ) | ((c ^ row) & SWZ);
-                  uint4 val = *reinterpret_cast<const uint4 *>(staging + row * Cfg::OUT_ROW_BYTES + pc * 16);
-                  uint8_t *dst = reinterpret_cast<uint8_t *>(p.out) +
-                                 ((long long)orow * p.ldo + ncol) * Cfg::OES;
-                  *reinterpret_cast<uint4 *>(dst) = val;
-                }
-              }
-            }
-          }
-          if (et == 0) {
             CB2_TRACE_EVENT(4, 9, tile);  // rows stored
-            CB2_PROF_MARK(5);  // staging -> global
-          }
     }
     if (et == 0)
       CB2_PROF_END2();
