@@ -365,6 +365,8 @@ void wgrad_layout(int num_sms, int max_ctas, int m_total, int n_total, long long
   const int per = wgrad_chunk_tiles((int)ntiles);
   L->n_chunks = per > 0 ? (int)((ntiles + per - 1) / per) : 0;
   L->row_capacity = (n_rows * std::min(kvs, 8 + kvs / 8) + 127) / 128 * 128;
+  if (ntiles <= kWgradOneBlockTiles)  // one launch makes the lists, each with room for every row
+    L->row_capacity = ntiles * 128 * kvs;
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   L->off_head = up(L->total);
   L->off_counts = L->off_head + 2 * kWgradMaxOffsets * 4;
@@ -420,14 +422,21 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
   p.lists = reinterpret_cast<const int *>(ws + L.off_lists);
   p.list_stride = L.list_stride;
   p.status = dev->status;
-  // Row lists where the caller allows them and the workspace has room, tiles otherwise.
-  const bool row_lists = (plan_flags & CB2_PLAN_ROW_LISTS) && p.mode == kWgradMaskConv && p.n_rows > 0 && workspace_bytes >= L.total_lists &&
-                         L.row_capacity < (1ll << 31);
-  if (row_lists) {
+  // Row lists where the caller allows them and the workspace has room, tiles otherwise.  A plan in such a
+  // workspace says for itself which of the two it holds, so one made either way can be reused.
+  const bool room = p.mode == kWgradMaskConv && p.n_rows > 0 && workspace_bytes >= L.total_lists &&
+                    L.row_capacity < (1ll << 31);
+  const bool row_lists = room && (plan_flags & CB2_PLAN_ROW_LISTS);
+  if (room) {
     p.row_head = reinterpret_cast<int *>(ws + L.off_head);
     p.rows = reinterpret_cast<const int *>(ws + L.off_rows);
   }
-  if (!reuse_plan && row_lists) {
+  if (!reuse_plan && row_lists && L.list_stride <= kWgradOneBlockTiles) {
+    wgrad_plan_rows_kernel<<<p.kv, kWgradPlanThreads, 0, stream>>>(p, reinterpret_cast<int *>(ws + L.off_lists),
+                                                                   reinterpret_cast<int *>(ws + L.off_rows), L.n_ctl);
+    CB2_CUDA(cudaGetLastError());
+    g_launches.fetch_add(1);
+  } else if (!reuse_plan && row_lists) {
     const dim3 grid(L.n_chunks, p.kv);
     uint4 *bits = reinterpret_cast<uint4 *>(ws + L.off_bits);
     int2 *counts = reinterpret_cast<int2 *>(ws + L.off_counts);

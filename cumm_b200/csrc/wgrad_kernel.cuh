@@ -124,9 +124,9 @@ __device__ __forceinline__ bool wgrad_tile_has(const WgradParams &p, int tile, i
 
 // ---------------------------------------------------------------- schedule
 // The work is the sequence of all (filter offset f, row tile carrying f) pairs, offsets in
-// ascending order, tiles in ascending order inside an offset: T steps in all.  CTA c of G takes
-// the steps [c*T/G, (c+1)*T/G) -- every CTA the same number, whatever the offsets' shares --
-// and each maximal run of one offset inside a CTA's range is a UNIT: it accumulates in TMEM
+// ascending order, tiles in ascending order inside an offset: T steps in all, with what an offset's
+// units cost charged in steps.  CTA c of G takes the steps [c*T/G, (c+1)*T/G) -- every CTA the same
+// number, whatever the offsets' shares -- and each maximal run of one offset inside a CTA's range is a UNIT: it accumulates in TMEM
 // and leaves one fp32 partial.  The units of an offset are consecutive in this numbering, and
 // there are at most G + kv - 1 of them.
 //
@@ -159,11 +159,23 @@ __device__ __forceinline__ void wgrad_scan4(const int (&v)[4], int (&excl)[4], i
     run += v[j];
   }
 }
-// Given the tile counts of this lane's offsets: P = steps before each offset, T = all steps,
-// c_first = CTA holding step P, S = units of the offset, U = units before it.
+// A unit costs its CTA about as much as kWgradUnitSteps steps (a partial sum stored, counted in, and
+// read again by whoever sums): every offset is charged that many steps before its own, or the CTAs that
+// get a dozen offsets of one or two steps each are the last to finish.  The cuts are made in charged steps.
+constexpr int kWgradUnitSteps = 2;
+// Given the step counts of this lane's offsets: P = charged steps before the offset's first own step,
+// T = all charged steps, c_first = CTA holding the offset's first step, S = units of the offset, U = units
+// before it.
 __device__ __forceinline__ void wgrad_plan_warp(const int (&cnt)[4], int G, int (&P)[4], int &T, int (&c_first)[4],
                                                 int (&S)[4], int (&U)[4]) {
-  wgrad_scan4(cnt, P, T);
+  int charged[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    charged[j] = cnt[j] > 0 ? cnt[j] + kWgradUnitSteps : 0;
+  wgrad_scan4(charged, P, T);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    P[j] += kWgradUnitSteps;
   // the CTA holding step x is the largest c with c*T/G <= x, i.e. ceil((x+1)*G/T) - 1
   auto chunk_of = [&](int x) -> int {
     const int c = (int)((((long long)x + 1) * G + T - 1) / T) - 1;
@@ -229,8 +241,11 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
     }
     running += all;
   }
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
     p.sched[f] = running;
+    if (p.row_head)
+      p.row_head[f] = -1;
+  }
 }
 
 // ---------------------------------------------------------------- plan with row lists
@@ -241,12 +256,88 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
 // ceil(pairs / 128) steps.  Two kernels make the lists: one marks, per (offset, tile), the rows that take
 // part (a 128-bit word) and counts them per chunk of tiles, the other turns counts into places and
 // writes the lists in sorted order, so the sums have one fixed order.  Offsets whose tiles are at least
-// four fifths full, and lists that find no room, are walked by tiles.
-constexpr int kWgradPlanThreads = 256;
+// four fifths full, and lists that find no room, are walked by tiles.  (100 003 rows of a scanned scene,
+// 64 channels: 8281 steps by tiles, 4030 by rows, 102 -> 54 us; 30 011 rows, 125 offsets: 16324 and
+// 3100, 218 -> 33 us and 21 us of planning.  At four fifths the shorter walk is worth the table read
+// that makes it.)
+constexpr int kWgradPlanThreads = 1024;  // a warp per tile of a group of 32
 constexpr int kWgradMaxChunks = 64;
 // tiles per chunk: whole groups of 32
 __host__ __device__ inline int wgrad_chunk_tiles(int ntiles) {
   return 32 * ((ntiles + 32 * kWgradMaxChunks - 1) / (32 * kWgradMaxChunks));
+}
+
+// Rows of tile t that take part at offset f, 32 per word (warp-collective); o = the output rows.
+__device__ __forceinline__ uint4 wgrad_tile_rows(const WgradParams &p, int t, int f, int (&o)[4]) {
+  const int lane = (int)lane_id();
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  if (wgrad_tile_has(p, t, f)) {
+    bool on[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = t * 128 + q * 32 + lane;
+      o[q] = r < p.n_rows ? __ldg(p.argsort + r) : -1;
+      on[q] = o[q] >= 0;
+      if (p.mask_width < 128 && on[q])
+        on[q] = (__ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5)) >> (f & 31)) & 1u;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      w[q] = __ballot_sync(0xffffffffu, on[q] && __ldg(p.indices + (long long)f * p.n_rows + o[q]) >= 0);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ bool wgrad_listed(long long rows, long long tiles) {
+  return 512 * tiles > 5 * rows;  // tiles less than four fifths full
+}
+
+// Up to kWgradOneBlockTiles tiles: both in one launch, a block per offset, every list with room for all
+// rows (so that no offset has to know the others' counts).
+constexpr int kWgradOneBlockTiles = 256;
+__global__ void __launch_bounds__(kWgradPlanThreads) wgrad_plan_rows_kernel(const WgradParams p, int *lists, int *rows,
+                                                                            int n_ctl) {
+  __shared__ int s_n[32];
+  const int f = blockIdx.x;
+  for (int i = f * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * blockDim.x)
+    p.ctl[i] = 0;
+  grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the plan
+  const int ntiles = (p.n_rows + 127) / 128;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long base = (long long)f * ((p.n_rows + 127) / 128 * 128);
+  int all_rows = 0, all_tiles = 0;
+  for (int t0 = 0; t0 < ntiles; t0 += 32) {
+    const int t = t0 + wid;
+    int o[4];
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (t < ntiles)
+      v = wgrad_tile_rows(p, t, f, o);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
+    __syncthreads();  // s_n of the previous round has been read
+    if (lane == 0)
+      s_n[wid] = n;
+    __syncthreads();
+    const int c = s_n[lane];
+    const unsigned any = __ballot_sync(0xffffffffu, c > 0);
+    const int round_rows = __reduce_add_sync(0xffffffffu, c);
+    int at = all_rows + __reduce_add_sync(0xffffffffu, lane < wid ? c : 0);
+    if (lane == 0 && n > 0)
+      lists[(long long)f * p.list_stride + all_tiles + __popc(any & ((1u << wid) - 1u))] = t;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if ((w[q] >> lane) & 1u)
+        rows[base + at + __popc(w[q] & ((1u << lane) - 1u))] = o[q];
+      at += __popc(w[q]);
+    }
+    all_rows += round_rows;
+    all_tiles += __popc(any);
+  }
+  if (threadIdx.x == 0) {
+    const bool listed = wgrad_listed(all_rows, all_tiles);
+    p.sched[f] = listed ? (all_rows + 127) / 128 : all_tiles;
+    p.row_head[f] = listed ? (int)base : -1;
+    p.row_head[kWgradMaxOffsets + f] = all_rows;
+  }
 }
 
 // grid (chunks, offsets); bits[f][tile][4], counts[f][chunk] = {rows, tiles with any}
@@ -261,22 +352,9 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_mark_rows_kernel(cons
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int rows = 0, tiles = 0;
   for (int t = chunk * per + wid; t < min((chunk + 1) * per, ntiles); t += kWgradPlanThreads / 32) {
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    if (wgrad_tile_has(p, t, f)) {
-      int o[4];
-      bool on[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = t * 128 + q * 32 + lane;
-        o[q] = r < p.n_rows ? __ldg(p.argsort + r) : -1;
-        on[q] = o[q] >= 0;
-        if (p.mask_width < 128 && on[q])
-          on[q] = (__ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5)) >> (f & 31)) & 1u;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        w[q] = __ballot_sync(0xffffffffu, on[q] && __ldg(p.indices + (long long)f * p.n_rows + o[q]) >= 0);
-    }
+    int o[4];
+    const uint4 v = wgrad_tile_rows(p, t, f, o);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
     rows += n;
     tiles += n > 0;
@@ -324,7 +402,7 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_list_rows_kernel(cons
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int g = 4 * lane + j;
-      listed[j] = 512ll * s_tiles[g] > 5ll * s_rows[g];  // tiles less than four fifths full
+      listed[j] = wgrad_listed(s_rows[g], s_tiles[g]);
       size[j] = listed[j] ? (s_rows[g] + 127) / 128 : 0;  // in steps
     }
     wgrad_scan4(size, first, total);
@@ -728,7 +806,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     const int g = (warp - 5) / Cfg::GW;
     const int quad = (warp - 5) % Cfg::GW * (32 / Cfg::GW) + lane;
     const bool has_quad = lane < 32 / Cfg::GW;
-    const bool first_lane = quad == 0;
+    const bool first_lane = (warp - 5) % Cfg::GW == 0 && lane == 0;
     if (g < Cfg::SA) {
       const int n_units = s_plan[0];
       const bool staged = s_plan[1] != 0;

@@ -116,6 +116,7 @@ def run_dense_conv(params) -> None:
     q.split_k_slices = params.split_k_slices
     q.workspace, q.stream, q.verbose = params.workspace, params.stream, params.verbose
     q.max_ctas = getattr(params, "max_ctas", 0)
+    q.row_lists = False  # every row has every neighbour but those at the border
     op = ConvOpType(int(desp.op_type))
     if op == ConvOpType.BackwardInput:
         q.indices, q.mask, q.mask_argsort = t["indices_bwd"], t["mask_bwd"], t["argsort_bwd"]

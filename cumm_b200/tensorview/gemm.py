@@ -494,6 +494,8 @@ class ConvParams:
         # Not in the reference: upper bound on the CTAs of the launch (0 = one per SM), for calls
         # that run side by side on different streams (``cb2_conv_args.max_ctas``).
         self.max_ctas = 0
+        # Not in the reference: the weight gradient's plan may list rows (``CB2_PLAN_ROW_LISTS``).
+        self.row_lists = True
 
 
 # --------------------------------------------------------------------------------------
@@ -776,9 +778,12 @@ def run_conv(params: ConvParams) -> None:
     if args.op_type == ConvOpType.BackwardWeight:  # the only operator that needs scratch
         need = L.cb2_conv_workspace_size(ctypes.byref(args))
         if need:
+            lists = params.row_lists
             args.workspace, args.workspace_bytes = _workspace_for(
-                args._device, stream, need, params.workspace, L.cb2_conv_workspace_size_lists(ctypes.byref(args)))
-            args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS  # this call's tables, planned for this call
+                args._device, stream, need, params.workspace,
+                L.cb2_conv_workspace_size_lists(ctypes.byref(args)) if lists else 0)
+            if lists:  # this call's tables, planned for this call
+                args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS
     # verbose: registers of the kernel and the time of this launch (cumm/conv/main.py:723-729)
     timer = params.timer
     enabled = timer is not None and getattr(timer, "enable", False)
