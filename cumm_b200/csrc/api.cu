@@ -620,6 +620,8 @@ int pairgen_layout(const cb2_pairgen_args *a, PairgenLayout *L) {
       b = t;
     }
     const int period = a->stride[i] / gcd;  // r takes every period-th value
+    L->g.period[i] = period;
+    L->g.drop[i] = a->dil[i] / gcd;
     per_input *= std::min(a->ksize[i], (a->ksize[i] + period - 1) / period);
   }
   L->list_cap = a->subm ? 0 : std::min<long long>(n_in * per_input, cells);
@@ -651,7 +653,7 @@ int pairgen_layout(const cb2_pairgen_args *a, PairgenLayout *L) {
   L->off_list_a = take(static_cast<size_t>(keys_cap) * 8);
   L->off_list_b = take(static_cast<size_t>(keys_cap) * 8);
   L->off_key_hist = take(keys_cap ? static_cast<size_t>(256) * ((keys_cap + cb2pg::kKeySortTile - 1) / cb2pg::kKeySortTile + 1) * 4 : 0);
-  L->hist_ints = cb2pg::sort_hist_ints(L->shape, L->nmax);
+  L->hist_ints = cb2pg::kSortHistInts * L->shape.passes;
   L->off_hist = take(2 * L->hist_ints * 4);
   for (int side = 0; side < 2; ++side) {
     const size_t n = static_cast<size_t>(side == 0 ? L->nmax : n_in);
@@ -729,9 +731,8 @@ int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, c
       o.chunk = j.side.chunk;
       o.n_chunks = (j.side.n + j.side.chunk - 1) / j.side.chunk;
       max_chunks = std::max(max_chunks, o.n_chunks);
-      const size_t hist_pass = static_cast<size_t>(o.n_chunks) * cb2pg::kSortBins;
-      o.hist = j.side.hist + p * hist_pass;
-      o.hist_next = to_go ? j.side.hist + (p + 1) * hist_pass : nullptr;
+      o.hist = j.side.hist + p * cb2pg::kSortHistInts;
+      o.hist_next = to_go ? j.side.hist + (p + 1) * cb2pg::kSortHistInts : nullptr;
       o.rows = j.side.rows;
       // results of the last pass in the result arrays, of the one before it in scratch, and so on
       o.vout = to_go % 2 ? j.v_tmp : j.argsort;
@@ -764,8 +765,8 @@ struct Fill {
     most = std::max<long long>(most, static_cast<long long>(bytes / 4));
   }
   void run(const DeviceState *dev, cudaStream_t s) const {
-    const long long blocks = std::min<long long>((most / 4 + 255) / 256 + 1, 8ll * dev->num_sms);
-    cb2pg::fill_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(r);
+    const long long blocks = std::min<long long>((most / 4 + 1023) / 1024 + 1, 8ll * dev->num_sms);
+    cb2pg::fill_kernel<<<dim3(static_cast<unsigned>(blocks), r.count), 256, 0, s>>>(r);
     g_launches.fetch_add(1);
   }
 };
@@ -828,9 +829,7 @@ int cb2_pairgen_count_outputs(const cb2_pairgen_args *a, int *n_out, void *strea
     const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
     fill.add(bm.words, static_cast<size_t>(L.bitmap_words) * 4, 0u);
     fill.run(dev, stream);
-    const long long threads = static_cast<long long>(a->n_in) * L.g.ksize[0] * L.g.ksize[1];
-    cb2pg::bitmap_mark_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(a->in_coords, a->n_in, L.g,
-                                                                                              bm.words);
+    cb2pg::bitmap_mark_kernel<<<(a->n_in + 127) / 128, 128, 0, stream>>>(a->in_coords, a->n_in, L.g, bm.words);
     cb2pg::bitmap_rank_kernel<<<bm.n_blocks, cb2pg::kBitmapThreads, 0, stream>>>(bm, counter);
     g_launches.fetch_add(2);
   } else {
@@ -891,11 +890,12 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
     const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
     fill.add(a->indices, static_cast<size_t>(L.g.kv) * n_out * 4, 0xffffffffu);
     fill.add(jobs[0].side.rows, static_cast<size_t>(n_out) * words * 4, 0u);
+    if (bwd)
+      fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
     cb2pg::bitmap_coords_kernel<<<blocks(bm.n_words), 256, 0, stream>>>(bm, n_out, L.g, a->out_coords);
-    const long long threads = static_cast<long long>(n_in) * L.g.ksize[0] * L.g.ksize[1];
-    cb2pg::bitmap_scatter_kernel<<<blocks(threads), 256, 0, stream>>>(a->in_coords, n_in, L.g, bm, jobs[0].side, words,
-                                                                      dev->status);
+    cb2pg::bitmap_scatter_kernel<<<(n_in + 127) / 128, 128, 0, stream>>>(a->in_coords, n_in, L.g, bm, jobs[0].side, words,
+                                                                         dev->status);
     const int bwd_blocks = bwd ? static_cast<int>(blocks(n_in)) : 0;
     auto kern = words > 1 ? cb2pg::bitmap_backward_kernel<4> : cb2pg::bitmap_backward_kernel<1>;
     kern<<<bwd_blocks + blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(a->in_coords, L.g, bm, jobs[0].side, jobs[1].side,
@@ -905,15 +905,15 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
   } else {
     cb2pg::HashView h;
     h.slots = reinterpret_cast<unsigned long long *>(ws + L.off_hash);
-    h.cap_mask = L.cap_in - 1;
-    h.exact = L.exact;
+    h.bucket_mask = L.cap_in / cb2pg::kBucket - 1;
     h.coords = a->in_coords;
     const bool mirror = bwd && L.mirror;
     fill.add(h.slots, static_cast<size_t>(L.cap_in) * 8, 0xffffffffu);
     if (bwd && !mirror)
       fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
-    cb2pg::hash_insert_kernel<<<blocks(n_in), 256, 0, stream>>>(a->in_coords, n_in, L.g, h, dev->status);
+    auto insert = L.exact ? cb2pg::hash_insert_kernel<true> : cb2pg::hash_insert_kernel<false>;
+    insert<<<blocks(n_in), 256, 0, stream>>>(a->in_coords, n_in, L.g, h, dev->status);
     const int32_t *out_coords = a->in_coords;
     if (!a->subm) {
       cb2pg::decode_out_coords_kernel<<<blocks(n_out), 256, 0, stream>>>(
@@ -921,7 +921,8 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
       out_coords = a->out_coords;
       g_launches.fetch_add(1);
     }
-    auto kern = words > 1 ? cb2pg::probe_kernel<4> : cb2pg::probe_kernel<1>;
+    auto kern = L.exact ? (words > 1 ? cb2pg::probe_kernel<4, true> : cb2pg::probe_kernel<1, true>)
+                        : (words > 1 ? cb2pg::probe_kernel<4, false> : cb2pg::probe_kernel<1, false>);
     kern<<<blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(out_coords, L.g, h, jobs[0].side, mirror ? jobs[1].side : none,
                                                             words, shape.width);
     g_launches.fetch_add(2);
@@ -955,7 +956,7 @@ static void seq_layout(int count, long long n, SeqLayout *L) {
   L->off_argsort = take(static_cast<size_t>(n) * 4);
   L->off_m = take(static_cast<size_t>(n) * 4);
   L->off_v = take(static_cast<size_t>(n) * 4);
-  L->off_hist = take(cb2pg::sort_hist_ints(shape, n) * 4);
+  L->off_hist = take(cb2pg::kSortHistInts * shape.passes * 4);
   L->total = off;
 }
 
@@ -1027,7 +1028,7 @@ int cb2_gemm_sequence_run(const cb2_gemm_sequence_args *a, void *stream_v) {
     Fill fill;
     fill.add(ws + L.off_tickets, 256, 0u);
     fill.add(table, static_cast<size_t>(a->count) * n * 4, 0xffffffffu);
-    fill.add(ws + L.off_hist, cb2pg::sort_hist_ints(shape, n) * 4, 0u);
+    fill.add(ws + L.off_hist, cb2pg::kSortHistInts * shape.passes * 4, 0u);
     fill.run(dev, stream);
     const long long pairs = lists.first[a->count];
     if (pairs > 0) {

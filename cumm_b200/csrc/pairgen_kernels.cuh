@@ -29,6 +29,8 @@ struct Geometry {
   int grid[3];    // input grid (z, y, x)
   int ogrid[3];   // output grid
   int ksize[3], stride[3], pad[3], dil[3];
+  int period[3];  // stride / gcd(stride, dil): the offsets through which a cell feeds outputs are this far apart
+  int drop[3];    // dil / gcd(stride, dil): and those outputs this far
   int kv;
   int batch_size;
 };
@@ -47,32 +49,66 @@ __device__ __forceinline__ unsigned long long linear_key(int b, int z, int y, in
 }
 
 // ---------------------------------------------------------------- hash table: voxel -> smallest row
-// One 8-byte word per slot, (tag << 32) | row, all ones = empty: a lookup is one load where a key
-// array and a row array took two dependent ones.  While the grid has fewer than 2^32 cells the tag
-// IS the linearised voxel (`exact`); above, it is 32 bits of another hash of it and a match is
-// confirmed against the row's coordinates.
+// One 8-byte word per slot, (tag << 32) | row, all ones = empty; four slots of one 32-byte sector make
+// a bucket and are read together.  Four consecutive cells share a bucket, so that the three neighbours
+// of one (z, y) line are found in one sector or two.  A full bucket runs over into the next.  While the
+// grid has fewer than 2^32 cells the tag IS the linearised voxel (EXACT, all in 32 bits); above, it is
+// 32 bits of a hash of it and a match is confirmed against the row's coordinates.
+constexpr int kBucket = 4;
 struct HashView {
   unsigned long long *slots;
-  uint32_t cap_mask;
-  int exact;
+  uint32_t bucket_mask;  // buckets - 1
   const int32_t *coords;
 };
-
-__device__ __forceinline__ uint32_t hash_tag(const HashView &h, unsigned long long key) {
-  return h.exact ? static_cast<uint32_t>(key) : static_cast<uint32_t>((key * 0x9e3779b97f4a7c15ULL) >> 32);
-}
+template <bool EXACT> struct HashKey;
+template <> struct HashKey<true> {
+  using Key = uint32_t;
+  static __device__ __forceinline__ uint32_t bucket(const HashView &h, Key key) {
+    uint32_t k = key >> 2;
+    k = (k ^ (k >> 16)) * 0x85ebca6bu;
+    k = (k ^ (k >> 13)) * 0xc2b2ae35u;
+    return (k ^ (k >> 16)) & h.bucket_mask;
+  }
+  static __device__ __forceinline__ uint32_t tag(Key key) { return key; }
+};
+template <> struct HashKey<false> {
+  using Key = unsigned long long;
+  static __device__ __forceinline__ uint32_t bucket(const HashView &h, Key key) { return mix64(key >> 2) & h.bucket_mask; }
+  static __device__ __forceinline__ uint32_t tag(Key key) { return static_cast<uint32_t>((key * 0x9e3779b97f4a7c15ULL) >> 32); }
+};
+template <bool EXACT>
 __device__ __forceinline__ bool hash_match(const HashView &h, unsigned long long entry, uint32_t tag, int b, int z,
                                            int y, int x) {
-  if (static_cast<uint32_t>(entry >> 32) != tag)
+  if (entry == kEmptyKey || static_cast<uint32_t>(entry >> 32) != tag)
     return false;
-  if (h.exact)
+  if (EXACT)
     return true;
   const int4 c = __ldg(reinterpret_cast<const int4 *>(h.coords) + static_cast<uint32_t>(entry));
   return c.x == b && c.y == z && c.z == y && c.w == x;
 }
+struct BucketWords {
+  ulonglong2 lo, hi;
+};
+__device__ __forceinline__ BucketWords load_bucket(const HashView &h, uint32_t bucket) {
+  const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(h.slots + static_cast<size_t>(bucket) * kBucket);
+  return {__ldg(p), __ldg(p + 1)};
+}
+// row of the voxel among a bucket's entries, -1 = not there, -2 = the bucket is full: look in the next
+template <bool EXACT>
+__device__ __forceinline__ int find_in_bucket(const HashView &h, const BucketWords &w, uint32_t tag, int b, int z, int y,
+                                              int x) {
+  const unsigned long long e[kBucket] = {w.lo.x, w.lo.y, w.hi.x, w.hi.y};
+#pragma unroll
+  for (int i = 0; i < kBucket; ++i)
+    if (hash_match<EXACT>(h, e[i], tag, b, z, y, x))
+      return static_cast<int>(static_cast<uint32_t>(e[i]));
+  return e[kBucket - 1] == kEmptyKey ? -1 : -2;
+}
 
+template <bool EXACT>
 __global__ void __launch_bounds__(256) hash_insert_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                           HashView h, int *status) {
+  using HK = HashKey<EXACT>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
@@ -82,19 +118,22 @@ __global__ void __launch_bounds__(256) hash_insert_kernel(const int32_t *__restr
     atomicCAS(status, 0, kStatusBadCoord);
     return;
   }
-  const unsigned long long key = linear_key(c.x, c.y, c.z, c.w, g.grid);
-  const uint32_t tag = hash_tag(h, key);
+  const typename HK::Key key = static_cast<typename HK::Key>(linear_key(c.x, c.y, c.z, c.w, g.grid));
+  const uint32_t tag = HK::tag(key);
   const unsigned long long entry = (static_cast<unsigned long long>(tag) << 32) | static_cast<uint32_t>(i);
-  uint32_t slot = mix64(key) & h.cap_mask;
-  for (uint32_t probe = 0; probe <= h.cap_mask; ++probe) {
-    const unsigned long long prev = atomicCAS(h.slots + slot, kEmptyKey, entry);
-    if (prev == kEmptyKey)
-      return;
-    if (hash_match(h, prev, tag, c.x, c.y, c.z, c.w)) {
-      atomicMin(h.slots + slot, entry);  // duplicates resolve to the first row, as a stable sort + search does
-      return;
+  uint32_t bucket = HK::bucket(h, key);
+  for (uint32_t probe = 0; probe <= h.bucket_mask; ++probe) {
+    unsigned long long *slot = h.slots + static_cast<size_t>(bucket) * kBucket;
+    for (int q = 0; q < kBucket; ++q, ++slot) {
+      const unsigned long long prev = atomicCAS(slot, kEmptyKey, entry);
+      if (prev == kEmptyKey)
+        return;
+      if (hash_match<EXACT>(h, prev, tag, c.x, c.y, c.z, c.w)) {
+        atomicMin(slot, entry);  // duplicates resolve to the first row, as a stable sort + search does
+        return;
+      }
     }
-    slot = (slot + 1) & h.cap_mask;
+    bucket = (bucket + 1) & h.bucket_mask;
   }
   atomicCAS(status, 0, kStatusTableFull);
 }
@@ -182,10 +221,12 @@ __global__ void __launch_bounds__(256) decode_out_coords_kernel(const unsigned l
 // for the 27 offsets of a 3x3x3 kernel).  The rows are cut into at most kSortChunks equal chunks, one
 // CTA each.  hist[pass][chunk][digit] counts the digits of the chunk's rows as they stand BEFORE that
 // pass: the kernel that makes the masks fills pass 0, every pass fills the next one's counts while it
-// scatters, so a pass is one launch (it was three: count, scan, scatter).
+// scatters, so a pass is one launch (it was three: count, scan, scatter).  Chunks lie 2 KB apart: with a
+// digit's counts side by side the updates of all CTAs met in the same few lines (45 instead of 28 us).
 constexpr int kSortDigitBits = 9;
 constexpr int kSortBins = 1 << kSortDigitBits;
 constexpr int kSortChunks = 74;     // two sides (forward and backward tables) fill 148 SMs
+constexpr size_t kSortHistInts = static_cast<size_t>(kSortBins) * kSortChunks;  // of a pass
 constexpr int kSortThreads = kSortBins;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 8;       // rows per thread and round
@@ -207,9 +248,16 @@ inline int sort_chunk(long long n) {  // rows per chunk
   const long long c = (least + kProbeThreads - 1) / kProbeThreads * kProbeThreads;
   return static_cast<int>(c < 2048 ? 2048 : c);
 }
-inline size_t sort_hist_ints(const SortShape &s, long long n_max) {  // room for any n up to n_max
-  const long long chunks = (n_max + 2047) / 2048;
-  return static_cast<size_t>(s.passes) * (chunks < kSortChunks ? chunks : kSortChunks) * kSortBins;
+// The lanes that hold the same digit (of `width` bits; lanes outside `valid` are nobody's peers): a vote
+// per bit, which is faster than match.any.
+__device__ __forceinline__ unsigned digit_peers(uint32_t digit, int width, unsigned valid) {
+  unsigned peers = valid;
+  for (int b = 0; b < width; ++b) {
+    const bool bit = (digit >> b) & 1u;
+    const unsigned v = __ballot_sync(0xffffffffu, bit);
+    peers &= bit ? v : ~v;
+  }
+  return peers;
 }
 
 // Counts the first digit of one row per thread into the block's chunk (all threads of a block of
@@ -219,14 +267,15 @@ __device__ __forceinline__ void count_first_digit(int *s_hist, bool valid, uint3
   for (int d = threadIdx.x; d < kSortBins; d += blockDim.x)
     s_hist[d] = 0;
   __syncthreads();
-  const uint32_t digit = valid ? (low_word & ((1u << width) - 1u)) : 0xffffffffu;
-  const unsigned peers = __match_any_sync(0xffffffffu, digit);  // most rows of a sparse scene share one mask
+  const uint32_t digit = low_word & ((1u << width) - 1u);
+  // most rows of a sparse scene share one mask
+  const unsigned peers = digit_peers(digit, width, __ballot_sync(0xffffffffu, valid));
   if (valid && static_cast<int>(threadIdx.x & 31) == __ffs(peers) - 1)
     atomicAdd(&s_hist[digit], __popc(peers));
   __syncthreads();
   for (int d = threadIdx.x; d < kSortBins; d += blockDim.x)
     if (s_hist[d])
-      atomicAdd(hist + static_cast<long long>(chunk_index) * kSortBins + d, s_hist[d]);
+      atomicAdd(hist + chunk_index * kSortBins + d, s_hist[d]);
   __syncthreads();
 }
 
@@ -240,17 +289,18 @@ struct MaskSide {
 
 // ---------------------------------------------------------------- indices[f, o] and masks
 // One thread per output voxel; consecutive threads write consecutive columns of every row of the
-// table.  Lookups are issued nine at a time: their first loads are in flight together, so a thread
-// waits for ceil(kv / 9) memory round trips instead of kv.
+// table.  Lookups are issued three at a time, so that their loads are in flight together.
 // `mirror` (submanifold convolutions whose offsets are symmetric): o' is o's neighbour at offset f
 // exactly if o is o's neighbour at offset kv - 1 - f, so the backward table is the forward one with
 // the offsets reversed and is written by the same thread.  A row that repeats another row's voxel
 // has no backward neighbours (nothing points at it).
-template <int NW>
+template <int NW, bool EXACT>
 __global__ void __launch_bounds__(kProbeThreads, 4) probe_kernel(const int32_t *__restrict__ out_coords, Geometry g,
                                                               const HashView h, const MaskSide side,
                                                               const MaskSide mirror, int words, int width) {
-  constexpr int B = 9;
+  constexpr int B = 3;
+  using HK = HashKey<EXACT>;
+  using Key = typename HK::Key;
   __shared__ int s_hist[kSortBins];
   const int o = blockIdx.x * kProbeThreads + threadIdx.x;
   const bool valid = o < side.n;
@@ -262,22 +312,25 @@ __global__ void __launch_bounds__(kProbeThreads, 4) probe_kernel(const int32_t *
   if (valid) {
     const int4 c = __ldg(reinterpret_cast<const int4 *>(out_coords) + o);
     const int z0 = c.y * g.stride[0] - g.pad[0], y0 = c.z * g.stride[1] - g.pad[1], x0 = c.w * g.stride[2] - g.pad[2];
+    // linear index of offset 0's cell; modulo the word where that cell lies outside, which is never looked up
+    const Key line = (static_cast<Key>(c.x) * g.grid[0] + z0) * g.grid[1] + y0;
     int rz = 0, ry = 0, rx = 0;
     bool repeats = false;
     for (int f0 = 0; f0 < g.kv; f0 += B) {
-      unsigned long long entry[B];
-      uint32_t slot[B], tag[B];
+      BucketWords found[B];
+      uint32_t bucket[B], tag[B];
+      bool in[B];
 #pragma unroll
       for (int j = 0; j < B; ++j) {
-        entry[j] = kEmptyKey;
-        slot[j] = tag[j] = 0u;
         const int z = z0 + rz * g.dil[0], y = y0 + ry * g.dil[1], x = x0 + rx * g.dil[2];
-        if (f0 + j < g.kv && z >= 0 && z < g.grid[0] && y >= 0 && y < g.grid[1] && x >= 0 && x < g.grid[2]) {
-          const unsigned long long key = linear_key(c.x, z, y, x, g.grid);
-          slot[j] = mix64(key) & h.cap_mask;
-          tag[j] = hash_tag(h, key);
-          entry[j] = __ldg(h.slots + slot[j]);
-        }
+        in[j] = f0 + j < g.kv && z >= 0 && z < g.grid[0] && y >= 0 && y < g.grid[1] && x >= 0 && x < g.grid[2];
+        const Key key = (line + static_cast<Key>(rz * g.dil[0]) * g.grid[1] + ry * g.dil[1]) * g.grid[2] + x;
+        bucket[j] = in[j] ? HK::bucket(h, key) : 0u;
+        tag[j] = HK::tag(key);
+        if (j > 0 && bucket[j] == bucket[j - 1])
+          found[j] = found[j - 1];
+        else
+          found[j] = load_bucket(h, bucket[j]);
         if (++rx == g.ksize[2]) {
           rx = 0;
           if (++ry == g.ksize[1]) {
@@ -291,17 +344,18 @@ __global__ void __launch_bounds__(kProbeThreads, 4) probe_kernel(const int32_t *
         const int f = f0 + j;
         if (f < g.kv) {
           int idx = -1;
-          unsigned long long e = entry[j];
-          uint32_t s = slot[j];
-          for (uint32_t probe = 0; probe <= h.cap_mask && e != kEmptyKey; ++probe) {
-            const int xy = g.ksize[1] * g.ksize[2];
-            if (hash_match(h, e, tag[j], c.x, z0 + f / xy * g.dil[0], y0 + f % xy / g.ksize[2] * g.dil[1],
-                           x0 + f % g.ksize[2] * g.dil[2])) {
-              idx = static_cast<int>(static_cast<uint32_t>(e));
-              break;
+          if (in[j]) {
+            int z = 0, y = 0, x = 0;
+            if (!EXACT) {
+              const int xy = g.ksize[1] * g.ksize[2];
+              z = z0 + f / xy * g.dil[0], y = y0 + f % xy / g.ksize[2] * g.dil[1], x = x0 + f % g.ksize[2] * g.dil[2];
             }
-            s = (s + 1) & h.cap_mask;
-            e = __ldg(h.slots + s);
+            idx = find_in_bucket<EXACT>(h, found[j], tag[j], c.x, z, y, x);
+            for (uint32_t probe = 0; idx == -2 && probe < h.bucket_mask; ++probe) {
+              bucket[j] = (bucket[j] + 1) & h.bucket_mask;
+              idx = find_in_bucket<EXACT>(h, load_bucket(h, bucket[j]), tag[j], c.x, z, y, x);
+            }
+            idx = max(idx, -1);
           }
           side.indices[static_cast<long long>(f) * side.n + o] = idx;
 #pragma unroll
@@ -396,61 +450,80 @@ struct FillRanges {
   uint32_t value[6];
   int count;
 };
-__global__ void __launch_bounds__(256) fill_kernel(const FillRanges r) {
+__global__ void __launch_bounds__(256) fill_kernel(const __grid_constant__ FillRanges r) {  // one grid row per range
   const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (int k = 0; k < r.count; ++k) {
-    const uint32_t v = r.value[k];
-    const long long head = min(r.words[k], static_cast<long long>((16u - (reinterpret_cast<uintptr_t>(r.ptr[k]) & 15u)) & 15u) / 4);
-    const long long n4 = (r.words[k] - head) / 4, tail = r.words[k] - head - 4 * n4;
-    uint4 *p4 = reinterpret_cast<uint4 *>(r.ptr[k] + head);
-    for (long long i = first; i < n4; i += step)
-      p4[i] = make_uint4(v, v, v, v);
-    if (first < head)
-      r.ptr[k][first] = v;
-    if (first < tail)
-      r.ptr[k][head + 4 * n4 + first] = v;
+  uint32_t *ptr = r.ptr[blockIdx.y];
+  const long long words = r.words[blockIdx.y];
+  const uint32_t v = r.value[blockIdx.y];
+  const long long head = min(words, static_cast<long long>((16u - (reinterpret_cast<uintptr_t>(ptr) & 15u)) & 15u) / 4);
+  const long long n4 = (words - head) / 4, tail = words - head - 4 * n4;
+  uint4 *p4 = reinterpret_cast<uint4 *>(ptr + head);
+#pragma unroll 4
+  for (long long i = first; i < n4; i += step)
+    p4[i] = make_uint4(v, v, v, v);
+  if (first < head)
+    ptr[first] = v;
+  if (first < tail)
+    ptr[head + 4 * n4 + first] = v;
+}
+
+// The outputs that read a cell, one axis: through offsets r, r + period, ... at positions p, p - drop, ...
+// Every lane walks its own offsets (two or fewer per axis for a 3x3x3 kernel of stride 2), where a loop
+// over all offsets would run each of them for the whole warp.
+struct AxisWalk {
+  int r, p;
+};
+__device__ __forceinline__ AxisWalk first_output(const Geometry &g, int axis, int at) {
+  AxisWalk w = {0, 0};
+  for (; w.r < g.period[axis]; ++w.r) {
+    const int num = at + g.pad[axis] - w.r * g.dil[axis];
+    w.p = num / g.stride[axis];
+    if (w.p * g.stride[axis] == num)
+      return w;
+  }
+  w.r = g.ksize[axis];  // none
+  return w;
+}
+// fn(f, cell) for every output cell the voxel feeds and the offset it feeds it through
+template <class Fn> __device__ __forceinline__ void for_each_output(const Geometry &g, const int4 &c, Fn fn) {
+  const AxisWalk wz = first_output(g, 0, c.y), wy = first_output(g, 1, c.z), wx = first_output(g, 2, c.w);
+  for (int rz = wz.r, oz = wz.p; rz < g.ksize[0]; rz += g.period[0], oz -= g.drop[0]) {
+    if (oz < 0 || oz >= g.ogrid[0])
+      continue;
+    for (int ry = wy.r, oy = wy.p; ry < g.ksize[1]; ry += g.period[1], oy -= g.drop[1]) {
+      if (oy < 0 || oy >= g.ogrid[1])
+        continue;
+      const uint32_t line = static_cast<uint32_t>((c.x * g.ogrid[0] + oz) * g.ogrid[1] + oy) * g.ogrid[2];
+      for (int rx = wx.r, ox = wx.p; rx < g.ksize[2]; rx += g.period[2], ox -= g.drop[2])
+        if (ox >= 0 && ox < g.ogrid[2])
+          fn((rz * g.ksize[1] + ry) * g.ksize[2] + rx, line + ox);
+    }
   }
 }
-
-// Output positions that read input coordinate `at` along one axis through offset r: at + pad - r * dil
-// divided by the stride, or -1.
-__device__ __forceinline__ int out_position(const Geometry &g, int axis, int at, int r) {
-  const int num = at + g.pad[axis] - r * g.dil[axis];
-  if (num < 0 || num % g.stride[axis] != 0)
-    return -1;
-  const int p = num / g.stride[axis];
-  return p < g.ogrid[axis] ? p : -1;
+__device__ __forceinline__ bool inside(const Geometry &g, const int4 &c) {
+  return c.x >= 0 && c.x < g.batch_size && c.y >= 0 && c.y < g.grid[0] && c.z >= 0 && c.z < g.grid[1] && c.w >= 0 &&
+         c.w < g.grid[2];
 }
 
-// One thread per (input voxel, rz, ry); bits of one word set together.
-__global__ void __launch_bounds__(256) bitmap_mark_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
+// One thread per input voxel; bits of one word set together.
+__global__ void __launch_bounds__(128) bitmap_mark_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                           uint32_t *words) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int planes = g.ksize[0] * g.ksize[1];
-  const int i = static_cast<int>(t / planes), zy = static_cast<int>(t % planes);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
   const int4 c = __ldg(reinterpret_cast<const int4 *>(coords) + i);
   if (c.x < 0 || c.x >= g.batch_size)
     return;  // reported with the other bad coordinates when the tables are filled
-  const int oz = out_position(g, 0, c.y, zy / g.ksize[1]), oy = out_position(g, 1, c.z, zy % g.ksize[1]);
-  if (oz < 0 || oy < 0)
-    return;
-  const uint32_t line = static_cast<uint32_t>(linear_key(c.x, oz, oy, 0, g.ogrid));
   uint32_t word = 0, bits = 0;
-  for (int rx = 0; rx < g.ksize[2]; ++rx) {
-    const int ox = out_position(g, 2, c.w, rx);
-    if (ox < 0)
-      continue;
-    const uint32_t cell = line + ox;
+  for_each_output(g, c, [&](int, uint32_t cell) {
     if (bits && (cell >> 5) != word) {
       atomicOr(words + word, bits);
       bits = 0;
     }
     word = cell >> 5;
     bits |= 1u << (cell & 31);
-  }
+  });
   if (bits)
     atomicOr(words + word, bits);
 }
@@ -553,38 +626,28 @@ __global__ void __launch_bounds__(256) bitmap_coords_kernel(const Bitmap bm, int
 
 // indices[f, o] = i and bit f of row o's mask for every output o that reads input i through f.  The table
 // and the masks start as -1 and 0; of several rows with one voxel the smallest wins.
-__global__ void __launch_bounds__(256) bitmap_scatter_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
+__global__ void __launch_bounds__(128) bitmap_scatter_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                              const Bitmap bm, const MaskSide out, int words, int *status) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int planes = g.ksize[0] * g.ksize[1];
-  const int i = static_cast<int>(t / planes), zy = static_cast<int>(t % planes);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
   const int4 c = __ldg(reinterpret_cast<const int4 *>(coords) + i);
-  if (c.x < 0 || c.x >= g.batch_size || c.y < 0 || c.y >= g.grid[0] || c.z < 0 || c.z >= g.grid[1] || c.w < 0 ||
-      c.w >= g.grid[2]) {
+  if (!inside(g, c)) {
     atomicCAS(status, 0, kStatusBadCoord);
     return;
   }
-  const int oz = out_position(g, 0, c.y, zy / g.ksize[1]), oy = out_position(g, 1, c.z, zy % g.ksize[1]);
-  if (oz < 0 || oy < 0)
-    return;
-  const uint32_t line = static_cast<uint32_t>(linear_key(c.x, oz, oy, 0, g.ogrid));
-  for (int rx = 0; rx < g.ksize[2]; ++rx) {
-    const int ox = out_position(g, 2, c.w, rx);
-    if (ox < 0)
-      continue;
-    const int o = bitmap_rank(bm, line + ox);
-    if (o >= out.n)
-      continue;
-    const int f = zy * g.ksize[2] + rx;
-    atomicMin(reinterpret_cast<uint32_t *>(out.indices) + static_cast<long long>(f) * out.n + o, static_cast<uint32_t>(i));
-    atomicOr(out.rows + static_cast<long long>(o) * words + (f >> 5), 1u << (f & 31));
-  }
+  for_each_output(g, c, [&](int f, uint32_t cell) {
+    const int o = bitmap_rank(bm, cell);
+    if (o < out.n) {
+      atomicMin(reinterpret_cast<uint32_t *>(out.indices) + static_cast<long long>(f) * out.n + o, static_cast<uint32_t>(i));
+      atomicOr(out.rows + static_cast<long long>(o) * words + (f >> 5), 1u << (f & 31));
+    }
+  });
 }
 
-// Blocks below `bwd_blocks`: the backward table, indices_bwd[f, i] = o where indices[f, o] = i, and its
-// masks.  The other blocks: first-digit counts of the forward masks that the scatter finished.
+// Blocks below `bwd_blocks`: the backward table, indices_bwd[f, i] = o where indices[f, o] = i (-1
+// before), and its masks.  The other blocks: first-digit counts of the forward masks that the scatter
+// finished.
 template <int NW>
 __global__ void __launch_bounds__(kProbeThreads) bitmap_backward_kernel(const int32_t *__restrict__ coords, Geometry g,
                                                                         const Bitmap bm, const MaskSide out,
@@ -607,29 +670,17 @@ __global__ void __launch_bounds__(kProbeThreads) bitmap_backward_kernel(const in
     m[w] = 0u;
   if (valid) {
     const int4 c = __ldg(reinterpret_cast<const int4 *>(coords) + i);
-    const bool ok = c.x >= 0 && c.x < g.batch_size && c.y >= 0 && c.y < g.grid[0] && c.z >= 0 && c.z < g.grid[1] &&
-                    c.w >= 0 && c.w < g.grid[2];
-    int f = 0;
-    for (int rz = 0; rz < g.ksize[0]; ++rz) {
-      const int oz = ok ? out_position(g, 0, c.y, rz) : -1;
-      for (int ry = 0; ry < g.ksize[1]; ++ry) {
-        const int oy = oz >= 0 ? out_position(g, 1, c.z, ry) : -1;
-        for (int rx = 0; rx < g.ksize[2]; ++rx, ++f) {
-          const int ox = oy >= 0 ? out_position(g, 2, c.w, rx) : -1;
-          int found = -1;
-          if (ox >= 0) {
-            const int o = bitmap_rank(bm, static_cast<uint32_t>(linear_key(c.x, oz, oy, ox, g.ogrid)));
-            if (o < out.n && __ldg(out.indices + static_cast<long long>(f) * out.n + o) == i)
-              found = o;
-          }
-          in.indices[static_cast<long long>(f) * in.n + i] = found;
+    if (inside(g, c))
+      for_each_output(g, c, [&](int f, uint32_t cell) {
+        const int o = bitmap_rank(bm, cell);
+        if (o < out.n && __ldg(out.indices + static_cast<long long>(f) * out.n + o) == i) {
+          in.indices[static_cast<long long>(f) * in.n + i] = o;
 #pragma unroll
           for (int w = 0; w < NW; ++w)
-            if (found >= 0 && (NW == 1 || (f >> 5) == w))
+            if (NW == 1 || (f >> 5) == w)
               m[w] |= 1u << (f & 31);
         }
-      }
-    }
+      });
 #pragma unroll
     for (int w = 0; w < NW; ++w)
       if (w < words)
@@ -654,7 +705,8 @@ struct SortSides {
   SortSide side[2];
 };
 template <bool WIDE>
-__global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const SortSides sides, int pass, const SortShape shape) {
+__global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_constant__ SortSides sides, int pass,
+                                                                 const SortShape shape) {
   const SortSide &s = sides.side[blockIdx.y];
   __shared__ int s_cnt[kSortWarps][kSortBins];
   __shared__ int s_base[kSortBins];
@@ -665,11 +717,16 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const SortSides
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   // where this chunk's rows of digit t go: rows with smaller digits, then those of earlier chunks
   int before = 0, all = 0;
-#pragma unroll 16
-  for (int c = 0; c < s.n_chunks; ++c) {
-    const int v = __ldg(s.hist + c * kSortBins + t);
-    all += v;
-    before += c < me ? v : 0;
+  for (int c0 = 0; c0 < s.n_chunks; c0 += 25) {  // 25 loads in flight: one after the other they were most of a pass
+    int v[25];
+#pragma unroll
+    for (int i = 0; i < 25; ++i)
+      v[i] = c0 + i < s.n_chunks ? __ldg(s.hist + (c0 + i) * kSortBins + t) : 0;
+#pragma unroll
+    for (int i = 0; i < 25; ++i) {
+      all += v[i];
+      before += c0 + i < me ? v[i] : 0;
+    }
   }
   int total;
   s_base[t] = block_scan_512(all, s_warp, total) + before;
@@ -704,7 +761,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const SortSides
     }
 #pragma unroll
     for (int it = 0; it < kSortItems; ++it) {
-      digit[it] = 0xffffffffu;
+      digit[it] = 0u;
       if (val[it] >= 0)
         digit[it] = WIDE ? wide_digit(val[it], bit0, digit_mask) : ((key[it] >> bit0) & digit_mask);
     }
@@ -712,7 +769,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const SortSides
     // rank inside the warp's 32 * kSortItems consecutive rows, in their order
 #pragma unroll
     for (int it = 0; it < kSortItems; ++it) {
-      const unsigned peers = __match_any_sync(0xffffffffu, digit[it]);
+      const unsigned peers = digit_peers(digit[it], shape.width, __ballot_sync(0xffffffffu, val[it] >= 0));
       rank[it] = 0;
       if (val[it] >= 0)
         rank[it] = s_cnt[warp][digit[it]] + __popc(peers & ((1u << lane) - 1u));
@@ -746,19 +803,29 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const SortSides
           const uint32_t next = WIDE ? wide_digit(val[it], bit1, next_mask) : ((key[it] >> bit1) & next_mask);
           where = static_cast<uint32_t>(pos / s.chunk) * kSortBins + next;
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, where);
-        if (valid && lane == __ffs(peers) - 1)
-          atomicAdd(s.hist_next + where, __popc(peers));
-      } else if (valid) {
-        if (WIDE) {
-          for (int w = 0; w < shape.words; ++w) {
-            const uint32_t m = __ldg(s.rows + static_cast<long long>(val[it]) * shape.words + w);
+        // Most rows of a sparse scene share one mask and stay together: the lanes that agree with the
+        // first one are counted in one update.
+        const uint32_t where0 = __shfl_sync(0xffffffffu, where, 0);
+        const unsigned agree = __ballot_sync(0xffffffffu, where == where0);
+        if (lane == 0 && valid)
+          atomicAdd(s.hist_next + where, __popc(agree));
+        else if (valid && where != where0)
+          atomicAdd(s.hist_next + where, 1);
+      } else {
+        const int run = valid ? pos >> 7 : -1;  // the same for tile masks
+        const int run0 = __shfl_sync(0xffffffffu, run, 0);
+        const bool agrees = valid && run == run0;
+        for (int w = 0; w < (WIDE ? shape.words : 1); ++w) {
+          uint32_t m = key[it];
+          if (WIDE && valid) {
+            m = __ldg(s.rows + static_cast<long long>(val[it]) * shape.words + w);
             s.kout[static_cast<long long>(pos) * shape.words + w] = m;
-            if (s.tile_masks)
-              atomicOr(s.tile_masks + static_cast<long long>(pos >> 7) * shape.words + w, m);
           }
-        } else if (s.tile_masks) {
-          atomicOr(s.tile_masks + (pos >> 7), key[it]);
+          if (s.tile_masks) {
+            const uint32_t any = __reduce_or_sync(0xffffffffu, agrees ? m : 0u);
+            if (valid && (lane == 0 || !agrees))
+              atomicOr(s.tile_masks + static_cast<long long>(run) * shape.words + w, lane == 0 ? any : m);
+          }
         }
       }
     }

@@ -63,7 +63,7 @@ def build_tables_gpu(in_coords, batch_size: int, grid: Sequence[int], ksize=(3, 
             mbwd = torch.empty((n_in,) + wide, dtype=torch.int32, device=dev)
             abwd = torch.empty((n_in,), dtype=torch.int32, device=dev)
             a.indices_bwd, a.mask_bwd, a.mask_argsort_bwd = ibwd.data_ptr(), mbwd.data_ptr(), abwd.data_ptr()
-        mask_output = torch.zeros(((n_out + 127) // 128,) + wide, dtype=torch.int32, device=dev)
+        mask_output = torch.empty(((n_out + 127) // 128,) + wide, dtype=torch.int32, device=dev)
         a.tile_masks = mask_output.data_ptr()
         _lib.raise_for(L.cb2_pairgen_run(ctypes.byref(a), ctypes.c_void_p(stream)))
     # the kernels enqueued above still read the workspace: it lives as long as the tables do
