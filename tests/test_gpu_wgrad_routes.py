@@ -75,6 +75,16 @@ def test_weight_gradient_in_scratch_of_either_size(torch):
         H.check_status()
         assert torch.equal(dw, results[0])
     assert torch.equal(results[0], results[1])
+    # a plan in a large workspace is reused as what it is: tiles then lists allowed, and the other way round
+    for first, then in ((0, 1 | _lib.CB2_PLAN_ROW_LISTS), (_lib.CB2_PLAN_ROW_LISTS, 1)):
+        args = _conv_args(p)
+        args.workspace, args.workspace_bytes = p.workspace.data_ptr(), p.workspace.numel()
+        for args.reuse_plan in (first, then):
+            p.weight.zero_()
+            _lib.raise_for(_lib.load().cb2_conv_run(ctypes.byref(args), None))
+            torch.cuda.synchronize()
+            H.check_status()
+            assert torch.equal(p.weight, dw)
     want = torch.zeros((27, K, C), dtype=torch.float64)
     for f in range(27):
         o = torch.nonzero(t.indices[f] >= 0).flatten().cpu()
