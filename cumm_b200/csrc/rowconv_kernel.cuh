@@ -5,7 +5,7 @@
 // for every filter offset present in the tile's OR-ed neighbour mask it gathers the 128
 // operand rows into a 128-byte-swizzled shared-memory tile (TMA tile::gather4 for rows of up
 // to 128 bytes, 16-byte cp.async for wider ones; missing neighbours read as zeros), brings the
-// matching weight slice in by TMA, and one thread issues tcgen05.mma into a TMEM accumulator.
+// matching weight slice in by TMA, and one warp issues tcgen05.mma into a TMEM accumulator.
 // Eight (fp16) or sixteen (int8) epilogue warps read the accumulator back, apply
 // alpha/beta/bias/activation (or the int8 requantisation) and write the rows to their scattered
 // destinations, whole 32-byte sectors per thread.  No atomics on data: every
@@ -74,7 +74,7 @@ struct RowConvParams {
 #define CB2_ROWCONV_NARROW_STAGES 6
 #endif
 #ifndef CB2_ROWCONV_WIDE_STAGES
-#define CB2_ROWCONV_WIDE_STAGES 3
+#define CB2_ROWCONV_WIDE_STAGES 4
 #endif
 #ifndef CB2_ROWCONV_EPI_PARTS
 #define CB2_ROWCONV_EPI_PARTS 4
@@ -92,10 +92,14 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int UMMA_K = 32 / ES;
   static constexpr int KRED = NATOM_K * ATOM_ELEMS;       // reduction elements per stage
   static constexpr int TILE_M = 128;
-  // A stages == producer groups.  The kernel with sixteen epilogue warps keeps to 24 warps: six per
+  // A stages == producer groups.  What bounds a step is not the bytes of a stage but how many steps are
+  // on their way, so narrow rows have six stages (three: 229 us, six: 218 us for a training step of a
+  // scanned scene at 64 channels, before the issuer was the limit) and wide fp16 rows four, which is
+  // what the shared memory holds (three: 150, four: 132 us for 60 000 rows at 256 channels).  The kernel with sixteen epilogue warps keeps to 24 warps: six per
   // SM sub-partition leave 80 registers per thread, seven would leave 72 and spill.
   static constexpr int SA =
-      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES) : CB2_ROWCONV_WIDE_STAGES;
+      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES)
+                                 : (KIND == 0 ? CB2_ROWCONV_WIDE_STAGES : 3);
   static constexpr int A_STAGE_BYTES = TILE_M * 128 * NATOM_K;
   static constexpr int B_SLOT_BYTES = BLOCK_N * 128 * NATOM_K;
   static constexpr int MW = MASK_WORDS;
@@ -121,13 +125,17 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // many warps each SM sub-partition can switch between, not by arithmetic throughput.
   static constexpr int EPI_HALVES = (KIND == 1 && BLOCK_N >= 128) ? CB2_ROWCONV_EPI_PARTS : 2;
   static constexpr int EPI_THREADS = 128 * EPI_HALVES;
+  // Groups of epilogue warps that take turns at the tiles: a requantised tile is a long chain per warp
+  // (read, convert, scale, convert, pack, store), and two tiles on their way at once fill its gaps
+  // (stride-2 int8 layer, 3839 tiles: 43.7 -> 42.1 us).
+  static constexpr int EPI_GROUPS = (KIND == 1 && BLOCK_N >= 128) ? 2 : 1;
   static constexpr int GROUP_THREADS = TMA_GATHER ? 32 : CB2_ROWCONV_GROUP_THREADS;
   static constexpr int FULL_A_COUNT = TMA_GATHER ? 1 : GROUP_THREADS;
   static constexpr int MMA_WARP = EPI_THREADS / 32;
   static constexpr int TMA_WARP = MMA_WARP + 1;
   static constexpr int FIRST_GATHER_WARP = TMA_WARP + 1;
   static constexpr int SCHED_WARP = FIRST_GATHER_WARP + SA * GROUP_THREADS / 32;  // the last warp hands out tiles
-  static constexpr int THREADS = (SCHED_WARP + 1) * 32;   // 544
+  static constexpr int THREADS = (SCHED_WARP + 1) * 32;
   static constexpr int RING_CONSUMER_WARPS = SCHED_WARP;   // every warp but the scheduler
   // shared memory map (offsets from a 1024-byte aligned base)
   static constexpr int OFF_A = 0;
@@ -229,11 +237,12 @@ __device__ __forceinline__ int ring_tile_masks(const RowConvParams &p, const int
 
 // Walks the tiles the scheduler publishes; every consumer warp of the CTA has one and runs the
 // identical walk, so their step counters agree.  next() reads a tile's header into registers, the same
-// in every lane, lets the role read its rows and gives the slot back at once; the role loops over the
-// tile's (filter offset, reduction pass) steps itself.  A walk that called a function per step, run by one
+// in every lane, lets the role read its rows and gives the slot back at once (the MMA issuer when it
+// has issued the tile: a slot stands for work not done yet, by which the scheduler decides whether
+// this CTA may draw more); the role loops over the tile's (filter offset, reduction pass) steps itself.  A walk that called a function per step, run by one
 // thread, had the MMA issuer at 1500 cycles per step (walk 360, waits 500, four MMAs 260, commits 130),
 // which paced every tile with several offsets.
-template <int MW> struct TileCursor {
+template <int MW, bool HOLD = false> struct TileCursor {
   static_assert(MW == 1 || MW == 4, "one mask word, or four");
   int slot = 0;
   uint32_t phase = 0;
@@ -274,6 +283,11 @@ template <int MW> struct TileCursor {
       offsets = __popcll(lo) + __popcll(hi);
     }
     read(sl);
+    if (!HOLD || tile < 0)
+      release(rv);
+    return tile >= 0 ? 1 : 0;
+  }
+  __device__ __forceinline__ void release(const RingView &rv) {
     __syncwarp();
     if (lane_id() == 0)
       mbar_arrive(rv.empty0 + 8u * slot);
@@ -281,7 +295,6 @@ template <int MW> struct TileCursor {
       slot = 0;
       phase ^= 1u;
     }
-    return tile >= 0 ? 1 : 0;
   }
   __device__ __forceinline__ int first_offset() const {
     if constexpr (MW == 1)
@@ -584,7 +597,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     }
     for (int s = 0; s < Cfg::NUM_ACC; ++s) {
       mbar_init(acc_full(s), 1);
-      mbar_init(acc_empty(s), Cfg::EPI_THREADS / 32);
+      mbar_init(acc_empty(s), Cfg::EPI_THREADS / 32 / Cfg::EPI_GROUPS);
     }
     mbar_init(final_bar, 1);
     for (int s = 0; s < Cfg::RING; ++s) {
@@ -641,12 +654,21 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     // of all epilogue warps into every tile.)
     const int et = threadIdx.x;
     const int erow = et & 127;   // the tile row this thread reads from TMEM (lane quarter = warp & 3)
-    const int half = et >> 7;    // which share of the columns
-    constexpr int COLS_PER_HALF = BLOCK_N / Cfg::EPI_HALVES;
+    constexpr int HALVES = Cfg::EPI_HALVES / Cfg::EPI_GROUPS;
+    const int half = (et >> 7) % HALVES;   // which share of the columns
+    const int group = (et >> 7) / HALVES;  // which of the tiles with work
+    int turn = 0;
+    constexpr int COLS_PER_HALF = BLOCK_N / HALVES;
     const bool sectors = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(p.ldo * Cfg::OES)) & 31u) == 0;
     int buf = 0;
     uint32_t acc_phase = 0;
     bool dep_waited = false;
+    auto next_acc = [&]() {
+      if (++buf == Cfg::NUM_ACC) {
+        buf = 0;
+        acc_phase ^= 1u;
+      }
+    };
     CB2_PROF_BEGIN();
     TileCursor<MW> tc;
     int o = -1;  // destination row of this thread's tile row
@@ -657,13 +679,22 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           const bool has_work = tc.offsets != 0;
           if (!has_work && p.skip_empty_tiles)
             continue;
+          if (Cfg::EPI_GROUPS > 1) {
+            const bool mine = turn == group;
+            turn = turn + 1 == Cfg::EPI_GROUPS ? 0 : turn + 1;
+            if (!mine) {
+              if (has_work)
+                next_acc();
+              continue;
+            }
+          }
           const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
           CB2_PROF_MARK(0);  // walk
           if (!dep_waited) {
             grid_dep_wait();
             dep_waited = true;
           }
-          if (et == 0 && p.mask_out && n0 == 0) {
+          if (erow == 0 && half == 0 && p.mask_out && n0 == 0) {
             if constexpr (MW == 1) {
               p.mask_out[tile] = tc.m;  // forward: not reversed
             } else {
@@ -838,10 +869,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             }
           }
           CB2_PROF_MARK(3);  // TMEM -> rows
-          if (has_work && ++buf == Cfg::NUM_ACC) {
-            buf = 0;
-            acc_phase ^= 1u;
-          }
+          if (has_work)
+            next_acc();
           if (et == 0)
             CB2_TRACE_EVENT(4, 9, tile);  // rows stored
     }
@@ -856,7 +885,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     const uint64_t bdesc_base = B_MN ? make_smem_desc(sbase + Cfg::OFF_B, p.b_lbo, p.b_sbo)
                                      : make_smem_desc(sbase + Cfg::OFF_B, 16, 1024);
     const int ksteps_last = (p.red - (kpasses - 1) * Cfg::KRED + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
-    TileCursor<MW> tc;
+    TileCursor<MW, true> tc;
     int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
     uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
     bool ok = true;
@@ -867,8 +896,10 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         ok = false;
         break;
       }
-      if (tc.offsets == 0)
+      if (tc.offsets == 0) {
+        tc.release(rv);
         continue;
+      }
       // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
       // are in the key: weights have as many columns)
       bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
@@ -937,6 +968,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         new_b = true;
         ++steps;
       }
+      tc.release(rv);
       last_key = (tc.last_offset() * kpasses + kpasses - 1) * p.nn + tc.n0;
       if (++buf == Cfg::NUM_ACC) {
         buf = 0;
