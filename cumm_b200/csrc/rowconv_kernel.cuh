@@ -108,6 +108,11 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr bool PARTS = KIND == 0;
   static constexpr int RING = MASK_WORDS == 1 ? CB2_ROWCONV_RING : CB2_ROWCONV_RING / 2;  // tile ring slots
   static constexpr int RING_SLOT_INTS = 136 + 128 * MASK_WORDS;  // header; 128 gather rows; 128 output rows / row masks
+  // int8 rows of up to 128 bytes: a stage holds the step's weight tile beside its rows, under the same pair
+  // of barriers -- one wait and one commit per step for the issuer (46.7 -> 43.7 us for the stride-2
+  // layer; the weights of a run of tiles with the same offset come from L2 each time).  fp16 keeps slots
+  // of their own: there it lost (135 -> 144 us for the scanned scene's step).
+  static constexpr bool JOINT = KIND == 1 && TMA_GATHER && NATOM_K == 1;
   // mbarriers: operand stages, accumulators, the final one, weight slots, tile ring
   static constexpr int BAR_EMPTY_A = SA, BAR_ACC_FULL = 2 * SA, BAR_ACC_EMPTY = BAR_ACC_FULL + 2,
                        BAR_FINAL = BAR_ACC_EMPTY + 2, BAR_FULL_B = BAR_FINAL + 1, BAR_EMPTY_B = BAR_FULL_B + 6,
@@ -117,7 +122,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + SA * 2 * 128 * 4 +
                                      2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (BAR_RING + 3 * RING) * 8 + 64 + 1024;
   static constexpr int SB_FIT = (232448 - FIXED_BYTES) / B_SLOT_BYTES;
-  static constexpr int SB = SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
+  static constexpr int SB = JOINT ? SA : SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
   static constexpr int NUM_ACC = 2;                       // TMEM accumulators: one fills while one drains
   static constexpr int TMEM_COLS = NUM_ACC * BLOCK_N;     // 128 or 256: power of two >= 32
   // Epilogue: several threads per tile row, each converting its share of the columns.  The
@@ -130,7 +135,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // (stride-2 int8 layer, 3839 tiles: 43.7 -> 42.1 us).
   static constexpr int EPI_GROUPS = (KIND == 1 && BLOCK_N >= 128) ? 2 : 1;
   static constexpr int GROUP_THREADS = TMA_GATHER ? 32 : CB2_ROWCONV_GROUP_THREADS;
-  static constexpr int FULL_A_COUNT = TMA_GATHER ? 1 : GROUP_THREADS;
+  static constexpr int FULL_A_COUNT = JOINT ? 2 : TMA_GATHER ? 1 : GROUP_THREADS;
   static constexpr int MMA_WARP = EPI_THREADS / 32;
   static constexpr int TMA_WARP = MMA_WARP + 1;
   static constexpr int FIRST_GATHER_WARP = TMA_WARP + 1;
@@ -237,12 +242,13 @@ __device__ __forceinline__ int ring_tile_masks(const RowConvParams &p, const int
 
 // Walks the tiles the scheduler publishes; every consumer warp of the CTA has one and runs the
 // identical walk, so their step counters agree.  next() reads a tile's header into registers, the same
-// in every lane, lets the role read its rows and gives the slot back at once (the MMA issuer when it
-// has issued the tile: a slot stands for work not done yet, by which the scheduler decides whether
-// this CTA may draw more); the role loops over the tile's (filter offset, reduction pass) steps itself.  A walk that called a function per step, run by one
+// in every lane, lets the role read its rows and gives the slot back at once; the role loops over the
+// tile's (filter offset, reduction pass) steps itself.  (With slots held until a tile has been issued
+// the look-ahead was too short for tiles with many offsets: 148 instead of 135 us for a training step of
+// a scanned scene at 64 channels.)  A walk that called a function per step, run by one
 // thread, had the MMA issuer at 1500 cycles per step (walk 360, waits 500, four MMAs 260, commits 130),
 // which paced every tile with several offsets.
-template <int MW, bool HOLD = false> struct TileCursor {
+template <int MW> struct TileCursor {
   static_assert(MW == 1 || MW == 4, "one mask word, or four");
   int slot = 0;
   uint32_t phase = 0;
@@ -283,11 +289,6 @@ template <int MW, bool HOLD = false> struct TileCursor {
       offsets = __popcll(lo) + __popcll(hi);
     }
     read(sl);
-    if (!HOLD || tile < 0)
-      release(rv);
-    return tile >= 0 ? 1 : 0;
-  }
-  __device__ __forceinline__ void release(const RingView &rv) {
     __syncwarp();
     if (lane_id() == 0)
       mbar_arrive(rv.empty0 + 8u * slot);
@@ -295,6 +296,7 @@ template <int MW, bool HOLD = false> struct TileCursor {
       slot = 0;
       phase ^= 1u;
     }
+    return tile >= 0 ? 1 : 0;
   }
   __device__ __forceinline__ int first_offset() const {
     if constexpr (MW == 1)
@@ -885,7 +887,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     const uint64_t bdesc_base = B_MN ? make_smem_desc(sbase + Cfg::OFF_B, p.b_lbo, p.b_sbo)
                                      : make_smem_desc(sbase + Cfg::OFF_B, 16, 1024);
     const int ksteps_last = (p.red - (kpasses - 1) * Cfg::KRED + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
-    TileCursor<MW, true> tc;
+    TileCursor<MW> tc;
     int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
     uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
     bool ok = true;
@@ -896,10 +898,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         ok = false;
         break;
       }
-      if (tc.offsets == 0) {
-        tc.release(rv);
+      if (tc.offsets == 0)
         continue;
-      }
       // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
       // are in the key: weights have as many columns)
       bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
@@ -909,21 +909,24 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       const int total = tc.offsets * kpasses;
       int kp = 0;
       for (int s = 0; s < total; ++s) {
-        if (new_b) {
-          if (last_key >= 0 && lane == 0)
-            tc_commit(empty_b(bslot));
-          last_key = 0;
-          if (++bslot == Cfg::SB) {
-            bslot = 0;
-            b_phase ^= 1u;
+        if constexpr (Cfg::JOINT) {
+          bslot = stage;
+        } else {
+          if (new_b) {
+            if (last_key >= 0 && lane == 0)
+              tc_commit(empty_b(bslot));
+            last_key = 0;
+            if (++bslot == Cfg::SB) {
+              bslot = 0;
+              b_phase ^= 1u;
+            }
           }
+          const bool b_there = mbar_test(full_b(bslot), b_phase);
+          if (!b_there)
+            ok = ok && mbar_wait(full_b(bslot), b_phase, abort_flag);
         }
-        const bool b_there = mbar_test(full_b(bslot), b_phase), a_there = mbar_test(full_a(stage), a_phase);
-        if (!b_there)
-          ok = ok && mbar_wait(full_b(bslot), b_phase, abort_flag);
         CB2_PROF_MARK(2);  // weight tile present
-        if (!a_there)
-          ok = ok && mbar_wait(full_a(stage), a_phase, abort_flag);
+        ok = ok && mbar_wait(full_a(stage), a_phase, abort_flag);
         CB2_PROF_MARK(3);  // rows present
         ok = __all_sync(0xffffffffu, ok);
         if (!ok)
@@ -968,7 +971,6 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         new_b = true;
         ++steps;
       }
-      tc.release(rv);
       last_key = (tc.last_offset() * kpasses + kpasses - 1) * p.nn + tc.n0;
       if (++buf == Cfg::NUM_ACC) {
         buf = 0;
@@ -1003,24 +1005,25 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         const int f = tc.take();
         for (int kp = 0; ok && kp < kpasses; ++kp) {
           const int key = (f * kpasses + kp) * p.nn + tc.n0;
-          if (key == last_key)
+          if (!Cfg::JOINT && key == last_key)
             continue;
           last_key = key;
-          ok = __all_sync(0xffffffffu, mbar_wait(empty_b(bslot), b_phase, abort_flag));
+          const uint32_t full = Cfg::JOINT ? full_a(bslot) : full_b(bslot);
+          ok = __all_sync(0xffffffffu, mbar_wait(Cfg::JOINT ? empty_a(bslot) : empty_b(bslot), b_phase, abort_flag));
           if (ok && lane == 0) {
             const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
             const uint32_t dst = sbase + Cfg::OFF_B + bslot * Cfg::B_SLOT_BYTES;
-            mbar_arrive_expect_tx(full_b(bslot), Cfg::B_SLOT_BYTES);
+            mbar_arrive_expect_tx(full, Cfg::B_SLOT_BYTES);
             if constexpr (!B_MN) {
               // [BLOCK_N rows x 128 B] per reduction atom; rows = output channels
 #pragma unroll
               for (int ka = 0; ka < NATOM_K; ++ka)
-                tma_load_3d(dst + ka * (BLOCK_N * 128), &tmap_b, full_b(bslot), kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS, f, n0);
+                tma_load_3d(dst + ka * (BLOCK_N * 128), &tmap_b, full, kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS, f, n0);
             } else {
               // [KRED rows x 128 B] per block of ATOM_ELEMS output channels; rows = reduction
 #pragma unroll
               for (int na = 0; na < BLOCK_N / Cfg::ATOM_ELEMS; ++na)
-                tma_load_3d(dst + na * (Cfg::KRED * 128), &tmap_b, full_b(bslot), n0 + na * Cfg::ATOM_ELEMS, f, kp * Cfg::KRED);
+                tma_load_3d(dst + na * (Cfg::KRED * 128), &tmap_b, full, n0 + na * Cfg::ATOM_ELEMS, f, kp * Cfg::KRED);
             }
           }
           __syncwarp();
