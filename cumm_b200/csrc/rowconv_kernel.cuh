@@ -132,8 +132,10 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int EPI_THREADS = 128 * EPI_HALVES;
   // Groups of epilogue warps that take turns at the tiles: a requantised tile is a long chain per warp
   // (read, convert, scale, convert, pack, store), and two tiles on their way at once fill its gaps
-  // (stride-2 int8 layer, 3839 tiles: 43.7 -> 42.1 us).
+  // (stride-2 int8 layer, 3839 tiles: 43.7 -> 42.1 us).  Each group owns one accumulator: it waits for and
+  // gives back every use of that one, in order, so that a barrier's parity never lies two uses back.
   static constexpr int EPI_GROUPS = (KIND == 1 && BLOCK_N >= 128) ? 2 : 1;
+  static_assert(EPI_GROUPS == 1 || EPI_GROUPS == NUM_ACC, "an accumulator belongs to one group");
   static constexpr int GROUP_THREADS = TMA_GATHER ? 32 : CB2_ROWCONV_GROUP_THREADS;
   static constexpr int FULL_A_COUNT = JOINT ? 2 : TMA_GATHER ? 1 : GROUP_THREADS;
   static constexpr int MMA_WARP = EPI_THREADS / 32;
@@ -658,8 +660,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     const int erow = et & 127;   // the tile row this thread reads from TMEM (lane quarter = warp & 3)
     constexpr int HALVES = Cfg::EPI_HALVES / Cfg::EPI_GROUPS;
     const int half = (et >> 7) % HALVES;   // which share of the columns
-    const int group = (et >> 7) / HALVES;  // which of the tiles with work
-    int turn = 0;
+    const int group = (et >> 7) / HALVES;  // which accumulator is this thread's (with several groups)
     constexpr int COLS_PER_HALF = BLOCK_N / HALVES;
     const bool sectors = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(p.ldo * Cfg::OES)) & 31u) == 0;
     int buf = 0;
@@ -681,14 +682,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           const bool has_work = tc.offsets != 0;
           if (!has_work && p.skip_empty_tiles)
             continue;
-          if (Cfg::EPI_GROUPS > 1) {
-            const bool mine = turn == group;
-            turn = turn + 1 == Cfg::EPI_GROUPS ? 0 : turn + 1;
-            if (!mine) {
-              if (has_work)
-                next_acc();
-              continue;
-            }
+          // A tile without work uses no accumulator and passes none on: whoever is next in turn stores it.
+          if (Cfg::EPI_GROUPS > 1 && buf != group) {
+            if (has_work)
+              next_acc();
+            continue;
           }
           const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
           CB2_PROF_MARK(0);  // walk

@@ -152,10 +152,12 @@ def run_conv_wgrad(torch, dout, x, tb, reduced_mask, *, kv=27, dw_init=None, bet
 
 
 def run_conv_s8(torch, x, w, scale, bias, tb, *, output_add=None, beta=0.0, act=Activation.None_, act_alpha=0.0,
-                tile=None):
+                tile=None, mask_filter=0xFFFFFFFF, max_ctas=0):
     K, kv, C = w.shape
     p = ConvParams(3, ConvOpType.Forward)
     p.conv_algo_desp = conv_desp(ConvOpType.Forward, C, K, int8_inference=True)
+    p.conv_algo_desp.dynamic_mask = kv > 32
+    p.mask_filter, p.max_ctas = mask_filter, max_ctas
     _apply_tile(p, tile)
     p.input = dev(x, torch)
     p.weight = dev(w, torch)

@@ -2,6 +2,8 @@
 gradient, int8 inference) through the operator surface / C ABI, against the CPU oracle.
 fp16 results within rtol 1e-2 / atol 1e-2 of the fp32-accumulated oracle; masks and int8
 outputs bit-exact."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -236,6 +238,41 @@ def test_int8_inference_bit_exact(torch, oracle, n, C, K):
                                 tb.mask_argsort)
     assert (want != 0).mean() > 0.5 and (np.abs(want.astype(int)) < 127).mean() > 0.5, "degenerate test data"
     assert (got == want).all(), f"{int((got != want).sum())} of {got.size} int8 outputs differ"
+
+
+@pytest.mark.parametrize("shuffled", [False, True])
+@pytest.mark.parametrize("ksize,n,C,mask_filter", [
+    ((3, 3, 3), 9000, 128, 0x2AAAAAA), ((3, 3, 3), 9000, 256, 0x1FF),
+    ((5, 5, 5), 2000, 128, 0x0F0F0F0F),  # four mask words
+])
+def test_int8_empty_tiles_between_others(torch, oracle, ksize, n, C, mask_filter, shuffled):
+    """Tiles without an offset between tiles of many, many tiles per CTA: the groups of epilogue warps
+    take turns at the accumulators, and an empty tile takes none."""
+    grid = (41, 400, 352)
+    tb = W.build_tables(W.sample_coords(n, 441, grid), grid=grid, ksize=ksize, stride=(2, 2, 2), subm=False)
+    rng = np.random.default_rng(442)
+    mask, argsort = tb.mask, tb.mask_argsort
+    whole = tb.n_out // 128
+    if shuffled:
+        order = np.concatenate([(rng.permutation(whole)[:, None] * 128 + np.arange(128)).ravel(),
+                                np.arange(whole * 128, tb.n_out)])
+        mask, argsort = mask[order], argsort[order]
+    tiles = np.bitwise_or.reduce(mask[:whole * 128].reshape(whole, 128, -1), axis=1)
+    work = ((tiles & np.uint32(mask_filter)) != 0).any(axis=1)
+    changes = int((work[1:] != work[:-1]).sum())
+    assert changes >= 20, "no empty tiles between others"
+    K = 128
+    x = rng.integers(-127, 128, (tb.n_in, C)).astype(np.int8)
+    w = rng.integers(-127, 128, (K, tb.kv, C)).astype(np.int8)
+    scale = (rng.uniform(1e-3, 1e-2, K) / 16).astype(np.float32)
+    bias = rng.standard_normal(K).astype(np.float32)
+    tb = dataclasses.replace(tb, mask=mask, mask_argsort=argsort)
+    want = oracle.mask_igemm_s8(x, w, np.zeros((tb.n_out, K), np.int8), scale, bias, tb.indices, tb.mask,
+                                tb.mask_argsort, mask_filter=mask_filter)
+    for max_ctas in (1, 3, 0):
+        got = H.run_conv_s8(torch, x, w, scale, bias, tb, mask_filter=mask_filter, max_ctas=max_ctas)
+        H.check_status()
+        assert (got == want).all(), f"{int((got != want).sum())} of {got.size} int8 outputs differ, max_ctas={max_ctas}"
 
 
 def test_int8_large_accumulators_bit_exact(torch, oracle):
