@@ -8,7 +8,7 @@
 // matching weight slice in by TMA, and one warp issues tcgen05.mma into a TMEM accumulator.
 // Eight (fp16) or sixteen (int8) epilogue warps read the accumulator back, apply
 // alpha/beta/bias/activation (or the int8 requantisation) and write the rows to their scattered
-// destinations, whole 32-byte sectors per thread.  No atomics on data: every
+// destinations, whole 32-byte sectors at a time.  No atomics on data: every
 // output row is owned by exactly one tile.
 //
 // What it computes follows the reference kernel's control flow
@@ -100,13 +100,26 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int SA =
       TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES)
                                  : (KIND == 0 ? CB2_ROWCONV_WIDE_STAGES : 3);
+  // Groups that gather: one warp per stage with the copy engine.  Groups of four warps are three, whatever the
+  // stages, and take the steps in turn: their copies are asynchronous, so a group fills a stage while its
+  // last is on the way.  A fourth group leaves 72 registers a thread instead of 80, which costs every role:
+  // 105 us for the forward pass of 960 000 uniform rows at 128 channels, 91 with three (150 000 rows:
+  // 28.9 and 28.0; 60 000 scanned rows at 256 channels: 125 and 120).
+  static constexpr int GROUPS = TMA_GATHER ? SA : 3;
   static constexpr int A_STAGE_BYTES = TILE_M * 128 * NATOM_K;
   static constexpr int B_SLOT_BYTES = BLOCK_N * 128 * NATOM_K;
   static constexpr int MW = MASK_WORDS;
   // Outputs wider than BLOCK_N: column parts drawn with the tiles (fp16), or one grid row per part
   // (int8, whose sixteen epilogue warps have no register to spare for a part that changes).
   static constexpr bool PARTS = KIND == 0;
-  static constexpr int RING = MASK_WORDS == 1 ? CB2_ROWCONV_RING : CB2_ROWCONV_RING / 2;  // tile ring slots
+  // tile ring slots (four mask words beside wide rows: what is left)
+  static constexpr int RING = MASK_WORDS == 1 ? CB2_ROWCONV_RING
+                              : KIND == 0 && !TMA_GATHER ? CB2_ROWCONV_RING / 2 - 1 : CB2_ROWCONV_RING / 2;
+  // fp16: each epilogue warp turns its 32 rows of 64 bytes around in 2 KB of its own before they are stored
+  // (600 000 uniform rows, forward: 50.5 -> 44.5 us at 64 channels, 74.5 -> 71.4 at 128).  int8 rows are half
+  // as long and their registers all taken: each thread stores its own 32 bytes.
+  static constexpr int EPI_WARP_BYTES = KIND == 0 ? 32 * 64 : 0;
+  static constexpr int EPI_BYTES = 8 * EPI_WARP_BYTES;
   static constexpr int RING_SLOT_INTS = 136 + 128 * MASK_WORDS;  // header; 128 gather rows; 128 output rows / row masks
   // int8 rows of up to 128 bytes: a stage holds the step's weight tile beside its rows, under the same pair
   // of barriers -- one wait and one commit per step for the issuer (46.7 -> 43.7 us for the stride-2
@@ -119,7 +132,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
                        BAR_RING = (BAR_EMPTY_B + 6 + 1) / 2 * 2;
   // Weight slots: as many as fit (2 to 6).  A tile whose mask carries many offsets needs a new
   // weight tile every step, and with two slots the L2 latency of that load bounds the step.
-  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + SA * 2 * 128 * 4 +
+  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + GROUPS * 2 * 128 * 4 + EPI_BYTES +
                                      2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (BAR_RING + 3 * RING) * 8 + 64 + 1024;
   static constexpr int SB_FIT = (232448 - FIXED_BYTES) / B_SLOT_BYTES;
   static constexpr int SB = JOINT ? SA : SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
@@ -136,19 +149,21 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // gives back every use of that one, in order, so that a barrier's parity never lies two uses back.
   static constexpr int EPI_GROUPS = (KIND == 1 && BLOCK_N >= 128) ? 2 : 1;
   static_assert(EPI_GROUPS == 1 || EPI_GROUPS == NUM_ACC, "an accumulator belongs to one group");
+  static_assert(EPI_BYTES == EPI_WARP_BYTES * EPI_THREADS / 32 || KIND == 1, "every epilogue warp has its bytes");
   static constexpr int GROUP_THREADS = TMA_GATHER ? 32 : CB2_ROWCONV_GROUP_THREADS;
   static constexpr int FULL_A_COUNT = JOINT ? 2 : TMA_GATHER ? 1 : GROUP_THREADS;
   static constexpr int MMA_WARP = EPI_THREADS / 32;
   static constexpr int TMA_WARP = MMA_WARP + 1;
   static constexpr int FIRST_GATHER_WARP = TMA_WARP + 1;
-  static constexpr int SCHED_WARP = FIRST_GATHER_WARP + SA * GROUP_THREADS / 32;  // the last warp hands out tiles
+  static constexpr int SCHED_WARP = FIRST_GATHER_WARP + GROUPS * GROUP_THREADS / 32;  // the last warp hands out tiles
   static constexpr int THREADS = (SCHED_WARP + 1) * 32;
   static constexpr int RING_CONSUMER_WARPS = SCHED_WARP;   // every warp but the scheduler
   // shared memory map (offsets from a 1024-byte aligned base)
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + SA * A_STAGE_BYTES;
-  static constexpr int OFF_ROWIDX = OFF_B + SB * B_SLOT_BYTES;       // SA * 2 * 128 ints
-  static constexpr int OFF_SCALE = OFF_ROWIDX + SA * 2 * 128 * 4;    // 2 * BLOCK_N floats
+  static constexpr int OFF_EPI = OFF_B + SB * B_SLOT_BYTES;          // EPI_WARP_BYTES per epilogue warp
+  static constexpr int OFF_ROWIDX = OFF_EPI + EPI_BYTES;             // GROUPS * 2 * 128 ints
+  static constexpr int OFF_SCALE = OFF_ROWIDX + GROUPS * 2 * 128 * 4;  // 2 * BLOCK_N floats
   static constexpr int OFF_RING = OFF_SCALE + 2 * BLOCK_N * 4;       // RING slots
   static constexpr int OFF_BARS = OFF_RING + RING * RING_SLOT_INTS * 4;  // BAR_RING + 3 * RING mbarriers
   static constexpr int OFF_MISC = OFF_BARS + (BAR_RING + 3 * RING) * 8;  // tmem ptr, abort, flags
@@ -557,7 +572,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   float *s_scale = reinterpret_cast<float *>(smem + Cfg::OFF_SCALE);
   float *s_bias = s_scale + BLOCK_N;
   volatile int *misc = reinterpret_cast<volatile int *>(smem + Cfg::OFF_MISC);
-  // misc[0] tmem base, misc[1] abort flag, misc[2..5] per-group wait results
+  // misc[0] tmem base, misc[1] abort flag, misc[4 + 2 g, 6 + 2 g) what gather group g's waits returned, one for
+  // each of its row buffers
   volatile int *abort_flag = misc + 1;
 
   const uint32_t bars = sbase + Cfg::OFF_BARS;
@@ -611,7 +627,6 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     }
     mbar_init_fence();
     misc[1] = 0;
-    misc[2] = misc[3] = misc[4] = misc[5] = 1;
     CB2_TRACE_SELECT(0);
   }
   if (KIND == 1) {
@@ -652,10 +667,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
 
   if (warp < Cfg::MMA_WARP) {
     // ======================= epilogue: TMEM -> registers -> scattered rows.  A thread holds 32
-    // consecutive columns of one row and stores them itself, 32 bytes at a time (whole sectors); nothing
-    // is staged, so every warp runs at its own pace and the accumulator is free again as soon as the
-    // last column has been read.  (Staging a tile in shared memory to store whole rows put two barriers
-    // of all epilogue warps into every tile.)
+    // consecutive columns of one row.  int8 stores them itself, 32 bytes at a time (whole sectors); an fp16
+    // warp passes its 32 rows through 2 KB of shared memory of its own, so that four lanes store 64 bytes
+    // side by side.  Either way every warp runs at its own pace and the accumulator is free again as soon
+    // as the last column has been read.  (Staging the whole tile put two barriers of all epilogue warps
+    // into every tile; storing 32 bytes a thread made 32 requests of every store of a warp.)
     const int et = threadIdx.x;
     const int erow = et & 127;   // the tile row this thread reads from TMEM (lane quarter = warp & 3)
     constexpr int HALVES = Cfg::EPI_HALVES / Cfg::EPI_GROUPS;
@@ -727,6 +743,27 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           // 16-byte pieces of this thread's row; the columns past nn are not stored
           auto store = [&](int ncol, const auto &packed) {
             constexpr int N = sizeof(packed) / 16, PIECE = 16 / Cfg::OES;
+            if constexpr (Cfg::EPI_WARP_BYTES > 0) {
+              // four lanes store 64 bytes of a row side by side (the exclusive or keeps a quarter warp's
+              // pieces in different banks)
+              const uint32_t buf_w = sbase + Cfg::OFF_EPI + warp * Cfg::EPI_WARP_BYTES;
+#pragma unroll
+              for (int q = 0; q < N; ++q)
+                st_shared_16(buf_w + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4), &packed[4 * q]);
+              __syncwarp();
+              const int q = lane & 3;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = i * 8 + (lane >> 2);
+                const int to = __shfl_sync(0xffffffffu, o, r);
+                const uint4 piece = ld_shared_16(buf_w + r * 64 + ((q ^ ((r >> 1) & 3)) << 4));
+                if (to >= 0 && ncol + q * PIECE < p.nn)
+                  *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) +
+                                             ((long long)to * p.ldo + ncol + q * PIECE) * Cfg::OES) = piece;
+              }
+              __syncwarp();
+              return;
+            }
             if (o < 0)
               return;
             uint8_t *dst = reinterpret_cast<uint8_t *>(p.out) + ((long long)o * p.ldo + ncol) * Cfg::OES;
@@ -1138,17 +1175,17 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     } else {
       constexpr int GT = Cfg::GROUP_THREADS;
       constexpr int RPT = (128 + GT - 1) / GT;                  // tile rows whose index each thread fetches
-      const int g = (warp - Cfg::FIRST_GATHER_WARP) / (GT / 32);  // 0..2
+      const int g = (warp - Cfg::FIRST_GATHER_WARP) / (GT / 32);
       const int gt = threadIdx.x - (Cfg::FIRST_GATHER_WARP * 32 + g * GT);
       constexpr int CPR = NATOM_K * 8;                  // 16-byte chunks per operand row
       constexpr int RSTEP = GT / CPR;
       const int c = gt % CPR;
       const int row0 = gt / CPR;
-      int *group_rowidx = rowidx + g * 256;  // two buffers, alternating per use of the stage
-      volatile int *my_flag = misc + 3 + g;
+      int *group_rowidx = rowidx + g * 256;  // two buffers, alternating per step of the group
+      volatile int *my_flag = misc + 4 + 2 * g;
       bool dep_waited = false, ok = true;
-      int stage = 0;       // stage of the CTA's next step
-      uint32_t use = 0;    // of this group's own stage
+      uint32_t steps = 0;  // the CTA's steps before this tile; step n fills stage n % SA and is group n % GROUPS'
+      uint32_t use = 0;    // steps this group has taken
       int o[RPT];
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
@@ -1161,79 +1198,95 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                              for (int r = 0; r < RPT; ++r)
                                o[r] = (gt + r * GT < 128) ? sl[8 + gt + r * GT] : -1;
                            })) > 0;) {
-        for (int left = tc.offsets; ok && left > 0; --left) {
-          const int f = tc.take();
-          for (int kp = 0; ok && kp < kpasses; ++kp) {
-            const bool mine = stage == g;
-            if (++stage == Cfg::SA)
-              stage = 0;
-            if (!mine)
-              continue;
-            int idx[RPT];
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-              idx[r] = -1;
-              if (o[r] >= 0) {
-                if (p.mode == kModeMaskConv)
-                  idx[r] = __ldg(p.indices + (long long)f * p.n_rows + o[r]);
-                else
-                  idx[r] = p.a_inds ? __ldg(p.a_inds + o[r]) : o[r];
-              }
-            }
-#pragma unroll
-            for (int r = 0; r < RPT; ++r)
-              if (idx[r] >= p.a_rows) {  // never dereference a row the caller did not provide
-                fail(kStatusBadIndex);
-                idx[r] = -1;
-              }
-            if (gt == 0) {
-              CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
-              const bool free = mbar_wait(empty_a(g), (use & 1) ^ 1, abort_flag);
-              CB2_TRACE_EVENT(g, 2, f);  // stage free
-              *my_flag = free ? 1 : 0;
-              if (!free)
-                fail(kStatusWaitTimeout);
-            }
-            // Double-buffered: a thread that runs ahead writes the other buffer than the one
-            // slower threads of the group may still be reading for the previous use.
-            int *my_rowidx = group_rowidx + (use & 1) * 128;
-#pragma unroll
-            for (int r = 0; r < RPT; ++r)
-              if (gt + r * GT < 128)
-                my_rowidx[gt + r * GT] = idx[r];
-            named_bar_sync(2 + g, Cfg::GROUP_THREADS);
-            ++use;
-            if (*my_flag == 0) {
-              ok = false;
-              break;
-            }
-            if (!dep_waited) {
-              grid_dep_wait();
-              dep_waited = true;
-            }
-            const uint32_t a_stage = sbase + Cfg::OFF_A + g * Cfg::A_STAGE_BYTES;
-            const int byte_off = kp * Cfg::KRED * Cfg::ES + c * 16;
-            const bool col_ok = byte_off < p.red * Cfg::ES;
-            const uint32_t dst_c = a_stage + (c >> 3) * (Cfg::TILE_M * 128);
-#pragma unroll
-            for (int i = 0; i < (128 + RSTEP - 1) / RSTEP; ++i) {
-              const int row = row0 + i * RSTEP;
-              if ((128 % RSTEP) != 0 && row >= 128)
-                break;
-              const int ridx = my_rowidx[row];
-              const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
-              const bool valid = col_ok && ridx >= 0;
-              const uint8_t *srcp = valid ? a_bytes + ((long long)ridx * p.lda) * Cfg::ES + byte_off : a_bytes;
-              cp_async_16(dst, srcp, valid ? 16u : 0u);
-            }
-            // The barrier is signalled by the copy engine when this thread's copies have landed;
-            // the thread itself runs on to its next step.  The consumer makes the data visible
-            // to the tensor core with a proxy fence after its wait.
-            cp_async_mbar_arrive_noinc(full_a(g));
-            if (gt == 0)
-              CB2_TRACE_EVENT(g, 3, f);  // copies issued
+        const int total = tc.offsets * kpasses;
+        int f = -1, upto = 0;  // the offset taken last, and the first step that needs the next one
+        auto look_up = [&](int step, int (&idx)[RPT]) {
+          while (step >= upto) {
+            f = tc.take();
+            upto += kpasses;
           }
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) {
+            idx[r] = -1;
+            if (o[r] >= 0) {
+              if (p.mode == kModeMaskConv)
+                idx[r] = __ldg(p.indices + (long long)f * p.n_rows + o[r]);
+              else
+                idx[r] = p.a_inds ? __ldg(p.a_inds + o[r]) : o[r];
+            }
+          }
+        };
+        // The neighbour indices of the group's next step in the tile are on their way while it waits for the
+        // stage and copies (100 000 scanned rows at 128 channels, forward: 66.5 -> 60.2 us).
+        int ahead[RPT];
+        const int turn = static_cast<int>(steps % Cfg::GROUPS);
+        int step = g - turn + (g < turn ? Cfg::GROUPS : 0);
+        if (step < total)
+          look_up(step, ahead);
+        for (; step < total; step += Cfg::GROUPS) {
+          const uint32_t n = steps + step;
+          const int st = static_cast<int>(n % Cfg::SA);
+          const uint32_t st_phase = ((n / Cfg::SA) & 1u) ^ 1u;
+          const int kp = step - (upto - kpasses);  // the step's offset is the one taken last
+          int idx[RPT];
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) {
+            idx[r] = ahead[r];
+            if (idx[r] >= p.a_rows) {  // never dereference a row the caller did not provide
+              fail(kStatusBadIndex);
+              idx[r] = -1;
+            }
+          }
+          if (step + Cfg::GROUPS < total)
+            look_up(step + Cfg::GROUPS, ahead);
+          if (gt == 0) {
+            CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
+            const bool free = mbar_wait(empty_a(st), st_phase, abort_flag);
+            CB2_TRACE_EVENT(g, 2, f);  // stage free
+            my_flag[use & 1] = free ? 1 : 0;
+            if (!free)
+              fail(kStatusWaitTimeout);
+          }
+          // Double-buffered, as the flag is: a thread that runs ahead writes the other buffer than the one
+          // slower threads of the group may still be reading for the previous step.
+          int *my_rowidx = group_rowidx + (use & 1) * 128;
+#pragma unroll
+          for (int r = 0; r < RPT; ++r)
+            if (gt + r * GT < 128)
+              my_rowidx[gt + r * GT] = idx[r];
+          named_bar_sync(2 + g, Cfg::GROUP_THREADS);
+          ++use;
+          if (my_flag[(use - 1) & 1] == 0) {
+            ok = false;
+            break;
+          }
+          if (!dep_waited) {
+            grid_dep_wait();
+            dep_waited = true;
+          }
+          const uint32_t a_stage = sbase + Cfg::OFF_A + st * Cfg::A_STAGE_BYTES;
+          const int byte_off = kp * Cfg::KRED * Cfg::ES + c * 16;
+          const bool col_ok = byte_off < p.red * Cfg::ES;
+          const uint32_t dst_c = a_stage + (c >> 3) * (Cfg::TILE_M * 128);
+#pragma unroll
+          for (int i = 0; i < (128 + RSTEP - 1) / RSTEP; ++i) {
+            const int row = row0 + i * RSTEP;
+            if ((128 % RSTEP) != 0 && row >= 128)
+              break;
+            const int ridx = my_rowidx[row];
+            const uint32_t dst = dst_c + (row >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4);
+            const bool valid = col_ok && ridx >= 0;
+            const uint8_t *srcp = valid ? a_bytes + ((long long)ridx * p.lda) * Cfg::ES + byte_off : a_bytes;
+            cp_async_16(dst, srcp, valid ? 16u : 0u);
+          }
+          // The barrier is signalled by the copy engine when this thread's copies have landed;
+          // the thread itself runs on to its next step.  The consumer makes the data visible
+          // to the tensor core with a proxy fence after its wait.
+          cp_async_mbar_arrive_noinc(full_a(st));
+          if (gt == 0)
+            CB2_TRACE_EVENT(g, 3, f);  // copies issued
         }
+        steps += total;
       }
       cp_async_wait_all();
     }

@@ -74,7 +74,7 @@ def mask_to_torch(mask, torch):
 
 
 def run_conv_fwd(torch, x, w, tb, *, out_init=None, beta=0.0, alpha=1.0, bias=None, act=Activation.None_,
-                 act_alpha=0.0, mask_filter=0xFFFFFFFF, want_mask_out=True, tile=None):
+                 act_alpha=0.0, mask_filter=0xFFFFFFFF, want_mask_out=True, tile=None, max_ctas=0):
     K, kv, C = w.shape
     p = ConvParams(3, ConvOpType.Forward)
     p.conv_algo_desp = conv_desp(ConvOpType.Forward, C, K)
@@ -91,7 +91,7 @@ def run_conv_fwd(torch, x, w, tb, *, out_init=None, beta=0.0, alpha=1.0, bias=No
         p.mask_output = mo
     p.alpha, p.beta = alpha, beta
     p.act_type, p.act_alpha = act, act_alpha
-    p.mask_filter = mask_filter
+    p.mask_filter, p.max_ctas = mask_filter, max_ctas
     if bias is not None:
         p.bias = dev(bias, torch)
     ConvMainUnitTest.implicit_gemm2(p)

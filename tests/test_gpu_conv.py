@@ -311,6 +311,22 @@ def test_int8_output_add_and_relu(torch, oracle):
     assert (got >= 0).all()
 
 
+@pytest.mark.parametrize("max_ctas", [1, 5])
+@pytest.mark.parametrize("C", [72, 128, 264])  # one pass with and without a ragged end, three passes
+@pytest.mark.parametrize("n,grid", [(129, (8, 24, 24)), (2300, (8, 24, 24)), (3000, (41, 300, 300))])
+def test_wide_rows_many_steps_per_cta(torch, oracle, n, grid, C, max_ctas):
+    """Four operand stages filled in turn by three groups: steps per tile from one to dozens, tiles of one
+    CTA one after the other, so that stage and group meet in every combination."""
+    tb = W.build_tables(W.sample_coords(n, 460 + n, grid), grid=grid)
+    rng = np.random.default_rng(461)
+    x = rng.standard_normal((tb.n_in, C)).astype(np.float16)
+    w = (rng.standard_normal((104, 27, C)) / np.sqrt(27 * C) * 4).astype(np.float16)
+    got, _ = H.run_conv_fwd(torch, x, w, tb, max_ctas=max_ctas)
+    H.check_status()
+    want = oracle.mask_igemm(x, w, np.zeros((n, 104), np.float16), tb.indices, tb.mask, tb.mask_argsort)
+    H.assert_close_f16(got, want, f"n={n} C={C} max_ctas={max_ctas}")
+
+
 def test_errors_surface_as_exceptions(torch):
     tb, x, w, _ = make(300, 501, 64, 64)
     p = ConvParams(3, ConvOpType.Forward)
