@@ -637,7 +637,8 @@ def run_gemm(params: GemmParams) -> None:
             args.workspace, args.workspace_bytes = _workspace_for(args._device, stream, need, params.workspace)
     timer = params.timer
     if timer is not None and getattr(timer, "enable", False):
-        with _TimerGuard(repr(params.algo_desp), timer, stream):
+        import torch
+        with torch.cuda.device(args._device), _TimerGuard(repr(params.algo_desp), timer, stream):
             _call_on(args._device, L.cb2_gemm_run, args, stream)
     else:
         _call_on(args._device, L.cb2_gemm_run, args, stream)
@@ -794,7 +795,8 @@ def run_conv(params: ConvParams) -> None:
     own = None
     if not enabled:
         timer = own = CUDAKernelTimer(True)
-    with _TimerGuard(name, timer, stream):
+    import torch
+    with torch.cuda.device(args._device), _TimerGuard(name, timer, stream):  # events of the call's device
         _call_on(args._device, L.cb2_conv_run, args, stream)
     if params.verbose:
         info = _lib.last_launch_info()

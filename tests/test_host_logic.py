@@ -302,3 +302,57 @@ def test_kernel_timer_names_follow_the_namespace_stack():
     off.push("x")
     off.record("start")
     assert off.insert_pair("", "a", "b") == "" and off._events == {}
+
+
+@pytest.mark.parametrize("kind", ["gemm", "conv", "verbose"])
+def test_timed_calls_record_their_events_on_the_calls_device(monkeypatch, kind):
+    """Tensors on device 1 while device 0 is current: device 1 is current when the events are
+    recorded and when the call is made, and device 0 again afterwards."""
+    import torch
+    import cumm_b200.tensorview.gemm as G
+    current, seen = [0], []
+
+    class Device:
+        def __init__(self, index):
+            self.index = index
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.index
+
+        def __exit__(self, *exc):
+            current[0] = self.before
+
+    class Timer(tv.CUDAKernelTimer):
+        def record(self, name, stream=0):
+            seen.append((name, current[0]))
+
+        def get_pair_duration(self, name):
+            return 0.0
+
+    class Library:
+        @staticmethod
+        def cb2_gemm_run(args, stream):
+            seen.append(("run", current[0]))
+            return 0
+
+        cb2_conv_run = cb2_gemm_run
+
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(G, "CUDAKernelTimer", Timer)
+    monkeypatch.setattr(G._lib, "load", lambda: Library)
+    monkeypatch.setattr(G._lib, "last_launch_info", lambda: {"num_regs": 0})
+    timer = None if kind == "verbose" else Timer(True)
+    if kind == "gemm":
+        p = GemmParams(timer)
+        p.algo_desp = H.gemm_desp(ShuffleStrideType.ShuffleAC)
+        args = _lib.GemmArgs()
+        monkeypatch.setattr(G, "_gemm_args", lambda params: args)
+    else:
+        p = ConvParams(3, ConvOpType.Forward, timer)
+        args = _lib.ConvArgs()
+        p.conv_algo_desp, p.verbose = H.conv_desp(ConvOpType.Forward, 64, 64), kind == "verbose"
+        monkeypatch.setattr(G, "_conv_args", lambda params: args)
+    args._device = 1
+    (G.run_gemm if kind == "gemm" else G.run_conv)(p)
+    assert seen == [("start", 1), ("run", 1), ("stop", 1)] and current == [0]
