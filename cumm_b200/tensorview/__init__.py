@@ -45,18 +45,19 @@ def itemsize(code: int) -> int:
     return _ITEMSIZE[int(code)]
 
 
-_TORCH_CODES = {}
+_TORCH_CODES = {}  # replaced as a whole on first use: another thread sees it empty or complete
 
 
 def _torch_dtype_code(dt) -> int:
+    global _TORCH_CODES
     if not _TORCH_CODES:
         import torch
-        for name, code in (("float32", float32), ("int32", int32), ("int16", int16), ("int8", int8),
-                           ("float64", float64), ("bool", bool_), ("uint8", uint8), ("float16", float16),
-                           ("int64", int64), ("bfloat16", bfloat16), ("uint16", uint16), ("uint32", uint32),
-                           ("uint64", uint64)):
-            if hasattr(torch, name):
-                _TORCH_CODES[getattr(torch, name)] = code
+        _TORCH_CODES = {getattr(torch, name): code
+                        for name, code in (("float32", float32), ("int32", int32), ("int16", int16), ("int8", int8),
+                                           ("float64", float64), ("bool", bool_), ("uint8", uint8),
+                                           ("float16", float16), ("int64", int64), ("bfloat16", bfloat16),
+                                           ("uint16", uint16), ("uint32", uint32), ("uint64", uint64))
+                        if hasattr(torch, name)}
     return _TORCH_CODES[dt]
 
 

@@ -356,3 +356,35 @@ def test_timed_calls_record_their_events_on_the_calls_device(monkeypatch, kind):
     args._device = 1
     (G.run_gemm if kind == "gemm" else G.run_conv)(p)
     assert seen == [("start", 1), ("run", 1), ("stop", 1)] and current == [0]
+
+
+def test_dtype_table_is_published_complete(monkeypatch):
+    """A second thread that asks for a dtype while the first is still filling the table."""
+    import sys
+    import threading
+    import torch
+    answers = []
+
+    def ask():
+        try:
+            answers.append(tv._torch_dtype_code(torch.bfloat16))
+        except KeyError as e:
+            answers.append(e)
+
+    class SlowTorch:
+        asked = False
+
+        def __getattr__(self, name):
+            if name == "int64" and not self.asked:
+                self.asked = True
+                t = threading.Thread(target=ask)
+                t.start()
+                t.join()
+            return getattr(torch, name)
+
+    monkeypatch.setattr(tv, "_TORCH_CODES", {})
+    monkeypatch.setitem(sys.modules, "torch", SlowTorch())
+    assert tv._torch_dtype_code(torch.float16) == tv.float16
+    assert answers == [tv.bfloat16]
+    with pytest.raises(KeyError):
+        tv._torch_dtype_code(torch.complex64)
