@@ -894,12 +894,12 @@ def prepare_conv(params: ConvParams, static_tables: bool = False, static_rows: b
     has a workspace of its own (two prepared weight gradients may overlap on the GPU).
     ``static_rows``, beside ``static_tables``: ``indices`` and ``mask_argsort`` keep their contents too, so
     that the weight gradient's plan may list rows (without ``static_tables`` it plans, and lists, on
-    every launch)."""
+    every launch); ``params.row_lists = False`` keeps any plan to row tiles and the scratch small."""
     L = _lib.load()
     args = _conv_args(params)
     keep = [params.input, params.weight, params.output, params.indices, params.mask, params.mask_argsort,
             params.mask_output, params.bias, params.scale, params.output_add]
-    if static_rows or not static_tables:
+    if params.row_lists and (static_rows or not static_tables):
         args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS
     _attach_workspace(L, args, params, keep, L.cb2_conv_workspace_size,
                       L.cb2_conv_workspace_size_lists if args.reuse_plan else None)

@@ -388,3 +388,52 @@ def test_dtype_table_is_published_complete(monkeypatch):
     assert answers == [tv.bfloat16]
     with pytest.raises(KeyError):
         tv._torch_dtype_code(torch.complex64)
+
+
+class SizesOnly:
+    """The two sizes of a weight gradient's scratch."""
+
+    @staticmethod
+    def cb2_conv_workspace_size(args):
+        return 1000
+
+    @staticmethod
+    def cb2_conv_workspace_size_lists(args):
+        return 5000
+
+
+@pytest.fixture
+def weight_gradient(monkeypatch):
+    """(params, argument record, sizes asked of the allocator) of a weight gradient whose call is never made."""
+    import torch
+    import cumm_b200.tensorview.gemm as G
+    p = conv_params(ConvOpType.BackwardWeight)
+    p.mask_width, p.split_k_slices = 128, 32
+    args = _conv_args(p)
+    sizes = []
+
+    def empty(n, **kw):
+        sizes.append(n)
+        return torch.zeros(n, dtype=torch.uint8)
+
+    monkeypatch.setattr(G, "_conv_args", lambda params: args)
+    monkeypatch.setattr(G._lib, "load", lambda: SizesOnly)
+    monkeypatch.setattr(G, "PreparedCall", lambda kind, args, *rest: args)
+    monkeypatch.setattr(G, "_call_on", lambda device, fn, args, stream: None)
+    monkeypatch.setattr(SizesOnly, "cb2_conv_run", None, raising=False)
+    monkeypatch.setattr(G, "_WORKSPACES", {})
+    monkeypatch.setattr(torch, "empty", empty)
+    return p, args, sizes
+
+
+@pytest.mark.parametrize("static_tables,static_rows,row_lists,size", [
+    (True, True, True, 5000), (False, False, True, 5000), (True, False, True, 1000),
+    (True, True, False, 1000), (False, False, False, 1000)])
+def test_prepared_weight_gradient_lists_rows_where_the_caller_allows(weight_gradient, static_tables, static_rows,
+                                                                     row_lists, size):
+    import cumm_b200.tensorview.gemm as G
+    p, args, sizes = weight_gradient
+    p.row_lists = row_lists
+    G.prepare_conv(p, static_tables, static_rows)
+    assert sizes == [size] and args.workspace_bytes == size
+    assert args.reuse_plan == (_lib.CB2_PLAN_ROW_LISTS if size == 5000 else 0)
