@@ -502,6 +502,20 @@ class ConvParams:
 # dispatch
 # --------------------------------------------------------------------------------------
 _WORKSPACES = {}
+_NO_ROOM = {}  # (device, stream) -> the fewest bytes that could not be had
+
+
+def _scratch(device: int, nbytes: int, best: int, have=None):
+    """A buffer of ``best`` bytes; where the card has no room for those, ``have`` or a new one of ``nbytes``,
+    which are enough."""
+    import torch
+    if best > nbytes:
+        try:
+            return torch.empty(best, dtype=torch.uint8, device=f"cuda:{device}")
+        except torch.cuda.OutOfMemoryError:
+            if have is not None and have.numel() >= nbytes:
+                return have
+    return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{device}")
 
 
 def _workspace_for(device: int, stream: int, nbytes: int, user_ws, best: int = 0):
@@ -512,19 +526,21 @@ def _workspace_for(device: int, stream: int, nbytes: int, user_ws, best: int = 0
     predecessor before it touches the workspace, so they do not race.  Callers that run weight
     gradients on several streams at once pass their own ``workspace`` (or use
     :func:`prepare_conv`, which gives every call its own).  ``best``: bytes with which the call runs
-    fastest, if those are more than it needs; a buffer of the caller's only has to hold ``nbytes``."""
+    fastest, if those are more than it needs; a buffer of the caller's only has to hold ``nbytes``, and so
+    has the cached one where the larger size cannot be had (which is then not asked for again)."""
     t = as_view(user_ws)
     if t is not None and t.nbytes() >= nbytes and t.data_ptr() % 256 == 0:
         return t.data_ptr(), t.nbytes()
     if t is not None and t.nbytes() < nbytes:
         raise RuntimeError(f"workspace at least {nbytes} bytes.")
-    import torch
-    nbytes = max(nbytes, best)
     key = (device, stream)
     buf = _WORKSPACES.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{device}")
-        _WORKSPACES[key] = buf
+    if best >= _NO_ROOM.get(key, best + 1):
+        best = 0
+    if buf is None or buf.numel() < max(nbytes, best):
+        buf = _WORKSPACES[key] = _scratch(device, nbytes, best, buf)
+        if buf.numel() < best:
+            _NO_ROOM[key] = best
     return buf.data_ptr(), buf.numel()
 
 
@@ -877,12 +893,9 @@ def _attach_workspace(L, args, params, keep, size_fn, best_fn=None) -> None:
     if need:
         t = as_view(params.workspace)
         if t is None or t.nbytes() < need:
-            import torch
-            if best_fn is not None:
-                need = max(need, best_fn(ctypes.byref(args)))
-            ws = torch.empty(need, dtype=torch.uint8, device=f"cuda:{args._device}")
+            ws = _scratch(args._device, need, best_fn(ctypes.byref(args)) if best_fn is not None else 0)
             keep.append(ws)
-            args.workspace, args.workspace_bytes = ws.data_ptr(), need
+            args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
         else:
             keep.append(params.workspace)
             args.workspace, args.workspace_bytes = t.data_ptr(), t.nbytes()

@@ -409,11 +409,14 @@ def weight_gradient(monkeypatch):
     import cumm_b200.tensorview.gemm as G
     p = conv_params(ConvOpType.BackwardWeight)
     p.mask_width, p.split_k_slices = 128, 32
+    p.room = 1 << 20
     args = _conv_args(p)
     sizes = []
 
     def empty(n, **kw):
         sizes.append(n)
+        if n > p.room:
+            raise torch.cuda.OutOfMemoryError()
         return torch.zeros(n, dtype=torch.uint8)
 
     monkeypatch.setattr(G, "_conv_args", lambda params: args)
@@ -422,6 +425,7 @@ def weight_gradient(monkeypatch):
     monkeypatch.setattr(G, "_call_on", lambda device, fn, args, stream: None)
     monkeypatch.setattr(SizesOnly, "cb2_conv_run", None, raising=False)
     monkeypatch.setattr(G, "_WORKSPACES", {})
+    monkeypatch.setattr(G, "_NO_ROOM", {}, raising=False)
     monkeypatch.setattr(torch, "empty", empty)
     return p, args, sizes
 
@@ -437,3 +441,24 @@ def test_prepared_weight_gradient_lists_rows_where_the_caller_allows(weight_grad
     G.prepare_conv(p, static_tables, static_rows)
     assert sizes == [size] and args.workspace_bytes == size
     assert args.reuse_plan == (_lib.CB2_PLAN_ROW_LISTS if size == 5000 else 0)
+
+
+def test_scratch_falls_back_to_what_the_call_needs(weight_gradient):
+    """A nearly full card: the room for row lists cannot be had, the call runs without; the cached
+    buffer is then kept, not asked for anew on each call."""
+    import torch
+    import cumm_b200.tensorview.gemm as G
+    p, args, sizes = weight_gradient
+    p.room = 3000
+    G.prepare_conv(p, True, True)
+    assert sizes == [5000, 1000] and args.workspace_bytes == 1000
+    for _ in range(2):
+        G.run_conv(p)
+        assert sizes == [5000, 1000] * 2 and args.workspace_bytes == 1000
+    # a buffer that is there already serves, too
+    G._NO_ROOM.clear()
+    G.run_conv(p)
+    assert sizes == [5000, 1000] * 2 + [5000] and args.workspace_bytes == 1000
+    p.room = 500
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        G.prepare_conv(p, True, True)
