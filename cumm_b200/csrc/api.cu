@@ -422,12 +422,11 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
   p.lists = reinterpret_cast<const int *>(ws + L.off_lists);
   p.list_stride = L.list_stride;
   p.status = dev->status;
-  // Row lists where the caller allows them and the workspace has room, tiles otherwise.  A plan in such a
-  // workspace says for itself which of the two it holds, so one made either way can be reused.
-  const bool room = p.mode == kWgradMaskConv && p.n_rows > 0 && workspace_bytes >= L.total_lists &&
-                    L.row_capacity < (1ll << 31);
-  const bool row_lists = room && (plan_flags & CB2_PLAN_ROW_LISTS);
-  if (room) {
+  // Row lists where the caller allows them and the workspace has room, tiles otherwise.  A plan that is
+  // there already says for itself which of the two it is, whatever this call's flags and size are.
+  const bool possible = p.mode == kWgradMaskConv && p.n_rows > 0 && L.row_capacity < (1ll << 31);
+  const bool row_lists = possible && workspace_bytes >= L.total_lists && (plan_flags & CB2_PLAN_ROW_LISTS);
+  if (possible && (reuse_plan || row_lists)) {
     p.row_head = reinterpret_cast<int *>(ws + L.off_head);
     p.rows = reinterpret_cast<const int *>(ws + L.off_rows);
   }

@@ -42,14 +42,14 @@ struct WgradParams {
   const int32_t *a_inds;   // pair-list mode
   const int32_t *b_inds;   //   "
   float *partials;         // workspace: [unit][m_tile][n_tile][128 x BLOCK_N] fp32
-  int *ctl;                // workspace, zero between calls: [0] CTAs that have left; [9 + 8 by, 13 + 8 by) bit
-                           // masks of the ready offsets of output tile by; from kWgradCtlBase on, per
+  int *ctl;                // workspace, zero between calls but for [1]: [0] CTAs that have left; [1] what the plan
+                           // is (kWgradPlanTiles, kWgradPlanRows); [9 + 8 by, 13 + 8 by) bit masks of the ready offsets of output tile by; from kWgradCtlBase on, per
                            // (f, by) at a pitch of four ints: units arrived
   int *sched;              // workspace header: [0,128) number of row tiles carrying offset f
   const int *lists;        // workspace: per offset, the ordered list of those tiles
   int list_stride;         // ints between two offsets' lists
-  int *row_head;           // workspace or null: [0,128) first entry of offset f's row list, -1 = walked by tiles;
-                           // [128,256) its entries
+  int *row_head;           // workspace or null, for plans with row lists: [0,128) first entry of offset f's row
+                           // list, -1 = walked by tiles; [128,256) its entries
   const int *rows;         // workspace: the row lists
   int *status;
   void *out;               // dW
@@ -138,6 +138,11 @@ __device__ __forceinline__ bool wgrad_tile_has(const WgradParams &p, int tile, i
 //   sched[f]                      tiles carrying offset f
 //   lists[f * list_stride + k]    the k-th of them
 
+// Which kind a plan is stands in a control word, not in what the caller says: a plan may be used again
+// through an argument record of another workspace size or with other flags than it was made with.
+enum : int { kWgradPlanTiles = 0, kWgradPlanRows = 1 };
+__device__ __forceinline__ int wgrad_ctl_start(int i, int plan) { return i == 1 ? plan : 0; }
+
 // One warp plans for up to 128 offsets: lane l owns offsets 4l .. 4l+3.
 constexpr int kWgradMaxOffsets = 128;
 // Exclusive prefix sum, in offset order, of four values per lane; `total` = the sum of all.
@@ -203,7 +208,7 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
   const int f = blockIdx.x;
   // the control words start from zero (every later call leaves them at zero again)
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * blockDim.x)
-    p.ctl[i] = 0;
+    p.ctl[i] = wgrad_ctl_start(i, kWgradPlanTiles);
   const int ntiles = (p.n_rows + 127) / 128;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the lists
@@ -241,11 +246,8 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
     }
     running += all;
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0)
     p.sched[f] = running;
-    if (p.row_head)
-      p.row_head[f] = -1;
-  }
 }
 
 // ---------------------------------------------------------------- plan with row lists
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_plan_rows_kernel(cons
   __shared__ int s_n[32];
   const int f = blockIdx.x;
   for (int i = f * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * blockDim.x)
-    p.ctl[i] = 0;
+    p.ctl[i] = wgrad_ctl_start(i, kWgradPlanRows);
   grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the plan
   const int ntiles = (p.n_rows + 127) / 128;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_mark_rows_kernel(cons
   __shared__ int2 s_sum[kWgradPlanThreads / 32];
   const int f = blockIdx.y, chunk = blockIdx.x;
   for (int i = (f * gridDim.x + chunk) * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * gridDim.y * blockDim.x)
-    p.ctl[i] = 0;
+    p.ctl[i] = wgrad_ctl_start(i, kWgradPlanRows);
   const int ntiles = (p.n_rows + 127) / 128;
   const int per = wgrad_chunk_tiles(ntiles);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -488,6 +490,7 @@ __device__ __forceinline__ void wgrad_load_plan(const WgradParams &p, const int 
     }
     wgrad_plan_warp(cnt, G, P, T, c_first, S, U);
     const int b0 = (int)(((long long)c * T) / G), b1 = (int)(((long long)(c + 1) * T) / G);
+    const bool lists_rows = p.row_head && __ldcg(p.ctl + 1) == kWgradPlanRows;
     int has[4], k0[4], k1[4], len[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -512,8 +515,8 @@ __device__ __forceinline__ void wgrad_load_plan(const WgradParams &p, const int 
       if (has[j]) {
         int *e = s_plan + 8 + 7 * slot[j];
         e[0] = 4 * lane + j;
-        e[5] = p.row_head ? __ldg(p.row_head + 4 * lane + j) : -1;
-        e[6] = p.row_head ? __ldg(p.row_head + kWgradMaxOffsets + 4 * lane + j) : 0;
+        e[5] = lists_rows ? __ldg(p.row_head + 4 * lane + j) : -1;
+        e[6] = lists_rows ? __ldg(p.row_head + kWgradMaxOffsets + 4 * lane + j) : 0;
         e[1] = k0[j];
         e[2] = k1[j];
         e[3] = U[j] + (c - c_first[j]);
@@ -1176,7 +1179,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
   if (misc[6]) {
     const int n_ctl = kWgradCtlBase + 4 * p.kv * gy;
     for (int i = threadIdx.x; i < n_ctl; i += Cfg::THREADS)
-      p.ctl[i] = 0;
+      if (i != 1)
+        p.ctl[i] = 0;
     __threadfence();
   }
   if (threadIdx.x == 0)

@@ -179,7 +179,8 @@ typedef struct cb2_conv_args {
    *   the neighbour tables only, so a training loop plans once per scene.  Bit 0 says so; bit 1
    *   (CB2_PLAN_ROW_LISTS, with or without bit 0) lets the plan list rows where the workspace has
    *   cb2_conv_workspace_size_lists() bytes: such a plan may be reused only while indices and
-   *   mask_argsort are as they were, too. */
+   *   mask_argsort are as they were, too.  A plan says for itself which kind it is: bit 1 and
+   *   workspace_bytes of the call that reuses it play no part. */
   void *sched_scratch;
   int max_ctas;
   int reuse_plan;

@@ -75,11 +75,16 @@ def test_weight_gradient_in_scratch_of_either_size(torch):
         H.check_status()
         assert torch.equal(dw, results[0])
     assert torch.equal(results[0], results[1])
-    # a plan in a large workspace is reused as what it is: tiles then lists allowed, and the other way round
-    for first, then in ((0, 1 | _lib.CB2_PLAN_ROW_LISTS), (_lib.CB2_PLAN_ROW_LISTS, 1)):
+    # a plan is reused as what it is: tiles then lists allowed, and the other way round; made in a record of
+    # the smaller size and used in one of the larger, and the other way round
+    lists = _lib.CB2_PLAN_ROW_LISTS
+    large, small = p.workspace.numel(), _lib.load().cb2_conv_workspace_size(ctypes.byref(_conv_args(p)))
+    for steps in (((0, large), (1 | lists, large)), ((lists, large), (1, large)),
+                  ((lists, small), (1 | lists, large)), ((lists, large), (1 | lists, small))):
         args = _conv_args(p)
-        args.workspace, args.workspace_bytes = p.workspace.data_ptr(), p.workspace.numel()
-        for args.reuse_plan in (first, then):
+        p.workspace.fill_(0x7f)  # nothing left of an earlier plan
+        args.workspace = p.workspace.data_ptr()
+        for args.reuse_plan, args.workspace_bytes in steps:
             p.weight.zero_()
             _lib.raise_for(_lib.load().cb2_conv_run(ctypes.byref(args), None))
             torch.cuda.synchronize()
