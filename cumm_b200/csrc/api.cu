@@ -440,9 +440,10 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
     uint4 *bits = reinterpret_cast<uint4 *>(ws + L.off_bits);
     int2 *counts = reinterpret_cast<int2 *>(ws + L.off_counts);
     wgrad_mark_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, L.n_ctl);
-    wgrad_list_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, reinterpret_cast<int *>(ws + L.off_lists),
-                                                                   reinterpret_cast<int *>(ws + L.off_rows), L.row_capacity);
     CB2_CUDA(cudaGetLastError());
+    CB2_CUDA(launch_after(1, wgrad_list_rows_kernel, grid, dim3(kWgradPlanThreads), 0, stream, p, bits, counts,
+                          reinterpret_cast<int *>(ws + L.off_lists), reinterpret_cast<int *>(ws + L.off_rows),
+                          L.row_capacity));
     g_launches.fetch_add(2);
   } else if (!reuse_plan) {
     // counts and lists of the row tiles per offset; control words to zero

@@ -258,10 +258,11 @@ __global__ void __launch_bounds__(1024) wgrad_plan_kernel(const WgradParams p, i
 // ceil(pairs / 128) steps.  Two kernels make the lists: one marks, per (offset, tile), the rows that take
 // part (a 128-bit word) and counts them per chunk of tiles, the other turns counts into places and
 // writes the lists in sorted order, so the sums have one fixed order.  Offsets whose tiles are at least
-// four fifths full, and lists that find no room, are walked by tiles.  (100 003 rows of a scanned scene,
-// 64 channels: 8281 steps by tiles, 4030 by rows, 102 -> 54 us; 30 011 rows, 125 offsets: 16324 and
-// 3100, 218 -> 33 us and 21 us of planning.  At four fifths the shorter walk is worth the table read
-// that makes it.)
+// four fifths full, and lists that find no room, are walked by tiles.  (The kernel by tiles and by rows, and
+// what planning adds: 100 003 rows of a scanned scene, 64 channels, 8234 and 4030 steps, 75 and 40 us, 3.5 and
+// 19 us; 34 000 rows, 125 offsets, 270 and 35 us, 5 and 32 us; 150 000 uniform rows, 128 channels, 34.0 and
+// 32.4 us, 3.6 and 13 us; 960 000 such rows, 105 us either way, 7 and 25 us -- there lists do not pay.  At four
+// fifths the shorter walk is worth the table read that makes it.)
 constexpr int kWgradPlanThreads = 1024;  // a warp per tile of a group of 32
 constexpr int kWgradMaxChunks = 64;
 // tiles per chunk: whole groups of 32
@@ -269,24 +270,23 @@ __host__ __device__ inline int wgrad_chunk_tiles(int ntiles) {
   return 32 * ((ntiles + 32 * kWgradMaxChunks - 1) / (32 * kWgradMaxChunks));
 }
 
-// Rows of tile t that take part at offset f, 32 per word (warp-collective); o = the output rows.
+// Rows of tile t, which carries offset f, that take part there, 32 per word (warp-collective); o = the
+// output rows.
 __device__ __forceinline__ uint4 wgrad_tile_rows(const WgradParams &p, int t, int f, int (&o)[4]) {
   const int lane = (int)lane_id();
-  uint32_t w[4] = {0u, 0u, 0u, 0u};
-  if (wgrad_tile_has(p, t, f)) {
-    bool on[4];
+  uint32_t w[4];
+  bool on[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = t * 128 + q * 32 + lane;
-      o[q] = r < p.n_rows ? __ldg(p.argsort + r) : -1;
-      on[q] = o[q] >= 0;
-      if (p.mask_width < 128 && on[q])
-        on[q] = (__ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5)) >> (f & 31)) & 1u;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      w[q] = __ballot_sync(0xffffffffu, on[q] && __ldg(p.indices + (long long)f * p.n_rows + o[q]) >= 0);
+  for (int q = 0; q < 4; ++q) {
+    const int r = t * 128 + q * 32 + lane;
+    o[q] = r < p.n_rows ? __ldg(p.argsort + r) : -1;
+    on[q] = o[q] >= 0;
+    if (p.mask_width < 128 && on[q])
+      on[q] = (__ldg(p.rmask + (long long)(r / p.mask_width) * p.words + (f >> 5)) >> (f & 31)) & 1u;
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    w[q] = __ballot_sync(0xffffffffu, on[q] && __ldg(p.indices + (long long)f * p.n_rows + o[q]) >= 0);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ bool wgrad_listed(long long rows, long long tiles) {
@@ -295,6 +295,8 @@ __device__ __forceinline__ bool wgrad_listed(long long rows, long long tiles) {
 
 // Up to kWgradOneBlockTiles tiles: both in one launch, a block per offset, every list with room for all
 // rows (so that no offset has to know the others' counts).
+// (Where the line lies: at 219 tiles, 27 offsets, planning adds 16 us so, at 266 tiles and 125 offsets in two
+// launches 32 us; at 390 tiles 13 rounds of 32 tiles would be in sequence.)
 constexpr int kWgradOneBlockTiles = 256;
 __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_plan_rows_kernel(const WgradParams p, int *lists, int *rows,
                                                                             int n_ctl) {
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_plan_rows_kernel(cons
     const int t = t0 + wid;
     int o[4];
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (t < ntiles)
+    if (t < ntiles && wgrad_tile_has(p, t, f))
       v = wgrad_tile_rows(p, t, f, o);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
@@ -347,21 +349,30 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_mark_rows_kernel(cons
                                                                             int n_ctl) {
   __shared__ int2 s_sum[kWgradPlanThreads / 32];
   const int f = blockIdx.y, chunk = blockIdx.x;
+  grid_dep_launch();  // the next kernel waits before it reads what this one writes
   for (int i = (f * gridDim.x + chunk) * blockDim.x + threadIdx.x; i < n_ctl; i += gridDim.x * gridDim.y * blockDim.x)
     p.ctl[i] = wgrad_ctl_start(i, kWgradPlanRows);
   const int ntiles = (p.n_rows + 127) / 128;
-  const int per = wgrad_chunk_tiles(ntiles);
+  const int per = wgrad_chunk_tiles(ntiles), run = per / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int t0 = chunk * per + wid * run, t1 = min(t0 + run, ntiles);
+  uint4 *mine = bits + (long long)f * p.list_stride;
   int rows = 0, tiles = 0;
-  for (int t = chunk * per + wid; t < min((chunk + 1) * per, ntiles); t += kWgradPlanThreads / 32) {
-    int o[4];
-    const uint4 v = wgrad_tile_rows(p, t, f, o);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    const int n = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
-    rows += n;
-    tiles += n > 0;
-    if (lane == 0)
-      bits[(long long)f * p.list_stride + t] = make_uint4(w[0], w[1], w[2], w[3]);
+  for (int first = t0; first < t1; first += 32) {
+    // the mask words of the warp's tiles in one load: away from the centre most have nothing to do
+    const bool has = first + lane < t1 && wgrad_tile_has(p, first + lane, f);
+    if (first + lane < t1 && !has)
+      mine[first + lane] = make_uint4(0u, 0u, 0u, 0u);
+    for (unsigned left = __ballot_sync(0xffffffffu, has); left; left &= left - 1) {
+      const int t = first + __ffs(left) - 1;
+      int o[4];
+      const uint4 v = wgrad_tile_rows(p, t, f, o);
+      const int n = __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+      rows += n;
+      tiles += n > 0;
+      if (lane == 0)
+        mine[t] = v;
+    }
   }
   if (lane == 0)
     s_sum[wid] = make_int2(rows, tiles);
@@ -374,29 +385,59 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_mark_rows_kernel(cons
   }
 }
 
+// A block of the second kernel whose chunk has none of the offset's rows is gone at once; the others add up the
+// counts with all warps, a warp per offset, their loads in flight together (with a thread per offset, one load
+// after the other, planning and the kernel took 163 instead of 130 us for 960 000 uniform rows, 54.5 instead
+// of 45.6 for 150 000, 123 instead of 118 for 300 000 scanned ones).  Warp w takes a contiguous run of the
+// chunk's tiles.
 __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_list_rows_kernel(const WgradParams p, const uint4 *bits,
                                                                             const int2 *counts, int *lists, int *rows,
                                                                             long long capacity) {
-  __shared__ int s_rows[kWgradMaxOffsets], s_tiles[kWgradMaxOffsets], s_base[kWgradMaxOffsets];
-  __shared__ int s_before[2];
-  __shared__ int s_place[32], s_count[2];
+  __shared__ int s_rows[kWgradMaxOffsets], s_tiles[kWgradMaxOffsets];
+  __shared__ int s_base, s_before[2];
+  __shared__ int2 s_n[32];
   const int f = blockIdx.y, chunk = blockIdx.x, n_chunks = gridDim.x;
-  grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the plan
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x < kWgradMaxOffsets) {
-    int r = 0, t = 0;
-    if ((int)threadIdx.x < p.kv) {
-#pragma unroll 8
-      for (int c = 0; c < n_chunks; ++c) {
-        if ((int)threadIdx.x == f && c == chunk)
-          s_before[0] = r, s_before[1] = t;
-        const int2 v = __ldg(counts + threadIdx.x * n_chunks + c);
-        r += v.x, t += v.y;
+  grid_dep_launch();  // the main kernel may set itself up meanwhile; it waits before reading the plan
+  grid_dep_wait();
+  if (chunk > 0 && __ldg(counts + f * n_chunks + chunk).x == 0)
+    return;
+#pragma unroll
+  for (int j = 0; j < kWgradMaxOffsets / 32; ++j) {
+    const int g = 32 * j + wid;
+    int2 all = make_int2(0, 0), before = make_int2(0, 0);
+    if (g < p.kv) {
+#pragma unroll
+      for (int i = 0; i < kWgradMaxChunks / 32; ++i) {
+        const int c = 32 * i + lane;
+        const int2 v = c < n_chunks ? __ldg(counts + g * n_chunks + c) : make_int2(0, 0);
+        all.x += v.x, all.y += v.y;
+        if (c < chunk)
+          before.x += v.x, before.y += v.y;
       }
     }
-    s_rows[threadIdx.x] = r;
-    s_tiles[threadIdx.x] = t;
+    all.x = __reduce_add_sync(0xffffffffu, all.x), all.y = __reduce_add_sync(0xffffffffu, all.y);
+    if (lane == 0)
+      s_rows[g] = all.x, s_tiles[g] = all.y;
+    if (g == f) {
+      before.x = __reduce_add_sync(0xffffffffu, before.x), before.y = __reduce_add_sync(0xffffffffu, before.y);
+      if (lane == 0)
+        s_before[0] = before.x, s_before[1] = before.y;
+    }
   }
+  const int ntiles = (p.n_rows + 127) / 128;
+  const int per = wgrad_chunk_tiles(ntiles), run = per / 32;
+  const int t0 = chunk * per + wid * run, t1 = min(min(t0 + run, (chunk + 1) * per), ntiles);
+  const uint4 *mine = bits + (long long)f * p.list_stride;
+  int2 n = make_int2(0, 0);
+  for (int t = t0 + lane; t < t1; t += 32) {
+    const uint4 w = __ldg(mine + t);
+    const int c = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+    n.x += c, n.y += c > 0;
+  }
+  n.x = __reduce_add_sync(0xffffffffu, n.x), n.y = __reduce_add_sync(0xffffffffu, n.y);
+  if (lane == 0)
+    s_n[wid] = n;
   __syncthreads();
   if (wid == 0) {
     int size[4], first[4], total;
@@ -410,54 +451,38 @@ __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_list_rows_kernel(cons
     wgrad_scan4(size, first, total);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      s_base[4 * lane + j] = listed[j] && 128ll * (first[j] + size[j]) <= capacity ? 128 * first[j] : -1;
-  }
-  __syncthreads();
-  const int base = s_base[f];
-  if (chunk == 0 && threadIdx.x == 0) {
-    p.sched[f] = base >= 0 ? (s_rows[f] + 127) / 128 : s_tiles[f];
-    p.row_head[f] = base;
-    p.row_head[kWgradMaxOffsets + f] = s_rows[f];
-  }
-  const int ntiles = (p.n_rows + 127) / 128;
-  const int per = wgrad_chunk_tiles(ntiles);
-  const int end = min((chunk + 1) * per, ntiles);
-  int before_rows = s_before[0], before_tiles = s_before[1];
-  const uint4 *mine = bits + (long long)f * p.list_stride;
-  for (int t0 = chunk * per; t0 < end; t0 += 32) {
-    if (wid == 0) {
-      const int t = t0 + lane;
-      const uint4 w = t < end ? __ldg(mine + t) : make_uint4(0u, 0u, 0u, 0u);
-      const int n = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
-      int incl = n;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d)
-          incl += v;
-      }
-      s_place[lane] = incl - n;
-      const unsigned any = __ballot_sync(0xffffffffu, n > 0);
-      if (base < 0 && n > 0)
-        lists[(long long)f * p.list_stride + before_tiles + __popc(any & ((1u << lane) - 1u))] = t;
-      if (lane == 31)
-        s_count[0] = incl, s_count[1] = __popc(any);
-    }
-    __syncthreads();
-    if (base >= 0)
-      for (int l = wid; l < 32 && t0 + l < end; l += kWgradPlanThreads / 32) {
-        const uint4 v = __ldg(mine + t0 + l);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        int at = base + before_rows + s_place[l];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if ((w[q] >> lane) & 1u)
-            rows[at + __popc(w[q] & ((1u << lane) - 1u))] = __ldg(p.argsort + (t0 + l) * 128 + q * 32 + lane);
-          at += __popc(w[q]);
+      if (4 * lane + j == f) {
+        const int base = listed[j] && 128ll * (first[j] + size[j]) <= capacity ? 128 * first[j] : -1;
+        s_base = base;
+        if (chunk == 0) {
+          p.sched[f] = base >= 0 ? size[j] : s_tiles[f];
+          p.row_head[f] = base;
+          p.row_head[kWgradMaxOffsets + f] = s_rows[f];
         }
       }
-    before_rows += s_count[0], before_tiles += s_count[1];
-    __syncthreads();
+  }
+  const int2 others = s_n[lane];
+  int at = s_before[0] + __reduce_add_sync(0xffffffffu, lane < wid ? others.x : 0);
+  int at_tile = s_before[1] + __reduce_add_sync(0xffffffffu, lane < wid ? others.y : 0);
+  __syncthreads();
+  const int base = s_base;
+  for (int t = t0; t < t1; ++t) {
+    const uint4 v = __ldg(mine + t);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    if ((v.x | v.y | v.z | v.w) == 0)
+      continue;
+    if (base < 0) {
+      if (lane == 0)
+        lists[(long long)f * p.list_stride + at_tile] = t;
+      ++at_tile;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if ((w[q] >> lane) & 1u)
+          rows[base + at + __popc(w[q] & ((1u << lane) - 1u))] = __ldg(p.argsort + t * 128 + q * 32 + lane);
+        at += __popc(w[q]);
+      }
+    }
   }
 }
 

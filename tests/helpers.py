@@ -127,10 +127,11 @@ def run_conv_dgrad(torch, dout, w, tb, *, din_init=None, beta=0.0, use_reverse=F
 
 
 def run_conv_wgrad(torch, dout, x, tb, reduced_mask, *, kv=27, dw_init=None, beta=0.0, alpha=1.0,
-                   mask_filter=0xFFFFFFFF, mask_width=128, fp32_out=False, tile=None):
+                   mask_filter=0xFFFFFFFF, mask_width=128, fp32_out=False, tile=None, row_lists=True):
     K, C = dout.shape[1], x.shape[1]
     p = ConvParams(3, ConvOpType.BackwardWeight)
     p.conv_algo_desp = conv_desp(ConvOpType.BackwardWeight, C, K)
+    p.conv_algo_desp.dynamic_mask, p.row_lists = kv > 32, row_lists
     _apply_tile(p, tile)
     p.input = dev(x, torch)
     dt = torch.float32 if fp32_out else torch.float16

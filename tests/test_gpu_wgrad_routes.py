@@ -24,8 +24,8 @@ def operands(tb, C, K, seed):
     return x, dout, w
 
 
-# (rows, grid): nothing but the centre; one row past a tile; half full (most offsets listed); three fifths
-# full (more pairs than the lists have room for, the last offsets walked by tiles); solid (nothing listed)
+# (rows, grid), all of up to 256 tiles, whose lists one launch makes and which always have room: nothing but
+# the centre; one row past a tile; half full (most offsets listed); three fifths full; solid (nothing listed)
 SCENES = [(1, (8, 24, 24)), (129, (8, 24, 24)), (2300, (8, 24, 24)), (2900, (8, 24, 24)), (4608, (8, 24, 24))]
 
 
@@ -39,6 +39,40 @@ def test_weight_gradient_by_rows(torch, oracle, n, grid, C, K):
     H.check_status()
     want = oracle.mask_igemm_wgrad(dout, x, np.zeros((K, 27, C), np.float16), tb.indices, tiles, tb.mask_argsort)
     H.assert_close_wgrad(got, want, tb.indices, f"n={n} C={C} K={K}")
+
+
+@pytest.mark.parametrize("ksize,n,grid,mask_width,mask_filter", [
+    # three fifths full: more listed pairs than there is room for, the last offsets are walked by tiles
+    ((3, 3, 3), 33500, (16, 60, 60), 128, 0xFFFFFFFF), ((3, 3, 3), 33500, (16, 60, 60), 32, 0xFFFFFFFF),
+    ((3, 3, 3), 33500, (16, 60, 60), 256, 0xFFFFFFFF), ((3, 3, 3), 33500, (16, 60, 60), 128, 0x5A5A5A5),
+    # a few rows per offset beside a full centre; the centre filtered out; nothing left
+    ((3, 3, 3), 32769, (41, 300, 300), 128, 0xFFFFFFFF), ((3, 3, 3), 40000, (41, 300, 300), 64, ~(1 << 13)),
+    ((3, 3, 3), 32769, (41, 300, 300), 128, 0),
+    # four mask words: all listed, and too many
+    ((5, 5, 5), 33000, (20, 120, 120), 128, 0xFFFFFFFF), ((5, 5, 5), 33000, (16, 80, 80), 128, 0xFFFFFFFF)])
+def test_row_lists_of_more_than_256_tiles(torch, ksize, n, grid, mask_width, mask_filter):
+    """The plan in three launches.  Integers sum exactly: lists and tiles give the same bits."""
+    tb = W.build_tables(W.sample_coords(n, 5, grid), grid=grid, ksize=ksize)
+    per_row = tb.num_pairs / n - 1
+    room = 8 + tb.kv // 8
+    if grid in ((16, 60, 60), (16, 80, 80)):
+        assert per_row > room, "the lists do not overflow"
+    rng = np.random.default_rng(n)
+    x = rng.integers(-2, 3, (n, 32)).astype(np.float16)
+    dout = rng.integers(-2, 3, (n, 40)).astype(np.float16)
+    masks = np.bitwise_or.reduceat(tb.mask, np.arange(0, n, mask_width), axis=0)
+    flt = mask_filter & 0xFFFFFFFF
+    by = [H.run_conv_wgrad(torch, dout, x, tb, masks, kv=tb.kv, mask_width=mask_width, mask_filter=flt, fp32_out=True,
+                           row_lists=lists) for lists in (True, False)]
+    H.check_status()
+    want = np.zeros((40, tb.kv, 32))
+    xs, ds = torch.from_numpy(x).cuda().double(), torch.from_numpy(dout).cuda().double()
+    for f in range(tb.kv):
+        if (flt >> (f % 32)) & 1:
+            o = np.flatnonzero(tb.indices[f] >= 0)
+            i = torch.from_numpy(tb.indices[f][o].astype(np.int64)).cuda()
+            want[:, f] = (ds[torch.from_numpy(o).cuda()].T @ xs[i]).cpu().numpy()
+    assert (by[0] == want).all() and (by[1] == want).all()
 
 
 def test_weight_gradient_in_scratch_of_either_size(torch):
