@@ -365,7 +365,7 @@ void wgrad_layout(int num_sms, int max_ctas, int m_total, int n_total, long long
   const int per = wgrad_chunk_tiles((int)ntiles);
   L->n_chunks = per > 0 ? (int)((ntiles + per - 1) / per) : 0;
   L->row_capacity = (n_rows * std::min(kvs, 8 + kvs / 8) + 127) / 128 * 128;
-  if (ntiles <= kWgradOneBlockTiles)  // one launch makes the lists, each with room for every row
+  if (ntiles <= kWgradRoomyTiles)
     L->row_capacity = ntiles * 128 * kvs;
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   L->off_head = up(L->total);
@@ -430,7 +430,7 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
     p.row_head = reinterpret_cast<int *>(ws + L.off_head);
     p.rows = reinterpret_cast<const int *>(ws + L.off_rows);
   }
-  if (!reuse_plan && row_lists && L.list_stride <= kWgradOneBlockTiles) {
+  if (!reuse_plan && row_lists && wgrad_one_block((p.n_rows + 127) / 128, p.kv)) {
     wgrad_plan_rows_kernel<<<p.kv, kWgradPlanThreads, 0, stream>>>(p, reinterpret_cast<int *>(ws + L.off_lists),
                                                                    reinterpret_cast<int *>(ws + L.off_rows), L.n_ctl);
     CB2_CUDA(cudaGetLastError());

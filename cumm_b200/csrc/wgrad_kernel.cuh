@@ -293,11 +293,14 @@ __device__ __forceinline__ bool wgrad_listed(long long rows, long long tiles) {
   return 512 * tiles > 5 * rows;  // tiles less than four fifths full
 }
 
-// Up to kWgradOneBlockTiles tiles: both in one launch, a block per offset, every list with room for all
-// rows (so that no offset has to know the others' counts).
-// (Where the line lies: at 219 tiles, 27 offsets, planning adds 16 us so, at 266 tiles and 125 offsets in two
-// launches 32 us; at 390 tiles 13 rounds of 32 tiles would be in sequence.)
-constexpr int kWgradOneBlockTiles = 256;
+// Few tiles: both in one launch, a block per offset, every list with room for all rows (so that no offset
+// has to know the others' counts).  A block takes 32 tiles at a time, one round after the other, so the line lies
+// low for as many offsets as blocks of two launches fill the chip with, and higher for more (planning and the
+// kernel in one and in two launches, scanned scenes: 27 offsets, 51 tiles 22.4 and 24.0 us, 79 tiles 25.8 and
+// 25.1, 219 tiles 35.3 and 29.2; 125 offsets, 51 tiles 24.6 and 28.0, 235 tiles 53.6 and 61.2; a uniform one
+// of 469 tiles 53.9 and 41.5).
+constexpr int kWgradRoomyTiles = 256;  // up to here the lists have room for all rows whichever way they are made
+__host__ __device__ inline bool wgrad_one_block(long long ntiles, int kv) { return ntiles <= (kv <= 32 ? 64 : kWgradRoomyTiles); }
 __global__ void __launch_bounds__(kWgradPlanThreads) wgrad_plan_rows_kernel(const WgradParams p, int *lists, int *rows,
                                                                             int n_ctl) {
   __shared__ int s_n[32];

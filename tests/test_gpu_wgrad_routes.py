@@ -24,7 +24,7 @@ def operands(tb, C, K, seed):
     return x, dout, w
 
 
-# (rows, grid), all of up to 256 tiles, whose lists one launch makes and which always have room: nothing but
+# (rows, grid), all of up to 64 tiles, whose lists one launch makes and which always have room: nothing but
 # the centre; one row past a tile; half full (most offsets listed); three fifths full; solid (nothing listed)
 SCENES = [(1, (8, 24, 24)), (129, (8, 24, 24)), (2300, (8, 24, 24)), (2900, (8, 24, 24)), (4608, (8, 24, 24))]
 
@@ -48,10 +48,14 @@ def test_weight_gradient_by_rows(torch, oracle, n, grid, C, K):
     # a few rows per offset beside a full centre; the centre filtered out; nothing left
     ((3, 3, 3), 32769, (41, 300, 300), 128, 0xFFFFFFFF), ((3, 3, 3), 40000, (41, 300, 300), 64, ~(1 << 13)),
     ((3, 3, 3), 32769, (41, 300, 300), 128, 0),
+    # around the line between one launch and two, and the last size whose lists have room for all rows
+    ((3, 3, 3), 8192, (16, 30, 30), 128, 0xFFFFFFFF), ((3, 3, 3), 8193, (16, 30, 30), 128, 0xFFFFFFFF),
+    ((3, 3, 3), 32768, (16, 59, 59), 128, 0xFFFFFFFF), ((5, 5, 5), 32768, (20, 120, 120), 128, 0xFFFFFFFF),
     # four mask words: all listed, and too many
     ((5, 5, 5), 33000, (20, 120, 120), 128, 0xFFFFFFFF), ((5, 5, 5), 33000, (16, 80, 80), 128, 0xFFFFFFFF)])
-def test_row_lists_of_more_than_256_tiles(torch, ksize, n, grid, mask_width, mask_filter):
-    """The plan in three launches.  Integers sum exactly: lists and tiles give the same bits."""
+def test_row_lists_in_two_launches(torch, ksize, n, grid, mask_width, mask_filter):
+    """Plans made by two kernels, and the last sizes that one makes.  Integers sum exactly: lists and tiles
+    give the same bits."""
     tb = W.build_tables(W.sample_coords(n, 5, grid), grid=grid, ksize=ksize)
     per_row = tb.num_pairs / n - 1
     room = 8 + tb.kv // 8
