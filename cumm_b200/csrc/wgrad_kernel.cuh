@@ -636,7 +636,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     mbar_init(final_bar, 1);
     mbar_init_fence();
     misc[1] = 0;
-    misc[2] = misc[3] = misc[4] = misc[5] = 1;
+    misc[2] = 1;
 #ifndef CB2_TRACE_WGRAD_CTA
 #define CB2_TRACE_WGRAD_CTA 0
 #endif
@@ -956,7 +956,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     const int g = (warp - 5) >> 2;
     const int gt = threadIdx.x - (5 * 32 + g * 128);
     int *group_rowidx = rowidx + g * 512;
-    volatile int *my_flag = misc + 3 + g;
+    volatile int *my_flag = misc + 8 + 2 * g;  // per row buffer: a thread that runs ahead writes the other one
     int step = 0;
     const uint8_t *a_bytes = reinterpret_cast<const uint8_t *>(p.dout);
     const uint8_t *b_bytes = reinterpret_cast<const uint8_t *>(p.x);
@@ -1000,7 +1000,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
             CB2_TRACE_EVENT(g, 1, step - 1 + (ib == 0x7fffffff));  // indices loaded
             bool ok = mbar_wait(empty_s(g), (use & 1) ^ 1, abort_flag);
             CB2_TRACE_EVENT(g, 2, step - 1);             // stage free
-            *my_flag = ok ? 1 : 0;
+            my_flag[use & 1] = ok ? 1 : 0;
             if (!ok)
               fail(kStatusWaitTimeout);
           }
@@ -1009,7 +1009,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           ridx_a[gt] = ia;
           ridx_b[gt] = ib;
           named_bar_sync(2 + g, 128);
-          if (*my_flag == 0)
+          if (my_flag[use & 1] == 0)
             return false;
           {
             // A rows: 256 B (128 channels of dout starting at m0), 16 chunks per row
