@@ -272,6 +272,13 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const void *tmap, uint
                "l"(tmap), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
                : "memory");
 }
+// The row a gather4 request names for tile row `at` (0 to 127): the row itself, or, where there is none, a
+// row number below zero of the tile row's own, which reads as zeros.  With -1 for every missing row all SMs
+// meet at one place: 128 rows of 128 bytes a step, half of them missing, took 0.61 us a step and SM, nine
+// tenths missing 0.98; with 128 different numbers 0.27, as with every row present.  (Layer of 125 offsets,
+// 30 011 scanned rows, 32 channels, forward: 108 -> 87 us.)
+__device__ __forceinline__ int row_or_zeros(int row, int at) { return row >= 0 ? row : -1 - at; }
+
 // ---------------------------------------------------------------- tcgen05 / TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst),

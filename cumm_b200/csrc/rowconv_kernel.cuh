@@ -1164,8 +1164,9 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             if (wanted) {
 #pragma unroll
               for (int ka = 0; ka < NATOM_K; ++ka)
-                tma_gather4(my_quad + ka * (Cfg::TILE_M * 128), &tmap_a, full_a(g),
-                            kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS, idx[0], idx[1], idx[2], idx[3]);
+                tma_gather4(my_quad + ka * (Cfg::TILE_M * 128), &tmap_a, full_a(g), kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS,
+                            row_or_zeros(idx[0], 4 * lane), row_or_zeros(idx[1], 4 * lane + 1),
+                            row_or_zeros(idx[2], 4 * lane + 2), row_or_zeros(idx[3], 4 * lane + 3));
             }
             dirty = need;
             if (lane == 0)

@@ -925,6 +925,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
             fail(kStatusBadIndex);
             ia[j] = ib[j] = -1;
           }
+          ia[j] = row_or_zeros(ia[j], 4 * quad + j);
+          ib[j] = row_or_zeros(ib[j], 4 * quad + j);
         }
         if (first_lane)
           CB2_TRACE_EVENT(g, 1, cur.tile + (ib[0] == 0x7fffffff));  // indices loaded
