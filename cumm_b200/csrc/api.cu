@@ -242,12 +242,11 @@ int plan_rowconv(int kind, int red, int nn, bool b_mn, int tile_n, int tile_k, R
 
 int launch_rowconv(const RowConvPlan &pl, const CUtensorMap &map, const CUtensorMap &map_a, bool tma_gather,
                    const RowConvParams &p, int gx, int gy, cudaStream_t s) {
-  // Kernel volumes above 32 (several mask words per row): one variant per shape, with the gather
-  // path that is the default for its row width.
+  // Kernel volumes above 32 (several mask words per row): one variant per shape.
 #define CB2_INST(K, A, N, M)                                                                      \
   if (pl.kind == K && pl.natom_k == A && pl.block_n == N && pl.b_mn == M) {                        \
     if (p.mask_words > 1)                                                                          \
-      return launch_rowconv_inst<K, A, N, M, (A == 1), 4>(map, map_a, p, gx, gy, s);               \
+      return launch_rowconv_inst<K, A, N, M, true, 4>(map, map_a, p, gx, gy, s);               \
     return tma_gather ? launch_rowconv_inst<K, A, N, M, true>(map, map_a, p, gx, gy, s)            \
                       : launch_rowconv_inst<K, A, N, M, false>(map, map_a, p, gx, gy, s);          \
   }
@@ -291,11 +290,9 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
                        b_mn ? kred : pl.block_n);
   if (rc)
     return rc;
-  // Operand rows of up to 128 bytes go through the copy engine (one tile::gather4 request per
-  // four rows); wider rows need a request per 128-byte column block, at which point the copy
-  // engine's request rate, not memory, bounds a step, and 16-byte cp.async is faster.
-  // CUMM_B200_GATHER forces one path for every width.
-  const bool tma_gather = (getenv("CUMM_B200_GATHER") && p.mask_words == 1) ? gather_mode() != 0 : pl.natom_k == 1;
+  // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes);
+  // CUMM_B200_GATHER=0 has 16-byte cp.async instead.
+  const bool tma_gather = p.mask_words > 1 || gather_mode() != 0;
   CUtensorMap map_a;
   memset(&map_a, 0, sizeof(map_a));
   if (tma_gather) {

@@ -74,6 +74,18 @@ __device__ __forceinline__ void trace_cta(int which, unsigned long long value) {
 #define CB2_TRACE_SELECT(on) ((void)0)
 #endif
 
+// True in one lane of a warp that is together; the compiler knows that what follows is run by one lane.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n"
+               ".reg .pred p;\n"
+               "elect.sync _|p, 0xffffffff;\n"
+               "selp.u32 %0, 1, 0, p;\n"
+               "}\n"
+               : "=r"(one));
+  return one != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -3,9 +3,9 @@
 // explicit row lists).  One persistent CTA per SM takes 128-row tiles of the (sorted)
 // output rows from a scheduler warp (global ticket counter, ring of tiles in shared memory);
 // for every filter offset present in the tile's OR-ed neighbour mask it gathers the 128
-// operand rows into a 128-byte-swizzled shared-memory tile (TMA tile::gather4 for rows of up
-// to 128 bytes, 16-byte cp.async for wider ones; missing neighbours read as zeros), brings the
-// matching weight slice in by TMA, and one warp issues tcgen05.mma into a TMEM accumulator.
+// operand rows into a 128-byte-swizzled shared-memory tile (TMA tile::gather4, a warp per 128-byte
+// column block of a stage; missing neighbours read as zeros), brings the
+// matching weight slice in by TMA, and one thread issues tcgen05.mma into a TMEM accumulator.
 // Eight (fp16) or sixteen (int8) epilogue warps read the accumulator back, apply
 // alpha/beta/bias/activation (or the int8 requantisation) and write the rows to their scattered
 // destinations, whole 32-byte sectors at a time.  No atomics on data: every
@@ -71,7 +71,7 @@ struct RowConvParams {
 #define CB2_ROWCONV_TICKET_BATCH 4
 #endif
 #ifndef CB2_ROWCONV_NARROW_STAGES
-#define CB2_ROWCONV_NARROW_STAGES 6
+#define CB2_ROWCONV_NARROW_STAGES 7
 #endif
 #ifndef CB2_ROWCONV_WIDE_STAGES
 #define CB2_ROWCONV_WIDE_STAGES 4
@@ -80,9 +80,12 @@ struct RowConvParams {
 #define CB2_ROWCONV_EPI_PARTS 4
 #endif
 
-// TMA_GATHER: operand rows are fetched by the TMA unit (tile::gather4, four rows per request,
-// one warp per group) instead of 16-byte cp.async issued by 128 threads per group.  The copy
-// engine path keeps the load/store queues of the SM free for the other roles.
+// TMA_GATHER: operand rows are fetched by the TMA unit (tile::gather4, four rows per request, a warp per
+// 128-byte column block of a stage) instead of 16-byte cp.async issued by 128 threads per group, which only
+// CUMM_B200_GATHER=0 still asks for.  The copy engine path keeps the load/store queues of the SM free for
+// the other roles and leaves the kernel of wide rows at 19 warps instead of 23.  (Rows of 256 bytes, cp.async
+// and gather4, forward: 150 000 uniform rows 28.3 and 26.3 us, 960 000 93.3 and 90.2, 60 000 scanned rows at
+// 256 channels 124 and 117.)
 // MASK_WORDS: mask words per row the ring slots have room for (1: kernel volumes up to 32; 4: up
 // to 128, the reference's "dynamic mask" kernels, cumm/gemm/blockmma/mma.py:78-270).
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MASK_WORDS = 1> struct RowConvCfg {
@@ -92,21 +95,20 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int UMMA_K = 32 / ES;
   static constexpr int KRED = NATOM_K * ATOM_ELEMS;       // reduction elements per stage
   static constexpr int TILE_M = 128;
-  // A stages == producer groups.  What bounds a step is not the bytes of a stage but how many steps are
-  // on their way, so narrow rows have six stages (three: 229 us, six: 218 us for a training step of a
-  // scanned scene at 64 channels, before the issuer was the limit) and wide fp16 rows four, which is
-  // what the shared memory holds (three: 150, four: 132 us for 60 000 rows at 256 channels).  The kernel with sixteen epilogue warps keeps to 24 warps: six per
-  // SM sub-partition leave 80 registers per thread, seven would leave 72 and spill.
+  // What bounds a step is not the bytes of a stage but how many steps are on their way, so narrow fp16 rows
+  // have seven stages (forward and input gradient of 100 003 scanned rows at 64 channels: six 36.4, seven 34.1,
+  // eight 36.0 us; 125 offsets, 30 011 rows: 61.9, 60.6, 58; 2000 rows: 15.4, 14.5, 14.5) and wide fp16 rows
+  // four, which is what the shared memory holds.  int8 keeps five beside sixteen epilogue warps: its stages
+  // hold the weights too.
   static constexpr int SA =
-      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 && BLOCK_N >= 128 ? CB2_ROWCONV_NARROW_STAGES - 1 : CB2_ROWCONV_NARROW_STAGES)
+      TMA_GATHER && NATOM_K == 1 ? (KIND == 1 ? (BLOCK_N >= 128 ? 5 : 6) : CB2_ROWCONV_NARROW_STAGES)
                                  : (KIND == 0 ? CB2_ROWCONV_WIDE_STAGES : 3);
-  // Groups that gather: one warp per stage with the copy engine.  Groups of four warps are three, whatever the
-  // stages, and take the steps in turn: their copies are asynchronous, so a group fills a stage while its
-  // last is on the way.  A fourth group leaves 72 registers a thread instead of 80, which costs every role:
-  // 105 us for the forward pass of 960 000 uniform rows at 128 channels, 91 with three (150 000 rows:
-  // 28.9 and 28.0; 60 000 scanned rows at 256 channels: 125 and 120).
+  // Groups that gather: one per stage with the copy engine.  Groups of four warps (cp.async) are three, whatever
+  // the stages, and take the steps in turn: their copies are asynchronous, so a group fills a stage while its
+  // last is on the way.
   static constexpr int GROUPS = TMA_GATHER ? SA : 3;
   static constexpr int A_STAGE_BYTES = TILE_M * 128 * NATOM_K;
+  static constexpr int ROWIDX_BYTES = TMA_GATHER ? 0 : GROUPS * 2 * 128 * 4;  // row numbers pass through registers
   static constexpr int B_SLOT_BYTES = BLOCK_N * 128 * NATOM_K;
   static constexpr int MW = MASK_WORDS;
   // Outputs wider than BLOCK_N: column parts drawn with the tiles (fp16), or one grid row per part
@@ -114,7 +116,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr bool PARTS = KIND == 0;
   // tile ring slots (four mask words beside wide rows: what is left)
   static constexpr int RING = MASK_WORDS == 1 ? CB2_ROWCONV_RING
-                              : KIND == 0 && !TMA_GATHER ? CB2_ROWCONV_RING / 2 - 1 : CB2_ROWCONV_RING / 2;
+                              : KIND == 0 && NATOM_K == 2 ? CB2_ROWCONV_RING / 2 - 1 : CB2_ROWCONV_RING / 2;
   // fp16: each epilogue warp turns its 32 rows of 64 bytes around in 2 KB of its own before they are stored
   // (600 000 uniform rows, forward: 50.5 -> 44.5 us at 64 channels, 74.5 -> 71.4 at 128).  int8 rows are half
   // as long and their registers all taken: each thread stores its own 32 bytes.
@@ -132,7 +134,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
                        BAR_RING = (BAR_EMPTY_B + 6 + 1) / 2 * 2;
   // Weight slots: as many as fit (2 to 6).  A tile whose mask carries many offsets needs a new
   // weight tile every step, and with two slots the L2 latency of that load bounds the step.
-  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + GROUPS * 2 * 128 * 4 + EPI_BYTES +
+  static constexpr int FIXED_BYTES = SA * A_STAGE_BYTES + ROWIDX_BYTES + EPI_BYTES +
                                      2 * BLOCK_N * 4 + RING * RING_SLOT_INTS * 4 + (BAR_RING + 3 * RING) * 8 + 64 + 1024;
   static constexpr int SB_FIT = (232448 - FIXED_BYTES) / B_SLOT_BYTES;
   static constexpr int SB = JOINT ? SA : SB_FIT < 2 ? 2 : (SB_FIT > 6 ? 6 : SB_FIT);
@@ -150,8 +152,8 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int EPI_GROUPS = (KIND == 1 && BLOCK_N >= 128) ? 2 : 1;
   static_assert(EPI_GROUPS == 1 || EPI_GROUPS == NUM_ACC, "an accumulator belongs to one group");
   static_assert(EPI_BYTES == EPI_WARP_BYTES * EPI_THREADS / 32 || KIND == 1, "every epilogue warp has its bytes");
-  static constexpr int GROUP_THREADS = TMA_GATHER ? 32 : CB2_ROWCONV_GROUP_THREADS;
-  static constexpr int FULL_A_COUNT = JOINT ? 2 : TMA_GATHER ? 1 : GROUP_THREADS;
+  static constexpr int GROUP_THREADS = TMA_GATHER ? 32 * NATOM_K : CB2_ROWCONV_GROUP_THREADS;
+  static constexpr int FULL_A_COUNT = JOINT ? 2 : TMA_GATHER ? NATOM_K : GROUP_THREADS;
   static constexpr int MMA_WARP = EPI_THREADS / 32;
   static constexpr int TMA_WARP = MMA_WARP + 1;
   static constexpr int FIRST_GATHER_WARP = TMA_WARP + 1;
@@ -162,8 +164,8 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + SA * A_STAGE_BYTES;
   static constexpr int OFF_EPI = OFF_B + SB * B_SLOT_BYTES;          // EPI_WARP_BYTES per epilogue warp
-  static constexpr int OFF_ROWIDX = OFF_EPI + EPI_BYTES;             // GROUPS * 2 * 128 ints
-  static constexpr int OFF_SCALE = OFF_ROWIDX + GROUPS * 2 * 128 * 4;  // 2 * BLOCK_N floats
+  static constexpr int OFF_ROWIDX = OFF_EPI + EPI_BYTES;             // ROWIDX_BYTES
+  static constexpr int OFF_SCALE = OFF_ROWIDX + ROWIDX_BYTES;  // 2 * BLOCK_N floats
   static constexpr int OFF_RING = OFF_SCALE + 2 * BLOCK_N * 4;       // RING slots
   static constexpr int OFF_BARS = OFF_RING + RING * RING_SLOT_INTS * 4;  // BAR_RING + 3 * RING mbarriers
   static constexpr int OFF_MISC = OFF_BARS + (BAR_RING + 3 * RING) * 8;  // tmem ptr, abort, flags
@@ -263,9 +265,7 @@ __device__ __forceinline__ int ring_tile_masks(const RowConvParams &p, const int
 // tile's (filter offset, reduction pass) steps itself.  (With slots held until a tile has been issued
 // the look-ahead was too short for tiles with many offsets: 148 instead of 135 us for a training step of
 // a scanned scene at 64 channels.)  Every lane polls for itself: with one lane polling and a shuffle the
-// forward pass of 960 000 uniform rows took 121 instead of 104 us.  A walk that called a function per step, run by one
-// thread, had the MMA issuer at 1500 cycles per step (walk 360, waits 500, four MMAs 260, commits 130),
-// which paced every tile with several offsets.
+// forward pass of 960 000 uniform rows took 121 instead of 104 us.
 template <int MW> struct TileCursor {
   static_assert(MW == 1 || MW == 4, "one mask word, or four");
   int slot = 0;
@@ -276,18 +276,24 @@ template <int MW> struct TileCursor {
   uint32_t m;
   unsigned long long lo, hi;  // four words
   // Returns 1 on a tile, 0 at the end, -1 when the wait gave up.  read(slot) runs before the slot is
-  // given back.
-  template <class ReadFn>
+  // given back.  ALONE: one thread walks for its warp (the MMA issuer).
+  template <bool ALONE = false, class ReadFn>
   __device__ __forceinline__ int next(const RowConvParams &p, const RingView &rv, ReadFn read) {
     const bool ok = mbar_wait(rv.full0 + 8u * slot, phase, rv.abort_flag);
-    if (!__all_sync(0xffffffffu, ok))
+    auto same = [](auto v) {
+      if constexpr (ALONE)
+        return v;
+      else
+        return __shfl_sync(0xffffffffu, v, 0);
+    };
+    if (ALONE ? !ok : !__all_sync(0xffffffffu, ok))
       return -1;
     const int *sl = rv.slot(slot);
     const int4 head = *reinterpret_cast<const int4 *>(sl);
-    tile = __shfl_sync(0xffffffffu, head.x, 0);
-    n0 = __shfl_sync(0xffffffffu, head.w, 0);
+    tile = same(head.x);
+    n0 = same(head.w);
     if constexpr (MW == 1) {
-      m = __shfl_sync(0xffffffffu, static_cast<uint32_t>(head.y), 0);
+      m = same(static_cast<uint32_t>(head.y));
       if (p.reverse_mask)
         m = __brev(m) >> (32 - p.kv);
       offsets = __popc(m);
@@ -296,8 +302,8 @@ template <int MW> struct TileCursor {
       auto join = [](int a, int b) {
         return (static_cast<unsigned long long>(static_cast<uint32_t>(b)) << 32) | static_cast<uint32_t>(a);
       };
-      lo = __shfl_sync(0xffffffffu, join(w.x, w.y), 0);
-      hi = __shfl_sync(0xffffffffu, join(w.z, w.w), 0);
+      lo = same(join(w.x, w.y));
+      hi = same(join(w.z, w.w));
       if (p.reverse_mask) {  // 128 bits reversed, then shifted down by 128 - kv
         const unsigned long long rl = __brevll(hi), rh = __brevll(lo);
         const int s = 128 - p.kv;
@@ -307,8 +313,9 @@ template <int MW> struct TileCursor {
       offsets = __popcll(lo) + __popcll(hi);
     }
     read(sl);
-    __syncwarp();
-    if (lane_id() == 0)
+    if constexpr (!ALONE)
+      __syncwarp();
+    if (ALONE || lane_id() == 0)
       mbar_arrive(rv.empty0 + 8u * slot);
     if (++slot == rv.ring) {
       slot = 0;
@@ -917,74 +924,79 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     if (et == 0)
       CB2_PROF_END2();
   } else if (warp == Cfg::MMA_WARP) {
-    // ======================= MMA issuer: the warp walks together (its state is the same in every
-    // lane), lane 0 issues
-    constexpr uint32_t idesc = make_idesc(KIND, false, B_MN, 128, BLOCK_N);
-    constexpr int KSTEPS_FULL = NATOM_K * 4;
-    const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_A, 16, 1024);
-    const uint64_t bdesc_base = B_MN ? make_smem_desc(sbase + Cfg::OFF_B, p.b_lbo, p.b_sbo)
-                                     : make_smem_desc(sbase + Cfg::OFF_B, 16, 1024);
-    const int ksteps_last = (p.red - (kpasses - 1) * Cfg::KRED + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
-    TileCursor<MW> tc;
-    int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
-    uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
-    bool ok = true;
-    CB2_PROF_BEGIN();
-    for (int more; ok && (more = tc.next(p, rv, [](const int *) {})) != 0;) {
-      CB2_PROF_MARK(0);  // next tile
-      if (more < 0) {
-        ok = false;
-        break;
-      }
-      if (tc.offsets == 0)
-        continue;
-      // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
-      // are in the key: weights have as many columns)
-      bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
-      ok = mbar_wait(acc_empty(buf), acc_phase, abort_flag);
-      CB2_PROF_MARK(1);  // accumulator free
-      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
-      const int total = tc.offsets * kpasses;
-      int kp = 0;
-      for (int s = 0; s < total; ++s) {
-        if constexpr (Cfg::JOINT) {
-          bslot = stage;
-        } else {
-          if (new_b) {
-            if (last_key >= 0 && lane == 0)
-              tc_commit(empty_b(bslot));
-            last_key = 0;
-            if (++bslot == Cfg::SB) {
-              bslot = 0;
-              b_phase ^= 1u;
-            }
+    // ======================= MMA issuer: one thread, from the walk to the commits.  It paces tiles with
+    // several offsets.  Elected, so that the compiler keeps descriptors in uniform registers: with lane 0
+    // chosen by its number four MMAs took 310 cycles of a step's 1000, elected 100; a thread that walks by itself
+    // needs no votes between them.  (Warp that walks together, lane 0 by number / the same, elected to issue /
+    // one thread, before the gathers were sped up: 30 011 rows of 125 offsets 87 / 79 / 77.8 us, 100 003 scanned
+    // rows at 64 channels 42.5 / 39.5 / 39.8, after: - / 73 / 60.6 and - / 35.7 / 34.1.)  Whoever is waited for
+    // next is looked at as soon as a step is committed.
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc(KIND, false, B_MN, 128, BLOCK_N);
+      constexpr int KSTEPS_FULL = NATOM_K * 4;
+      const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_A, 16, 1024);
+      const uint64_t bdesc_base = B_MN ? make_smem_desc(sbase + Cfg::OFF_B, p.b_lbo, p.b_sbo)
+                                       : make_smem_desc(sbase + Cfg::OFF_B, 16, 1024);
+      const int ksteps_last = (p.red - (kpasses - 1) * Cfg::KRED + Cfg::UMMA_K - 1) / Cfg::UMMA_K;
+      TileCursor<MW> tc;
+      int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
+      uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
+      bool ok = true;
+      CB2_PROF_BEGIN();
+      for (int more; ok && (more = tc.template next<true>(p, rv, [](const int *) {})) != 0;) {
+        CB2_PROF_MARK(0);  // next tile
+        if (more < 0) {
+          ok = false;
+          break;
+        }
+        if (tc.offsets == 0)
+          continue;
+        // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
+        // are in the key: weights have as many columns)
+        const bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
+        auto next_b = [&]() {
+          if (++bslot == Cfg::SB) {
+            bslot = 0;
+            b_phase ^= 1u;
           }
-          const bool b_there = mbar_test(full_b(bslot), b_phase);
+        };
+        if (!Cfg::JOINT && new_b) {
+          if (last_key >= 0)
+            tc_commit(empty_b(bslot));
+          next_b();
+        }
+        ok = mbar_wait(acc_empty(buf), acc_phase, abort_flag);
+        CB2_PROF_MARK(1);  // accumulator free
+        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BLOCK_N);
+        const int total = tc.offsets * kpasses;
+        int kp = 0;
+        bool a_there = mbar_test(full_a(stage), a_phase), b_there = Cfg::JOINT || mbar_test(full_b(bslot), b_phase);
+        for (int s = 0; s < total; ++s) {
+          if constexpr (Cfg::JOINT)
+            bslot = stage;
           if (!b_there)
             ok = ok && mbar_wait(full_b(bslot), b_phase, abort_flag);
-        }
-        CB2_PROF_MARK(2);  // weight tile present
-        ok = ok && mbar_wait(full_a(stage), a_phase, abort_flag);
-        CB2_PROF_MARK(3);  // rows present
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok)
-          break;
-        if constexpr (!TMA_GATHER)
-          fence_proxy_async_smem();  // gathered rows were written through the generic proxy
-        tc_fence_after();
-        // descriptors differ from the stage's / slot's base descriptor only in the start address field
-        // (bits 0-13, units of 16 bytes)
-        const uint64_t adesc0 = adesc_base + static_cast<uint64_t>((stage * Cfg::A_STAGE_BYTES) >> 4);
-        const uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((bslot * Cfg::B_SLOT_BYTES) >> 4);
-        auto issue = [&](int ks, uint32_t acc) {
-          const int ka = ks >> 2, kk = ks & 3;
-          const uint64_t adesc = adesc0 + static_cast<uint64_t>((ka * (Cfg::TILE_M * 128) + kk * 32) >> 4);
-          const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(B_MN ? (((ka * 4 + kk) * (Cfg::UMMA_K * 128)) >> 4)
-                                                                     : ((ka * (BLOCK_N * 128) + kk * 32) >> 4));
-          tc_mma<KIND>(d_tmem, adesc, bdesc, idesc, acc);
-        };
-        const bool last_pass = ++kp == kpasses;
-        if (lane == 0) {
+          CB2_PROF_MARK(2);  // weight tile present
+          if (!a_there)
+            ok = ok && mbar_wait(full_a(stage), a_phase, abort_flag);
+          CB2_PROF_MARK(3);  // rows present
+          if (!ok)
+            break;
+          if constexpr (!TMA_GATHER)
+            fence_proxy_async_smem();  // gathered rows were written through the generic proxy
+          tc_fence_after();
+          // descriptors differ from the stage's / slot's base descriptor only in the start address field
+          // (bits 0-13, units of 16 bytes)
+          const uint64_t adesc0 = adesc_base + static_cast<uint64_t>((stage * Cfg::A_STAGE_BYTES) >> 4);
+          const uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((bslot * Cfg::B_SLOT_BYTES) >> 4);
+          auto issue = [&](int ks, uint32_t acc) {
+            const int ka = ks >> 2, kk = ks & 3;
+            const uint64_t adesc = adesc0 + static_cast<uint64_t>((ka * (Cfg::TILE_M * 128) + kk * 32) >> 4);
+            const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(B_MN ? (((ka * 4 + kk) * (Cfg::UMMA_K * 128)) >> 4)
+                                                                       : ((ka * (BLOCK_N * 128) + kk * 32) >> 4));
+            tc_mma<KIND>(d_tmem, adesc, bdesc, idesc, acc);
+          };
+          const bool last_pass = ++kp == kpasses;
           if (!last_pass || ksteps_last == KSTEPS_FULL) {
 #pragma unroll
             for (int ks = 0; ks < KSTEPS_FULL; ++ks)
@@ -995,27 +1007,31 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           }
           CB2_PROF_MARK(5);  // MMAs issued
           tc_commit(empty_a(stage));
-          if (s == total - 1)
+          if (last_pass)
+            kp = 0;
+          if (++stage == Cfg::SA) {
+            stage = 0;
+            a_phase ^= 1u;
+          }
+          ++steps;
+          if (s == total - 1) {
             tc_commit(acc_full(buf));
+          } else {
+            if (!Cfg::JOINT) {
+              tc_commit(empty_b(bslot));
+              next_b();
+              b_there = mbar_test(full_b(bslot), b_phase);
+            }
+            a_there = mbar_test(full_a(stage), a_phase);
+          }
+          CB2_PROF_MARK(6);  // commits
         }
-        __syncwarp();
-        CB2_PROF_MARK(6);  // commits
-        if (last_pass)
-          kp = 0;
-        if (++stage == Cfg::SA) {
-          stage = 0;
-          a_phase ^= 1u;
+        last_key = (tc.last_offset() * kpasses + kpasses - 1) * p.nn + tc.n0;
+        if (++buf == Cfg::NUM_ACC) {
+          buf = 0;
+          acc_phase ^= 1u;
         }
-        new_b = true;
-        ++steps;
       }
-      last_key = (tc.last_offset() * kpasses + kpasses - 1) * p.nn + tc.n0;
-      if (++buf == Cfg::NUM_ACC) {
-        buf = 0;
-        acc_phase ^= 1u;
-      }
-    }
-    if (lane == 0) {
       CB2_TRACE_CTA(2, (unsigned long long)steps);
       CB2_PROF_END();
       if (!ok) {
@@ -1081,97 +1097,98 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   } else {
     // ======================= operand-row gather: group g owns stage g
     if constexpr (TMA_GATHER) {
-      // One warp per group; lane L fetches tile rows 4L .. 4L+3 ("its quad") with one request
-      // per 128-byte column block.  A quad none of whose rows has a neighbour at this offset is
+      // One warp per group and 128-byte column block; lane L fetches tile rows 4L .. 4L+3 ("its quad") with
+      // one request.  A quad none of whose rows has a neighbour at this offset is
       // not requested at all -- for the offsets away from the centre that is most quads, and the
       // copy engine's request rate is what bounds such steps.  The stage therefore keeps the
       // invariant "a quad that was not requested holds zeros": it is cleared once here, and a
-      // quad that was filled in the previous use and is not refilled now is cleared again.
-      const int g = warp - Cfg::FIRST_GATHER_WARP;
+      // quad that was filled in the previous use and is not needed now is requested with no row at all
+      // (cleared by stores and a proxy fence instead: 36.5 against 36.0 us, 100 003 scanned rows at 64 channels).
+      // The neighbour indices of the group's next step in the tile are on their way while it waits for its stage
+      // (the same scene: 39.8 -> 36.4 us; 125 offsets, 30 011 rows: 77 -> 61).
+      const int g = (warp - Cfg::FIRST_GATHER_WARP) / NATOM_K;
+      const int part = (warp - Cfg::FIRST_GATHER_WARP) % NATOM_K;
       if (lane == 0)
         tma_prefetch_desc(&tmap_a);
-      const uint32_t first_quad = sbase + Cfg::OFF_A + g * Cfg::A_STAGE_BYTES;
+      const uint32_t first_quad = sbase + Cfg::OFF_A + g * Cfg::A_STAGE_BYTES + part * (Cfg::TILE_M * 128);
       const uint32_t my_quad = first_quad + lane * (4 * 128);
-      // The warp clears one quad at a time, every lane 16 of its 512 bytes: with a quad per lane the
-      // lanes' addresses are 512 bytes apart and all meet in the same banks.
-      auto clear_quads = [&](uint32_t quads) {
-        for (; quads; quads &= quads - 1) {
-          const uint32_t at = first_quad + (__ffs(quads) - 1) * (4 * 128) + lane * 16;
-#pragma unroll
-          for (int ka = 0; ka < NATOM_K; ++ka)
-            st_shared_zero16(at + ka * (Cfg::TILE_M * 128));
-        }
-        fence_proxy_async_smem();  // generic-proxy stores, read by the tensor core
-      };
-      clear_quads(0xffffffffu);
+      for (int q = 0; q < 32; ++q)
+        st_shared_zero16(first_quad + q * (4 * 128) + lane * 16);
+      fence_proxy_async_smem();  // generic-proxy stores, read by the tensor core
       __syncwarp();
       uint32_t dirty = 0;  // quads of this stage that hold gathered rows
       bool dep_waited = false, ok = true;
-      int stage = 0;         // stage of the CTA's next step
-      uint32_t phase = 1;    // of this warp's own stage
+      int stage = 0;         // stage of the CTA's next tile's first step
+      uint32_t phase = 1;    // of this group's own stage
       TileCursor<MW> tc;
       int4 o = make_int4(-1, -1, -1, -1);
       for (int more; ok && (more = tc.next(p, rv, [&](const int *sl) {
                              o = *reinterpret_cast<const int4 *>(sl + 8 + lane * 4);
                            })) != 0;) {
         ok = more > 0;
-        for (int left = ok ? tc.offsets : 0; ok && left > 0; --left) {
-          const int f = tc.take();
-          for (int kp = 0; kp < kpasses; ++kp) {
-            const bool mine = stage == g;
-            if (++stage == Cfg::SA)
-              stage = 0;
-            if (!mine)
-              continue;
-            const int row[4] = {o.x, o.y, o.z, o.w};
-            int idx[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-              idx[r] = -1;
-              if (row[r] >= 0) {
-                if (p.mode == kModeMaskConv)
-                  idx[r] = __ldg(p.indices + (long long)f * p.n_rows + row[r]);
-                else
-                  idx[r] = p.a_inds ? __ldg(p.a_inds + row[r]) : row[r];
-              }
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-              if (idx[r] >= p.a_rows) {  // reported; the copy engine would read such a row as zeros
-                fail(kStatusBadIndex);
-                idx[r] = -1;
-              }
-            if (lane == 0)
-              CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
-            ok = mbar_wait_warp(empty_a(g), phase, abort_flag);
-            if (!ok)
-              break;
-            phase ^= 1u;
-            if (!dep_waited) {
-              grid_dep_wait();
-              dep_waited = true;
-            }
-            const bool wanted = (idx[0] & idx[1] & idx[2] & idx[3]) >= 0;  // some row index is not -1
-            const uint32_t need = __ballot_sync(0xffffffffu, wanted);
-            if (dirty & ~need)
-              clear_quads(dirty & ~need);
-            __syncwarp();
-            if (lane == 0) {
-              CB2_TRACE_EVENT(g, 2, f);  // stage free
-              mbar_arrive_expect_tx(full_a(g), static_cast<uint32_t>(__popc(need)) * (NATOM_K * 512));
-            }
-            __syncwarp();
-            if (wanted) {
-#pragma unroll
-              for (int ka = 0; ka < NATOM_K; ++ka)
-                tma_gather4(my_quad + ka * (Cfg::TILE_M * 128), &tmap_a, full_a(g), kp * Cfg::KRED + ka * Cfg::ATOM_ELEMS,
-                            row_or_zeros(idx[0], 4 * lane), row_or_zeros(idx[1], 4 * lane + 1),
-                            row_or_zeros(idx[2], 4 * lane + 2), row_or_zeros(idx[3], 4 * lane + 3));
-            }
-            dirty = need;
-            if (lane == 0)
-              CB2_TRACE_EVENT(g, 3, f);  // copies issued
+        const int total = ok ? tc.offsets * kpasses : 0;
+        int f = -1, upto = 0;  // the offset taken last, and the first step that needs the next one
+        auto look_up = [&](int step, int (&idx)[4], int &kp) {
+          while (step >= upto) {
+            f = tc.take();
+            upto += kpasses;
           }
+          kp = step - (upto - kpasses);
+          const int row[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            idx[r] = -1;
+            if (row[r] >= 0) {
+              if (p.mode == kModeMaskConv)
+                idx[r] = __ldg(p.indices + (long long)f * p.n_rows + row[r]);
+              else
+                idx[r] = p.a_inds ? __ldg(p.a_inds + row[r]) : row[r];
+            }
+          }
+        };
+        int ahead[4], ahead_kp = 0;
+        int step = g - stage + (g < stage ? Cfg::SA : 0);
+        stage = (stage + total) % Cfg::SA;
+        if (step < total)
+          look_up(step, ahead, ahead_kp);
+        for (; step < total; step += Cfg::SA) {
+          int idx[4];
+          const int kp = ahead_kp;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            idx[r] = ahead[r];
+            if (idx[r] >= p.a_rows) {  // reported; the copy engine would read such a row as zeros
+              fail(kStatusBadIndex);
+              idx[r] = -1;
+            }
+          }
+          if (step + Cfg::SA < total)
+            look_up(step + Cfg::SA, ahead, ahead_kp);
+          if (lane == 0)
+            CB2_TRACE_EVENT(g, 1, f + (idx[0] == 0x7fffffff));  // index loaded
+          ok = mbar_wait_warp(empty_a(g), phase, abort_flag);
+          if (!ok)
+            break;
+          phase ^= 1u;
+          if (!dep_waited) {
+            grid_dep_wait();
+            dep_waited = true;
+          }
+          const bool wanted = (idx[0] & idx[1] & idx[2] & idx[3]) >= 0;  // some row index is not -1
+          const uint32_t need = __ballot_sync(0xffffffffu, wanted);
+          const uint32_t ask = need | dirty;
+          if (lane == 0) {
+            CB2_TRACE_EVENT(g, 2, f);  // stage free
+            mbar_arrive_expect_tx(full_a(g), static_cast<uint32_t>(__popc(ask)) * 512);
+          }
+          __syncwarp();
+          if ((ask >> lane) & 1u)
+            tma_gather4(my_quad, &tmap_a, full_a(g), kp * Cfg::KRED + part * Cfg::ATOM_ELEMS,
+                        row_or_zeros(idx[0], 4 * lane), row_or_zeros(idx[1], 4 * lane + 1),
+                        row_or_zeros(idx[2], 4 * lane + 2), row_or_zeros(idx[3], 4 * lane + 3));
+          dirty = need;
+          if (lane == 0)
+            CB2_TRACE_EVENT(g, 3, f);  // copies issued
         }
       }
       if (!ok && lane == 0)

@@ -327,6 +327,22 @@ def test_wide_rows_many_steps_per_cta(torch, oracle, n, grid, C, max_ctas):
     H.assert_close_f16(got, want, f"n={n} C={C} max_ctas={max_ctas}")
 
 
+@pytest.mark.parametrize("max_ctas", [1, 5])
+@pytest.mark.parametrize("C", [8, 40, 64, 200])  # one pass with and without a ragged end, four passes of 64
+@pytest.mark.parametrize("n,grid", [(1, (8, 24, 24)), (2300, (8, 24, 24)), (3000, (41, 300, 300))])
+def test_narrow_rows_many_steps_per_cta(torch, oracle, n, grid, C, max_ctas):
+    """The same for the seven stages of narrow rows: quads of a stage that hold rows in one step and none in
+    the next, steps whose indices were looked up while the one before was waited for."""
+    tb = W.build_tables(W.sample_coords(n, 470 + n, grid), grid=grid)
+    rng = np.random.default_rng(471)
+    x = rng.standard_normal((tb.n_in, C)).astype(np.float16)
+    w = (rng.standard_normal((48, 27, C)) / np.sqrt(27 * C) * 4).astype(np.float16)
+    got, _ = H.run_conv_fwd(torch, x, w, tb, max_ctas=max_ctas, tile=[128, 64, 64])
+    H.check_status()
+    want = oracle.mask_igemm(x, w, np.zeros((n, 48), np.float16), tb.indices, tb.mask, tb.mask_argsort)
+    H.assert_close_f16(got, want, f"n={n} C={C} max_ctas={max_ctas}")
+
+
 def test_errors_surface_as_exceptions(torch):
     tb, x, w, _ = make(300, 501, 64, 64)
     p = ConvParams(3, ConvOpType.Forward)
