@@ -242,11 +242,13 @@ int plan_rowconv(int kind, int red, int nn, bool b_mn, int tile_n, int tile_k, R
 
 int launch_rowconv(const RowConvPlan &pl, const CUtensorMap &map, const CUtensorMap &map_a, bool tma_gather,
                    const RowConvParams &p, int gx, int gy, cudaStream_t s) {
-  // Kernel volumes above 32 (several mask words per row): one variant per shape.
+  // Kernel volumes above 32 (several mask words per row): no cp.async variant for rows of up to 128
+  // bytes.
 #define CB2_INST(K, A, N, M)                                                                      \
   if (pl.kind == K && pl.natom_k == A && pl.block_n == N && pl.b_mn == M) {                        \
     if (p.mask_words > 1)                                                                          \
-      return launch_rowconv_inst<K, A, N, M, true, 4>(map, map_a, p, gx, gy, s);               \
+      return tma_gather ? launch_rowconv_inst<K, A, N, M, true, 4>(map, map_a, p, gx, gy, s)       \
+                        : launch_rowconv_inst<K, A, N, M, A == 1, 4>(map, map_a, p, gx, gy, s);    \
     return tma_gather ? launch_rowconv_inst<K, A, N, M, true>(map, map_a, p, gx, gy, s)            \
                       : launch_rowconv_inst<K, A, N, M, false>(map, map_a, p, gx, gy, s);          \
   }
@@ -290,9 +292,16 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
                        b_mn ? kred : pl.block_n);
   if (rc)
     return rc;
-  // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes);
-  // CUMM_B200_GATHER=0 has 16-byte cp.async instead.
-  const bool tma_gather = p.mask_words > 1 || gather_mode() != 0;
+  // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes) where the rows
+  // lie so that no 128-byte column block crosses a 128-byte line; others by 16-byte cp.async, which spreads the
+  // lines' sectors over more requests in flight.  (60 000 scanned rows, forward, us, gather4 and cp.async: 24
+  // channels 38.4 and 37.3, 40 36.5 and 34.5, 72 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
+  // 46.9, 120 57.9 and 52.8, but 128 44.4 and 46.8; 64 channels, 100 003 rows, 34 and 43.)  CUMM_B200_GATHER forces one path.  Rows of up to 128 bytes with several mask
+  // words have gather4 only.
+  const uint64_t pitch = static_cast<uint64_t>(p.lda) * es;
+  const uint64_t line = std::min<uint64_t>(pitch, 128);
+  const bool in_lines = 128 % line == 0 && pitch % line == 0 && reinterpret_cast<uintptr_t>(p.a) % line == 0;
+  const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) || (getenv("CUMM_B200_GATHER") ? gather_mode() != 0 : in_lines);
   CUtensorMap map_a;
   memset(&map_a, 0, sizeof(map_a));
   if (tma_gather) {

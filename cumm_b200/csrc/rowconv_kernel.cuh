@@ -4,7 +4,7 @@
 // output rows from a scheduler warp (global ticket counter, ring of tiles in shared memory);
 // for every filter offset present in the tile's OR-ed neighbour mask it gathers the 128
 // operand rows into a 128-byte-swizzled shared-memory tile (TMA tile::gather4, a warp per 128-byte
-// column block of a stage; missing neighbours read as zeros), brings the
+// column block of a stage, or 16-byte cp.async; missing neighbours read as zeros), brings the
 // matching weight slice in by TMA, and one thread issues tcgen05.mma into a TMEM accumulator.
 // Eight (fp16) or sixteen (int8) epilogue warps read the accumulator back, apply
 // alpha/beta/bias/activation (or the int8 requantisation) and write the rows to their scattered
@@ -81,11 +81,11 @@ struct RowConvParams {
 #endif
 
 // TMA_GATHER: operand rows are fetched by the TMA unit (tile::gather4, four rows per request, a warp per
-// 128-byte column block of a stage) instead of 16-byte cp.async issued by 128 threads per group, which only
-// CUMM_B200_GATHER=0 still asks for.  The copy engine path keeps the load/store queues of the SM free for
+// 128-byte column block of a stage) instead of 16-byte cp.async issued by 128 threads per group (see run_rowconv for
+// which).  The copy engine path keeps the load/store queues of the SM free for
 // the other roles and leaves the kernel of wide rows at 19 warps instead of 23.  (Rows of 256 bytes, cp.async
-// and gather4, forward: 150 000 uniform rows 28.3 and 26.3 us, 960 000 93.3 and 90.2, 60 000 scanned rows at
-// 256 channels 124 and 117.)
+// and gather4, forward: 150 000 uniform rows 28.3 and 26.3 us, 960 000 93.3 and 87.5, 60 000 scanned rows at
+// 256 channels 124 and 112.)
 // MASK_WORDS: mask words per row the ring slots have room for (1: kernel volumes up to 32; 4: up
 // to 128, the reference's "dynamic mask" kernels, cumm/gemm/blockmma/mma.py:78-270).
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MASK_WORDS = 1> struct RowConvCfg {
