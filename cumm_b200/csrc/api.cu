@@ -292,16 +292,14 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
                        b_mn ? kred : pl.block_n);
   if (rc)
     return rc;
-  // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes) where the rows
-  // lie so that no 128-byte column block crosses a 128-byte line; others by 16-byte cp.async, which spreads the
-  // lines' sectors over more requests in flight.  (60 000 scanned rows, forward, us, gather4 and cp.async: 24
-  // channels 38.4 and 37.3, 40 36.5 and 34.5, 72 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
-  // 46.9, 120 57.9 and 52.8, but 128 44.4 and 46.8; 64 channels, 100 003 rows, 34 and 43.)  CUMM_B200_GATHER forces one path.  Rows of up to 128 bytes with several mask
-  // words have gather4 only.
-  const uint64_t pitch = static_cast<uint64_t>(p.lda) * es;
-  const uint64_t line = std::min<uint64_t>(pitch, 128);
-  const bool in_lines = 128 % line == 0 && pitch % line == 0 && reinterpret_cast<uintptr_t>(p.a) % line == 0;
-  const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) || (getenv("CUMM_B200_GATHER") ? gather_mode() != 0 : in_lines);
+  // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes), but rows of
+  // more than 128 bytes whose column blocks cross 128-byte lines by 16-byte cp.async.  (60 000 scanned rows,
+  // forward, us, gather4 and cp.async: 72 channels 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
+  // 46.9, 120 57.9 and 52.8, 128 44.4 and 46.8; of one column block: 40 36.5 and 34.5, 64 -- 100 003 rows -- 34 and
+  // 43; int8 128, stride 2, 41 and 70.)  CUMM_B200_GATHER forces one path.
+  const bool in_lines = (reinterpret_cast<uintptr_t>(p.a) | static_cast<uintptr_t>(p.lda * es)) % 128 == 0;
+  const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) ||
+                          (getenv("CUMM_B200_GATHER") ? gather_mode() != 0 : (pl.natom_k == 1 || in_lines));
   CUtensorMap map_a;
   memset(&map_a, 0, sizeof(map_a));
   if (tma_gather) {
