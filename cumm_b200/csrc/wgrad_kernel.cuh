@@ -167,7 +167,9 @@ __device__ __forceinline__ void wgrad_scan4(const int (&v)[4], int (&excl)[4], i
 // A unit costs its CTA about as much as kWgradUnitSteps steps (a partial sum stored, counted in, and
 // read again by whoever sums): every offset is charged that many steps before its own, or the CTAs that
 // get a dozen offsets of one or two steps each are the last to finish.  The cuts are made in charged steps.
-constexpr int kWgradUnitSteps = 2;
+// (Two, three, four and six steps, us: 150 000 uniform rows at 128 channels 32.0, 31.1, 31.5, 33.3; 60 000, 128 to 64
+// 20.8, 19.6, 21.0, 21.0; 1600 scanned rows 17.7, 17.3, 16.8, 16.3; 100 003 at 64 channels 35.2, 35.4, 35.3, 35.4.)
+constexpr int kWgradUnitSteps = 3;
 // Given the step counts of this lane's offsets: P = charged steps before the offset's first own step,
 // T = all charged steps, c_first = CTA holding the offset's first step, S = units of the offset, U = units
 // before it.
@@ -769,6 +771,11 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     int stage = 0, acc_use = 0;
     uint32_t phase = 0;
     bool ok_all = true;
+    // The lane that issues.  Elected, the descriptors stay in uniform registers and a step costs the issuer a third:
+    // 100 003 scanned rows at 64 channels 40.2 -> 35.3 us, 30 011 rows of 125 offsets 31.7 -> 27.4.  Launches of
+    // the widest tiles, three stages, wait for memory; stages given back sooner only crowd it (960 000
+    // uniform rows 106.2 -> 108.4).
+    auto issuer = [&]() { return Cfg::SA > 3 ? elect_one() : lane == 0; };
     const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES, 128 * 128, 1024);
     const uint64_t bdesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES + Cfg::A_BYTES, 128 * 128, 1024);
     wgrad_walk(
@@ -794,7 +801,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           const uint64_t adesc = adesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
           const uint64_t bdesc = bdesc_base + static_cast<uint64_t>((stage * Cfg::STAGE_BYTES) >> 4);
           const int rows = __shfl_sync(0xffffffffu, wgrad_step_rows(p, e, tile), 0);
-          if (lane == 0) {
+          if (issuer()) {
             if (rows >= 128) {
 #pragma unroll
               for (int ks = 0; ks < 8; ++ks)
@@ -815,14 +822,14 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
         },
         [&](int, int, int active) -> bool {
           if (active > 0) {
-            if (lane == 0)
+            if (issuer())
               tc_commit(acc_full(acc_use & 1));
             __syncwarp();
             ++acc_use;
           }
           return true;
         });
-    if (lane == 0 && ok_all) {
+    if (ok_all && issuer()) {
       tc_commit(final_bar);
       if (!mbar_wait(final_bar, 0, abort_flag))
         fail(kStatusWaitTimeout);
