@@ -164,7 +164,7 @@ int gather_mode() {
 // (only with CUMM_B200_PDL=2): the fp16 convolution row kernels.  CUMM_B200_PDL=0 launches everything the
 // ordinary way.
 template <class Kern, class... Args>
-cudaError_t launch_after(int level, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                          Args... args) {
   static const int enabled = [] {
     const char *v = getenv("CUMM_B200_PDL");
@@ -177,19 +177,72 @@ cudaError_t launch_after(int level, Kern kern, dim3 grid, dim3 block, size_t sme
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  if (pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MW = 1>
+// How many CTAs share an item's filter offsets in a launch whose items leave most SMs idle: 4 or 8 where the clusters
+// fit the CTAs the launch may have and are all resident at once (each has one item), and a CTA has two offsets of a
+// full tile or more; else 1.  `resident`: per device, clusters of 4 and 8 CTAs of this kernel that it holds, plus
+// one (0 = not asked yet).
+using ResidentClusters = std::atomic<int>[kMaxDevices][2];
+template <class Kern>
+int cluster_split(Kern kern, ResidentClusters &resident, int threads, int smem, int max_ctas, long long items, int kv) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+    return 1;
+  for (int e = 1; e >= 0; --e) {
+    const int split = 4 << e;
+    if (items * split > max_ctas || kv < 2 * split)
+      continue;
+    int n = resident[dev][e].load();
+    if (n == 0) {
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(split);
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = split;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int found = 0;
+      if (cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        found = 0;
+      }
+      n = found + 1;
+      resident[dev][e].store(n);
+    }
+    if (items <= n - 1)
+      return split;
+  }
+  return 1;
+}
+
+template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MW = 1, bool SPLIT = false>
 int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const RowConvParams &p, int gx, int gy,
-                        cudaStream_t stream) {
+                        int max_ctas, cudaStream_t stream) {
   using Cfg = RowConvCfg<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW>;
-  auto kern = rowconv_kernel<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW>;
+  auto kern = rowconv_kernel<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, SPLIT>;
+  if constexpr (!SPLIT && KIND == 0 && TMA_GATHER) {
+    const long long items = (p.n_rows + 127) / 128 * static_cast<long long>(p.n_parts);
+    if (p.mode == kModeMaskConv && 4 * items <= max_ctas && p.kv >= 8)
+      return launch_rowconv_inst<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, true>(map, map_a, p, gx, gy, max_ctas, stream);
+  }
   static std::atomic<uint64_t> configured{0};  // bit per device
   static std::atomic<int> regs{0};
   int dev = 0;
@@ -199,6 +252,12 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
     regs.store(kernel_regs(kern));
     configured.fetch_or(1ull << dev);
   }
+  RowConvParams q = p;
+  q.split = 1;
+  if constexpr (SPLIT) {
+    static ResidentClusters resident;
+    q.split = cluster_split(kern, resident, Cfg::THREADS, Cfg::SMEM_BYTES, max_ctas, gx, p.kv);
+  }
   g_last_launch.num_regs = regs.load();
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
@@ -206,9 +265,10 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   // overlapping each kernel's set-up with its predecessor's tail nearly halves the run.  For the
   // convolutions it measured +4 % for the int8 kernels (long epilogue tail) and neutral to
   // slightly worse for fp16, so only the former take part by default.
-  const int pdl_level = p.mode != kModeMaskConv ? 1 : (KIND == 1 ? 1 : 2);
-  CB2_CUDA(launch_after(pdl_level, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, map,
-                        map_a, p));
+  // So do launches that clusters share: they leave SMs free for their successor, and draw no tickets.
+  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || q.split > 1 ? 1 : 2;
+  CB2_CUDA(launch_after(pdl_level, q.split, kern, dim3(gx * q.split, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
+                        map, map_a, q));
   g_launches.fetch_add(1);
   return CB2_OK;
 }
@@ -241,16 +301,16 @@ int plan_rowconv(int kind, int red, int nn, bool b_mn, int tile_n, int tile_k, R
 }
 
 int launch_rowconv(const RowConvPlan &pl, const CUtensorMap &map, const CUtensorMap &map_a, bool tma_gather,
-                   const RowConvParams &p, int gx, int gy, cudaStream_t s) {
+                   const RowConvParams &p, int gx, int gy, int max_ctas, cudaStream_t s) {
   // Kernel volumes above 32 (several mask words per row): no cp.async variant for rows of up to 128
   // bytes.
 #define CB2_INST(K, A, N, M)                                                                      \
   if (pl.kind == K && pl.natom_k == A && pl.block_n == N && pl.b_mn == M) {                        \
     if (p.mask_words > 1)                                                                          \
-      return tma_gather ? launch_rowconv_inst<K, A, N, M, true, 4>(map, map_a, p, gx, gy, s)       \
-                        : launch_rowconv_inst<K, A, N, M, A == 1, 4>(map, map_a, p, gx, gy, s);    \
-    return tma_gather ? launch_rowconv_inst<K, A, N, M, true>(map, map_a, p, gx, gy, s)            \
-                      : launch_rowconv_inst<K, A, N, M, false>(map, map_a, p, gx, gy, s);          \
+      return tma_gather ? launch_rowconv_inst<K, A, N, M, true, 4>(map, map_a, p, gx, gy, max_ctas, s)       \
+                        : launch_rowconv_inst<K, A, N, M, A == 1, 4>(map, map_a, p, gx, gy, max_ctas, s);    \
+    return tma_gather ? launch_rowconv_inst<K, A, N, M, true>(map, map_a, p, gx, gy, max_ctas, s)            \
+                      : launch_rowconv_inst<K, A, N, M, false>(map, map_a, p, gx, gy, max_ctas, s);          \
   }
   CB2_INST(0, 1, 64, false)
   CB2_INST(0, 1, 128, false)
@@ -330,7 +390,7 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
   CB2_CHECK_RT(items < (1ll << 30), "too many output tiles (%lld)", items);
   const int sms = (max_ctas > 0 && max_ctas < dev->num_sms) ? max_ctas : dev->num_sms;
   const int gx = static_cast<int>(std::min<long long>(std::max(sms / gy, 1), items));
-  return launch_rowconv(pl, map, map_a, tma_gather, p, gx, gy, stream);
+  return launch_rowconv(pl, map, map_a, tma_gather, p, gx, gy, sms, stream);
 }
 
 // ---------------------------------------------------------------- weight gradient
@@ -396,7 +456,7 @@ int launch_wgrad_inst(const CUtensorMap &ma, const CUtensorMap &mb, const WgradP
   g_last_launch.num_regs = regs.load();
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
-  CB2_CUDA(launch_after(1, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, ma, mb, p));
+  CB2_CUDA(launch_after(1, 1, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, ma, mb, p));
   g_launches.fetch_add(1);
   return CB2_OK;
 }
@@ -445,7 +505,7 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
     int2 *counts = reinterpret_cast<int2 *>(ws + L.off_counts);
     wgrad_mark_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, L.n_ctl);
     CB2_CUDA(cudaGetLastError());
-    CB2_CUDA(launch_after(1, wgrad_list_rows_kernel, grid, dim3(kWgradPlanThreads), 0, stream, p, bits, counts,
+    CB2_CUDA(launch_after(1, 1, wgrad_list_rows_kernel, grid, dim3(kWgradPlanThreads), 0, stream, p, bits, counts,
                           reinterpret_cast<int *>(ws + L.off_lists), reinterpret_cast<int *>(ws + L.off_rows),
                           L.row_capacity));
     g_launches.fetch_add(2);

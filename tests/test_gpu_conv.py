@@ -343,6 +343,66 @@ def test_narrow_rows_many_steps_per_cta(torch, oracle, n, grid, C, max_ctas):
     H.assert_close_f16(got, want, f"n={n} C={C} max_ctas={max_ctas}")
 
 
+@pytest.mark.parametrize("ksize,n,C,K", [((3, 3, 3), 1, 64, 64), ((3, 3, 3), 129, 40, 72), ((3, 3, 3), 2304, 64, 128),
+                                         ((3, 3, 3), 2200, 256, 256), ((3, 3, 3), 4500, 128, 64),
+                                         ((2, 2, 2), 700, 64, 64), ((5, 5, 5), 900, 32, 48)])
+def test_offsets_shared_by_a_cluster(torch, oracle, ksize, n, C, K):
+    """Launches of few tiles, whose offsets the CTAs of a cluster share (eight or four of them, one or two column
+    parts, one or four mask words), with everything an epilogue can do; against the oracle, and against the same call on
+    few CTAs, which nobody shares."""
+    rng = np.random.default_rng(480 + n)
+    subm = ksize[0] % 2 == 1
+    tb = W.build_tables(W.sample_coords(n, 480 + n, (8, 24, 24)), grid=(8, 24, 24), ksize=ksize, subm=subm,
+                        stride=(1, 1, 1) if subm else (2, 2, 2))
+    words, tiles = (tb.kv + 31) // 32, (tb.n_out + 127) // 128
+    x = rng.standard_normal((tb.n_in, C)).astype(np.float16)
+    dout = rng.standard_normal((tb.n_out, K)).astype(np.float16)
+    w = (rng.standard_normal((K, tb.kv, C)) / np.sqrt(tb.kv * C) * 4).astype(np.float16)
+    bias = rng.standard_normal(K).astype(np.float16)
+    init = rng.standard_normal((tb.n_out, K)).astype(np.float16)
+    mo_want = np.zeros((tiles, words) if words > 1 else tiles, np.uint32)
+
+    def call(op, max_ctas, **more):
+        p = ConvParams(3, op)
+        p.conv_algo_desp = H.conv_desp(op, C, K)
+        p.conv_algo_desp.dynamic_mask = words > 1
+        p.weight, p.max_ctas = H.dev(w, torch), max_ctas
+        for k, v in more.items():
+            setattr(p, k, v)
+        ConvMainUnitTest.implicit_gemm2(p)
+        torch.cuda.synchronize()
+        H.check_status()
+
+    results = {}
+    for max_ctas in (0, 3):
+        fwd = dict(input=H.dev(x, torch), indices=H.dev(tb.indices, torch), mask=H.mask_to_torch(tb.mask, torch),
+                   mask_argsort=H.dev(tb.mask_argsort, torch))
+        for name, kw in (("bias and ReLU", dict(bias=H.dev(bias, torch), beta=1.0, act_type=Activation.ReLU)),
+                         ("into what is there", dict(alpha=0.5, beta=0.75))):
+            out, mo = H.dev(init, torch), torch.zeros(mo_want.shape, dtype=torch.int32, device="cuda")
+            call(ConvOpType.Forward, max_ctas, output=out, mask_output=mo, **fwd, **kw)
+            results[max_ctas, name] = out.cpu().numpy(), mo.cpu().numpy().view(np.uint32)
+        din = torch.full((tb.n_in, C), 3.0, dtype=torch.float16, device="cuda")
+        call(ConvOpType.BackwardInput, max_ctas, input=din, output=H.dev(dout, torch), indices=H.dev(tb.indices_bwd, torch),
+             mask=H.mask_to_torch(tb.mask_bwd, torch), mask_argsort=H.dev(tb.mask_argsort_bwd, torch))
+        results[max_ctas, "din"] = din.cpu().numpy(), None
+    sums = oracle.mask_igemm(x, w, np.zeros((tb.n_out, K), np.float16), tb.indices, tb.mask, tb.mask_argsort,
+                             mask_out=mo_want).astype(np.float32)
+    want = {"bias and ReLU": np.maximum(sums + bias.astype(np.float32), 0),
+            "into what is there": 0.5 * sums + 0.75 * init.astype(np.float32),
+            "din": oracle.mask_igemm(dout, w, np.full((tb.n_in, C), 3.0, np.float16), tb.indices_bwd, tb.mask_bwd,
+                                     tb.mask_argsort_bwd, is_dgrad=True)}
+    for name, ref in want.items():
+        for max_ctas in (0, 3):
+            got, mo = results[max_ctas, name]
+            H.assert_close_f16(got, ref.astype(np.float16), f"{name} max_ctas={max_ctas}")
+            if mo is not None:
+                assert (mo == mo_want).all(), "tile masks must be bit-exact"
+        # fp32 sums in another order, rounded once: two results differ by a last place or so
+        a, b = (results[m, name][0].astype(np.float32) for m in (0, 3))
+        assert np.abs(a - b).max() <= 2.0 ** -9 * max(1.0, np.abs(b).max()), name
+
+
 def test_errors_surface_as_exceptions(torch):
     tb, x, w, _ = make(300, 501, 64, 64)
     p = ConvParams(3, ConvOpType.Forward)
