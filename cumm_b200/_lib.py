@@ -243,6 +243,17 @@ def load() -> ctypes.CDLL:
     return L
 
 
+def load_host():
+    """The extension that reads parameter records (``csrc/host_args.cpp``); raises if it has not been built."""
+    import torch  # noqa: F401  (its libraries are the extension's)
+    try:
+        from . import _host
+    except ImportError as e:
+        raise RuntimeError(f"cumm_b200/_host.so is missing or does not load ({e}): the native code has not been built "
+                           "(run `python -c 'import cumm_b200.build as b; b.build()'`).") from e
+    return _host
+
+
 def last_error() -> str:
     return load().cb2_last_error().decode("utf-8", "replace")
 

@@ -1,0 +1,374 @@
+// The host side of a call in native code: reads a GemmParams / ConvParams record as the Python layer
+// (cumm_b200/tensorview/gemm.py, _gemm_args and _conv_args) does, and launches.  It answers for the ordinary
+// call only -- torch tensors on the current device, a descriptor of this library's kernels, no timer -- and
+// returns None for everything else, wrong or merely unusual, before anything has been launched: the Python
+// layer then takes the call, with its checks and its errors.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <ATen/core/Tensor.h>
+#include <c10/core/impl/DeviceGuardImplInterface.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstring>
+
+#include "../../include/cumm_b200.h"
+
+namespace {
+
+using RunGemm = int (*)(const cb2_gemm_args *, void *);
+using RunConv = int (*)(const cb2_conv_args *, void *);
+RunGemm g_run_gemm = nullptr;
+RunConv g_run_conv = nullptr;
+PyObject *g_gemm_params, *g_gemm_desp, *g_conv_params, *g_conv_desp;  // the record classes
+
+#define CB2_NAMES(X)                                                                                                  \
+  X(_a) X(_b) X(_c) X(_d) X(a_inds) X(b_inds) X(c_inds) X(alpha) X(beta) X(act_alpha) X(act_beta) X(act_type)          \
+  X(stream) X(timer) X(max_ctas) X(split_k_slices) X(_algo_desp) X(_conv_algo_desp) X(dtype_a) X(dtype_b) X(dtype_c)   \
+  X(dacc) X(dcomp) X(trans_a_) X(trans_b_) X(trans_c_) X(tile_shape) X(warp_tile_shape) X(tensorop) X(num_stage)       \
+  X(algo) X(shuffle_type) X(element_per_access_a) X(element_per_access_b) X(element_per_access_c) X(input) X(weight)   \
+  X(output) X(output_add) X(bias) X(scale) X(indices) X(mask) X(mask_argsort) X(mask_output) X(mask_width)             \
+  X(mask_filter) X(reverse_mask) X(verbose) X(op_type) X(ndim) X(mask_sparse) X(dynamic_mask) X(is_int8_inference)     \
+  X(split_k_serial_) X(split_k_parallel_)
+#define X(n) PyObject *k_##n;
+CB2_NAMES(X)
+#undef X
+
+// Not the ordinary call: whoever finds out throws, nothing has been launched yet.
+struct Unusual {};
+inline void need(bool ok) {
+  if (!ok)
+    throw Unusual();
+}
+
+struct Ref {
+  PyObject *p;
+  explicit Ref(PyObject *o) : p(o) {}
+  Ref(const Ref &) = delete;
+  Ref &operator=(const Ref &) = delete;
+  ~Ref() { Py_XDECREF(p); }
+};
+
+struct Record {
+  PyObject *o;
+  PyObject *get(PyObject *key) const {
+    PyObject *v = PyObject_GetAttr(o, key);
+    if (!v)
+      PyErr_Clear();
+    need(v != nullptr);
+    return v;
+  }
+  long long integer(PyObject *key) const {
+    Ref v(get(key));
+    need(PyLong_Check(v.p));
+    const long long r = PyLong_AsLongLong(v.p);
+    if (r == -1 && PyErr_Occurred()) {
+      PyErr_Clear();
+      throw Unusual();
+    }
+    return r;
+  }
+  int small(PyObject *key) const {
+    const long long r = integer(key);
+    need(r >= -(1ll << 31) && r < (1ll << 31));
+    return static_cast<int>(r);
+  }
+  bool flag(PyObject *key) const {
+    Ref v(get(key));
+    need(PyBool_Check(v.p));
+    return v.p == Py_True;
+  }
+  float real(PyObject *key) const {
+    Ref v(get(key));
+    need(PyFloat_CheckExact(v.p) || PyLong_CheckExact(v.p));
+    const double r = PyFloat_AsDouble(v.p);
+    if (r == -1.0 && PyErr_Occurred()) {
+      PyErr_Clear();
+      throw Unusual();
+    }
+    return static_cast<float>(r);
+  }
+  bool none(PyObject *key) const {
+    Ref v(get(key));
+    return v.p == Py_None;
+  }
+  void triple(PyObject *key, int (&out)[3]) const {
+    Ref v(get(key));
+    need(PyList_CheckExact(v.p) && PyList_GET_SIZE(v.p) == 3);
+    for (int i = 0; i < 3; ++i) {
+      PyObject *e = PyList_GET_ITEM(v.p, i);
+      need(PyLong_CheckExact(e));
+      const long r = PyLong_AsLong(e);
+      if (r == -1 && PyErr_Occurred())
+        PyErr_Clear();
+      need(r > 0 && r < (1 << 20));
+      out[i] = static_cast<int>(r);
+    }
+  }
+};
+
+// A CUDA tensor with at least one element, or none.
+struct View {
+  const at::Tensor *t = nullptr;
+  int64_t dim(int i) const { return t->size(i); }
+  int64_t stride(int i) const { return t->stride(i); }
+  int n_dims() const { return static_cast<int>(t->dim()); }
+  void *data() const { return t ? t->data_ptr() : nullptr; }
+  explicit operator bool() const { return t != nullptr; }
+};
+View view(const Record &r, PyObject *key, bool may_be_none) {
+  Ref v(r.get(key));  // the record holds it for the length of the call
+  View w;
+  if (v.p == Py_None) {
+    need(may_be_none);
+    return w;
+  }
+  need(THPVariable_CheckExact(v.p));
+  w.t = &THPVariable_Unpack(v.p);
+  need(w.t->is_cuda() && w.t->layout() == at::kStrided && w.t->numel() > 0);
+  return w;
+}
+int size32(int64_t v) {
+  need(v >= 0 && v < (1ll << 31));
+  return static_cast<int>(v);
+}
+int dtype_code(const at::Tensor &t) {
+  switch (t.scalar_type()) {
+  case at::kHalf:
+    return CB2_DTYPE_F16;
+  case at::kChar:
+    return CB2_DTYPE_I8;
+  case at::kFloat:
+    return CB2_DTYPE_F32;
+  default:
+    throw Unusual();
+  }
+}
+void *stream_of(const Record &p) { return reinterpret_cast<void *>(static_cast<intptr_t>(p.integer(k_stream))); }
+bool on_current_device(const View &v) {
+  return c10::impl::getDeviceGuardImpl(at::kCUDA)->getDevice().index() == v.t->get_device();
+}
+
+struct Desp {
+  int tile[3];
+  int epa[3];
+  bool ta, tb, tc;
+};
+// GemmAlgoDesp.check_valid, and the fields both kinds of call use
+Desp read_desp(const Record &d) {
+  Desp r;
+  const int a = d.small(k_trans_a_), b = d.small(k_trans_b_), c = d.small(k_trans_c_);
+  need((a == 0 || a == 1) && (b == 0 || b == 1) && (c == 0 || c == 1));
+  r.ta = a, r.tb = b, r.tc = c;
+  {
+    Ref algo(d.get(k_algo));
+    need(PyUnicode_CheckExact(algo.p) && PyUnicode_GET_LENGTH(algo.p) > 0);
+  }
+  int other[3];
+  d.triple(k_tile_shape, r.tile);
+  d.triple(k_warp_tile_shape, other);
+  d.triple(k_tensorop, other);
+  need(d.small(k_dtype_a) != -1 && d.small(k_dtype_b) != -1 && d.small(k_dtype_c) != -1 && d.small(k_dacc) != -1 &&
+       d.small(k_dcomp) != -1 && d.small(k_num_stage) > 0);
+  r.epa[0] = d.small(k_element_per_access_a);
+  r.epa[1] = d.small(k_element_per_access_b);
+  r.epa[2] = d.small(k_element_per_access_c);
+  need(r.tile[0] == 128);
+  return r;
+}
+bool divides(int epa, long long v) { return epa <= 0 || v % epa == 0; }
+
+// The flat record of a GEMM call whose tensors are on the current device: plain or scattered rows.
+void read_gemm(PyObject *params, cb2_gemm_args &g) {
+  need(g_run_gemm && reinterpret_cast<PyObject *>(Py_TYPE(params)) == g_gemm_params);
+  const Record p{params};
+  need(p.none(k_timer) && p.none(k__d) && p.none(k_b_inds));
+  Ref desp(p.get(k__algo_desp));
+  need(reinterpret_cast<PyObject *>(Py_TYPE(desp.p)) == g_gemm_desp);
+  const Record d{desp.p};
+  const Desp ds = read_desp(d);
+  const int shuffle = d.small(k_shuffle_type);
+  need((shuffle == CB2_SHUFFLE_AC || shuffle == CB2_SHUFFLE_NONE) && !ds.ta && !ds.tc);
+  need(p.small(k_split_k_slices) == 1);
+  const View a = view(p, k__a, false), b = view(p, k__b, false), c = view(p, k__c, false);
+  need(a.n_dims() == 2 && b.n_dims() == 2 && c.n_dims() == 2);
+  need(a.t->get_device() == c.t->get_device() && b.t->get_device() == c.t->get_device() && on_current_device(c));
+  const View ai = view(p, k_a_inds, true), ci = view(p, k_c_inds, shuffle != CB2_SHUFFLE_AC);
+  need((!ai || ai.n_dims() > 0) && (!ci || ci.n_dims() > 0));
+  g.m = size32(shuffle == CB2_SHUFFLE_AC && ai ? ai.dim(0) : a.dim(0));
+  g.k = size32(a.dim(1));
+  g.n = size32(b.dim(ds.tb ? 0 : 1));
+  need(b.dim(ds.tb ? 1 : 0) == g.k && c.dim(1) == g.n && (shuffle == CB2_SHUFFLE_AC || c.dim(0) == g.m));
+  // the leading dimensions GemmAlgoDesp.supported looks at
+  need(divides(ds.epa[0], g.k) && divides(ds.epa[1], ds.tb ? g.k : g.n) && divides(ds.epa[2], g.n));
+  g.ptr_A = a.data(), g.ptr_B = b.data(), g.ptr_C = c.data();
+  g.stride_A = a.stride(0), g.stride_B = b.stride(0), g.stride_C = c.stride(0);
+  if (shuffle == CB2_SHUFFLE_AC) {
+    g.indiceA = static_cast<const int32_t *>(ai.data());
+    g.indiceBorC = static_cast<const int32_t *>(ci.data());
+  }
+  g.alpha = p.real(k_alpha), g.beta = p.real(k_beta);
+  g.act_alpha = p.real(k_act_alpha), g.act_beta = p.real(k_act_beta);
+  g.act_type = p.small(k_act_type);
+  g.split_k_slices = 1;
+  g.dtype_a = d.small(k_dtype_a), g.dtype_b = d.small(k_dtype_b), g.dtype_c = d.small(k_dtype_c);
+  g.trans_b = ds.tb;
+  g.shuffle_type = shuffle;
+  g.rows_A = size32(a.dim(0)), g.rows_B = size32(b.dim(0));
+  g.tile_n = ds.tile[1], g.tile_k = ds.tile[2];
+  g.max_ctas = p.small(k_max_ctas);
+}
+
+// The flat record of a convolution call whose tensors are on the current device.
+void read_conv(PyObject *params, cb2_conv_args &g) {
+  need(g_run_conv && reinterpret_cast<PyObject *>(Py_TYPE(params)) == g_conv_params);
+  const Record p{params};
+  need(p.none(k_timer) && !p.flag(k_verbose));
+  Ref desp(p.get(k__conv_algo_desp));
+  need(reinterpret_cast<PyObject *>(Py_TYPE(desp.p)) == g_conv_desp);
+  const Record d{desp.p};
+  const int op = d.small(k_op_type);
+  need(op >= CB2_CONV_FORWARD && op <= CB2_CONV_BACKWARD_WEIGHT && d.flag(k_mask_sparse));
+  const bool fwd = op == CB2_CONV_FORWARD, wgrad = op == CB2_CONV_BACKWARD_WEIGHT, int8 = d.flag(k_is_int8_inference);
+  const Desp ds = read_desp(d);
+  g.split_k_slices = p.small(k_split_k_slices);
+  need(g.split_k_slices <= 1 || d.small(k_split_k_serial_) == 1 || d.small(k_split_k_parallel_) == 1);
+  const View in = view(p, k_input, false), w = view(p, k_weight, false), out = view(p, k_output, false);
+  need(in.n_dims() == 2 && out.n_dims() == 2 && w.n_dims() == 3);
+  need(in.t->is_contiguous() && w.t->is_contiguous() && out.t->is_contiguous());
+  const View add = view(p, k_output_add, true), bias = view(p, k_bias, true), scale = view(p, k_scale, true);
+  const View ind = view(p, k_indices, false), mask = view(p, k_mask, false), order = view(p, k_mask_argsort, false),
+             mask_out = view(p, k_mask_output, true);
+  g.K = size32(w.dim(0)), g.kernel_volume = size32(w.dim(1)), g.C = size32(w.dim(2));
+  need(in.dim(1) == g.C && out.dim(1) == g.K);
+  need(int8 ? (bias && scale) : !add);
+  if (add)
+    need(add.t->scalar_type() == out.t->scalar_type() && add.t->sizes() == out.t->sizes());
+  const int kv = g.kernel_volume, words = (kv + 31) / 32;
+  need(ind.n_dims() == 2 && ind.dim(0) == kv && kv >= 1 && kv <= 128 && (kv <= 32 || d.flag(k_dynamic_mask)));
+  g.N = size32(ind.dim(1));
+  need(g.N == (fwd || wgrad ? out : in).dim(0));
+  g.mask_width = p.small(k_mask_width);
+  // what ConvAlgoDesp.supported looks at
+  const long long m = wgrad ? g.K : g.N, n = fwd ? g.K : wgrad ? 1ll * g.C * kv : g.C,
+                  k = wgrad ? g.N : 1ll * kv * (fwd ? g.C : g.K);
+  need(divides(ds.epa[0], ds.ta ? m : k) && divides(ds.epa[1], ds.tb ? k : n) && divides(ds.epa[2], ds.tc ? m : n));
+  need(ds.epa[0] != 0 && (fwd ? g.C : g.K) % ds.epa[0] == 0);
+  if (wgrad)
+    need(ds.epa[1] != 0 && g.C % ds.epa[1] == 0 && g.mask_width > 0 && g.mask_width % ds.tile[2] == 0);
+  const View &a = fwd ? in : out, &b = wgrad ? in : w, &c = fwd ? out : wgrad ? w : in;
+  need(on_current_device(c));
+  g.ptr_A = a.data(), g.ptr_B = b.data(), g.ptr_C = c.data();
+  g.ptr_D = add ? add.data() : (int8 || !bias) ? c.data() : bias.data();
+  g.d_is_bias = bias && !int8 && !add;
+  g.bias_pointer = bias.data(), g.scale_pointer = scale.data();
+  g.alpha = p.real(k_alpha), g.beta = p.real(k_beta);
+  g.act_alpha = p.real(k_act_alpha), g.act_beta = p.real(k_act_beta);
+  g.act_type = p.small(k_act_type);
+  g.mask_ptr = static_cast<const uint32_t *>(mask.data());
+  g.mask_out_ptr = static_cast<uint32_t *>(mask_out.data());
+  g.indice_ptr = static_cast<const int32_t *>(ind.data());
+  g.mask_argsort_ptr = static_cast<const int32_t *>(order.data());
+  g.mask_filter = static_cast<uint32_t>(p.integer(k_mask_filter));
+  g.reverse_mask = p.flag(k_reverse_mask);
+  g.ndim = d.small(k_ndim);
+  g.mode = 1;
+  g.groups = 1;
+  g.op_type = op;
+  g.dtype_a = dtype_code(*a.t), g.dtype_b = dtype_code(*b.t), g.dtype_c = dtype_code(*c.t);
+  g.is_int8_inference = int8;
+  g.rows_A = size32(a.dim(0)), g.rows_B = size32(b.dim(0));
+  g.mask_words = size32(mask.t->numel());
+  need(wgrad || g.mask_words >= static_cast<long long>(g.N) * words);
+  if (fwd && mask_out)
+    need(mask_out.t->numel() >= (static_cast<long long>(g.N) + 127) / 128 * words);
+  g.tile_n = ds.tile[1], g.tile_k = wgrad ? 0 : ds.tile[2];
+  g.max_ctas = p.small(k_max_ctas);
+}
+
+template <class Args, class Run> PyObject *launch(Run run, const Args &a, void *stream) {
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = run(&a, stream);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// run_gemm(params), run_conv(params): the call's return code, or None.  The weight gradient needs scratch, which
+// the Python layer keeps.
+PyObject *run_gemm(PyObject *, PyObject *params) {
+  cb2_gemm_args g;
+  memset(&g, 0, sizeof(g));
+  void *stream;
+  try {
+    read_gemm(params, g);
+    stream = stream_of(Record{params});
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+  return launch(g_run_gemm, g, stream);
+}
+PyObject *run_conv(PyObject *, PyObject *params) {
+  cb2_conv_args g;
+  memset(&g, 0, sizeof(g));
+  void *stream;
+  try {
+    read_conv(params, g);
+    need(g.op_type != CB2_CONV_BACKWARD_WEIGHT);
+    stream = stream_of(Record{params});
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+  return launch(g_run_conv, g, stream);
+}
+
+// gemm_args(params, address), conv_args(params, address): fill the flat record there; True, or None.
+template <class Args> PyObject *fill(PyObject *args, void (*read)(PyObject *, Args &)) {
+  PyObject *params;
+  unsigned long long address;
+  if (!PyArg_ParseTuple(args, "OK", &params, &address))
+    return nullptr;
+  Args g;
+  memset(&g, 0, sizeof(g));
+  try {
+    read(params, g);
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+  memcpy(reinterpret_cast<void *>(static_cast<uintptr_t>(address)), &g, sizeof(g));
+  Py_RETURN_TRUE;
+}
+PyObject *gemm_args(PyObject *, PyObject *args) { return fill<cb2_gemm_args>(args, read_gemm); }
+PyObject *conv_args(PyObject *, PyObject *args) { return fill<cb2_conv_args>(args, read_conv); }
+
+// setup(GemmParams, GemmAlgoDesp, ConvParams, ConvAlgoDesp, address of cb2_gemm_run, of cb2_conv_run)
+PyObject *setup(PyObject *, PyObject *args) {
+  unsigned long long gemm, conv;
+  PyObject *c[4];
+  if (!PyArg_ParseTuple(args, "OOOOKK", &c[0], &c[1], &c[2], &c[3], &gemm, &conv))
+    return nullptr;
+  for (PyObject *o : c)
+    Py_INCREF(o);  // for the life of the process
+  g_gemm_params = c[0], g_gemm_desp = c[1], g_conv_params = c[2], g_conv_desp = c[3];
+  g_run_gemm = reinterpret_cast<RunGemm>(gemm);
+  g_run_conv = reinterpret_cast<RunConv>(conv);
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {{"setup", setup, METH_VARARGS, nullptr},
+                         {"run_gemm", run_gemm, METH_O, nullptr},
+                         {"run_conv", run_conv, METH_O, nullptr},
+                         {"gemm_args", gemm_args, METH_VARARGS, nullptr},
+                         {"conv_args", conv_args, METH_VARARGS, nullptr},
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+} // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+#define X(n)                                                                                                          \
+  if (!(k_##n = PyUnicode_InternFromString(#n)))                                                                      \
+    return nullptr;
+  CB2_NAMES(X)
+#undef X
+  return PyModule_Create(&module);
+}

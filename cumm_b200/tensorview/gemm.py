@@ -192,7 +192,14 @@ class GemmAlgoDesp:
 
     def copy(self):
         import copy
-        return copy.deepcopy(self)
+        new = object.__new__(type(self))
+        for k, v in vars(self).items():  # numbers, names and lists of numbers: nothing a deep copy would find more in
+            if type(v) is list and all(type(e) is int for e in v):
+                v = list(v)
+            elif not isinstance(v, (int, float, str)):
+                v = copy.deepcopy(v)
+            new.__dict__[k] = v
+        return new
 
     def query_workspace_size(self, m: int, n: int, k: int, split_k_slices: int) -> int:
         """params.h:115-132 (the reference's formula, a pure function of the record)."""
@@ -370,7 +377,7 @@ class GemmParams:
     """params.h:329-390.  Tensors may be ``torch.Tensor`` (CUDA) or ``tensorview.Tensor``."""
 
     def __init__(self, timer=None):
-        self.algo_desp = GemmAlgoDesp()
+        self._algo_desp = None
         self._a = None
         self._b = None
         self._c = None
@@ -387,8 +394,29 @@ class GemmParams:
         self.act_type = Activation.None_
         self.stream = 0
         self.timer = timer
-        self.nvrtc_params = NVRTCParams()
+        self._nvrtc_params = None
         self.max_ctas = 0  # not in the reference: see ConvParams.max_ctas
+
+    # made when first asked for: most callers bring a descriptor of their own
+    @property
+    def algo_desp(self) -> GemmAlgoDesp:
+        if self._algo_desp is None:
+            self._algo_desp = GemmAlgoDesp()
+        return self._algo_desp
+
+    @algo_desp.setter
+    def algo_desp(self, v):
+        self._algo_desp = v
+
+    @property
+    def nvrtc_params(self) -> NVRTCParams:
+        if self._nvrtc_params is None:
+            self._nvrtc_params = NVRTCParams()
+        return self._nvrtc_params
+
+    @nvrtc_params.setter
+    def nvrtc_params(self, v):
+        self._nvrtc_params = v
 
     # setters copy the dtype into the descriptor (params.h:366-388)
     @property
@@ -462,7 +490,8 @@ class ConvParams:
     """params.h:392-428."""
 
     def __init__(self, ndim: int, op_type, timer=None):
-        self.conv_algo_desp = ConvAlgoDesp(ndim, op_type)
+        self._kind = (int(ndim), ConvOpType(int(op_type)))
+        self._conv_algo_desp = None
         self.input = None
         self.weight = None
         self.output = None
@@ -490,12 +519,25 @@ class ConvParams:
         self.indices = None
         self.mask_output = None
         self.stream = 0
-        self.nvrtc_params = NVRTCParams()
+        self._nvrtc_params = None
         # Not in the reference: upper bound on the CTAs of the launch (0 = one per SM), for calls
         # that run side by side on different streams (``cb2_conv_args.max_ctas``).
         self.max_ctas = 0
         # Not in the reference: the weight gradient's plan may list rows (``CB2_PLAN_ROW_LISTS``).
         self.row_lists = True
+
+    # made when first asked for, as in GemmParams
+    @property
+    def conv_algo_desp(self) -> ConvAlgoDesp:
+        if self._conv_algo_desp is None:
+            self._conv_algo_desp = ConvAlgoDesp(*self._kind)
+        return self._conv_algo_desp
+
+    @conv_algo_desp.setter
+    def conv_algo_desp(self, v):
+        self._conv_algo_desp = v
+
+    nvrtc_params = GemmParams.nvrtc_params
 
 
 # --------------------------------------------------------------------------------------
@@ -641,9 +683,32 @@ def _gemm_args(params: GemmParams) -> _lib.GemmArgs:
     return args
 
 
+_HOST = None
+
+
+def _host():
+    """The native reader of the records (csrc/host_args.cpp), which answers for the ordinary call and leaves
+    every other to the functions here."""
+    global _HOST
+    if _HOST is None:
+        host, L = _lib.load_host(), _lib.load()
+        real = isinstance(L, ctypes.CDLL)  # something that stands in for the library is called from Python only
+        address = lambda name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value if real else 0
+        host.setup(GemmParams, GemmAlgoDesp, ConvParams, ConvAlgoDesp, address("cb2_gemm_run"), address("cb2_conv_run"))
+        if not real:
+            return host
+        _HOST = host
+    return _HOST
+
+
 def run_gemm(params: GemmParams) -> None:
     """What ``GemmMainUnitTest.matmul2`` does (cumm/gemm/main.py:1178-1335): validate,
     pick a kernel for the descriptor, launch on ``params.stream``."""
+    rc = (_HOST or _host()).run_gemm(params)
+    if rc is not None:
+        if rc:
+            _lib.raise_for(rc)
+        return
     L = _lib.load()
     args = _gemm_args(params)
     stream = int(params.stream)
@@ -785,12 +850,23 @@ def _conv_args(params: ConvParams) -> _lib.ConvArgs:
 
 def run_conv(params: ConvParams) -> None:
     """What ``ConvMainUnitTest.implicit_gemm2`` does (cumm/conv/main.py:485-745)."""
+    host = _HOST or _host()
+    rc = host.run_conv(params)
+    if rc is not None:
+        if rc:
+            _lib.raise_for(rc)
+        return
     if not params.conv_algo_desp.mask_sparse:
         # dense convolution: the same kernels over the neighbour table of the full grid
         from ..dense import run_dense_conv
         return run_dense_conv(params)
     L = _lib.load()
-    args = _conv_args(params)
+    args = _lib.ConvArgs()
+    if host.conv_args(params, ctypes.addressof(args)):
+        import torch
+        args._device = torch.cuda.current_device()
+    else:
+        args = _conv_args(params)
     stream = int(params.stream)
     if args.op_type == ConvOpType.BackwardWeight:  # the only operator that needs scratch
         need = L.cb2_conv_workspace_size(ctypes.byref(args))
