@@ -621,10 +621,11 @@ __device__ __forceinline__ uint4 rowconv_finish8(const RowConvParams &p, const f
 // SPLIT: a launch with so few items that most SMs would be idle.  What such a launch takes is one tile's offsets,
 // one after the other, so a cluster of `split` CTAs shares an item's offsets: each sums its own in tensor memory and
 // leaves the sums, fp32, in its shared memory; then each makes the output rows of its share of the tile from the
-// sums of all, in the order of the CTAs, through distributed shared memory.  (Forward, us, without and with: 2000
-// rows of a crop at 64 channels 14.6 and 11.5, scanned scenes of 4000 rows, 64 to 32, 13.0 and 10.6, 1600 at 128
-// 18.0 and 12.9.  Clusters of two, for up to half as many items as SMs, gained 8 % on 9000 scanned rows and lost 6 %
-// on uniform ones, most of whose tiles have one offset.)
+// sums of all, in the order of the CTAs, through distributed shared memory.  (Forward, us, without, with, and with
+// launches that start under their predecessor's tail: 2000 rows of a crop at 64 channels 14.6, 11.5, 8.2, scanned scenes
+// of 4000 rows, 64 to 32, 13.0, 10.6, 9.4, 1600 at 128 18.0, 12.9, 11.4; 2000 uniform rows 7.2, 7.5, 5.0.  Clusters of
+// two, for up to half as many items as SMs, gained 8 % on 9000 scanned rows and lost 6 % on uniform ones, most of
+// whose tiles have one offset.)
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MASK_WORDS = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(RowConvCfg<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MASK_WORDS>::THREADS, 1)
 rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_a,
