@@ -163,6 +163,10 @@ int gather_mode() {
 // weight-gradient kernels, the gather-GEMM-scatter calls and the int8 convolutions; level 2
 // (only with CUMM_B200_PDL=2): the fp16 convolution row kernels.  CUMM_B200_PDL=0 launches everything the
 // ordinary way.
+// The kernels of table generation take part too, but none triggers its dependent: a dependent's launch overlaps the
+// predecessor's end and no more (150 000 uniform rows, us: ordinary launches 85.4 and, stride 2, 186; so 76.5 and 170;
+// triggered as soon as a kernel starts 91.5 and 199, its successor's waiting blocks hold the SMs).  It also means that whoever reads
+// the tables before its own griddepcontrol.wait finds them complete.
 template <class Kern, class... Args>
 cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                          Args... args) {
@@ -806,11 +810,8 @@ int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, c
       o.tile_masks = to_go ? nullptr : j.tile_masks;
     }
     const dim3 grid(max_chunks, count);
-    if (shape.words > 1)
-      cb2pg::sort_pass_kernel<true><<<grid, cb2pg::kSortThreads, 0, s>>>(sides, p, shape);
-    else
-      cb2pg::sort_pass_kernel<false><<<grid, cb2pg::kSortThreads, 0, s>>>(sides, p, shape);
-    CB2_CUDA(cudaGetLastError());
+    auto kern = shape.words > 1 ? cb2pg::sort_pass_kernel<true> : cb2pg::sort_pass_kernel<false>;
+    CB2_CUDA(launch_after(1, 1, kern, grid, dim3(cb2pg::kSortThreads), 0, s, sides, p, shape));
     g_launches.fetch_add(1);
   }
   return CB2_OK;
@@ -893,8 +894,10 @@ int cb2_pairgen_count_outputs(const cb2_pairgen_args *a, int *n_out, void *strea
     const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
     fill.add(bm.words, static_cast<size_t>(L.bitmap_words) * 4, 0u);
     fill.run(dev, stream);
-    cb2pg::bitmap_mark_kernel<<<(a->n_in + 127) / 128, 128, 0, stream>>>(a->in_coords, a->n_in, L.g, bm.words);
-    cb2pg::bitmap_rank_kernel<<<bm.n_blocks, cb2pg::kBitmapThreads, 0, stream>>>(bm, counter);
+    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_mark_kernel, dim3((a->n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
+                          a->n_in, L.g, bm.words));
+    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_rank_kernel, dim3(bm.n_blocks), dim3(cb2pg::kBitmapThreads), 0, stream, bm,
+                          counter));
     g_launches.fetch_add(2);
   } else {
     fill.add(set_keys, static_cast<size_t>(L.cap_set) * 8, 0xffffffffu);
@@ -957,13 +960,14 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
     if (bwd)
       fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
-    cb2pg::bitmap_coords_kernel<<<blocks(bm.n_words), 256, 0, stream>>>(bm, n_out, L.g, a->out_coords);
-    cb2pg::bitmap_scatter_kernel<<<(n_in + 127) / 128, 128, 0, stream>>>(a->in_coords, n_in, L.g, bm, jobs[0].side, words,
-                                                                         dev->status);
+    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_coords_kernel, dim3(blocks(bm.n_words)), dim3(256), 0, stream, bm, n_out, L.g,
+                          a->out_coords));
+    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_scatter_kernel, dim3((n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
+                          n_in, L.g, bm, jobs[0].side, words, dev->status));
     const int bwd_blocks = bwd ? static_cast<int>(blocks(n_in)) : 0;
     auto kern = words > 1 ? cb2pg::bitmap_backward_kernel<4> : cb2pg::bitmap_backward_kernel<1>;
-    kern<<<bwd_blocks + blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(a->in_coords, L.g, bm, jobs[0].side, jobs[1].side,
-                                                                         bwd_blocks, words, shape.width);
+    CB2_CUDA(launch_after(1, 1, kern, dim3(bwd_blocks + blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, a->in_coords,
+                          L.g, bm, jobs[0].side, jobs[1].side, bwd_blocks, words, shape.width));
     CB2_CUDA(cudaGetLastError());
     g_launches.fetch_add(3);
   } else {
@@ -977,7 +981,7 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
       fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
     auto insert = L.exact ? cb2pg::hash_insert_kernel<true> : cb2pg::hash_insert_kernel<false>;
-    insert<<<blocks(n_in), 256, 0, stream>>>(a->in_coords, n_in, L.g, h, dev->status);
+    CB2_CUDA(launch_after(1, 1, insert, dim3(blocks(n_in)), dim3(256), 0, stream, a->in_coords, n_in, L.g, h, dev->status));
     const int32_t *out_coords = a->in_coords;
     if (!a->subm) {
       cb2pg::decode_out_coords_kernel<<<blocks(n_out), 256, 0, stream>>>(
@@ -987,8 +991,8 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
     }
     auto kern = L.exact ? (words > 1 ? cb2pg::probe_kernel<4, true> : cb2pg::probe_kernel<1, true>)
                         : (words > 1 ? cb2pg::probe_kernel<4, false> : cb2pg::probe_kernel<1, false>);
-    kern<<<blocks(n_out), cb2pg::kProbeThreads, 0, stream>>>(out_coords, L.g, h, jobs[0].side, mirror ? jobs[1].side : none,
-                                                            words, shape.width);
+    CB2_CUDA(launch_after(1, 1, kern, dim3(blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, out_coords, L.g, h,
+                          jobs[0].side, mirror ? jobs[1].side : none, words, shape.width));
     g_launches.fetch_add(2);
     if (bwd && !mirror) {
       cb2pg::invert_table_kernel<<<blocks(static_cast<long long>(n_out) * L.g.kv), 256, 0, stream>>>(

@@ -109,6 +109,7 @@ __device__ __forceinline__ int find_in_bucket(const HashView &h, const BucketWor
 template <bool EXACT>
 __global__ void __launch_bounds__(256) hash_insert_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                           HashView h, int *status) {
+  cb2::grid_dep_wait();
   using HK = HashKey<EXACT>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
@@ -301,6 +302,7 @@ template <int NW, bool EXACT>
 __global__ void __launch_bounds__(kProbeThreads, 4) probe_kernel(const int32_t *__restrict__ out_coords, Geometry g,
                                                               const HashView h, const MaskSide side,
                                                               const MaskSide mirror, int words, int width) {
+  cb2::grid_dep_wait();
   constexpr int B = 3;
   using HK = HashKey<EXACT>;
   using Key = typename HK::Key;
@@ -512,6 +514,7 @@ __device__ __forceinline__ bool inside(const Geometry &g, const int4 &c) {
 // One thread per input voxel; bits of one word set together.
 __global__ void __launch_bounds__(128) bitmap_mark_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                           uint32_t *words) {
+  cb2::grid_dep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
@@ -559,6 +562,7 @@ __device__ __forceinline__ int block_scan_512(int v, int *s_warp, int &total) {
 // counters[0] = all set bits, counters[1] = blocks that have counted (zero before the launch).  The
 // block that counts last scans the block sums: nobody waits for anybody.
 __global__ void __launch_bounds__(kBitmapThreads) bitmap_rank_kernel(const Bitmap bm, int *counters) {
+  cb2::grid_dep_wait();
   __shared__ int s_warp[16];
   __shared__ int s_last;
   const int w0 = blockIdx.x * kBitmapBlockWords + threadIdx.x * kBitmapWordsPerThread;
@@ -608,6 +612,7 @@ __device__ __forceinline__ int bitmap_rank(const Bitmap &bm, uint32_t cell) {
 
 // coordinates of the active outputs, in row order; one thread per word
 __global__ void __launch_bounds__(256) bitmap_coords_kernel(const Bitmap bm, int n_out, Geometry g, int32_t *out_coords) {
+  cb2::grid_dep_wait();
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= bm.n_words)
     return;
@@ -631,6 +636,7 @@ __global__ void __launch_bounds__(256) bitmap_coords_kernel(const Bitmap bm, int
 // and the masks start as -1 and 0; of several rows with one voxel the smallest wins.
 __global__ void __launch_bounds__(128) bitmap_scatter_kernel(const int32_t *__restrict__ coords, int n, Geometry g,
                                                              const Bitmap bm, const MaskSide out, int words, int *status) {
+  cb2::grid_dep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n)
     return;
@@ -656,6 +662,7 @@ __global__ void __launch_bounds__(kProbeThreads) bitmap_backward_kernel(const in
                                                                         const Bitmap bm, const MaskSide out,
                                                                         const MaskSide in, int bwd_blocks, int words,
                                                                         int width) {
+  cb2::grid_dep_wait();
   __shared__ int s_hist[kSortBins];
   if (static_cast<int>(blockIdx.x) >= bwd_blocks) {
     const int block = blockIdx.x - bwd_blocks;
@@ -710,6 +717,7 @@ struct SortSides {
 template <bool WIDE>
 __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_constant__ SortSides sides, int pass,
                                                                  const SortShape shape) {
+  cb2::grid_dep_wait();
   const SortSide &s = sides.side[blockIdx.y];
   __shared__ int s_cnt[kSortWarps][kSortBins];
   __shared__ int s_base[kSortBins];
