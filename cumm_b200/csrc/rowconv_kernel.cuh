@@ -161,6 +161,7 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int SCHED_WARP = FIRST_GATHER_WARP + GROUPS * GROUP_THREADS / 32;  // the last warp hands out tiles
   static constexpr int THREADS = (SCHED_WARP + 1) * 32;
   static constexpr int RING_CONSUMER_WARPS = SCHED_WARP;   // every warp but the scheduler
+  static constexpr int CLEARED_THREADS = EPI_THREADS + GROUPS * GROUP_THREADS;  // SPLIT: stages cleared, sums may come
   // shared memory map (offsets from a 1024-byte aligned base)
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + SA * A_STAGE_BYTES;
@@ -771,6 +772,10 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         acc_phase ^= 1u;
       }
     };
+    // The sums will lie where the gather warps clear their stages, and a warp without a step of its own has nothing
+    // else that orders its clearing before them.
+    if constexpr (SPLIT)
+      named_bar_sync(1, Cfg::CLEARED_THREADS);
     CB2_PROF_BEGIN();
     TileCursor<MW> tc;
     int o = -1;  // destination row of this thread's tile row
@@ -821,8 +826,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                                 static_cast<uint32_t>(buf * BLOCK_N);
           if constexpr (SPLIT) {
             if (misc[2] == 0) {
-              // the operand stages are idle: every MMA of the CTA has completed.  Four columns of row r at
-              // [column / 4][r], so that a warp's rows lie side by side
+              // The operand stages are idle: every MMA of the CTA has completed, and every stage was cleared before
+              // this warp began.  Four columns of row r at [column / 4][r], so that a warp's rows lie side by side
 #pragma unroll 1
               for (int round = 0; round < COLS_PER_HALF / 32; ++round) {
                 uint32_t v[32];
@@ -1208,6 +1213,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       for (int q = 0; q < 32; ++q)
         st_shared_zero16(first_quad + q * (4 * 128) + lane * 16);
       fence_proxy_async_smem();  // generic-proxy stores, read by the tensor core
+      if constexpr (SPLIT)
+        named_bar_arrive(1, Cfg::CLEARED_THREADS);
       __syncwarp();
       uint32_t dirty = 0;  // quads of this stage that hold gathered rows
       bool dep_waited = false, ok = true;

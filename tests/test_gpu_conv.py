@@ -403,6 +403,30 @@ def test_offsets_shared_by_a_cluster(torch, oracle, ksize, n, C, K):
         assert np.abs(a - b).max() <= 2.0 ** -9 * max(1.0, np.abs(b).max()), name
 
 
+@pytest.mark.parametrize("C,K", [(64, 64), (40, 128), (128, 128)])
+@pytest.mark.parametrize("offsets", [4, 5, 8, 9])
+def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, offsets):
+    """Items of four to nine offsets on clusters of eight CTAs: most of a CTA's gather warps have no step, and clear
+    their stages where the CTA's sums will lie while another warp's rows are already on their way.  Many launches, all the same."""
+    mask_filter = sum(1 << f for f in (13, 4, 22, 10, 16, 12, 14, 1, 25)[:offsets])
+    tb, x, w, dout = make(2300, 495, C, K)
+    want = oracle.mask_igemm(x, w, np.zeros((tb.n_out, K), np.float16), tb.indices, tb.mask, tb.mask_argsort,
+                             mask_filter=mask_filter)
+    p = ConvParams(3, ConvOpType.Forward)
+    p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, C, K)
+    p.input, p.weight, p.mask_filter = H.dev(x, torch), H.dev(w, torch), mask_filter
+    p.indices, p.mask, p.mask_argsort = H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
+    outs = [torch.full((tb.n_out, K), 7.0, dtype=torch.float16, device="cuda") for _ in range(50)]
+    torch.cuda.synchronize()
+    for p.output in outs:
+        ConvMainUnitTest.implicit_gemm2(p)
+    torch.cuda.synchronize()
+    H.check_status()
+    H.assert_close_f16(outs[0].cpu().numpy(), want, f"{offsets} offsets")
+    for i, out in enumerate(outs):
+        assert torch.equal(out, outs[0]), f"launch {i} differs from the first"
+
+
 def test_errors_surface_as_exceptions(torch):
     tb, x, w, _ = make(300, 501, 64, 64)
     p = ConvParams(3, ConvOpType.Forward)
