@@ -251,10 +251,8 @@ __device__ __forceinline__ float4 ld_cluster_16(uint32_t addr) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ int ld_cluster_int(uint32_t addr) {
-  int v;
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
+__device__ __forceinline__ void ld_cluster_2ints(uint32_t addr, int &a, int &b) {
+  asm volatile("ld.shared::cluster.v2.s32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
 }
 
 // ---------------------------------------------------------------- named barriers

@@ -365,12 +365,18 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // The first batch of tickets is requested at kernel entry (first_ticket_request), long before the
 // scheduler can use it: the counter's round trip, and an L2 prefetch of the first tile's words,
 // run while the CTA sets up its barriers and tensor memory.
-// SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `solo` (shared memory) says
-// that the item has so few that the first CTA keeps them all: the exchange would cost more than they do.
+// SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
+// becomes what that makes of the CTA; it stays kSplitUnknown in one that gives up before its item is known.
 constexpr int kSplitSoloOffsets = 3;
+enum SplitState {
+  kSplitUnknown = 0,
+  kSplitSolo,     // the item has so few offsets that the first CTA keeps them all: the exchange would cost more than they do
+  kSplitNothing,  // shared, none of the offsets is this CTA's
+  kSplitSums      // shared, the epilogue warps leave this CTA's sums in shared memory and count themselves
+};
 template <int MW, bool SPLIT>
 __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int block_n,
-                                              int kpasses, int first_base, int first_cnt, volatile int *solo) {
+                                              int kpasses, int first_base, int first_cnt, volatile int *split_state) {
   const int nitems = ntiles * p.n_parts;
   constexpr int STEP_BUDGET = CB2_ROWCONV_STEP_BUDGET;  // steps a CTA may hold (drawn, not read by every role)
   const int lane = (int)lane_id();
@@ -455,7 +461,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
           }
           offsets = kept;
           if (lane == 0)
-            *solo = alone ? 1 : 0;
+            *split_state = alone ? kSplitSolo : kept ? kSplitSums : kSplitNothing;
         }
       }
       const int nsteps = (sl[0] >= 0) ? max(1, offsets * kpasses) : 1;
@@ -490,6 +496,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // tables whose tiles can be fetched with two 16-byte copies per lane
   const bool wide_copies = conv && MW == 1 && p.mask_words == 1 &&
                            ((reinterpret_cast<uintptr_t>(p.argsort) | reinterpret_cast<uintptr_t>(p.mask)) & 15u) == 0;
+  bool ended = false;
   for (;;) {
     account();
     bool may_draw = can_draw();
@@ -503,7 +510,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
                           ? mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag)
                           : mbar_wait_warp(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1, rv.abort_flag);
       if (!ok)
-        return;
+        break;  // gave up
       continue;
     }
     const int si = issued % rv.ring;
@@ -565,17 +572,19 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
     if (lane == 0)
       CB2_TRACE_EVENT(6, 16, tile);  // tile drawn, fetch issued
     ++issued;
-    if (tile < 0)
+    if (tile < 0) {
+      ended = true;
       break;
+    }
   }
   // publish what is still in flight (the end marker at the latest)
-  while (accounted < issued) {
-    if (!mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag))
-      return;
-    account();
+  while (ended && accounted < issued) {
+    ended = mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag);
+    if (ended)
+      account();
   }
   // the last CTA to run out of tiles puts the two counters back to zero for the next launch
-  if (dynamic && lane == 0) {
+  if (ended && dynamic && lane == 0) {
     if (next_cnt != 0)  // an outstanding request must have been served before the counters may be reset
       asm volatile("" ::"r"(next_base) : "memory");
     __threadfence();
@@ -653,9 +662,9 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   float *s_scale = reinterpret_cast<float *>(smem + Cfg::OFF_SCALE);
   float *s_bias = s_scale + BLOCK_N;
   volatile int *misc = reinterpret_cast<volatile int *>(smem + Cfg::OFF_MISC);
-  // misc[0] tmem base, misc[1] abort flag, misc[2] SPLIT: the item is the first CTA's alone, misc[3] SPLIT: there
-  // are sums in this CTA's shared memory, misc[4 + 2 g, 6 + 2 g) what gather group g's waits returned, one for
-  // each of its row buffers
+  // misc[0] tmem base, misc[1] abort flag, misc[2] SPLIT: a SplitState, misc[3] SPLIT: epilogue warps whose sums are
+  // in this CTA's shared memory, misc[4 + 2 g, 6 + 2 g) what gather group g's waits returned, one for each of its
+  // row buffers
   volatile int *abort_flag = misc + 1;
 
   const uint32_t bars = sbase + Cfg::OFF_BARS;
@@ -784,7 +793,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                     })) > 0;) {
           const int tile = tc.tile;
           const bool has_work = tc.offsets != 0;
-          if (!has_work && (p.skip_empty_tiles || (SPLIT && (cluster_rank() != 0 || misc[2] == 0))))
+          if (!has_work && (p.skip_empty_tiles || (SPLIT && (cluster_rank() != 0 || misc[2] != kSplitSolo))))
             continue;
           // A tile without work uses no accumulator and passes none on: whoever is next in turn stores it.
           if (Cfg::EPI_GROUPS > 1 && buf != group) {
@@ -825,7 +834,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           const uint32_t trow = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) +
                                 static_cast<uint32_t>(buf * BLOCK_N);
           if constexpr (SPLIT) {
-            if (misc[2] == 0) {
+            if (misc[2] != kSplitSolo) {
               // The operand stages are idle: every MMA of the CTA has completed, and every stage was cleared before
               // this warp began.  Four columns of row r at [column / 4][r], so that a warp's rows lie side by side
 #pragma unroll 1
@@ -838,8 +847,9 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                 for (int q = 0; q < 8; ++q)
                   st_shared_16(sbase + ((col0 / 4 + q) * 128 + erow) * 16, &v[4 * q]);
               }
-              if (et == 0)
-                misc[3] = 1;
+              __syncwarp();
+              if (lane == 0)
+                atomicAdd(const_cast<int *>(misc + 3), 1);
               next_acc();
               continue;
             }
@@ -1417,16 +1427,22 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if constexpr (SPLIT) {
-    if (misc[2] == 0) {  // the same in all CTAs of the cluster; one that gave up leaves, and is not waited for
-      cluster_sync();
+    // Every CTA of the cluster passes both barriers, whatever became of its waits: none leaves while another may read
+    // its shared memory.  Rows are made only where every CTA has what its state promises; where one gave up (the status
+    // word says so) the item's rows stay as they were, and the slot its rows would be read from may not even be filled.
+    cluster_sync();
+    if (misc[2] != kSplitSolo) {
+      int state = kSplitNothing, warps = 0;  // of the CTA whose rank is this lane's number
+      if (lane < p.split)
+        ld_cluster_2ints(cluster_map(sbase + Cfg::OFF_MISC + 8, lane), state, warps);
+      const bool sums = state == kSplitSums && warps == Cfg::EPI_THREADS / 32;
+      const unsigned have = __ballot_sync(0xffffffffu, sums);
+      const bool whole = __all_sync(0xffffffffu, sums || state == kSplitNothing);
       grid_dep_wait();
       const int rows = 128 / p.split, first = (int)cluster_rank() * rows;
       const int *sl = rv.slot(0);  // the item's: the ring's first, and never used again
       const int n0 = sl[3];
-      unsigned have = 0;
-      for (int c = 0; c < p.split; ++c)
-        have |= ld_cluster_int(cluster_map(sbase + Cfg::OFF_MISC + 12, c)) ? 1u << c : 0u;
-      if (have != 0 || !p.skip_empty_tiles)
+      if (whole && (have != 0 || !p.skip_empty_tiles))
         for (int i = threadIdx.x; i < rows * (BLOCK_N / 8); i += Cfg::THREADS) {
           const int row = first + i % rows, col = i / rows * 8;
           const int to = sl[8 + row];
@@ -1444,8 +1460,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
               rowconv_finish8(p, v, to, n0 + col);
         }
       __syncwarp();
-      cluster_sync();  // the others have read this CTA's sums
     }
+    cluster_sync();
   }
   if (threadIdx.x == 0)
     CB2_TRACE_CTA(1, 0);

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import helpers as H
+from cumm_b200 import _lib
 from cumm_b200 import workloads as W
 from cumm_b200.tensorview.gemm import Activation, ConvOpType, ConvParams
 from cumm_b200.conv.main import ConvMainUnitTest
@@ -425,6 +426,44 @@ def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, offsets):
     H.assert_close_f16(outs[0].cpu().numpy(), want, f"{offsets} offsets")
     for i, out in enumerate(outs):
         assert torch.equal(out, outs[0]), f"launch {i} differs from the first"
+
+
+@pytest.mark.parametrize("C", [64, 128])
+def test_bad_row_index_stays_in_its_shared_tile(torch, oracle, C):
+    """A row index beyond the operand sets the abort flag of one CTA of a cluster (the flag that a wait which gives
+    up sets, too).  The launch ends, the status word tells, the other tiles are right, rows of its own tile are either
+    as they were or made with the bad row missing, and the next launch finds nothing of it."""
+    tb, x, w, _ = make(900, 497, C, C)
+    f = 13
+    bad = int(tb.mask_argsort[3 * 128 + 5])  # a row of the fourth tile
+    broken = tb.indices.copy()
+    broken[f, bad] = tb.n_in
+    missing = tb.indices.copy()
+    missing[f, bad] = -1
+    zeros = np.zeros((tb.n_out, C), np.float16)
+    right = oracle.mask_igemm(x, w, zeros.copy(), tb.indices, tb.mask, tb.mask_argsort)
+    without = oracle.mask_igemm(x, w, zeros.copy(), missing, tb.mask, tb.mask_argsort)
+    room = torch.full((tb.n_out + 256, C), 7.0, dtype=torch.float16, device="cuda")
+    out = room[128:128 + tb.n_out]
+    p = ConvParams(3, ConvOpType.Forward)
+    p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, C, C)
+    p.input, p.weight, p.output = H.dev(x, torch), H.dev(w, torch), out
+    p.mask, p.mask_argsort = H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
+    tables = {"broken": H.dev(broken, torch), "right": H.dev(tb.indices, torch)}
+    torch.cuda.synchronize()
+    p.indices = tables["broken"]
+    ConvMainUnitTest.implicit_gemm2(p)
+    assert _lib.device_status() == 2
+    got = out.cpu().numpy()
+    own = np.isin(np.arange(tb.n_out), tb.mask_argsort[3 * 128:4 * 128])
+    H.assert_close_f16(got[~own], right[~own], "other tiles")
+    rows = own & ~(got == 7.0).all(axis=1)
+    H.assert_close_f16(got[rows], without[rows], "the tile's own rows")
+    p.indices = tables["right"]
+    ConvMainUnitTest.implicit_gemm2(p)
+    H.check_status()
+    H.assert_close_f16(out.cpu().numpy(), right, "the launch after it")
+    assert bool((room[:128] == 7.0).all()) and bool((room[128 + tb.n_out:] == 7.0).all())
 
 
 def test_errors_surface_as_exceptions(torch):
