@@ -160,13 +160,15 @@ int gather_mode() {
 // Launch with programmatic stream serialisation: the kernel may be scheduled while its
 // predecessor on the stream is still running and synchronises with it through
 // griddepcontrol.wait in its own code.  `level` 1 (on by default): the chain of the three
-// weight-gradient kernels, the gather-GEMM-scatter calls and the int8 convolutions; level 2
-// (only with CUMM_B200_PDL=2): the fp16 convolution row kernels.  CUMM_B200_PDL=0 launches everything the
-// ordinary way.
+// weight-gradient kernels, the gather-GEMM-scatter calls, the int8 convolutions and the fp16 ones whose items clusters
+// share; level 2 (only with CUMM_B200_PDL=2): the other fp16 convolution row kernels.  CUMM_B200_PDL=0 launches
+// everything the ordinary way.
 // The kernels of table generation take part too, but none triggers its dependent: a dependent's launch overlaps the
 // predecessor's end and no more (150 000 uniform rows, us: ordinary launches 85.4 and, stride 2, 186; so 76.5 and 170;
-// triggered as soon as a kernel starts 91.5 and 199, its successor's waiting blocks hold the SMs).  It also means that whoever reads
-// the tables before its own griddepcontrol.wait finds them complete.
+// triggered as soon as a kernel starts 91.5 and 199, its successor's waiting blocks hold the SMs).
+// int8 convolutions and gather-GEMM-scatter calls read their tables and row lists before their own wait (if they waited:
+// int8, stride 2 from 150 000 rows, 40.9 -> 42.4 us).  PTX asks a dependent to wait where its prerequisite
+// issues launch_dependents; the kernels that make tables here do not, so their blocks have all ended by then.
 template <class Kern, class... Args>
 cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                          Args... args) {

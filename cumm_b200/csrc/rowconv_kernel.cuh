@@ -443,7 +443,6 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
         if (sl[0] >= 0) {
           const int rank = (int)cluster_rank();
           if (rank == 0 && lane == 0 && p.mask_out && sl[3] == 0) {
-            grid_dep_wait();
 #pragma unroll
             for (int w = 0; w < MW; ++w)
               if (w < p.mask_words)
@@ -496,6 +495,8 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // tables whose tiles can be fetched with two 16-byte copies per lane
   const bool wide_copies = conv && MW == 1 && p.mask_words == 1 &&
                            ((reinterpret_cast<uintptr_t>(p.argsort) | reinterpret_cast<uintptr_t>(p.mask)) & 15u) == 0;
+  if (SPLIT)
+    grid_dep_wait();  // the predecessor may have written the tables; who gathers learns its rows from here
   bool ended = false;
   for (;;) {
     account();
@@ -647,10 +648,12 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   if (threadIdx.x == 0)
     CB2_TRACE_CTA(0, 0);
   // Programmatic dependent launch: the next kernel on the stream may be scheduled onto SMs as
-  // they free up, and this one may itself have started before its predecessor finished.  What
-  // runs ahead is the set-up, the scheduler's tickets and mask words and the first row-index
-  // loads -- tables no kernel of this library writes.  Every role calls grid_dep_wait() before
-  // it first touches operand rows, weights or the output.
+  // they free up, and this one may itself have started before its predecessor finished.  What runs
+  // ahead is the set-up and, but for SPLIT, the scheduler's tickets, row lists and mask words, the first row-index
+  // loads and int8's scale and bias: a predecessor that writes those must not let its dependents start early
+  // (see launch_after).  With SPLIT the scheduler waits before it reads a table, so that a small
+  // convolution may follow whatever made its tables, at the price of its first lookups' overlap.  Every role calls
+  // grid_dep_wait() before it first touches operand rows, weights or the output.
   grid_dep_launch();
   // 1024-byte alignment: required by the 128-byte swizzle atoms of TMA and tcgen05.
   const uint32_t raw_addr = smem_u32(smem_raw);

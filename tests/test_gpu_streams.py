@@ -94,3 +94,105 @@ def test_the_same_prepared_call_back_to_back(cuda_lib, oracle):
         stream.synchronize()
     H.check_status()
     assert (out.cpu().numpy() == want).all(), "graph of back-to-back launches, replayed"
+
+
+def _small_scenes(oracle, channels, count, n=2000, grid=(8, 24, 24)):
+    """Scenes of one row count, weights for a layer per step of ``channels``, and what the layers make of them."""
+    rng = np.random.default_rng(731)
+    ws = [(rng.standard_normal((K, 27, C)) / np.sqrt(27 * C)).astype(np.float16) for C, K in zip(channels, channels[1:])]
+    scenes = []
+    for i in range(count):
+        coords = W.sample_coords(n, 730 + i, grid)
+        tb = W.build_tables(coords, grid=grid)
+        x = rng.standard_normal((n, channels[0])).astype(np.float16)
+        want = [x]
+        for w in ws:
+            want.append(oracle.mask_igemm(want[-1], w, np.zeros((n, w.shape[0]), np.float16), tb.indices, tb.mask,
+                                          tb.mask_argsort))
+        scenes.append((coords, tb, x, want[1:]))
+    return ws, scenes
+
+
+def _forward(p, x, w, out, indices, mask, argsort, stream=0):
+    from cumm_b200.conv.main import ConvMainUnitTest
+    p.input, p.weight, p.output = x, w, out
+    p.indices, p.mask, p.mask_argsort, p.stream = indices, mask, argsort, stream
+    ConvMainUnitTest.implicit_gemm2(p)
+
+
+def _params(ws):
+    from cumm_b200.tensorview.gemm import ConvOpType, ConvParams
+    ps = []
+    for w in ws:
+        p = ConvParams(3, ConvOpType.Forward)
+        p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, w.shape[2], w.shape[0])
+        ps.append(p)
+    return ps
+
+
+def test_small_layers_directly_behind_their_table_build(cuda_lib, oracle):
+    """Tables of one scene after the other, and layer into layer of each, on one stream without a synchronisation: the
+    tables of the next scene come to lie where the last one's were, activations are overwritten.  The launches
+    are those that clusters share, which start under their predecessor's end."""
+    import torch
+    from cumm_b200.pairgen import build_tables_gpu
+    grid = (8, 24, 24)
+    ws, scenes = _small_scenes(oracle, (64, 64, 128, 48), 6)
+    wd, ps = [H.dev(w, torch) for w in ws], _params(ws)
+    coords, xs = [H.dev(s[0], torch) for s in scenes], [H.dev(s[2], torch) for s in scenes]
+    acts = [torch.zeros((2000, w.shape[0]), dtype=torch.float16, device="cuda") for w in ws]
+    outs = []
+    torch.cuda.synchronize()
+    for rounds in range(5):
+        for i in range(len(scenes)):
+            t = build_tables_gpu(coords[i], 1, grid)
+            h = xs[i]
+            for p, w, act in zip(ps, wd, acts):
+                _forward(p, h, w, act, t.indices, t.mask, t.mask_argsort)
+                h = act
+            outs.append((i, [a.clone() for a in acts]))
+    torch.cuda.synchronize()
+    H.check_status()
+    for k, (i, got) in enumerate(outs):
+        for layer, (g, want) in enumerate(zip(got, scenes[i][3])):
+            H.assert_close_f16(g.cpu().numpy(), want, f"pass {k}, scene {i}, layer {layer}")
+
+
+def test_small_layers_captured_behind_the_kernels_that_write_their_tables(cuda_lib, oracle):
+    """The same as a graph: kernels write the tables in place, the layers follow at once; replayed on other tables."""
+    import torch
+    ws, scenes = _small_scenes(oracle, (64, 64, 128), 4)
+    wd, ps = [H.dev(w, torch) for w in ws], _params(ws)
+    hold = lambda tb: [H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)]
+    src, here = hold(scenes[0][1]), hold(scenes[0][1])
+    x = H.dev(scenes[0][2], torch)
+    acts = [torch.zeros((2000, w.shape[0]), dtype=torch.float16, device="cuda") for w in ws]
+    stream = torch.cuda.Stream()
+
+    def step():
+        h = x
+        for p, w, act in zip(ps, wd, acts):
+            for a, b in zip(src, here):
+                torch.add(a, 0, out=b)
+            _forward(p, h, w, act, *here, stream=stream.cuda_stream)
+            h = act
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        step()
+        stream.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            step()
+            step()
+        for rounds in range(12):
+            _, tb, feats, want = scenes[rounds % 4]
+            for a, b in zip(src, hold(tb)):
+                a.copy_(b)
+            x.copy_(H.dev(feats, torch))
+            g.replay()
+            g.replay()
+            got = [a.cpu().numpy() for a in acts]
+            for layer in range(len(ws)):
+                H.assert_close_f16(got[layer], want[layer], f"replay {rounds}, layer {layer}")
+    H.check_status()
