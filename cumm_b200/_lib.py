@@ -41,6 +41,7 @@ EXPORTED_SYMBOLS = (
     "cb2_enumerate_gemm_desps",
     "cb2_enumerate_conv_desps",
     "cb2_last_launch_info",
+    "cb2_last_launch_cluster",
     "cb2_dense_tables_run",
     "cb2_gemm_sequence_workspace_size",
     "cb2_gemm_sequence_run",
@@ -239,6 +240,8 @@ def load() -> ctypes.CDLL:
     L.cb2_dense_tables_run.argtypes = [ctypes.POINTER(DenseTablesArgs), ctypes.c_void_p]
     L.cb2_last_launch_info.restype = ctypes.c_int
     L.cb2_last_launch_info.argtypes = [ctypes.POINTER(ctypes.c_int)] * 3
+    L.cb2_last_launch_cluster.restype = ctypes.c_int
+    L.cb2_last_launch_cluster.argtypes = []
     _lib = L
     return L
 
@@ -288,10 +291,12 @@ def kernel_table(which: str):
 
 def last_launch_info() -> dict:
     """Registers per thread, threads per CTA and dynamic shared memory of the last kernel this
-    host thread launched through the library (``cb2_last_launch_info``)."""
+    host thread launched through the library (``cb2_last_launch_info``), and how many CTAs shared an
+    output tile in it (``cb2_last_launch_cluster``)."""
     r, t, m = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     load().cb2_last_launch_info(ctypes.byref(r), ctypes.byref(t), ctypes.byref(m))
-    return {"num_regs": r.value, "num_threads": t.value, "smem_bytes": m.value}
+    return {"num_regs": r.value, "num_threads": t.value, "smem_bytes": m.value,
+            "cluster": load().cb2_last_launch_cluster()}
 
 
 def launch_count() -> int:

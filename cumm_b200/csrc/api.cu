@@ -27,7 +27,7 @@ using namespace cb2;
 thread_local std::string g_err;
 std::atomic<uint64_t> g_launches{0};
 struct LaunchInfo {
-  int num_regs = 0, num_threads = 0, smem_bytes = 0;
+  int num_regs = 0, num_threads = 0, smem_bytes = 0, cluster = 1;
 };
 thread_local LaunchInfo g_last_launch;
 template <class Kern> int kernel_regs(Kern kern) {
@@ -200,13 +200,13 @@ cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 bloc
 
 // How many CTAs share an item's filter offsets in a launch whose items leave most SMs idle: 4 or 8 where the clusters
 // fit the CTAs the launch may have and are all resident at once (each has one item), and a CTA has two offsets of a
-// full tile or more; else 1.  `resident`: per device, clusters of 4 and 8 CTAs of this kernel that it holds, plus
-// one (0 = not asked yet).
+// full tile or more; else 1, and the ordinary kernel runs.  (148 SMs hold 15 clusters of eight and 33 of four.)  `resident`: per device, clusters of 4 and 8 CTAs of this
+// kernel that it holds, plus one (0 = not known yet: not asked, or without an answer).
 using ResidentClusters = std::atomic<int>[kMaxDevices][2];
 template <class Kern>
 int cluster_split(Kern kern, ResidentClusters &resident, int threads, int smem, int max_ctas, long long items, int kv) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+  if (4 * items > max_ctas || kv < 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
     return 1;
   for (int e = 1; e >= 0; --e) {
     const int split = 4 << e;
@@ -226,9 +226,10 @@ int cluster_split(Kern kern, ResidentClusters &resident, int threads, int smem, 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       int found = 0;
-      if (cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        found = 0;
+        return 1;
       }
       n = found + 1;
       resident[dev][e].store(n);
@@ -245,9 +246,15 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   using Cfg = RowConvCfg<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW>;
   auto kern = rowconv_kernel<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, SPLIT>;
   if constexpr (!SPLIT && KIND == 0 && TMA_GATHER) {
+    static ResidentClusters resident;
     const long long items = (p.n_rows + 127) / 128 * static_cast<long long>(p.n_parts);
-    if (p.mode == kModeMaskConv && 4 * items <= max_ctas && p.kv >= 8)
-      return launch_rowconv_inst<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, true>(map, map_a, p, gx, gy, max_ctas, stream);
+    RowConvParams shared = p;
+    shared.split = p.mode != kModeMaskConv ? 1
+                                           : cluster_split(rowconv_kernel<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, true>,
+                                                           resident, Cfg::THREADS, Cfg::SMEM_BYTES, max_ctas, items, p.kv);
+    if (shared.split > 1)
+      return launch_rowconv_inst<KIND, NATOM_K, BLOCK_N, B_MN, TMA_GATHER, MW, true>(map, map_a, shared, gx, gy, max_ctas,
+                                                                                     stream);
   }
   static std::atomic<uint64_t> configured{0};  // bit per device
   static std::atomic<int> regs{0};
@@ -258,23 +265,19 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
     regs.store(kernel_regs(kern));
     configured.fetch_or(1ull << dev);
   }
-  RowConvParams q = p;
-  q.split = 1;
-  if constexpr (SPLIT) {
-    static ResidentClusters resident;
-    q.split = cluster_split(kern, resident, Cfg::THREADS, Cfg::SMEM_BYTES, max_ctas, gx, p.kv);
-  }
+  const int cluster = SPLIT ? p.split : 1;
   g_last_launch.num_regs = regs.load();
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
+  g_last_launch.cluster = cluster;
   // A gather-GEMM-scatter call is one of a run of small kernels (one per filter offset), where
   // overlapping each kernel's set-up with its predecessor's tail nearly halves the run.  For the
   // convolutions it measured +4 % for the int8 kernels (long epilogue tail) and neutral to
   // slightly worse for fp16, so only the former take part by default.
   // So do launches that clusters share: they leave SMs free for their successor, and draw no tickets.
-  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || q.split > 1 ? 1 : 2;
-  CB2_CUDA(launch_after(pdl_level, q.split, kern, dim3(gx * q.split, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
-                        map, map_a, q));
+  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || SPLIT ? 1 : 2;
+  CB2_CUDA(launch_after(pdl_level, cluster, kern, dim3(gx * cluster, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
+                        map, map_a, p));
   g_launches.fetch_add(1);
   return CB2_OK;
 }
@@ -462,6 +465,7 @@ int launch_wgrad_inst(const CUtensorMap &ma, const CUtensorMap &mb, const WgradP
   g_last_launch.num_regs = regs.load();
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
+  g_last_launch.cluster = 1;
   CB2_CUDA(launch_after(1, 1, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, ma, mb, p));
   g_launches.fetch_add(1);
   return CB2_OK;
@@ -1354,6 +1358,8 @@ int cb2_last_launch_info(int *num_regs, int *num_threads, int *smem_bytes) {
     *smem_bytes = g_last_launch.smem_bytes;
   return CB2_OK;
 }
+
+int cb2_last_launch_cluster(void) { return g_last_launch.cluster; }
 
 int cb2_device_status(int *status) {
   DeviceState *dev;

@@ -419,6 +419,9 @@ int cb2_device_status(int *status);
  * from cudaFuncGetAttributes, cumm/conv/main.py:723-729).  Any pointer may be null. */
 int cb2_last_launch_info(int *num_regs, int *num_threads, int *smem_bytes);
 
+/* CTAs that shared an output tile's filter offsets in that launch: 4 or 8 for convolutions of few tiles, else 1. */
+int cb2_last_launch_cluster(void);
+
 /* Number of kernels this library has launched from the calling process (all threads). */
 uint64_t cb2_launch_count(void);
 

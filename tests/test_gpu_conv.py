@@ -404,13 +404,29 @@ def test_offsets_shared_by_a_cluster(torch, oracle, ksize, n, C, K):
         assert np.abs(a - b).max() <= 2.0 ** -9 * max(1.0, np.abs(b).max()), name
 
 
+@pytest.mark.parametrize("n,C,K,ksize,max_ctas,clusters", [
+    (1, 64, 64, 3, 0, [8]), (1024, 128, 64, 3, 0, [8]),           # 1 and 8 items
+    (1000, 64, 256, 3, 0, [8, 4]), (2304, 64, 64, 3, 0, [8, 4]),  # 16, 18: clusters of eight that fit depend on the card
+    (2305, 64, 64, 3, 0, [4]), (4096, 64, 64, 3, 0, [4]),        # 19 and 32 items: eight CTAs each are more than SMs
+    (4608, 64, 64, 3, 0, [4, 1]), (4737, 64, 64, 3, 0, [1]),     # 36 items, 38: four CTAs each are more than SMs
+    (700, 64, 64, 2, 0, [4]),                                    # 8 offsets: two for each of four CTAs
+    (1024, 64, 64, 3, 63, [4]), (1024, 64, 64, 3, 31, [1]),      # a share of the SMs
+    (1024, 72, 64, 3, 0, [1])])                                  # rows that come by cp.async
+def test_which_launches_clusters_share(torch, n, C, K, ksize, max_ctas, clusters):
+    tb = W.build_tables(W.sample_coords(n, 490 + n, (12, 24, 24)), grid=(12, 24, 24), ksize=(ksize,) * 3)
+    assert tb.n_out == n
+    H.run_conv_fwd(torch, np.zeros((n, C), np.float16), np.zeros((K, ksize ** 3, C), np.float16), tb, max_ctas=max_ctas)
+    assert _lib.last_launch_info()["cluster"] in clusters
+    H.check_status()
+
+
 @pytest.mark.parametrize("C,K", [(64, 64), (40, 128), (128, 128)])
 @pytest.mark.parametrize("offsets", [4, 5, 8, 9])
 def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, offsets):
     """Items of four to nine offsets on clusters of eight CTAs: most of a CTA's gather warps have no step, and clear
     their stages where the CTA's sums will lie while another warp's rows are already on their way.  Many launches, all the same."""
     mask_filter = sum(1 << f for f in (13, 4, 22, 10, 16, 12, 14, 1, 25)[:offsets])
-    tb, x, w, dout = make(2300, 495, C, K)
+    tb, x, w, dout = make(1500, 495, C, K)
     want = oracle.mask_igemm(x, w, np.zeros((tb.n_out, K), np.float16), tb.indices, tb.mask, tb.mask_argsort,
                              mask_filter=mask_filter)
     p = ConvParams(3, ConvOpType.Forward)
@@ -421,6 +437,7 @@ def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, offsets):
     torch.cuda.synchronize()
     for p.output in outs:
         ConvMainUnitTest.implicit_gemm2(p)
+        assert _lib.last_launch_info()["cluster"] == 8
     torch.cuda.synchronize()
     H.check_status()
     H.assert_close_f16(outs[0].cpu().numpy(), want, f"{offsets} offsets")
