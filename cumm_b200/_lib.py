@@ -246,15 +246,29 @@ def load() -> ctypes.CDLL:
     return L
 
 
+def host_path() -> Path:
+    """Where the extension that reads parameter records (``csrc/host_args.cpp``) lies.  It uses torch's and Python's own
+    types, so the name says which of each it was built for: another one's is never loaded."""
+    import sysconfig
+
+    import torch
+    return _HERE / f"_host.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
 def load_host():
-    """The extension that reads parameter records (``csrc/host_args.cpp``); raises if it has not been built."""
-    import torch  # noqa: F401  (its libraries are the extension's)
+    """That extension; None, with a warning, where there is none for this torch and this Python: the Python layer
+    reads the records itself, which takes longer and gives the same calls."""
+    import importlib.util
+    import warnings
     try:
-        from . import _host
+        spec = importlib.util.spec_from_file_location("cumm_b200._host", host_path())
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
     except ImportError as e:
-        raise RuntimeError(f"cumm_b200/_host.so is missing or does not load ({e}): the native code has not been built "
-                           "(run `python -c 'import cumm_b200.build as b; b.build()'`).") from e
-    return _host
+        warnings.warn(f"the native reader of parameter records does not load ({e}); every call takes some 20 us longer on "
+                      "the host (run `python -c 'import cumm_b200.build as b; b.build()'`)", RuntimeWarning, stacklevel=2)
+        return None
+    return module
 
 
 def last_error() -> str:

@@ -1,16 +1,18 @@
 """In-tree build of the CUDA library (``cumm_b200/libcumm_b200.so``, sm_100a) and of the extension that reads
-parameter records (``cumm_b200/_host.so``)."""
+parameter records (``_lib.host_path()``), which the library does without where it cannot be built."""
 from __future__ import annotations
 
 import os
 import shutil
 import subprocess
+import warnings
 from pathlib import Path
+
+from ._lib import host_path
 
 _HERE = Path(__file__).resolve().parent
 CSRC = _HERE / "csrc"
 OUT = _HERE / "libcumm_b200.so"
-HOST_OUT = _HERE / "_host.so"
 SOURCES = ["api.cu"]
 HOST_SOURCES = ["host_args.cpp"]
 HEADERS = sorted(p.name for p in CSRC.glob("*.cuh"))
@@ -23,12 +25,13 @@ def _nvcc() -> str:
     return cand
 
 
+def _stale(out: Path, sources) -> bool:
+    deps = [CSRC / s for s in sources] + [_HERE.parent / "include" / "cumm_b200.h"]
+    return not out.exists() or any(d.exists() and d.stat().st_mtime > out.stat().st_mtime for d in deps)
+
+
 def needs_build() -> bool:
-    if not (OUT.exists() and HOST_OUT.exists()):
-        return True
-    t = min(OUT.stat().st_mtime, HOST_OUT.stat().st_mtime)
-    deps = [CSRC / s for s in SOURCES + HOST_SOURCES + HEADERS] + [_HERE.parent / "include" / "cumm_b200.h"]
-    return any(d.exists() and d.stat().st_mtime > t for d in deps)
+    return _stale(OUT, SOURCES + HEADERS) or _stale(host_path(), HOST_SOURCES)
 
 
 def _build_host() -> None:
@@ -40,7 +43,7 @@ def _build_host() -> None:
     if cxx is None:
         raise RuntimeError("g++ not found")
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", str(HOST_OUT)]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", str(host_path())]
     cmd += ["-I" + p for p in (sysconfig.get_paths()["include"], str(root / "include"),
                                str(root / "include" / "torch" / "csrc" / "api" / "include"))]
     cmd += [str(CSRC / s) for s in HOST_SOURCES]
@@ -49,16 +52,23 @@ def _build_host() -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    if not force and not needs_build():
-        return OUT
+    if force or _stale(OUT, SOURCES + HEADERS):
+        _build_library(verbose)
+    if force or _stale(host_path(), HOST_SOURCES):
+        try:
+            _build_host()
+        except (RuntimeError, OSError, subprocess.CalledProcessError) as e:
+            warnings.warn(f"the native reader of parameter records was not built: {e}", RuntimeWarning, stacklevel=2)
+    return OUT
+
+
+def _build_library(verbose: bool) -> None:
     cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
            "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared", "-o", str(OUT)]
     if verbose:
         cmd += ["-Xptxas", "-v"]
     cmd += [str(CSRC / s) for s in SOURCES]
     subprocess.run(cmd, check=True, cwd=str(CSRC))
-    _build_host()
-    return OUT
 
 
 if __name__ == "__main__":

@@ -686,12 +686,32 @@ def _gemm_args(params: GemmParams) -> _lib.GemmArgs:
 _HOST = None
 
 
+class _NoHost:
+    """Where the native reader does not load: it answers for no call."""
+
+    @staticmethod
+    def run_gemm(params):
+        return None
+
+    run_conv = run_gemm
+
+    @staticmethod
+    def gemm_args(params, address):
+        return None
+
+    conv_args = gemm_args
+
+
 def _host():
     """The native reader of the records (csrc/host_args.cpp), which answers for the ordinary call and leaves
     every other to the functions here."""
     global _HOST
     if _HOST is None:
-        host, L = _lib.load_host(), _lib.load()
+        L = _lib.load()
+        host = _lib.load_host()
+        if host is None:
+            _HOST = _NoHost
+            return _HOST
         real = isinstance(L, ctypes.CDLL)  # something that stands in for the library is called from Python only
         address = lambda name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value if real else 0
         host.setup(GemmParams, GemmAlgoDesp, ConvParams, ConvAlgoDesp, address("cb2_gemm_run"), address("cb2_conv_run"))

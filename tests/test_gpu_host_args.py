@@ -128,3 +128,30 @@ def test_other_calls_are_left_to_the_general_path(torch):
     with pytest.raises(RuntimeError, match="can't find any suitable algo"):
         GemmMainUnitTest.matmul2(p)
     H.check_status()
+
+
+def test_same_results_without_the_native_reader(torch, monkeypatch):
+    """A layer's calls of both kinds with the extension and without it."""
+    import cumm_b200.tensorview.gemm as G
+    rng = np.random.default_rng(7)
+    fill = lambda t: t.copy_(H.dev(rng.standard_normal(tuple(t.shape)).astype(np.float16), torch))
+    calls = [(conv(torch, op), run) for op in (ConvOpType.Forward, ConvOpType.BackwardInput, ConvOpType.BackwardWeight)
+             for run in [ConvMainUnitTest.implicit_gemm2]] + [(gemm(torch), GemmMainUnitTest.matmul2)]
+    results = []
+    for p, run in calls:
+        out = p.c if isinstance(p, GemmParams) else (p.output, p.input, p.weight)[int(p.conv_algo_desp.op_type)]
+        for t in (p.a, p.b, p.c) if isinstance(p, GemmParams) else (p.input, p.weight, p.output):
+            if t is not out:
+                fill(t)
+        if isinstance(p, ConvParams) and p.conv_algo_desp.op_type == ConvOpType.BackwardWeight:
+            p.mask.fill_(0x7FFFFFF)
+        run(p)
+        results.append((p, run, out, out.clone()))
+        assert out.abs().max() > 0
+    monkeypatch.setattr(_lib, "load_host", lambda: None)
+    monkeypatch.setattr(G, "_HOST", None)
+    for p, run, out, want in results:
+        out.zero_()
+        run(p)
+        assert torch.equal(out, want)
+    H.check_status()

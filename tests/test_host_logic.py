@@ -462,3 +462,36 @@ def test_scratch_falls_back_to_what_the_call_needs(weight_gradient):
     p.room = 500
     with pytest.raises(torch.cuda.OutOfMemoryError):
         G.prepare_conv(p, True, True)
+
+
+def test_the_native_reader_may_be_missing(monkeypatch, tmp_path):
+    """Built for another torch or Python, or not at all: a warning once, and the Python layer reads every record."""
+    import cumm_b200.tensorview.gemm as G
+    from cumm_b200 import build
+    import torch
+    assert torch.__version__ in _lib.host_path().name and _lib.host_path().exists()
+    assert _lib.load_host() is not None
+    (tmp_path / "broken.so").write_bytes(b"not a library")
+    for path in (tmp_path / "none.so", tmp_path / "broken.so"):
+        monkeypatch.setattr(_lib, "host_path", lambda: path)
+        with pytest.warns(RuntimeWarning, match="does not load"):
+            assert _lib.load_host() is None
+        monkeypatch.setattr(G, "_HOST", None)
+        with pytest.warns(RuntimeWarning, match="does not load"):
+            host = G._host()
+        assert G._host() is host and host.run_gemm(None) is None and host.conv_args(None, 0) is None
+        with pytest.raises(RuntimeError, match="must be set"):
+            G.run_gemm(GemmParams())
+        with pytest.raises(RuntimeError, match="must not empty"):
+            p = ConvParams(3, ConvOpType.Forward)
+            p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, 64, 64)
+            G.run_conv(p)
+    # a tree built for another torch is out of date, and one whose extension cannot be built still gets its library
+    monkeypatch.setattr(build, "host_path", lambda: tmp_path / "none.so")
+    assert build.needs_build()
+    built = []
+    monkeypatch.setattr(build, "_build_library", lambda verbose: built.append(verbose))
+    monkeypatch.setattr(build.shutil, "which", lambda name: None)
+    with pytest.warns(RuntimeWarning, match="was not built"):
+        assert build.build(force=True) == build.OUT
+    assert built == [False]
