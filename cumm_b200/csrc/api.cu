@@ -365,8 +365,9 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
   // more than 128 bytes whose column blocks cross 128-byte lines by 16-byte cp.async.  (60 000 scanned rows,
   // forward, us, gather4 and cp.async: 72 channels 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
   // 46.9, 120 57.9 and 52.8, 128 44.4 and 46.8; of one column block: 40 36.5 and 34.5, 64 -- 100 003 rows -- 34 and
-  // 43; int8 128, stride 2, 41 and 70.)  CUMM_B200_GATHER forces one path.
-  const bool in_lines = (reinterpret_cast<uintptr_t>(p.a) | static_cast<uintptr_t>(p.lda * es)) % 128 == 0;
+  // 43; int8 128, stride 2, 41 and 70.)  Wide rows that overlap, or are all one (a stride below the width), are no
+  // tensor that a map describes: cp.async takes them.  CUMM_B200_GATHER forces one path.
+  const bool in_lines = (reinterpret_cast<uintptr_t>(p.a) | static_cast<uintptr_t>(p.lda * es)) % 128 == 0 && p.lda >= p.red;
   const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) ||
                           (getenv("CUMM_B200_GATHER") ? gather_mode() != 0 : (pl.natom_k == 1 || in_lines));
   CUtensorMap map_a;

@@ -169,6 +169,32 @@ def test_out_of_range_row_index_sets_status_not_fault(torch):
     assert (p.c[7] == 0).all()
 
 
+@pytest.mark.parametrize("shuffle", [ShuffleStrideType.ShuffleAC, ShuffleStrideType.NoShuffle])
+@pytest.mark.parametrize("k,stride", [(128, 0), (128, 64), (200, 128), (128, 128), (128, 192), (136, 192)])
+def test_wide_rows_of_any_stride(torch, oracle, shuffle, k, stride):
+    """Operand rows of more than 128 bytes whose stride is a multiple of a line: one row for all, rows that overlap, rows
+    side by side and apart.  The ones at less than their width apart are views that only cp.async can gather."""
+    m, n = 300, 64
+    rng = np.random.default_rng(k + stride)
+    flat = rng.uniform(-1, 1, m * 192 + k).astype(np.float16)
+    a = np.lib.stride_tricks.as_strided(flat, (m, k), (2 * stride, 2))
+    b = rng.uniform(-1, 1, (n, k)).astype(np.float16)
+    ai, ci = rng.permutation(m).astype(np.int32), rng.permutation(m).astype(np.int32)
+    p = GemmParams()
+    p.algo_desp = H.gemm_desp(shuffle, n=n, k=k)
+    p.a, p.b = H.dev(flat, torch).as_strided((m, k), (stride, 1)), H.dev(b, torch)
+    p.c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+    if shuffle == ShuffleStrideType.ShuffleAC:
+        p.a_inds, p.c_inds = H.dev(ai, torch), H.dev(ci, torch)
+    else:
+        ai = ci = np.arange(m, dtype=np.int32)
+    GemmMainUnitTest.matmul2(p)
+    torch.cuda.synchronize()
+    H.check_status()
+    want = oracle.gemm_shuffle_ac(np.ascontiguousarray(a), b, np.zeros((m, n), np.float16), ai, ci)
+    H.assert_close_f16(p.c.cpu().numpy(), want, f"k={k} stride={stride}")
+
+
 @pytest.mark.parametrize("tile_n,tile_k", [(64, 64), (64, 128), (128, 64), (128, 128)])
 def test_shuffle_ac_every_tile_shape(torch, oracle, tile_n, tile_k):
     """The descriptor's tile shape selects the kernel variant; all of them compute the same thing."""
