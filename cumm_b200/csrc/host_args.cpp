@@ -106,6 +106,28 @@ struct Record {
   }
 };
 
+// The types that the Python layer has a code for; a tensor of any other is refused there.
+bool has_code(at::ScalarType t) {
+  switch (t) {
+  case at::kFloat:
+  case at::kInt:
+  case at::kShort:
+  case at::kChar:
+  case at::kDouble:
+  case at::kBool:
+  case at::kByte:
+  case at::kHalf:
+  case at::kLong:
+  case at::kBFloat16:
+  case at::kUInt16:
+  case at::kUInt32:
+  case at::kUInt64:
+    return true;
+  default:
+    return false;
+  }
+}
+
 // A CUDA tensor with at least one element, or none.
 struct View {
   const at::Tensor *t = nullptr;
@@ -124,7 +146,7 @@ View view(const Record &r, PyObject *key, bool may_be_none) {
   }
   need(THPVariable_CheckExact(v.p));
   w.t = &THPVariable_Unpack(v.p);
-  need(w.t->is_cuda() && w.t->layout() == at::kStrided && w.t->numel() > 0);
+  need(w.t->is_cuda() && w.t->layout() == at::kStrided && w.t->numel() > 0 && has_code(w.t->scalar_type()));
   return w;
 }
 int size32(int64_t v) {

@@ -122,6 +122,16 @@ def test_other_calls_are_left_to_the_general_path(torch):
         assert native(p) is None, text
         with pytest.raises(error, match=text):
             (ConvMainUnitTest.implicit_gemm2 if isinstance(p, ConvParams) else GemmMainUnitTest.matmul2)(p)
+    # types without a code of the operator surface, in every place where the reader does not look at the type itself
+    odd = lambda t: t.new_empty(tuple(t.shape), dtype=torch.complex64)
+    for make, names in ((lambda: gemm(torch), ("a_inds", "c_inds")),
+                        (lambda: change(fwd(), bias=zeros(72)), ("indices", "mask", "mask_argsort", "mask_output", "bias"))):
+        for name in names:
+            p = make()
+            setattr(p, name, odd(getattr(p, name)))
+            assert native(p) is None, name
+            with pytest.raises(KeyError):
+                (ConvMainUnitTest.implicit_gemm2 if isinstance(p, ConvParams) else GemmMainUnitTest.matmul2)(p)
     # what only the library refuses comes back from the native path as the same error
     p = gemm(torch)
     p.algo_desp.tile_shape = [128, 32, 64]
