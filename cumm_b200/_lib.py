@@ -265,7 +265,7 @@ def load_host():
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
     except ImportError as e:
-        warnings.warn(f"the native reader of parameter records does not load ({e}); every call takes some 20 us longer on "
+        warnings.warn(f"the native reader of parameter records does not load ({e}); a call takes 8 to 12 us longer on "
                       "the host (run `python -c 'import cumm_b200.build as b; b.build()'`)", RuntimeWarning, stacklevel=2)
         return None
     return module

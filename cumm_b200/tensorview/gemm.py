@@ -876,13 +876,15 @@ def run_conv(params: ConvParams) -> None:
         if rc:
             _lib.raise_for(rc)
         return
-    if not params.conv_algo_desp.mask_sparse:
+    desp = params.conv_algo_desp
+    if not desp.mask_sparse:
         # dense convolution: the same kernels over the neighbour table of the full grid
         from ..dense import run_dense_conv
         return run_dense_conv(params)
     L = _lib.load()
     args = _lib.ConvArgs()
-    if host.conv_args(params, ctypes.addressof(args)):
+    # the reader leaves the weight gradient's launch to this function; any other call it has just declined
+    if desp.op_type == ConvOpType.BackwardWeight and host.conv_args(params, ctypes.addressof(args)):
         import torch
         args._device = torch.cuda.current_device()
     else:
