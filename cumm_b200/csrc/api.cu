@@ -199,9 +199,13 @@ cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 bloc
 }
 
 // How many CTAs share an item's filter offsets in a launch whose items leave most SMs idle: 4 or 8 where the clusters
-// fit the CTAs the launch may have and are all resident at once (each has one item), and a CTA has two offsets of a
-// full tile or more; else 1, and the ordinary kernel runs.  (148 SMs hold 15 clusters of eight and 33 of four.)  `resident`: per device, clusters of 4 and 8 CTAs of this
-// kernel that it holds, plus one (0 = not known yet: not asked, or without an answer).
+// fit the CTAs the launch may have and are all resident at once (each has one item; 148 SMs hold 33 clusters of four and
+// 15 of eight), else 1, and the ordinary kernel runs.  Four from two offsets a CTA on, eight from eight.  (Forward, us,
+// one CTA, four, eight.  125 offsets, 1900 rows of a crop at 32 channels: 49.7, 19.5, 17.1.  27 offsets at 64 channels,
+// crops of 1000 and 1900 rows: 14.2, 9.9, 9.5 and 14.9, 10.4, 10.6; 1900 uniform rows, whose tiles stay with one CTA of the
+// cluster: 7.2, 6.9, 7.4.  8 offsets, 2000 and 3800 rows: 8.8, 8.8 and 9.6, 9.6, at 128 channels 12.4, 10.9.)
+// `resident`: per device, clusters of 4 and 8 CTAs of this kernel that it holds, plus one (0 = not known yet: not
+// asked, or without an answer).
 using ResidentClusters = std::atomic<int>[kMaxDevices][2];
 template <class Kern>
 int cluster_split(Kern kern, ResidentClusters &resident, int threads, int smem, int max_ctas, long long items, int kv) {
@@ -210,7 +214,7 @@ int cluster_split(Kern kern, ResidentClusters &resident, int threads, int smem, 
     return 1;
   for (int e = 1; e >= 0; --e) {
     const int split = 4 << e;
-    if (items * split > max_ctas || kv < 2 * split)
+    if (items * split > max_ctas || kv < (e ? 64 : 8))
       continue;
     int n = resident[dev][e].load();
     if (n == 0) {

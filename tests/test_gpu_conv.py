@@ -405,39 +405,49 @@ def test_offsets_shared_by_a_cluster(torch, oracle, ksize, n, C, K):
 
 
 @pytest.mark.parametrize("n,C,K,ksize,max_ctas,clusters", [
-    (1, 64, 64, 3, 0, [8]), (1024, 128, 64, 3, 0, [8]),           # 1 and 8 items
-    (1000, 64, 256, 3, 0, [8, 4]), (2304, 64, 64, 3, 0, [8, 4]),  # 16, 18: clusters of eight that fit depend on the card
-    (2305, 64, 64, 3, 0, [4]), (4096, 64, 64, 3, 0, [4]),        # 19 and 32 items: eight CTAs each are more than SMs
+    (1, 64, 64, 5, 0, [8]), (1024, 128, 64, 5, 0, [8]), (1024, 64, 64, 5, 63, [4]),  # 1 and 8 items; a share of the SMs
+    (1000, 64, 256, 5, 0, [8, 4]), (2304, 64, 64, 5, 0, [8, 4]),  # 16, 18: clusters of eight that fit depend on the card
+    (2305, 64, 64, 5, 0, [4]), (4096, 64, 64, 5, 0, [4]),        # 19 and 32 items: eight CTAs each are more than SMs
+    (1, 64, 64, 3, 0, [4]), (4096, 64, 64, 3, 0, [4]), (700, 64, 64, 2, 0, [4]),  # fewer than 64 offsets, as few as 8
     (4608, 64, 64, 3, 0, [4, 1]), (4737, 64, 64, 3, 0, [1]),     # 36 items, 38: four CTAs each are more than SMs
-    (700, 64, 64, 2, 0, [4]),                                    # 8 offsets: two for each of four CTAs
-    (1024, 64, 64, 3, 63, [4]), (1024, 64, 64, 3, 31, [1]),      # a share of the SMs
+    (1024, 64, 64, 3, 31, [1]),
     (1024, 72, 64, 3, 0, [1])])                                  # rows that come by cp.async
 def test_which_launches_clusters_share(torch, n, C, K, ksize, max_ctas, clusters):
     tb = W.build_tables(W.sample_coords(n, 490 + n, (12, 24, 24)), grid=(12, 24, 24), ksize=(ksize,) * 3)
     assert tb.n_out == n
-    H.run_conv_fwd(torch, np.zeros((n, C), np.float16), np.zeros((K, ksize ** 3, C), np.float16), tb, max_ctas=max_ctas)
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")
+    p = ConvParams(3, ConvOpType.Forward)
+    p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, C, K)
+    p.conv_algo_desp.dynamic_mask, p.max_ctas = tb.kv > 32, max_ctas
+    p.input, p.weight, p.output = z(n, C), z(K, tb.kv, C), z(n, K)
+    p.indices, p.mask, p.mask_argsort = H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
+    ConvMainUnitTest.implicit_gemm2(p)
     assert _lib.last_launch_info()["cluster"] in clusters
     H.check_status()
 
 
 @pytest.mark.parametrize("C,K", [(64, 64), (40, 128), (128, 128)])
-@pytest.mark.parametrize("offsets", [4, 5, 8, 9])
-def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, offsets):
-    """Items of four to nine offsets on clusters of eight CTAs: most of a CTA's gather warps have no step, and clear
-    their stages where the CTA's sums will lie while another warp's rows are already on their way.  Many launches, all the same."""
+@pytest.mark.parametrize("ksize,offsets", [(3, 4), (3, 5), (3, 8), (3, 9), (5, 1), (5, 2)])
+def test_cluster_whose_ctas_have_one_step(torch, oracle, C, K, ksize, offsets):
+    """Items of four to nine offsets on clusters of four CTAs, of four and eight (one and two of each mask word) on
+    clusters of eight: most of a CTA's gather warps have no step, and clear their stages where the CTA's sums will lie
+    while another warp's rows are already on their way.  Many launches, all the same."""
     mask_filter = sum(1 << f for f in (13, 4, 22, 10, 16, 12, 14, 1, 25)[:offsets])
-    tb, x, w, dout = make(1500, 495, C, K)
+    tb, x, w, dout = make(1500, 495, C, K, ksize=(ksize,) * 3)
+    tiles = [np.bitwise_or.reduce(tb.mask[i:i + 128] & np.uint32(mask_filter)) for i in range(0, tb.n_out, 128)]
+    assert ksize == 5 or max(bin(m).count("1") for m in tiles) == offsets
     want = oracle.mask_igemm(x, w, np.zeros((tb.n_out, K), np.float16), tb.indices, tb.mask, tb.mask_argsort,
                              mask_filter=mask_filter)
     p = ConvParams(3, ConvOpType.Forward)
     p.conv_algo_desp = H.conv_desp(ConvOpType.Forward, C, K)
+    p.conv_algo_desp.dynamic_mask = tb.kv > 32
     p.input, p.weight, p.mask_filter = H.dev(x, torch), H.dev(w, torch), mask_filter
     p.indices, p.mask, p.mask_argsort = H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
     outs = [torch.full((tb.n_out, K), 7.0, dtype=torch.float16, device="cuda") for _ in range(50)]
     torch.cuda.synchronize()
     for p.output in outs:
         ConvMainUnitTest.implicit_gemm2(p)
-        assert _lib.last_launch_info()["cluster"] == 8
+        assert _lib.last_launch_info()["cluster"] == (4 if ksize == 3 else 8)
     torch.cuda.synchronize()
     H.check_status()
     H.assert_close_f16(outs[0].cpu().numpy(), want, f"{offsets} offsets")
