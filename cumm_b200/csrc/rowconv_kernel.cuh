@@ -653,8 +653,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   // loads and int8's scale and bias: a predecessor that writes those must not let its dependents start early
   // (see launch_after).  With SPLIT the scheduler waits before it reads a table, so that a small
   // convolution may follow whatever made its tables, at the price of its first lookups' overlap.  Every role calls
-  // grid_dep_wait() before it first touches operand rows, weights or the output.
-  grid_dep_launch();
+  // grid_dep_wait() before it first touches operand rows, weights or the output.  The weight warp lets the next kernel
+  // begin.
   // 1024-byte alignment: required by the 128-byte swizzle atoms of TMA and tcgen05.
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
@@ -1164,6 +1164,9 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     if (lane == 0)
       tma_prefetch_desc(&tmap_b);
     grid_dep_wait();
+    // Only now: the next launch may begin while this one runs, but not while this one's predecessor does.  A record has
+    // two pairs of ticket counters, and three launches of it in flight would have two that draw from one.
+    grid_dep_launch();
     for (int more; ok && (more = tc.next(p, rv, [](const int *) {})) != 0;) {
       ok = more > 0;
       for (int left = ok ? tc.offsets : 0; ok && left > 0; --left) {

@@ -95,7 +95,7 @@ typedef struct cb2_gemm_args {
    *   running at the same time on another stream.  Give every captured or replayed call its own;
    *   a caller that launches the SAME record twice in a row alternates between two such blocks
    *   (with programmatic dependent launch the second launch may draw tickets while the first
-   *   still runs).
+   *   still runs; a third does not begin before the first has ended).
    * max_ctas: upper bound on the CTAs of the launch (0 = one per SM).  The kernels are persistent
    *   and sized to one CTA per SM; calls that are meant to run side by side on different streams
    *   (forward, backward input and backward weight of one layer) each take a share.
@@ -169,7 +169,7 @@ typedef struct cb2_conv_args {
    *   running at the same time on another stream.  Give every captured or replayed call its own;
    *   a caller that launches the SAME record twice in a row alternates between two such blocks
    *   (with programmatic dependent launch the second launch may draw tickets while the first
-   *   still runs).
+   *   still runs; a third does not begin before the first has ended).
    * max_ctas: upper bound on the CTAs of the launch (0 = one per SM).  The kernels are persistent
    *   and sized to one CTA per SM; calls that are meant to run side by side on different streams
    *   (forward, backward input and backward weight of one layer) each take a share.

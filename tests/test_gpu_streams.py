@@ -196,3 +196,53 @@ def test_small_layers_captured_behind_the_kernels_that_write_their_tables(cuda_l
             for layer in range(len(ws)):
                 H.assert_close_f16(got[layer], want[layer], f"replay {rounds}, layer {layer}")
     H.check_status()
+
+
+def test_every_launch_of_a_chain_does_its_work_once(cuda_lib):
+    """One record launched many times in a row, each launch adding one to every output in place: a tile that a launch
+    leaves out or does twice stays visible.  Launches of fewer tiles than SMs, some of many offsets and most of one, so
+    that a launch's successors find SMs free while its heaviest tiles still run."""
+    import torch
+    from cumm_b200.layer import make_desp
+    from cumm_b200.tensorview.gemm import ConvOpType, ConvParams, GemmParams, ShuffleStrideType, prepare_conv, prepare_gemm
+    side = np.arange(17, dtype=np.int32)
+    block = np.stack(np.meshgrid([0], side + 3, side + 9, side + 9, indexing="ij"), -1).reshape(-1, 4)
+    sparse = W.sample_coords(5000, 741, (41, 300, 300))
+    coords = np.unique(np.concatenate([block, sparse]), axis=0).astype(np.int32)
+    tb = W.build_tables(np.random.default_rng(742).permutation(coords), grid=(41, 300, 300))
+    n, C, launches = tb.n_out, 128, 100
+    assert 128 * 70 < n < 128 * 80
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        out = torch.zeros((n, C), dtype=torch.int8, device="cuda")
+        p = ConvParams(3, ConvOpType.Forward)
+        p.conv_algo_desp = make_desp(ConvOpType.Forward, True, C, C)
+        p.input = torch.ones((n, C), dtype=torch.int8, device="cuda")
+        p.weight = torch.ones((C, 27, C), dtype=torch.int8, device="cuda")
+        p.output = p.output_add = out
+        p.scale, p.bias = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+        p.beta, p.stream = 1.0, stream.cuda_stream
+        p.indices, p.mask, p.mask_argsort = H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
+        a = torch.zeros((n, 64), dtype=torch.float16, device="cuda")
+        a[:, 0] = 1
+        q = GemmParams()
+        q.algo_desp = H.gemm_desp(ShuffleStrideType.ShuffleAC, trans_b=True, n=64, k=64)
+        q.a, q.b, q.c = a, torch.ones((64, 64), dtype=torch.float16, device="cuda"), torch.zeros_like(a)
+        q.a_inds = q.c_inds = torch.randperm(n, device="cuda").int()
+        q.beta, q.stream = 1.0, stream.cuda_stream
+        stream.synchronize()
+        for call, dst in ((prepare_conv(p), out), (prepare_gemm(q), q.c)):
+            for _ in range(launches):
+                call.launch()
+            stream.synchronize()
+            assert bool((dst == launches).all()), "eager launches"
+            dst.zero_()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                for _ in range(launches // 4):
+                    call.launch()
+            for _ in range(4):
+                g.replay()
+            stream.synchronize()
+            assert bool((dst == launches).all()), "captured launches"
+    H.check_status()
