@@ -167,9 +167,10 @@ __device__ __forceinline__ void wgrad_scan4(const int (&v)[4], int (&excl)[4], i
 // A unit costs its CTA about as much as kWgradUnitSteps steps (a partial sum stored, counted in, and
 // read again by whoever sums): every offset is charged that many steps before its own, or the CTAs that
 // get a dozen offsets of one or two steps each are the last to finish.  The cuts are made in charged steps.
-// (Two, three, four and six steps, us: 150 000 uniform rows at 128 channels 32.0, 31.1, 31.5, 33.3; 60 000, 128 to 64
-// 20.8, 19.6, 21.0, 21.0; 1600 scanned rows 17.7, 17.3, 16.8, 16.3; 100 003 at 64 channels 35.2, 35.4, 35.3, 35.4.)
-constexpr int kWgradUnitSteps = 3;
+// (Over 247 shapes of 1500 to 490 000 rows two and three steps are the same in the mean, and three moves the cuts
+// by luck, us: 150 000 uniform rows at 128 channels 27.7 and 26.5, 80 000 20.6 and 21.2, 10 000 scanned ones 20.3
+// and 20.9; 104 to 72 channels, stride 2 from 150 000 uniform rows 58 and 64, 150 000 scanned ones 73.4 and 76.0.)
+constexpr int kWgradUnitSteps = 2;
 // Given the step counts of this lane's offsets: P = charged steps before the offset's first own step,
 // T = all charged steps, c_first = CTA holding the offset's first step, S = units of the offset, U = units
 // before it.
