@@ -1216,8 +1216,10 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       // not requested at all -- for the offsets away from the centre that is most quads, and the
       // copy engine's request rate is what bounds such steps.  The stage therefore keeps the
       // invariant "a quad that was not requested holds zeros": it is cleared once here, and a
-      // quad that was filled in the previous use and is not needed now is requested with no row at all
-      // (cleared by stores and a proxy fence instead: 36.5 against 36.0 us, 100 003 scanned rows at 64 channels).
+      // quad that was filled in the previous use and is not needed now is requested with no row at all (fp16)
+      // or cleared by stores again (int8).  (Scanned rows, forward, us, requested and cleared: fp16, 100 003 at 64 channels
+      // 36.0 and 36.5, 40 to 72 channels 40 000 28.2 and 31.1, 80 000 53.2 and 48.4, 150 000 64.5 and 70.3; int8, 112 to 32,
+      // 40 000 24.5 and 23.9, 80 000 34.2 and 30.6, 150 000 at 32 to 96 50.3 and 46.9, at 128 44.0 and 44.0.)
       // The neighbour indices of the group's next step in the tile are on their way while it waits for its stage
       // (the same scene: 39.8 -> 36.4 us; 125 offsets, 30 011 rows: 77 -> 61).
       const int g = (warp - Cfg::FIRST_GATHER_WARP) / NATOM_K;
@@ -1292,7 +1294,13 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           }
           const bool wanted = (idx[0] & idx[1] & idx[2] & idx[3]) >= 0;  // some row index is not -1
           const uint32_t need = __ballot_sync(0xffffffffu, wanted);
-          const uint32_t ask = need | dirty;
+          const uint32_t ask = KIND == 1 ? need : need | dirty;
+          if (KIND == 1 && (dirty & ~need)) {
+            for (uint32_t q = dirty & ~need; q; q &= q - 1)
+              st_shared_zero16(first_quad + (__ffs(q) - 1) * (4 * 128) + lane * 16);
+            fence_proxy_async_smem();  // as at the start
+            __syncwarp();              // before lane 0 arrives
+          }
           if (lane == 0) {
             CB2_TRACE_EVENT(g, 2, f);  // stage free
             mbar_arrive_expect_tx(full_a(g), static_cast<uint32_t>(__popc(ask)) * 512);
