@@ -277,8 +277,8 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   // A gather-GEMM-scatter call is one of a run of small kernels (one per filter offset), where
   // overlapping each kernel's set-up with its predecessor's tail nearly halves the run.  For the
   // convolutions it measured +4 % for the int8 kernels (long epilogue tail) and neutral to
-  // slightly worse for fp16, so only the former take part by default.
-  // So do launches that clusters share: they leave SMs free for their successor, and draw no tickets.
+  // slightly worse for fp16, so only the former take part by default, and launches that clusters share: they leave
+  // SMs free for their successor.
   const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || SPLIT ? 1 : 2;
   CB2_CUDA(launch_after(pdl_level, cluster, kern, dim3(gx * cluster, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
                         map, map_a, p));
@@ -368,8 +368,10 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
   // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes), but rows of
   // more than 128 bytes whose column blocks cross 128-byte lines by 16-byte cp.async.  (60 000 scanned rows,
   // forward, us, gather4 and cp.async: 72 channels 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
-  // 46.9, 120 57.9 and 52.8, 128 44.4 and 46.8; of one column block: 40 36.5 and 34.5, 64 -- 100 003 rows -- 34 and
-  // 43; int8 128, stride 2, 41 and 70.)  Wide rows that overlap, or are all one (a stride below the width), are no
+  // 46.9, 120 57.9 and 52.8, 128 44.4 and 46.8, 136 86.7 and 81.9, 160 75.3 and 75.4, 192 69.6 and 76.8, 200 94.1 and
+  // 85.3, 224 76.1 and 78.5, 248 95.6 and 89.6, 256 72.3 and 78.3, 320 101 and 111, 512 134 and 148; 150 000 uniform rows
+  // 136 41.6 and 38.4, 192 33.3 and 35.0, 256 35.3 and 36.7; of one column block: 40 36.5 and 34.5, 64 -- 100 003
+  // rows -- 34 and 43; int8 128, stride 2, 41 and 70.)  Wide rows that overlap, or are all one (a stride below the width), are no
   // tensor that a map describes: cp.async takes them.  CUMM_B200_GATHER forces one path.
   const bool in_lines = (reinterpret_cast<uintptr_t>(p.a) | static_cast<uintptr_t>(p.lda * es)) % 128 == 0 && p.lda >= p.red;
   const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) ||

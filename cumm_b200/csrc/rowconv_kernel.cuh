@@ -367,6 +367,8 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // run while the CTA sets up its barriers and tensor memory.
 // SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
 // becomes what that makes of the CTA; it stays kSplitUnknown in one that gives up before its item is known.
+// (Items of up to 0, 3 and 7 offsets kept, forward, us: 1900 and 4000 uniform rows at 64 channels 8.4, 6.9, 6.9 and 9.1, 7.7,
+// 7.7; 8 offsets, 3800 rows at 64 and 128 9.6, 9.6, 9.2 and 10.9, 10.9, 11.4.)
 constexpr int kSplitSoloOffsets = 3;
 enum SplitState {
   kSplitUnknown = 0,
@@ -633,8 +635,8 @@ __device__ __forceinline__ uint4 rowconv_finish8(const RowConvParams &p, const f
 // one after the other, so a cluster of `split` CTAs shares an item's offsets: each sums its own in tensor memory and
 // leaves the sums, fp32, in its shared memory; then each makes the output rows of its share of the tile from the
 // sums of all, in the order of the CTAs, through distributed shared memory.  (Forward, us, without, with, and with
-// launches that start under their predecessor's tail: 2000 rows of a crop at 64 channels 14.6, 11.5, 8.2, scanned scenes
-// of 4000 rows, 64 to 32, 13.0, 10.6, 9.4, 1600 at 128 18.0, 12.9, 11.4; 2000 uniform rows 7.2, 7.5, 5.0.  Clusters of
+// launches that start under their predecessor's tail: 2000 rows of a crop at 64 channels 14.9, 11.5, 10.3, scanned scenes
+// of 4000 rows, 64 to 32, 12.9, 10.4, 9.3, 1600 at 128 18.5, 12.6, 11.0; 2000 uniform rows 7.2, 7.9, 6.7.  Clusters of
 // two, for up to half as many items as SMs, gained 8 % on 9000 scanned rows and lost 6 % on uniform ones, most of
 // whose tiles have one offset.)
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MASK_WORDS = 1, bool SPLIT = false>

@@ -773,9 +773,10 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     uint32_t phase = 0;
     bool ok_all = true;
     // The lane that issues.  Elected, the descriptors stay in uniform registers and a step costs the issuer a third:
-    // 100 003 scanned rows at 64 channels 40.2 -> 35.3 us, 30 011 rows of 125 offsets 31.7 -> 27.4.  Launches of
-    // the widest tiles, three stages, wait for memory; stages given back sooner only crowd it (960 000
-    // uniform rows 106.2 -> 108.4).
+    // 100 003 scanned rows at 64 channels 40.2 -> 35.3 us, 30 011 rows of 125 offsets 31.7 -> 27.4.  At the widest
+    // tiles, three stages, it makes no difference but on the largest scenes, which it slows down (128 channels, lane 0
+    // and elected: 20 000 scanned rows 23.9 and 23.5, 60 000 37.8 and 37.1, 100 003 50.8 and 50.7, 150 000 uniform ones
+    // 30.9 and 31.0, 400 000 55.9 and 56.2, 960 000 104.5 and 106.6).
     auto issuer = [&]() { return Cfg::SA > 3 ? elect_one() : lane == 0; };
     const uint64_t adesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES, 128 * 128, 1024);
     const uint64_t bdesc_base = make_smem_desc(sbase + Cfg::OFF_STAGES + Cfg::A_BYTES, 128 * 128, 1024);
@@ -783,7 +784,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
         p.lists, p.list_stride, s_plan, s_tiles,
         [&](int tile, const int *e, bool first) -> bool {
           const int buf = acc_use & 1;
-          // the warp walks together, its state the same in every lane; lane 0 issues
+          // the warp walks together, its state the same in every lane; one lane issues
           bool ok = true;
           if (first)
             ok = mbar_wait(acc_empty(buf), ((acc_use >> 1) & 1) ^ 1, abort_flag);
@@ -839,7 +840,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
   } else if constexpr (GATHER == kGatherTma4) {
     // ======================= gather both operands: the GW warps of group g own stage g, steps g,
     // g + SA, ... of this CTA.  A lane fetches a quad of four tile rows, one request per column block and
-    // operand; a row of -1 is out of bounds and reads as zeros.  The row numbers run ahead of the copies:
+    // operand; a missing row is asked for out of bounds and reads as zeros.  The row numbers run ahead of the copies:
     // while the group waits for its stage, the neighbour indices of its next step and the sort order of
     // the one after are on their way.
     const int g = (warp - 5) / Cfg::GW;

@@ -172,7 +172,10 @@ typedef struct cb2_conv_args {
    *   still runs; a third does not begin before the first has ended).
    * max_ctas: upper bound on the CTAs of the launch (0 = one per SM).  The kernels are persistent
    *   and sized to one CTA per SM; calls that are meant to run side by side on different streams
-   *   (forward, backward input and backward weight of one layer) each take a share.
+   *   (forward, backward input and backward weight of one layer) each take a share.  A last place of the results may
+   *   depend on it: fp16 forward and backward input of few tiles add a tile's offsets on several CTAs where the bound
+   *   leaves room for them (cb2_last_launch_cluster), on one otherwise; fp32 sums in a fixed order either way, as the
+   *   weight gradient's, whose partial sums are cut by the number of CTAs.
    * reuse_plan (backward weight only): the workspace still holds the plan of an earlier, stream-ordered
    *   call on the same workspace with the same reduced masks (contents, not just address), row count,
    *   mask_width, mask_filter, tile_n and max_ctas -- skip the planning kernel.  The plan depends on

@@ -316,8 +316,9 @@ def test_int8_output_add_and_relu(torch, oracle):
 @pytest.mark.parametrize("C", [72, 128, 264])  # one pass with and without a ragged end, three passes
 @pytest.mark.parametrize("n,grid", [(129, (8, 24, 24)), (2300, (8, 24, 24)), (3000, (41, 300, 300))])
 def test_wide_rows_many_steps_per_cta(torch, oracle, n, grid, C, max_ctas):
-    """Four operand stages filled in turn by three groups: steps per tile from one to dozens, tiles of one
-    CTA one after the other, so that stage and group meet in every combination."""
+    """Four operand stages, filled in turn by three groups (72 and 264 channels, cp.async) or by a group each (128,
+    gather4): steps per tile from one to dozens, tiles of one CTA one after the other, so that stage and group meet
+    in every combination."""
     tb = W.build_tables(W.sample_coords(n, 460 + n, grid), grid=grid)
     rng = np.random.default_rng(461)
     x = rng.standard_normal((tb.n_in, C)).astype(np.float16)
