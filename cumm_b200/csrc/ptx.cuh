@@ -177,6 +177,26 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The same for a condition that the whole warp looks at together.
+template <class Cond> __device__ __forceinline__ bool wait_for(Cond cond, volatile int *abort_flag) {
+  unsigned long long t0 = 0;
+  for (uint32_t i = 0; !cond(); ++i) {
+    __nanosleep(20);
+    if ((i & 63u) == 63u) {
+      const unsigned long long now = __shfl_sync(0xffffffffu, global_timer_ns(), 0);
+      if (__any_sync(0xffffffffu, *abort_flag != 0))
+        return false;
+      if (t0 == 0)
+        t0 = now;
+      else if (now - t0 > kWaitLimitNs) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
 // Warp-collective wait: lane 0 polls, the other lanes sleep at the shuffle.  Keeps the
 // number of spinning threads per SM small (one per warp), which matters because pollers
 // compete for issue slots with the warps that do the work.

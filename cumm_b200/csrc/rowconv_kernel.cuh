@@ -65,9 +65,6 @@ struct RowConvParams {
 #ifndef CB2_ROWCONV_RING
 #define CB2_ROWCONV_RING 12
 #endif
-#ifndef CB2_ROWCONV_STEP_BUDGET
-#define CB2_ROWCONV_STEP_BUDGET 12
-#endif
 #ifndef CB2_ROWCONV_TICKET_BATCH
 #define CB2_ROWCONV_TICKET_BATCH 4
 #endif
@@ -123,6 +120,11 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   // as long and their registers all taken: each thread stores its own 32 bytes.
   static constexpr int EPI_WARP_BYTES = KIND == 0 ? 32 * 64 : 0;
   static constexpr int EPI_BYTES = 8 * EPI_WARP_BYTES;
+  static constexpr bool DEALT = KIND == 0;  // a CTA's first ticket is its own number
+  // steps a CTA may hold (drawn, not issued) and still draw: what a ticket, the tile's words, its indices and its first
+  // rows take.  (6, 8, 12, 16: 100 003 scanned rows at 64 channels 33.6, 30.4, 27.6, 27.7 us, 150 000 at 128 65.9,
+  // 64.5, 64.5, 64.7, 150 000 uniform ones 22.0, 21.7, 22.0, 22.4.)
+  static constexpr int STEP_BUDGET = NATOM_K == 1 ? 12 : 8;
   static constexpr int RING_SLOT_INTS = 136 + 128 * MASK_WORDS;  // header; 128 gather rows; 128 output rows / row masks
   // int8 rows of up to 128 bytes: a stage holds the step's weight tile beside its rows, under the same pair
   // of barriers -- one wait and one commit per step for the issuer (46.7 -> 43.7 us for the stride-2
@@ -362,10 +364,9 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// The first batch of tickets is requested at kernel entry (first_ticket_request), long before the
-// scheduler can use it: the counter's round trip, and an L2 prefetch of the first tile's words,
-// run while the CTA sets up its barriers and tensor memory.
-// SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
+// An L2 prefetch of the first tile's words runs while the CTA sets up its barriers and tensor memory.
+// `progress` (shared memory): steps that the MMA issuer has issued, tiles without an offset counted as one.
+// `first`, `dealt`: see below.  SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
 // becomes what that makes of the CTA; it stays kSplitUnknown in one that gives up before its item is known.
 // (Items of up to 0, 3 and 7 offsets kept, forward, us: 1900 and 4000 uniform rows at 64 channels 8.4, 6.9, 6.9 and 9.1, 7.7,
 // 7.7; 8 offsets, 3800 rows at 64 and 128 9.6, 9.6, 9.2 and 10.9, 10.9, 11.4.)
@@ -376,41 +377,40 @@ enum SplitState {
   kSplitNothing,  // shared, none of the offsets is this CTA's
   kSplitSums      // shared, the epilogue warps leave this CTA's sums in shared memory and count themselves
 };
-template <int MW, bool SPLIT>
+template <int MW, bool SPLIT, int STEP_BUDGET>
 __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int block_n,
-                                              int kpasses, int first_base, int first_cnt, volatile int *split_state) {
+                                              int kpasses, int first, int dealt, volatile int *progress, volatile int *split_state) {
   const int nitems = ntiles * p.n_parts;
-  constexpr int STEP_BUDGET = CB2_ROWCONV_STEP_BUDGET;  // steps a CTA may hold (drawn, not read by every role)
   const int lane = (int)lane_id();
   const bool dynamic = !SPLIT && p.tickets != nullptr && gridDim.y == 1;
   const bool conv = p.mode == kModeMaskConv;
   int drawn = 0;
-  // Tickets come in batches and the next batch is requested before the current one is used up:
-  // the counter's round trip through L2 would otherwise be paid per tile.  Batches shrink to
-  // one ticket as the counter nears the end so the tail stays balanced.
+  // `first` is the CTA's first ticket, the others come from the counter, which begins behind the `dealt` ones that
+  // every CTA has as its own number.  Where tiles are light they come
+  // in batches and the next batch is requested before the current one is used up: the counter's round trip through
+  // L2 would otherwise be paid per tile.  Batches shrink to one ticket as the counter nears the end so the tail stays
+  // balanced.  A ticket that is on its way is a tile nobody else can take, so that heavy tiles are asked for
+  // one at a time and not before the CTA is about to need one.  (Ahead of time for tiles of up to 2, 4, 6 and 12 steps:
+  // 100 003 scanned rows at 64 channels 27.8, 28.2, 30.4, 30.2 us, 60 000, 104 to 72, 39.9, 39.9, 42.3, 45.7.)
   constexpr int MAX_BATCH = CB2_ROWCONV_TICKET_BATCH;
-  int cur_base = 0, cur_left = 0, next_base = 0, next_cnt = 0;
+  int cur_base = first, cur_left = 1, next_base = 0, next_cnt = 0;
   auto request = [&](int seen, int last_steps) {
-    // (the first tiles carry the most offsets: four of those in one hand set the length of a launch.  The
-    // line matters little -- 960 000 uniform rows, forward: 92.0 us, 92.5 with batches for every tile, 97.9
-    // with one ticket at a time throughout; scanned scenes the same with each)
+    // (the first tiles carry the most offsets: four of those in one hand set the length of a launch)
     int b = last_steps > 2 ? 1 : (nitems - seen) / ((int)gridDim.x * 4);
     next_cnt = b < 1 ? 1 : (b > MAX_BATCH ? MAX_BATCH : b);
     if (lane == 0)
-      next_base = atomicAdd(p.tickets, next_cnt);
+      next_base = dealt + atomicAdd(p.tickets, next_cnt);
   };
-  if (dynamic) {
-    next_base = first_base;  // requested at kernel entry (lane 0 holds the counter's answer)
-    next_cnt = first_cnt;
-  }
   auto draw = [&](int last_steps) -> int {
     int t;
     if (dynamic) {
       if (cur_left == 0) {
+        if (next_cnt == 0)
+          request(cur_base, last_steps);
         cur_base = __shfl_sync(0xffffffffu, next_base, 0);
         cur_left = next_cnt;
         next_cnt = 0;
-        if (cur_base < nitems)
+        if (cur_base < nitems && last_steps <= 2)
           request(cur_base, last_steps);
       }
       t = cur_base++;
@@ -426,11 +426,13 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   const uint32_t slots_addr = smem_u32(rv.slots);
   // Tiles a CTA has drawn cannot be taken over by an idle CTA, so the look-ahead is bounded by
   // WORK, not by tiles: a CTA draws while the steps it holds (one per offset in a tile's mask, until
-  // the last role has read the tile) are within STEP_BUDGET.  Until a tile's mask has landed it is
-  // charged what the previous tile cost -- tiles arrive heaviest first, so that is an upper
-  // estimate -- and the very first one is charged the whole budget: a CTA learns what its
-  // first tile weighs before it takes a second.
-  int issued = 0, accounted = 0, released = 0, held_steps = 0;
+  // they have been issued) are within STEP_BUDGET.  Until a tile's mask has landed it is
+  // charged what the previous tiles cost, half-way back to it where the last was lighter, and the very first one is
+  // charged the whole budget: a CTA learns what its first tile weighs before it takes a second.  (Forward, us, tiles held
+  // until every role had read them, then until issued, then with charges that remember heavier tiles: 60 000 scanned
+  // rows, 104 to 72 channels, 48.1, 48.6, 39.4, 150 000 at 128 70.1, 74.1, 64.5, 100 003 at 64 30.5, 31.2, 27.8; 125 offsets,
+  // 30 011 rows 59.7, 52.6, 52.4.)
+  int issued = 0, accounted = 0, released = 0, drawn_steps = 0;
   int guess = (conv && dynamic) ? STEP_BUDGET + 1 : 1;
   // The scheduler's own instructions are what paces a CTA whose tiles carry one offset each: every
   // poll here is made by all lanes at once (a vote instead of a test by one lane and a shuffle), and releases are only looked at when the
@@ -466,7 +468,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
         }
       }
       const int nsteps = (sl[0] >= 0) ? max(1, offsets * kpasses) : 1;
-      held_steps += nsteps - sl[2];
+      drawn_steps += nsteps - sl[2];
       __syncwarp();
       if (lane == 0) {
         uint32_t any = 0;
@@ -477,23 +479,22 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
             sl[4 + w] = static_cast<int>(km[w]);
         }
         sl[1] = static_cast<int>(any);
-        sl[2] = nsteps;
         CB2_TRACE_EVENT(6, 14, sl[0]);  // tile published
         mbar_arrive(rv.full0 + 8u * (accounted % rv.ring));
       }
       __syncwarp();
-      guess = nsteps;
+      guess = max(nsteps, (guess + nsteps) / 2);
       ++accounted;
     }
   };
   auto account_released = [&]() {
     while (released < accounted &&
            __any_sync(0xffffffffu, mbar_poll(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1))) {
-      held_steps -= rv.slot(released % rv.ring)[2];
       ++released;
     }
   };
-  auto can_draw = [&]() { return (held_steps <= STEP_BUDGET || released == issued) && (issued - released < rv.ring); };
+  auto within_budget = [&]() { return SPLIT || __any_sync(0xffffffffu, drawn_steps - *progress <= STEP_BUDGET); };
+  auto can_draw = [&]() { return issued - released < rv.ring && within_budget(); };
   // tables whose tiles can be fetched with two 16-byte copies per lane
   const bool wide_copies = conv && MW == 1 && p.mask_words == 1 &&
                            ((reinterpret_cast<uintptr_t>(p.argsort) | reinterpret_cast<uintptr_t>(p.mask)) & 15u) == 0;
@@ -508,10 +509,14 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
       may_draw = can_draw();
     }
     if (!may_draw) {
-      // first learn what the tiles in flight weigh, then wait for the oldest one to be read
-      const bool ok = accounted < issued
-                          ? mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag)
-                          : mbar_wait_warp(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1, rv.abort_flag);
+      // first learn what the tiles in flight weigh, then wait for the oldest one to be read or for steps to be issued
+      bool ok = true;
+      if (accounted < issued)
+        ok = mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag);
+      else if (issued - released >= rv.ring)
+        ok = mbar_wait_warp(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1, rv.abort_flag);
+      else if constexpr (!SPLIT)
+        ok = wait_for([&]() { return within_budget(); }, rv.abort_flag);
       if (!ok)
         break;  // gave up
       continue;
@@ -540,7 +545,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
       sl[2] = guess;
       sl[3] = part * block_n;
     }
-    held_steps += guess;
+    drawn_steps += guess;
     if (wide_copies && tile >= 0 && (tile + 1) * 128 <= p.n_rows) {
       cp_async_16(sa + (8 + 4 * lane) * 4, p.argsort + tile * 128 + 4 * lane, 16u);
       cp_async_16(sa + (136 + 4 * lane) * 4, p.mask + tile * 128 + 4 * lane, 16u);
@@ -667,7 +672,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   float *s_scale = reinterpret_cast<float *>(smem + Cfg::OFF_SCALE);
   float *s_bias = s_scale + BLOCK_N;
   volatile int *misc = reinterpret_cast<volatile int *>(smem + Cfg::OFF_MISC);
-  // misc[0] tmem base, misc[1] abort flag, misc[2] SPLIT: a SplitState, misc[3] SPLIT: epilogue warps whose sums are
+  // misc[0] tmem base, misc[1] abort flag, misc[15] steps issued, misc[2] SPLIT: a SplitState, misc[3] SPLIT: epilogue warps whose sums are
   // in this CTA's shared memory, misc[4 + 2 g, 6 + 2 g) what gather group g's waits returned, one for each of its
   // row buffers
   volatile int *abort_flag = misc + 1;
@@ -694,13 +699,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   const int ntiles = (p.n_rows + 127) / 128;
   const int kpasses = (p.red + Cfg::KRED - 1) / Cfg::KRED;
 
-  // Scheduler warp: ask for the first tickets now; their round trip overlaps the set-up below.
-  int early_base = 0, early_cnt = 0;
-  if (!SPLIT && warp == Cfg::SCHED_WARP && p.tickets != nullptr && gridDim.y == 1) {
-    early_cnt = 1;
-    if (lane == 0)
-      early_base = atomicAdd(p.tickets, early_cnt);
-  }
+  // Scheduler warp: the first ticket.  (int8 asks the counter: its tiles in the order in which the CTAs arrive.  Stride 2
+  // from 150 000 uniform rows, 39.6 us, and 41.6 by the CTAs' numbers, whose first rows arrive later.)
+  int first_ticket = blockIdx.x;
+  if (!SPLIT && !Cfg::DEALT && warp == Cfg::SCHED_WARP && p.tickets != nullptr && gridDim.y == 1 && lane == 0)
+    first_ticket = atomicAdd(p.tickets, 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::SA; ++s) {
@@ -725,6 +728,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     misc[1] = 0;
     misc[2] = 0;
     misc[3] = 0;
+    misc[15] = 0;
     CB2_TRACE_SELECT(0);
   }
   if (KIND == 1) {
@@ -738,10 +742,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     tmem_alloc(sbase + Cfg::OFF_MISC, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
-  if (warp == Cfg::SCHED_WARP && early_cnt > 0 && p.mode == kModeMaskConv) {
+  if (warp == Cfg::SCHED_WARP)
+    first_ticket = __shfl_sync(0xffffffffu, first_ticket, 0);
+  if (!SPLIT && warp == Cfg::SCHED_WARP && p.mode == kModeMaskConv) {
     // the first tile's sort order and masks: 128 ints each, four 128-byte lines each
-    const int first = __shfl_sync(0xffffffffu, early_base, 0);
-    const int tile = ntiles - 1 - first / p.n_parts;
+    const int tile = ntiles - 1 - first_ticket / p.n_parts;
     if (tile >= 0 && lane < 8) {
       const int r = tile * 128 + (lane & 3) * 32;
       if (r < p.n_rows) {
@@ -1055,6 +1060,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       int stage = 0, bslot = Cfg::SB - 1, buf = 0, last_key = -1, steps = 0;
       uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
       bool ok = true;
+      volatile int *const progress = misc + 15;
       CB2_PROF_BEGIN();
       for (int more; ok && (more = tc.template next<true>(p, rv, [](const int *) {})) != 0;) {
         CB2_PROF_MARK(0);  // next tile
@@ -1062,8 +1068,12 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           ok = false;
           break;
         }
-        if (tc.offsets == 0)
+        if (tc.offsets == 0) {
+          ++steps;  // what the scheduler charged
+          if constexpr (!SPLIT)
+            *progress = steps;
           continue;
+        }
         // consecutive steps of a tile never share a weight tile; consecutive tiles may (kpasses and n0
         // are in the key: weights have as many columns)
         const bool new_b = (tc.first_offset() * kpasses) * p.nn + tc.n0 != last_key;
@@ -1127,6 +1137,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             a_phase ^= 1u;
           }
           ++steps;
+          if constexpr (!SPLIT)
+            *progress = steps;
           if (s == total - 1) {
             tc_commit(acc_full(buf));
           } else {
@@ -1209,7 +1221,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
-    scheduler_run<MW, SPLIT>(p, rv, ntiles, BLOCK_N, kpasses, early_base, early_cnt, misc + 2);
+    scheduler_run<MW, SPLIT, Cfg::STEP_BUDGET>(p, rv, ntiles, BLOCK_N, kpasses, first_ticket, Cfg::DEALT ? (int)gridDim.x : 0, misc + 15, misc + 2);
   } else {
     // ======================= operand-row gather: group g owns stage g
     if constexpr (TMA_GATHER) {
