@@ -161,7 +161,7 @@ int gather_mode() {
 // predecessor on the stream is still running and synchronises with it through
 // griddepcontrol.wait in its own code.  `level` 1 (on by default): the chain of the three
 // weight-gradient kernels, the gather-GEMM-scatter calls, the int8 convolutions and the fp16 ones whose items clusters
-// share; level 2 (only with CUMM_B200_PDL=2): the other fp16 convolution row kernels.  CUMM_B200_PDL=0 launches
+// share or whose tables are known to be as they were; level 2 (only with CUMM_B200_PDL=2): the other fp16 convolution row kernels.  CUMM_B200_PDL=0 launches
 // everything the ordinary way.
 // The kernels of table generation take part too, but none triggers its dependent: a dependent's launch overlaps the
 // predecessor's end and no more (150 000 uniform rows, us: ordinary launches 85.4 and, stride 2, 186; so 76.5 and 170;
@@ -276,10 +276,13 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   g_last_launch.cluster = cluster;
   // A gather-GEMM-scatter call is one of a run of small kernels (one per filter offset), where
   // overlapping each kernel's set-up with its predecessor's tail nearly halves the run.  For the
-  // convolutions it measured +4 % for the int8 kernels (long epilogue tail) and neutral to
-  // slightly worse for fp16, so only the former take part by default, and launches that clusters share: they leave
-  // SMs free for their successor.
-  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || SPLIT ? 1 : 2;
+  // convolutions it measured +4 % for the int8 kernels (long epilogue tail).  fp16 launches that clusters share take
+  // part, they leave SMs free for their successor, and those whose tables an earlier call has found as they are:
+  // what they gain is that tickets, masks and indices are read under the predecessor's end.  (Forward, input and weight
+  // gradient in turn, us, ordinary launches, overlapped but waiting before a table is read, overlapped: 150 000 uniform
+  // rows at 128 channels 84.0, 86.0, 77.8, 100 003 scanned ones at 64 100.1, 101.6, 94.2, stride 2 from 40 009, 32 to 64,
+  // 46.6, 44.8, 41.0, 9000 at 128 62.0, 60.2, 56.1, 125 offsets, 30 011 rows, 136.2, 135.8, 127.5.)
+  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || SPLIT || p.tables_fixed ? 1 : 2;
   CB2_CUDA(launch_after(pdl_level, cluster, kern, dim3(gx * cluster, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
                         map, map_a, p));
   g_launches.fetch_add(1);
@@ -1657,6 +1660,7 @@ int cb2_conv_run(const cb2_conv_args *a, void *stream_v) {
   p.kv = a->kernel_volume;
   p.mask_words = (a->kernel_volume + 31) / 32;
   p.mode = kModeMaskConv;
+  p.tables_fixed = a->reuse_plan & 1;
   p.skip_empty_tiles = dgrad ? 1 : 0;
   p.reverse_mask = (dgrad && a->reverse_mask) ? 1 : 0;
   p.mask_filter = a->mask_filter;

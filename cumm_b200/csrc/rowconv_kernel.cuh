@@ -51,6 +51,7 @@ struct RowConvParams {
   int mode;
   int src_mode;
   int split;               // CTAs of a cluster that share an item's offsets (kernels with SPLIT)
+  int tables_fixed;        // indices, mask and argsort are as an earlier call on this stream found them
   int skip_empty_tiles;    // input-gradient: a tile whose mask is 0 is left untouched
   int reverse_mask;
   uint32_t mask_filter;
@@ -483,7 +484,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
         mbar_arrive(rv.full0 + 8u * (accounted % rv.ring));
       }
       __syncwarp();
-      guess = max(nsteps, (guess + nsteps) / 2);
+      guess = accounted == 0 ? nsteps : max(nsteps, (guess + nsteps) / 2);
       ++accounted;
     }
   };
@@ -498,7 +499,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // tables whose tiles can be fetched with two 16-byte copies per lane
   const bool wide_copies = conv && MW == 1 && p.mask_words == 1 &&
                            ((reinterpret_cast<uintptr_t>(p.argsort) | reinterpret_cast<uintptr_t>(p.mask)) & 15u) == 0;
-  if (SPLIT)
+  if (SPLIT && !p.tables_fixed)
     grid_dep_wait();  // the predecessor may have written the tables; who gathers learns its rows from here
   bool ended = false;
   for (;;) {
@@ -659,7 +660,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   // ahead is the set-up and, but for SPLIT, the scheduler's tickets, row lists and mask words, the first row-index
   // loads and int8's scale and bias: a predecessor that writes those must not let its dependents start early
   // (see launch_after).  With SPLIT the scheduler waits before it reads a table, so that a small
-  // convolution may follow whatever made its tables, at the price of its first lookups' overlap.  Every role calls
+  // convolution may follow whatever made its tables, at the price of its first lookups' overlap -- but not where the
+  // caller has said that an earlier call found the tables as they are.  Every role calls
   // grid_dep_wait() before it first touches operand rows, weights or the output.  The weight warp lets the next kernel
   // begin.
   // 1024-byte alignment: required by the 128-byte swizzle atoms of TMA and tcgen05.

@@ -958,8 +958,9 @@ class PreparedCall:
     tickets while its predecessor on the stream still runs, and that predecessor can be the
     same call.
     ``static_tables``: the caller promises that the neighbour tables (for the weight gradient:
-    the reduced masks) keep their contents while the call is in use; the weight gradient then
-    plans its schedule on the first launch only (``reuse_plan``)."""
+    the reduced masks) keep their contents while the call is in use; from the second launch on the
+    weight gradient then does without planning its schedule, and the other convolutions read their
+    tables while their predecessor on the stream still runs (``reuse_plan``)."""
 
     def __init__(self, kind: str, args, device: int, stream: int, keep, static_tables: bool = False):
         import torch
@@ -971,7 +972,8 @@ class PreparedCall:
         self._tickets = torch.zeros(8, dtype=torch.int32, device=f"cuda:{device}")
         self._turn = 0
         args.sched_scratch = self._tickets.data_ptr()
-        self._plan_once = bool(static_tables) and bool(args.workspace)
+        self._fixed = bool(static_tables) and (bool(args.workspace) or
+                                               (kind == "conv" and args.op_type != int(ConvOpType.BackwardWeight)))
         L = _lib.load()
         self._fn = L.cb2_conv_run if kind == "conv" else L.cb2_gemm_run
 
@@ -982,7 +984,7 @@ class PreparedCall:
         rc = self._fn(ctypes.byref(self._args), ctypes.c_void_p(s))
         if rc:
             _lib.raise_for(rc)
-        if self._plan_once:
+        if self._fixed:
             self._args.reuse_plan |= 1
 
 

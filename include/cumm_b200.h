@@ -176,7 +176,10 @@ typedef struct cb2_conv_args {
    *   depend on it: fp16 forward and backward input of few tiles add a tile's offsets on several CTAs where the bound
    *   leaves room for them (cb2_last_launch_cluster), on one otherwise; fp32 sums in a fixed order either way, as the
    *   weight gradient's, whose partial sums are cut by the number of CTAs.
-   * reuse_plan (backward weight only): the workspace still holds the plan of an earlier, stream-ordered
+   * reuse_plan, forward and backward input: bit 0 says that indice_ptr, mask_ptr and mask_argsort_ptr hold what they
+   *   held when an earlier, stream-ordered call read them.  An fp16 launch then reads them while its predecessor on the
+   *   stream still runs; without it only launches that a caller chains with CUMM_B200_PDL=2, and int8 ones, do.
+   *   Backward weight: the workspace still holds the plan of an earlier, stream-ordered
    *   call on the same workspace with the same reduced masks (contents, not just address), row count,
    *   mask_width, mask_filter, tile_n and max_ctas -- skip the planning kernel.  The plan depends on
    *   the neighbour tables only, so a training loop plans once per scene.  Bit 0 says so; bit 1

@@ -246,3 +246,50 @@ def test_every_launch_of_a_chain_does_its_work_once(cuda_lib):
             stream.synchronize()
             assert bool((dst == launches).all()), "captured launches"
     H.check_status()
+
+
+@pytest.mark.parametrize("n,grid,C", [(2000, (8, 24, 24), 64), (9000, (8, 48, 48), 128), (30011, (12, 80, 80), 32)])
+def test_layers_that_read_what_their_predecessor_writes(cuda_lib, n, grid, C):
+    """Two prepared layers over fixed tables, forward and backward, each launch reading what the one before it wrote:
+    from the second round on they read their tables and plans while that one still runs.  Input rows change every
+    round; results are those of calls with everything in between waited for, bit for bit."""
+    import torch
+    from cumm_b200.layer import DeviceTables, SparseConvLayer
+    rng = np.random.default_rng(741)
+    t = DeviceTables.from_host(W.build_tables(W.sample_coords(n, 740, grid), grid=grid), "cuda")
+    half = lambda *shape: H.dev((rng.standard_normal(shape) / 8).astype(np.float16), torch)
+    rows, grads = [half(n, C) for _ in range(4)], [half(n, C) for _ in range(4)]
+    ws = [half(C, t.kv, C), half(C, t.kv, C)]
+
+    def layers(stream):
+        b = {k: torch.zeros((n, C), dtype=torch.float16, device="cuda") for k in ("x", "y", "z", "dz", "dy", "dx")}
+        b.update({k: torch.zeros((C, t.kv, C), dtype=torch.float16, device="cuda") for k in ("dw1", "dw2")})
+        one = SparseConvLayer(t, ws[0], b["x"], b["y"], b["dy"], b["dx"], b["dw1"], stream=stream.cuda_stream)
+        two = SparseConvLayer(t, ws[1], b["y"], b["z"], b["dz"], b["dy"], b["dw2"], stream=stream.cuda_stream)
+        return b, [one.fwd, two.fwd, two.dgrad, two.wgrad, one.wgrad, one.dgrad]
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        want_b, alone = layers(stream)
+        b, calls = layers(stream)
+        for i in range(4):
+            for buf in (want_b, b):
+                buf["x"].copy_(rows[i])
+                buf["dz"].copy_(grads[i])
+            for c in alone:
+                stream.synchronize()
+                c.launch()
+            stream.synchronize()
+            if i < 2:
+                for c in calls:
+                    c.launch()
+            else:  # captured, the round twice over
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=stream):
+                    for c in calls + calls:
+                        c.launch()
+                g.replay()
+            stream.synchronize()
+            H.check_status()
+            for k, v in want_b.items():
+                assert torch.equal(v, b[k]), (i, k)
