@@ -505,6 +505,7 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
   p.partials = reinterpret_cast<float *>(ws + L.off_partials);
   p.lists = reinterpret_cast<const int *>(ws + L.off_lists);
   p.list_stride = L.list_stride;
+  p.plan_fixed = reuse_plan ? 1 : 0;
   p.status = dev->status;
   // Row lists where the caller allows them and the workspace has room, tiles otherwise.  A plan that is
   // there already says for itself which of the two it is, whatever this call's flags and size are.
