@@ -1122,13 +1122,16 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             tc_mma<KIND>(d_tmem, adesc, bdesc, idesc, acc);
           };
           const bool last_pass = ++kp == kpasses;
+          // unrolled either way: addresses worked out in a loop cost more than the MMAs
           if (!last_pass || ksteps_last == KSTEPS_FULL) {
 #pragma unroll
             for (int ks = 0; ks < KSTEPS_FULL; ++ks)
               issue(ks, (s == 0 && ks == 0) ? 0u : 1u);
           } else {
-            for (int ks = 0; ks < ksteps_last; ++ks)
-              issue(ks, (s == 0 && ks == 0) ? 0u : 1u);
+#pragma unroll
+            for (int ks = 0; ks < KSTEPS_FULL - 1; ++ks)
+              if (ks < ksteps_last)
+                issue(ks, (s == 0 && ks == 0) ? 0u : 1u);
           }
           CB2_PROF_MARK(5);  // MMAs issued
           tc_commit(empty_a(stage));
