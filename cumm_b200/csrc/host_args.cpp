@@ -28,7 +28,7 @@ PyObject *g_gemm_params, *g_gemm_desp, *g_conv_params, *g_conv_desp;  // the rec
   X(algo) X(shuffle_type) X(element_per_access_a) X(element_per_access_b) X(element_per_access_c) X(input) X(weight)   \
   X(output) X(output_add) X(bias) X(scale) X(indices) X(mask) X(mask_argsort) X(mask_output) X(mask_width)             \
   X(mask_filter) X(reverse_mask) X(verbose) X(op_type) X(ndim) X(mask_sparse) X(dynamic_mask) X(is_int8_inference)     \
-  X(split_k_serial_) X(split_k_parallel_)
+  X(split_k_serial_) X(split_k_parallel_) X(padding) X(stride) X(dilation)
 #define X(n) PyObject *k_##n;
 CB2_NAMES(X)
 #undef X
@@ -252,6 +252,73 @@ bool read_gemm(PyObject *params, cb2_gemm_args &g, bool) {
   return true;
 }
 
+// What both kinds of convolution calls say about their tensors: rows of channels, and the neighbour tables.
+struct ConvTensors {
+  View in, w, out, add, ind, mask, order, mask_out;
+  int64_t rows_in, rows_out;
+  int C, K, kv;
+  bool dynamic;  // the descriptor allows more than 32 offsets
+};
+
+// The rest of a convolution's record, and its checks.
+void fill_conv(const Record &p, const Record &d, const Desp &ds, int op, const ConvTensors &t, cb2_conv_args &g) {
+  const bool fwd = op == CB2_CONV_FORWARD, wgrad = op == CB2_CONV_BACKWARD_WEIGHT, int8 = d.flag(k_is_int8_inference);
+  g.split_k_slices = p.small(k_split_k_slices);
+  need(g.split_k_slices <= 1 || d.small(k_split_k_serial_) == 1 || d.small(k_split_k_parallel_) == 1);
+  const View bias = view(p, k_bias, true), scale = view(p, k_scale, true);
+  g.K = t.K, g.kernel_volume = t.kv, g.C = t.C;
+  need(int8 ? (bias && scale) : !t.add);
+  if (t.add)
+    need(t.add.t->scalar_type() == t.out.t->scalar_type() && t.add.t->sizes() == t.out.t->sizes());
+  const int kv = g.kernel_volume, words = (kv + 31) / 32;
+  need(t.ind.n_dims() == 2 && t.ind.dim(0) == kv && kv >= 1 && kv <= 128 && (kv <= 32 || t.dynamic));
+  g.N = size32(t.ind.dim(1));
+  need(g.N == (fwd || wgrad ? t.rows_out : t.rows_in));
+  // what ConvAlgoDesp.supported looks at
+  const long long m = wgrad ? g.K : g.N, n = fwd ? g.K : wgrad ? 1ll * g.C * kv : g.C,
+                  k = wgrad ? g.N : 1ll * kv * (fwd ? g.C : g.K);
+  need(divides(ds.epa[0], ds.ta ? m : k) && divides(ds.epa[1], ds.tb ? k : n) && divides(ds.epa[2], ds.tc ? m : n));
+  need(ds.epa[0] != 0 && (fwd ? g.C : g.K) % ds.epa[0] == 0);
+  if (wgrad)
+    need(ds.epa[1] != 0 && g.C % ds.epa[1] == 0 && g.mask_width > 0 && g.mask_width % ds.tile[2] == 0);
+  const View &a = fwd ? t.in : t.out, &b = wgrad ? t.in : t.w, &c = fwd ? t.out : wgrad ? t.w : t.in;
+  need(on_current_device(c));
+  g.ptr_A = a.data(), g.ptr_B = b.data(), g.ptr_C = c.data();
+  g.ptr_D = t.add ? t.add.data() : (int8 || !bias) ? c.data() : bias.data();
+  g.d_is_bias = bias && !int8 && !t.add;
+  g.bias_pointer = bias.data(), g.scale_pointer = scale.data();
+  g.alpha = p.real(k_alpha), g.beta = p.real(k_beta);
+  g.act_alpha = p.real(k_act_alpha), g.act_beta = p.real(k_act_beta);
+  g.act_type = p.small(k_act_type);
+  g.mask_ptr = static_cast<const uint32_t *>(t.mask.data());
+  g.mask_out_ptr = static_cast<uint32_t *>(t.mask_out.data());
+  g.indice_ptr = static_cast<const int32_t *>(t.ind.data());
+  g.mask_argsort_ptr = static_cast<const int32_t *>(t.order.data());
+  g.ndim = d.small(k_ndim);
+  g.mode = 1;
+  g.groups = 1;
+  g.op_type = op;
+  g.dtype_a = dtype_code(*a.t), g.dtype_b = dtype_code(*b.t), g.dtype_c = dtype_code(*c.t);
+  g.is_int8_inference = int8;
+  const auto rows = [&](const View &v) { return size32(&v == &t.in ? t.rows_in : &v == &t.out ? t.rows_out : t.K); };
+  g.rows_A = rows(a), g.rows_B = rows(b);
+  g.mask_words = size32(t.mask.t->numel());
+  need(wgrad || g.mask_words >= static_cast<long long>(g.N) * words);
+  if (fwd && t.mask_out)
+    need(t.mask_out.t->numel() >= (static_cast<long long>(g.N) + 127) / 128 * words);
+  g.tile_n = ds.tile[1], g.tile_k = wgrad ? 0 : ds.tile[2];
+  g.max_ctas = p.small(k_max_ctas);
+}
+
+// The record of a convolution in the ordinary call, its descriptor and its operator; false: some other kind.
+bool conv_record(PyObject *params, PyObject *desp) {
+  if (!g_run_conv || reinterpret_cast<PyObject *>(Py_TYPE(params)) != g_conv_params ||
+      reinterpret_cast<PyObject *>(Py_TYPE(desp)) != g_conv_desp)
+    return false;
+  const Record p{params};
+  return p.none(k_timer) && !p.flag(k_verbose) && p.is_tensor(k_output);
+}
+
 // The flat record of a convolution call whose tensors are on the current device.
 bool read_conv(PyObject *params, cb2_conv_args &g, bool with_weight_gradient) {
   if (!g_run_conv || reinterpret_cast<PyObject *>(Py_TYPE(params)) != g_conv_params)
@@ -267,61 +334,104 @@ bool read_conv(PyObject *params, cb2_conv_args &g, bool with_weight_gradient) {
   if (op < CB2_CONV_FORWARD || op > CB2_CONV_BACKWARD_WEIGHT || (op == CB2_CONV_BACKWARD_WEIGHT && !with_weight_gradient) ||
       !d.flag(k_mask_sparse))
     return false;
-  const bool fwd = op == CB2_CONV_FORWARD, wgrad = op == CB2_CONV_BACKWARD_WEIGHT, int8 = d.flag(k_is_int8_inference);
   const Desp ds = read_desp(d);
-  g.split_k_slices = p.small(k_split_k_slices);
-  need(g.split_k_slices <= 1 || d.small(k_split_k_serial_) == 1 || d.small(k_split_k_parallel_) == 1);
-  const View in = view(p, k_input, false), w = view(p, k_weight, false), out = view(p, k_output, false);
-  need(in.n_dims() == 2 && out.n_dims() == 2 && w.n_dims() == 3);
-  need(in.t->is_contiguous() && w.t->is_contiguous() && out.t->is_contiguous());
-  const View add = view(p, k_output_add, true), bias = view(p, k_bias, true), scale = view(p, k_scale, true);
-  const View ind = view(p, k_indices, false), mask = view(p, k_mask, false), order = view(p, k_mask_argsort, false),
-             mask_out = view(p, k_mask_output, true);
-  g.K = size32(w.dim(0)), g.kernel_volume = size32(w.dim(1)), g.C = size32(w.dim(2));
-  need(in.dim(1) == g.C && out.dim(1) == g.K);
-  need(int8 ? (bias && scale) : !add);
-  if (add)
-    need(add.t->scalar_type() == out.t->scalar_type() && add.t->sizes() == out.t->sizes());
-  const int kv = g.kernel_volume, words = (kv + 31) / 32;
-  need(ind.n_dims() == 2 && ind.dim(0) == kv && kv >= 1 && kv <= 128 && (kv <= 32 || d.flag(k_dynamic_mask)));
-  g.N = size32(ind.dim(1));
-  need(g.N == (fwd || wgrad ? out : in).dim(0));
+  ConvTensors t;
+  t.in = view(p, k_input, false), t.w = view(p, k_weight, false), t.out = view(p, k_output, false);
+  need(t.in.n_dims() == 2 && t.out.n_dims() == 2 && t.w.n_dims() == 3);
+  need(t.in.t->is_contiguous() && t.w.t->is_contiguous() && t.out.t->is_contiguous());
+  t.add = view(p, k_output_add, true);
+  t.ind = view(p, k_indices, false), t.mask = view(p, k_mask, false), t.order = view(p, k_mask_argsort, false),
+  t.mask_out = view(p, k_mask_output, true);
+  t.K = size32(t.w.dim(0)), t.kv = size32(t.w.dim(1)), t.C = size32(t.w.dim(2));
+  need(t.in.dim(1) == t.C && t.out.dim(1) == t.K);
+  t.rows_in = t.in.dim(0), t.rows_out = t.out.dim(0);
+  t.dynamic = t.kv <= 32 || d.flag(k_dynamic_mask);
   g.mask_width = p.small(k_mask_width);
-  // what ConvAlgoDesp.supported looks at
-  const long long m = wgrad ? g.K : g.N, n = fwd ? g.K : wgrad ? 1ll * g.C * kv : g.C,
-                  k = wgrad ? g.N : 1ll * kv * (fwd ? g.C : g.K);
-  need(divides(ds.epa[0], ds.ta ? m : k) && divides(ds.epa[1], ds.tb ? k : n) && divides(ds.epa[2], ds.tc ? m : n));
-  need(ds.epa[0] != 0 && (fwd ? g.C : g.K) % ds.epa[0] == 0);
-  if (wgrad)
-    need(ds.epa[1] != 0 && g.C % ds.epa[1] == 0 && g.mask_width > 0 && g.mask_width % ds.tile[2] == 0);
-  const View &a = fwd ? in : out, &b = wgrad ? in : w, &c = fwd ? out : wgrad ? w : in;
-  need(on_current_device(c));
-  g.ptr_A = a.data(), g.ptr_B = b.data(), g.ptr_C = c.data();
-  g.ptr_D = add ? add.data() : (int8 || !bias) ? c.data() : bias.data();
-  g.d_is_bias = bias && !int8 && !add;
-  g.bias_pointer = bias.data(), g.scale_pointer = scale.data();
-  g.alpha = p.real(k_alpha), g.beta = p.real(k_beta);
-  g.act_alpha = p.real(k_act_alpha), g.act_beta = p.real(k_act_beta);
-  g.act_type = p.small(k_act_type);
-  g.mask_ptr = static_cast<const uint32_t *>(mask.data());
-  g.mask_out_ptr = static_cast<uint32_t *>(mask_out.data());
-  g.indice_ptr = static_cast<const int32_t *>(ind.data());
-  g.mask_argsort_ptr = static_cast<const int32_t *>(order.data());
   g.mask_filter = static_cast<uint32_t>(p.integer(k_mask_filter));
   g.reverse_mask = p.flag(k_reverse_mask);
-  g.ndim = d.small(k_ndim);
-  g.mode = 1;
-  g.groups = 1;
-  g.op_type = op;
-  g.dtype_a = dtype_code(*a.t), g.dtype_b = dtype_code(*b.t), g.dtype_c = dtype_code(*c.t);
-  g.is_int8_inference = int8;
-  g.rows_A = size32(a.dim(0)), g.rows_B = size32(b.dim(0));
-  g.mask_words = size32(mask.t->numel());
-  need(wgrad || g.mask_words >= static_cast<long long>(g.N) * words);
-  if (fwd && mask_out)
-    need(mask_out.t->numel() >= (static_cast<long long>(g.N) + 127) / 128 * words);
-  g.tile_n = ds.tile[1], g.tile_k = wgrad ? 0 : ds.tile[2];
-  g.max_ctas = p.small(k_max_ctas);
+  fill_conv(p, d, ds, op, t, g);
+  return true;
+}
+
+// ---------------------------------------------------------------- dense convolutions (cumm_b200/dense.py)
+// Extents of a dense call, the spatial ones padded to three axes in front; as _geometry there works them out.
+struct DenseShape {
+  int64_t batch, C, K;
+  int64_t in[3], out[3], k[3];
+  int pad[3], stride[3], dil[3];
+};
+void axes(const Record &p, PyObject *key, int ndim, int otherwise, int (&v)[3], int fill) {
+  Ref l(p.get(key));
+  need(PyList_CheckExact(l.p));
+  const Py_ssize_t n = PyList_GET_SIZE(l.p);
+  need(n == 0 || n == ndim);
+  for (int a = 0; a < 3; ++a)
+    v[a] = fill;
+  for (int a = 0; a < ndim; ++a) {
+    int r = otherwise;
+    if (n) {
+      PyObject *e = PyList_GET_ITEM(l.p, a);
+      need(PyLong_CheckExact(e));
+      const long x = PyLong_AsLong(e);
+      if (x == -1 && PyErr_Occurred())
+        PyErr_Clear();
+      need(x >= 0 && x < (1 << 20));
+      r = static_cast<int>(x);
+    }
+    v[3 - ndim + a] = r;
+  }
+}
+// false: not the ordinary dense call
+bool dense_shape(const Record &p, const Record &d, DenseShape &s) {
+  if (d.flag(k_mask_sparse))
+    return false;
+  const int ndim = d.small(k_ndim);
+  need(ndim >= 1 && ndim <= 3);
+  const View in = view(p, k_input, false), w = view(p, k_weight, false), out = view(p, k_output, false);
+  need(in.n_dims() == ndim + 2 && w.n_dims() == ndim + 2 && out.n_dims() == ndim + 2);
+  need(in.t->is_contiguous() && w.t->is_contiguous() && out.t->is_contiguous() && p.none(k_output_add));
+  s.batch = in.dim(0), s.C = in.dim(ndim + 1), s.K = w.dim(0);
+  need(w.dim(ndim + 1) == s.C && out.dim(ndim + 1) == s.K && out.dim(0) == s.batch);
+  axes(p, k_padding, ndim, 0, s.pad, 0), axes(p, k_stride, ndim, 1, s.stride, 1), axes(p, k_dilation, ndim, 1, s.dil, 1);
+  for (int a = 0; a < 3; ++a)
+    s.in[a] = s.out[a] = s.k[a] = 1;
+  for (int a = 3 - ndim; a < 3; ++a) {
+    s.in[a] = in.dim(1 + a - (3 - ndim)), s.k[a] = w.dim(1 + a - (3 - ndim)), s.out[a] = out.dim(1 + a - (3 - ndim));
+    const int64_t span = s.in[a] + 2ll * s.pad[a] - s.dil[a] * (s.k[a] - 1) - 1;
+    need(s.stride[a] >= 1 && s.dil[a] >= 1 && span >= 0 && s.out[a] == span / s.stride[a] + 1);
+  }
+  return true;
+}
+View tensor(PyObject *o) {
+  need(THPVariable_CheckExact(o));
+  View v;
+  v.t = &THPVariable_Unpack(o);
+  return v;
+}
+// `tables`: (indices_fwd, indices_bwd, mask_fwd, mask_bwd, argsort_fwd, argsort_bwd, tile_masks) of the call's shape
+bool read_dense(PyObject *params, PyObject *tables, cb2_conv_args &g) {
+  Ref desp(Record{params}.get(k__conv_algo_desp));
+  if (!conv_record(params, desp.p) || !PyTuple_CheckExact(tables) || PyTuple_GET_SIZE(tables) != 7)
+    return false;
+  const Record p{params}, d{desp.p};
+  DenseShape s;
+  if (!dense_shape(p, d, s))
+    return false;
+  const int op = d.small(k_op_type);
+  need(op >= CB2_CONV_FORWARD && op <= CB2_CONV_BACKWARD_WEIGHT);
+  const Desp ds = read_desp(d);
+  ConvTensors t;
+  t.in = view(p, k_input, false), t.w = view(p, k_weight, false), t.out = view(p, k_output, false);
+  t.rows_in = s.batch * s.in[0] * s.in[1] * s.in[2], t.rows_out = s.batch * s.out[0] * s.out[1] * s.out[2];
+  t.C = size32(s.C), t.K = size32(s.K), t.kv = size32(s.k[0] * s.k[1] * s.k[2]);
+  t.dynamic = true;
+  const bool bwd = op == CB2_CONV_BACKWARD_INPUT, wgrad = op == CB2_CONV_BACKWARD_WEIGHT;
+  t.ind = tensor(PyTuple_GET_ITEM(tables, bwd ? 1 : 0));
+  t.mask = tensor(PyTuple_GET_ITEM(tables, wgrad ? 6 : bwd ? 3 : 2));
+  t.order = tensor(PyTuple_GET_ITEM(tables, bwd ? 5 : 4));
+  g.mask_width = wgrad ? 128 : -1;
+  g.mask_filter = 0xffffffffu;
+  fill_conv(p, d, ds, op, t, g);
   return true;
 }
 
@@ -360,6 +470,45 @@ PyObject *run_conv(PyObject *, PyObject *params) {
     Py_RETURN_NONE;
   }
   return launch(g_run_conv, g, stream);
+}
+
+// dense_key(params): what a dense call's tables are found by, or None.
+PyObject *dense_key(PyObject *, PyObject *params) {
+  try {
+    DenseShape s;
+    Ref desp(Record{params}.get(k__conv_algo_desp));
+    if (!conv_record(params, desp.p) || !dense_shape(Record{params}, Record{desp.p}, s))
+      Py_RETURN_NONE;
+    Ref out(Record{params}.get(k_output));
+    return Py_BuildValue("(iL(LLL)(LLL)(LLL)(iii)(iii)(iii))", static_cast<int>(THPVariable_Unpack(out.p).get_device()),
+                         (long long)s.batch, (long long)s.in[0], (long long)s.in[1], (long long)s.in[2], (long long)s.out[0],
+                         (long long)s.out[1], (long long)s.out[2], (long long)s.k[0], (long long)s.k[1], (long long)s.k[2],
+                         s.stride[0], s.stride[1], s.stride[2], s.pad[0], s.pad[1], s.pad[2], s.dil[0], s.dil[1], s.dil[2]);
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+}
+// run_dense(params, tables, address): forward and input gradient are launched (the return code); the weight gradient's
+// flat record is left at the address (True).  None: the Python layer takes the call.
+PyObject *run_dense(PyObject *, PyObject *args) {
+  PyObject *params, *tables;
+  unsigned long long address;
+  if (!PyArg_ParseTuple(args, "OOK", &params, &tables, &address))
+    return nullptr;
+  cb2_conv_args g;
+  memset(&g, 0, sizeof(g));
+  void *stream;
+  try {
+    if (!read_dense(params, tables, g))
+      Py_RETURN_NONE;
+    stream = stream_of(Record{params});
+  } catch (...) {
+    Py_RETURN_NONE;
+  }
+  if (g.op_type != CB2_CONV_BACKWARD_WEIGHT)
+    return launch(g_run_conv, g, stream);
+  memcpy(reinterpret_cast<void *>(static_cast<uintptr_t>(address)), &g, sizeof(g));
+  Py_RETURN_TRUE;
 }
 
 // gemm_args(params, address), conv_args(params, address): fill the flat record there; True, or None.
@@ -401,6 +550,8 @@ PyMethodDef methods[] = {{"setup", setup, METH_VARARGS, nullptr},
                          {"run_conv", run_conv, METH_O, nullptr},
                          {"gemm_args", gemm_args, METH_VARARGS, nullptr},
                          {"conv_args", conv_args, METH_VARARGS, nullptr},
+                         {"dense_key", dense_key, METH_O, nullptr},
+                         {"run_dense", run_dense, METH_VARARGS, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

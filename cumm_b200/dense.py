@@ -86,13 +86,30 @@ def _tables(device: int, geom, stream: int) -> dict:
         _lib.raise_for(_lib.load().cb2_dense_tables_run(ctypes.byref(a), ctypes.c_void_p(int(stream))))
     # the reduced masks of the weight gradient: every tile carries every offset
     t["tile_masks"] = t["mask_fwd"][:tiles].clone()
+    t["native"] = tuple(t[name] for name in ("indices_fwd", "indices_bwd", "mask_fwd", "mask_bwd", "argsort_fwd",
+                                             "argsort_bwd", "tile_masks"))
     _TABLES[key] = t
     return t
 
 
-def run_dense_conv(params) -> None:
-    """Forward / backward input / backward weight of a dense convolution (see the module text)."""
-    from .tensorview.gemm import ConvOpType, ConvParams, run_conv
+def run_dense_conv(params, host=None) -> None:
+    """Forward / backward input / backward weight of a dense convolution (see the module text).  ``host``: the
+    native reader of the records, which answers for the ordinary call over a grid whose tables are there."""
+    from .tensorview.gemm import ConvOpType, ConvParams, _attach_scratch, _call_on, run_conv
+    t = _TABLES.get(host.dense_key(params)) if host is not None else None
+    if t is not None:
+        args = _lib.ConvArgs()
+        rc = host.run_dense(params, t["native"], ctypes.addressof(args))
+        if rc is True:
+            import torch
+            args._device, stream = torch.cuda.current_device(), int(params.stream)
+            L = _lib.load()
+            _attach_scratch(L, args, stream, params.workspace, False)  # every row has every neighbour but those at the border
+            return _call_on(args._device, L.cb2_conv_run, args, stream)
+        if rc is not None:
+            if rc:
+                _lib.raise_for(rc)
+            return
     desp = params.conv_algo_desp
     geom = _geometry(params)
     C, K = geom[7], geom[8]

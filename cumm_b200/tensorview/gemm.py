@@ -701,6 +701,10 @@ class _NoHost:
 
     conv_args = gemm_args
 
+    @staticmethod
+    def dense_key(params):
+        return None
+
 
 def _host():
     """The native reader of the records (csrc/host_args.cpp), which answers for the ordinary call and leaves
@@ -868,6 +872,16 @@ def _conv_args(params: ConvParams) -> _lib.ConvArgs:
     return args
 
 
+def _attach_scratch(L, args, stream: int, workspace, lists: bool) -> None:
+    """What a weight gradient that plans for itself needs, the only operator that needs scratch."""
+    need = L.cb2_conv_workspace_size(ctypes.byref(args))
+    if need:
+        args.workspace, args.workspace_bytes = _workspace_for(
+            args._device, stream, need, workspace, L.cb2_conv_workspace_size_lists(ctypes.byref(args)) if lists else 0)
+        if lists:  # this call's tables, planned for this call
+            args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS
+
+
 def run_conv(params: ConvParams) -> None:
     """What ``ConvMainUnitTest.implicit_gemm2`` does (cumm/conv/main.py:485-745)."""
     host = _HOST or _host()
@@ -880,7 +894,7 @@ def run_conv(params: ConvParams) -> None:
     if not desp.mask_sparse:
         # dense convolution: the same kernels over the neighbour table of the full grid
         from ..dense import run_dense_conv
-        return run_dense_conv(params)
+        return run_dense_conv(params, host)
     L = _lib.load()
     args = _lib.ConvArgs()
     # the reader leaves the weight gradient's launch to this function; any other call it has just declined
@@ -890,15 +904,8 @@ def run_conv(params: ConvParams) -> None:
     else:
         args = _conv_args(params)
     stream = int(params.stream)
-    if args.op_type == ConvOpType.BackwardWeight:  # the only operator that needs scratch
-        need = L.cb2_conv_workspace_size(ctypes.byref(args))
-        if need:
-            lists = params.row_lists
-            args.workspace, args.workspace_bytes = _workspace_for(
-                args._device, stream, need, params.workspace,
-                L.cb2_conv_workspace_size_lists(ctypes.byref(args)) if lists else 0)
-            if lists:  # this call's tables, planned for this call
-                args.reuse_plan = _lib.CB2_PLAN_ROW_LISTS
+    if args.op_type == ConvOpType.BackwardWeight:
+        _attach_scratch(L, args, stream, params.workspace, params.row_lists)
     # verbose: registers of the kernel and the time of this launch (cumm/conv/main.py:723-729)
     timer = params.timer
     enabled = timer is not None and getattr(timer, "enable", False)

@@ -92,3 +92,58 @@ def test_dense_convolution_checks_shapes(cuda_lib):
     p.output = torch.zeros((64, 16), dtype=torch.float16, device="cuda")
     with pytest.raises(RuntimeError, match="channels-last"):
         ConvMainUnitTest.implicit_gemm2(p)
+
+
+@pytest.mark.parametrize("shape,ksize,padding,stride,dilation,dtype", [
+    ((2, 6, 10, 12), (3, 3, 3), [1, 1, 1], [2, 1, 2], [], "float16"),
+    ((1, 20, 24), (3, 3), [2, 2], [], [2, 2], "float32"),
+    ((3, 200), (5,), [], [2], [1], "float16"),
+    ((1, 5, 8, 8), (3, 5, 5), [1, 2, 2], [1, 1, 1], [1, 1, 1], "float16"),
+])
+def test_dense_calls_read_in_native_code_are_those_read_in_python(cuda_lib, shape, ksize, padding, stride, dilation, dtype):
+    """The second call over a grid is read and launched by the extension: the same results, bit for bit, as the call
+    read in Python, with a bias and an activation, with a source of its own, and with an fp32 weight gradient."""
+    import torch
+    from cumm_b200.dense import _TABLES, run_dense_conv
+    from cumm_b200.tensorview.gemm import Activation, _host
+    C, K, ndim = 16, 24, len(ksize)
+    half = lambda *s: torch.randn(s, device="cuda").half()
+    full = lambda v, d: v if v else [d] * ndim
+    osp = [(shape[1 + a] + 2 * full(padding, 0)[a] - full(dilation, 1)[a] * (ksize[a] - 1) - 1) // full(stride, 1)[a] + 1
+           for a in range(ndim)]
+    x, w, dout = half(*shape, C), half(K, *ksize, C), half(shape[0], *osp, K)
+    dw = torch.randn((K, *ksize, C), device="cuda").to(getattr(torch, dtype))
+
+    def call(op, host, inp, weight, output, **more):
+        p = dense_params(op, ndim, C, K, padding, stride, dilation)
+        p.input, p.weight, p.output = inp, weight, output
+        for k, v in more.items():
+            setattr(p, k, v)
+        run_dense_conv(p, host)
+        torch.cuda.synchronize()
+        return p
+
+    F, D, W = ConvOpType.Forward, ConvOpType.BackwardInput, ConvOpType.BackwardWeight
+    bias = half(K)
+    for op, out, more in ((F, "out", dict(bias=bias, beta=1.0, act_type=Activation.ReLU)), (F, "out", dict(alpha=0.5, beta=2.0)),
+                          (D, "in", {}), (W, "w", {}), (W, "w", dict(beta=0.5))):
+        made = []
+        for host in (None, _host()):
+            t = {"in": x.clone(), "w": dw.clone() if op == W else w, "out": dout.clone()}
+            p = call(op, host, t["in"], t["w"], t["out"], **more)
+            made.append(t[out])
+        assert torch.equal(*made), (op, more)
+        # and it was the extension that answered
+        import ctypes
+        from cumm_b200 import _lib
+        tables = _TABLES[_host().dense_key(p)]["native"]
+        assert _host().run_dense(p, tables, ctypes.addressof(_lib.ConvArgs())) == (True if op == W else 0)
+    # what it leaves to Python: lists of the wrong length, an output that does not fit
+    for field, value in (("padding", [1] * (ndim + 1)), ("output", dout[..., :8].contiguous())):
+        p = dense_params(F, ndim, C, K, padding, stride, dilation)
+        p.input, p.weight, p.output = x, w, dout
+        setattr(p, field, value)
+        with pytest.raises(RuntimeError):
+            run_dense_conv(p, _host())
+    torch.cuda.synchronize()
+    H.check_status()
