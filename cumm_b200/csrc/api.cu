@@ -809,8 +809,10 @@ int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, c
     cb2pg::SortSides sides;
     memset(&sides, 0, sizeof(sides));
     const int to_go = shape.passes - 1 - p;
+    bool few = true;
     for (int q = 0; q < count; ++q) {
       const MaskSort &j = jobs[q];
+      few = few && j.side.chunk <= cb2pg::kSortThreads * cb2pg::kSortItemsSmall;
       cb2pg::SortSide &o = sides.side[q];
       o.n = j.side.n;
       o.chunk = j.side.chunk;
@@ -827,7 +829,8 @@ int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, c
       o.tile_masks = to_go ? nullptr : j.tile_masks;
     }
     const dim3 grid(max_chunks, count);
-    auto kern = shape.words > 1 ? cb2pg::sort_pass_kernel<true> : cb2pg::sort_pass_kernel<false>;
+    auto kern = few ? (shape.words > 1 ? cb2pg::sort_pass_kernel<true, true> : cb2pg::sort_pass_kernel<false, true>)
+                    : (shape.words > 1 ? cb2pg::sort_pass_kernel<true, false> : cb2pg::sort_pass_kernel<false, false>);
     CB2_CUDA(launch_after(1, 1, kern, grid, dim3(cb2pg::kSortThreads), 0, s, sides, p, shape));
     g_launches.fetch_add(1);
   }

@@ -19,6 +19,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace cb2pg {
 
@@ -233,7 +234,10 @@ constexpr int kSortChunks = 74;
 constexpr size_t kSortHistInts = static_cast<size_t>(kSortBins) * kSortChunks;  // of a pass
 constexpr int kSortThreads = kSortBins;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 8;       // rows per thread and round
+// Rows per thread and round: as many as a chunk needs, up to eight.  (Table sets of chunks of 2048 rows, eight and four, us:
+// 150 000 uniform rows 75.9 and 71.7, scanned ones 107.4 and 104.8, 125 offsets, 30 011 rows, 419 and 379; of chunks of 6656, stride 2
+// from 150 000 rows, 164.8 and 172.1.)
+constexpr int kSortItems = 8, kSortItemsSmall = 4;
 constexpr int kProbeThreads = 256;  // chunks are whole multiples of this
 
 struct SortShape {
@@ -714,10 +718,12 @@ struct SortSide {
 struct SortSides {
   SortSide side[2];
 };
-template <bool WIDE>
+// FEW: chunks of kSortItemsSmall rows per thread.
+template <bool WIDE, bool FEW>
 __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_constant__ SortSides sides, int pass,
                                                                  const SortShape shape) {
   cb2::grid_dep_wait();
+  constexpr int kItems = FEW ? kSortItemsSmall : kSortItems;
   const SortSide &s = sides.side[blockIdx.y];
   __shared__ int s_cnt[kSortWarps][kSortBins];
   __shared__ int s_base[kSortBins];
@@ -728,16 +734,38 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_co
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   // where this chunk's rows of digit t go: rows with smaller digits, then those of earlier chunks
   int before = 0, all = 0;
-  for (int c0 = 0; c0 < s.n_chunks; c0 += 25) {  // 25 loads in flight: one after the other they were most of a pass
-    int v[25];
+  // All loads in flight together: one after the other they were most of a pass, three times 25 of them still 3 us of a set of
+  // 150 000 rows (78.9 -> 75.9); for few chunks the 74 cost as much as they save (20 000 rows 57.2 -> 60.7).  The loop of
+  // one round, as it is written for chunks of few rows, is faster than its body alone there (72 and 78 us) and slower
+  // where a thread has eight rows (174 and 164, stride 2).
+  auto count = [&](auto many) {
+    constexpr int N = decltype(many)::value;
+    int v[N];
 #pragma unroll
-    for (int i = 0; i < 25; ++i)
-      v[i] = c0 + i < s.n_chunks ? __ldg(s.hist + (c0 + i) * kSortBins + t) : 0;
+    for (int i = 0; i < N; ++i)
+      v[i] = i < s.n_chunks ? __ldg(s.hist + i * kSortBins + t) : 0;
 #pragma unroll
-    for (int i = 0; i < 25; ++i) {
+    for (int i = 0; i < N; ++i) {
       all += v[i];
-      before += c0 + i < me ? v[i] : 0;
+      before += i < me ? v[i] : 0;
     }
+  };
+  if (s.n_chunks <= 25) {
+    count(std::integral_constant<int, 25>());
+  } else if constexpr (FEW) {
+    for (int c0 = 0; c0 < s.n_chunks; c0 += kSortChunks) {
+      int v[kSortChunks];
+#pragma unroll
+      for (int i = 0; i < kSortChunks; ++i)
+        v[i] = c0 + i < s.n_chunks ? __ldg(s.hist + (c0 + i) * kSortBins + t) : 0;
+#pragma unroll
+      for (int i = 0; i < kSortChunks; ++i) {
+        all += v[i];
+        before += c0 + i < me ? v[i] : 0;
+      }
+    }
+  } else {
+    count(std::integral_constant<int, kSortChunks>());
   }
   int total;
   s_base[t] = block_scan_512(all, s_warp, total) + before;
@@ -753,14 +781,14 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_co
     const uint32_t hi = (bit & 31) + kSortDigitBits > 32 && (bit >> 5) + 1 < shape.words ? __ldg(r + 1) : 0u;
     return __funnelshift_r(lo, hi, bit & 31) & mask;
   };
-  for (int tile = begin; tile < end; tile += kSortThreads * kSortItems) {
+  for (int tile = begin; tile < end; tile += kSortThreads * kItems) {
     for (int w = 0; w < kSortWarps; ++w)
       s_cnt[w][t] = 0;
-    uint32_t key[kSortItems], digit[kSortItems];
-    int val[kSortItems], rank[kSortItems];
-    const int base = tile + warp * 32 * kSortItems + lane;
+    uint32_t key[kItems], digit[kItems];
+    int val[kItems], rank[kItems];
+    const int base = tile + warp * 32 * kItems + lane;
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
+    for (int it = 0; it < kItems; ++it) {
       const int idx = base + it * 32;
       val[it] = -1;
       key[it] = 0u;
@@ -771,15 +799,15 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_co
       }
     }
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
+    for (int it = 0; it < kItems; ++it) {
       digit[it] = 0u;
       if (val[it] >= 0)
         digit[it] = WIDE ? wide_digit(val[it], bit0, digit_mask) : ((key[it] >> bit0) & digit_mask);
     }
     __syncthreads();
-    // rank inside the warp's 32 * kSortItems consecutive rows, in their order
+    // rank inside the warp's 32 * kItems consecutive rows, in their order
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
+    for (int it = 0; it < kItems; ++it) {
       const unsigned peers = digit_peers(digit[it], shape.width, __ballot_sync(0xffffffffu, val[it] >= 0));
       rank[it] = 0;
       if (val[it] >= 0)
@@ -800,7 +828,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_co
     s_base[t] = run;
     __syncthreads();
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
+    for (int it = 0; it < kItems; ++it) {
       const bool valid = val[it] >= 0;
       const int pos = valid ? s_cnt[warp][digit[it]] + rank[it] : 0;
       if (valid) {
