@@ -159,10 +159,9 @@ int gather_mode() {
 
 // Launch with programmatic stream serialisation: the kernel may be scheduled while its
 // predecessor on the stream is still running and synchronises with it through
-// griddepcontrol.wait in its own code.  `level` 1 (on by default): the chain of the three
-// weight-gradient kernels, the gather-GEMM-scatter calls, the int8 convolutions and the fp16 ones whose items clusters
-// share or whose tables are known to be as they were; level 2 (only with CUMM_B200_PDL=2): the other fp16 convolution row kernels.  CUMM_B200_PDL=0 launches
-// everything the ordinary way.
+// griddepcontrol.wait in its own code.  CUMM_B200_PDL=0 launches everything the ordinary way.
+// The planning kernels of the weight gradient do not take part: their blocks would wait beside the row kernel before them (a
+// training step with 125 offsets 155.8 -> 177.7 us).
 // The kernels of table generation take part too, but none triggers its dependent: a dependent's launch overlaps the
 // predecessor's end and no more (150 000 uniform rows, us: ordinary launches 85.4 and, stride 2, 186; so 76.5 and 170;
 // triggered as soon as a kernel starts 91.5 and 199, its successor's waiting blocks hold the SMs).
@@ -170,13 +169,12 @@ int gather_mode() {
 // int8, stride 2 from 150 000 rows, 40.9 -> 42.4 us).  PTX asks a dependent to wait where its prerequisite
 // issues launch_dependents; the kernels that make tables here do not, so their blocks have all ended by then.
 template <class Kern, class... Args>
-cudaError_t launch_after(int level, int cluster, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+cudaError_t launch_after(int cluster, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                          Args... args) {
-  static const int enabled = [] {
+  static const bool pdl = [] {
     const char *v = getenv("CUMM_B200_PDL");
-    return v ? atoi(v) : 1;
+    return !v || atoi(v) > 0;
   }();
-  const bool pdl = enabled >= level;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid;
@@ -274,17 +272,14 @@ int launch_rowconv_inst(const CUtensorMap &map, const CUtensorMap &map_a, const 
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
   g_last_launch.cluster = cluster;
-  // A gather-GEMM-scatter call is one of a run of small kernels (one per filter offset), where
-  // overlapping each kernel's set-up with its predecessor's tail nearly halves the run.  For the
-  // convolutions it measured +4 % for the int8 kernels (long epilogue tail).  fp16 launches that clusters share take
-  // part, they leave SMs free for their successor, and those whose tables an earlier call has found as they are:
-  // what they gain is that tickets, masks and indices are read under the predecessor's end.  (Forward, input and weight
-  // gradient in turn, us, ordinary launches, overlapped but waiting before a table is read, overlapped: 150 000 uniform
-  // rows at 128 channels 84.0, 86.0, 77.8, 100 003 scanned ones at 64 100.1, 101.6, 94.2, stride 2 from 40 009, 32 to 64,
-  // 46.6, 44.8, 41.0, 9000 at 128 62.0, 60.2, 56.1, 125 offsets, 30 011 rows, 136.2, 135.8, 127.5.)
-  const int pdl_level = p.mode != kModeMaskConv || KIND == 1 || SPLIT || p.tables_fixed ? 1 : 2;
-  CB2_CUDA(launch_after(pdl_level, cluster, kern, dim3(gx * cluster, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream,
-                        map, map_a, p));
+  // Every row kernel's launch and set-up overlaps its predecessor's end.  It nearly halves a run of gather-GEMM-scatter
+  // calls; int8 convolutions gain 4 %; fp16 ones, which wait before they read a table: one forward after the other, us,
+  // 58 787 uniform rows, 40 to 56, 14.7 -> 11.5, 42 077 at 128 18.3 -> 15.9, 60 000 scanned ones at 256 102.4 -> 99.0, training steps
+  // that plan each time 1 to 13 % less.  With tables that an earlier call found as they are, tickets, masks and indices are
+  // read under the predecessor's end, too.  (Forward, input and weight gradient in turn, ordinary launches and
+  // overlapped: 150 000 uniform rows at 128 channels 84.0 and 77.8, 100 003 scanned ones at 64 100.1 and 94.2, stride 2 from
+  // 40 009, 32 to 64, 46.6 and 41.0, 9000 at 128 62.0 and 56.1, 125 offsets, 30 011 rows, 136.2 and 127.5.)
+  CB2_CUDA(launch_after(cluster, kern, dim3(gx * cluster, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, map, map_a, p));
   g_launches.fetch_add(1);
   return CB2_OK;
 }
@@ -476,7 +471,7 @@ int launch_wgrad_inst(const CUtensorMap &ma, const CUtensorMap &mb, const WgradP
   g_last_launch.num_threads = Cfg::THREADS;
   g_last_launch.smem_bytes = Cfg::SMEM_BYTES;
   g_last_launch.cluster = 1;
-  CB2_CUDA(launch_after(1, 1, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, ma, mb, p));
+  CB2_CUDA(launch_after(1, kern, dim3(gx, gy), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, ma, mb, p));
   g_launches.fetch_add(1);
   return CB2_OK;
 }
@@ -526,7 +521,7 @@ int run_wgrad(DeviceState *dev, WgradParams &p, int tile_n, int max_ctas, int pl
     int2 *counts = reinterpret_cast<int2 *>(ws + L.off_counts);
     wgrad_mark_rows_kernel<<<grid, kWgradPlanThreads, 0, stream>>>(p, bits, counts, L.n_ctl);
     CB2_CUDA(cudaGetLastError());
-    CB2_CUDA(launch_after(1, 1, wgrad_list_rows_kernel, grid, dim3(kWgradPlanThreads), 0, stream, p, bits, counts,
+    CB2_CUDA(launch_after(1, wgrad_list_rows_kernel, grid, dim3(kWgradPlanThreads), 0, stream, p, bits, counts,
                           reinterpret_cast<int *>(ws + L.off_lists), reinterpret_cast<int *>(ws + L.off_rows),
                           L.row_capacity));
     g_launches.fetch_add(2);
@@ -831,7 +826,7 @@ int sort_masks(const MaskSort *jobs, int count, const cb2pg::SortShape &shape, c
     const dim3 grid(max_chunks, count);
     auto kern = few ? (shape.words > 1 ? cb2pg::sort_pass_kernel<true, true> : cb2pg::sort_pass_kernel<false, true>)
                     : (shape.words > 1 ? cb2pg::sort_pass_kernel<true, false> : cb2pg::sort_pass_kernel<false, false>);
-    CB2_CUDA(launch_after(1, 1, kern, grid, dim3(cb2pg::kSortThreads), 0, s, sides, p, shape));
+    CB2_CUDA(launch_after(1, kern, grid, dim3(cb2pg::kSortThreads), 0, s, sides, p, shape));
     g_launches.fetch_add(1);
   }
   return CB2_OK;
@@ -914,9 +909,9 @@ int cb2_pairgen_count_outputs(const cb2_pairgen_args *a, int *n_out, void *strea
     const cb2pg::Bitmap bm = pairgen_bitmap(L, ws);
     fill.add(bm.words, static_cast<size_t>(L.bitmap_words) * 4, 0u);
     fill.run(dev, stream);
-    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_mark_kernel, dim3((a->n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
+    CB2_CUDA(launch_after(1, cb2pg::bitmap_mark_kernel, dim3((a->n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
                           a->n_in, L.g, bm.words));
-    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_rank_kernel, dim3(bm.n_blocks), dim3(cb2pg::kBitmapThreads), 0, stream, bm,
+    CB2_CUDA(launch_after(1, cb2pg::bitmap_rank_kernel, dim3(bm.n_blocks), dim3(cb2pg::kBitmapThreads), 0, stream, bm,
                           counter));
     g_launches.fetch_add(2);
   } else {
@@ -980,13 +975,13 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
     if (bwd)
       fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
-    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_coords_kernel, dim3(blocks(bm.n_words)), dim3(256), 0, stream, bm, n_out, L.g,
+    CB2_CUDA(launch_after(1, cb2pg::bitmap_coords_kernel, dim3(blocks(bm.n_words)), dim3(256), 0, stream, bm, n_out, L.g,
                           a->out_coords));
-    CB2_CUDA(launch_after(1, 1, cb2pg::bitmap_scatter_kernel, dim3((n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
+    CB2_CUDA(launch_after(1, cb2pg::bitmap_scatter_kernel, dim3((n_in + 127) / 128), dim3(128), 0, stream, a->in_coords,
                           n_in, L.g, bm, jobs[0].side, words, dev->status));
     const int bwd_blocks = bwd ? static_cast<int>(blocks(n_in)) : 0;
     auto kern = words > 1 ? cb2pg::bitmap_backward_kernel<4> : cb2pg::bitmap_backward_kernel<1>;
-    CB2_CUDA(launch_after(1, 1, kern, dim3(bwd_blocks + blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, a->in_coords,
+    CB2_CUDA(launch_after(1, kern, dim3(bwd_blocks + blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, a->in_coords,
                           L.g, bm, jobs[0].side, jobs[1].side, bwd_blocks, words, shape.width));
     CB2_CUDA(cudaGetLastError());
     g_launches.fetch_add(3);
@@ -1001,7 +996,7 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
       fill.add(a->indices_bwd, static_cast<size_t>(L.g.kv) * n_in * 4, 0xffffffffu);
     fill.run(dev, stream);
     auto insert = L.exact ? cb2pg::hash_insert_kernel<true> : cb2pg::hash_insert_kernel<false>;
-    CB2_CUDA(launch_after(1, 1, insert, dim3(blocks(n_in)), dim3(256), 0, stream, a->in_coords, n_in, L.g, h, dev->status));
+    CB2_CUDA(launch_after(1, insert, dim3(blocks(n_in)), dim3(256), 0, stream, a->in_coords, n_in, L.g, h, dev->status));
     const int32_t *out_coords = a->in_coords;
     if (!a->subm) {
       cb2pg::decode_out_coords_kernel<<<blocks(n_out), 256, 0, stream>>>(
@@ -1011,7 +1006,7 @@ int cb2_pairgen_run(const cb2_pairgen_args *a, void *stream_v) {
     }
     auto kern = L.exact ? (words > 1 ? cb2pg::probe_kernel<4, true> : cb2pg::probe_kernel<1, true>)
                         : (words > 1 ? cb2pg::probe_kernel<4, false> : cb2pg::probe_kernel<1, false>);
-    CB2_CUDA(launch_after(1, 1, kern, dim3(blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, out_coords, L.g, h,
+    CB2_CUDA(launch_after(1, kern, dim3(blocks(n_out)), dim3(cb2pg::kProbeThreads), 0, stream, out_coords, L.g, h,
                           jobs[0].side, mirror ? jobs[1].side : none, words, shape.width));
     g_launches.fetch_add(2);
     if (bwd && !mirror) {

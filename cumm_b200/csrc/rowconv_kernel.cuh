@@ -378,7 +378,7 @@ enum SplitState {
   kSplitNothing,  // shared, none of the offsets is this CTA's
   kSplitSums      // shared, the epilogue warps leave this CTA's sums in shared memory and count themselves
 };
-template <int MW, bool SPLIT, int STEP_BUDGET>
+template <int MW, bool SPLIT, int STEP_BUDGET, bool WAIT_FIRST>
 __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int block_n,
                                               int kpasses, int first, int dealt, volatile int *progress, volatile int *split_state) {
   const int nitems = ntiles * p.n_parts;
@@ -499,7 +499,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // tables whose tiles can be fetched with two 16-byte copies per lane
   const bool wide_copies = conv && MW == 1 && p.mask_words == 1 &&
                            ((reinterpret_cast<uintptr_t>(p.argsort) | reinterpret_cast<uintptr_t>(p.mask)) & 15u) == 0;
-  if (SPLIT && !p.tables_fixed)
+  if (WAIT_FIRST && conv && !p.tables_fixed)
     grid_dep_wait();  // the predecessor may have written the tables; who gathers learns its rows from here
   bool ended = false;
   for (;;) {
@@ -657,10 +657,10 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     CB2_TRACE_CTA(0, 0);
   // Programmatic dependent launch: the next kernel on the stream may be scheduled onto SMs as
   // they free up, and this one may itself have started before its predecessor finished.  What runs
-  // ahead is the set-up and, but for SPLIT, the scheduler's tickets, row lists and mask words, the first row-index
-  // loads and int8's scale and bias: a predecessor that writes those must not let its dependents start early
-  // (see launch_after).  With SPLIT the scheduler waits before it reads a table, so that a small
-  // convolution may follow whatever made its tables, at the price of its first lookups' overlap -- but not where the
+  // ahead is the set-up and, but for fp16 convolutions, the scheduler's tickets, row lists and mask words, the first
+  // row-index loads and int8's scale and bias: a predecessor that writes those must not let its dependents start early
+  // (see launch_after).  In an fp16 convolution the scheduler waits before it reads a table, so that it may follow
+  // whatever made its tables, at the price of its first lookups' overlap -- but not where the
   // caller has said that an earlier call found the tables as they are.  Every role calls
   // grid_dep_wait() before it first touches operand rows, weights or the output.  The weight warp lets the next kernel
   // begin.
@@ -1226,7 +1226,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
-    scheduler_run<MW, SPLIT, Cfg::STEP_BUDGET>(p, rv, ntiles, BLOCK_N, kpasses, first_ticket, Cfg::DEALT ? (int)gridDim.x : 0, misc + 15, misc + 2);
+    scheduler_run<MW, SPLIT, Cfg::STEP_BUDGET, KIND == 0>(p, rv, ntiles, BLOCK_N, kpasses, first_ticket, Cfg::DEALT ? (int)gridDim.x : 0, misc + 15, misc + 2);
   } else {
     // ======================= operand-row gather: group g owns stage g
     if constexpr (TMA_GATHER) {
