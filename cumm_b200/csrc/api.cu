@@ -198,10 +198,14 @@ cudaError_t launch_after(int cluster, Kern kern, dim3 grid, dim3 block, size_t s
 
 // How many CTAs share an item's filter offsets in a launch whose items leave most SMs idle: 4 or 8 where the clusters
 // fit the CTAs the launch may have and are all resident at once (each has one item; 148 SMs hold 33 clusters of four and
-// 15 of eight), else 1, and the ordinary kernel runs.  Four from two offsets a CTA on, eight from eight.  (Forward, us,
-// one CTA, four, eight.  125 offsets, 1900 rows of a crop at 32 channels: 49.7, 19.5, 17.1.  27 offsets at 64 channels,
-// crops of 1000 and 1900 rows: 14.2, 9.9, 9.5 and 14.9, 10.4, 10.6; 1900 uniform rows, whose tiles stay with one CTA of the
-// cluster: 7.2, 6.9, 7.4.  8 offsets, 2000 and 3800 rows: 8.8, 8.8 and 9.6, 9.6, at 128 channels 12.4, 10.9.)
+// 15 of eight), else 1, and the ordinary kernel runs.  Four from two offsets a CTA on, eight from
+// eight.  That line was laid before every launch overlapped its predecessor; by the figures now four CTAs pay from 16 offsets on,
+// at 128 channels from 12.  It stays where callers (cb2_last_launch_cluster) and tests know it.  (One forward after the other over
+// fixed tables, us, one CTA and four.  8 offsets: crops of 1000, 1900 and 3800 rows at 64 channels 4.8 and 6.2, 5.0 and 6.3,
+// 5.6 and 9.2, 1900 at 128 7.8 and 7.7; 12: 5.8 and 6.3, 6.5 and 6.7, 6.8 and 9.4, at 128 10.2 and 8.5; 18: 7.7 and 7.0, 8.3 and 7.3, 8.5
+// and 10.0, 13.4 and 9.4; 27: 10.0 and 7.5, 10.7 and 7.9, 11.1 and 10.8, 18.2 and 10.5, scanned scenes of 2000 rows 9.5 and 7.1, uniform
+// ones, whose tiles stay with one CTA of the cluster, 3.9 and 4.5.  125 offsets at 32 channels, one CTA, four and eight: crops of 1900
+// rows 45.4, 15.5 and 16.2; four and eight: of 1000 rows 14.1 and 11.7, scanned scenes of 1000 rows 12.0 and 8.9.)
 // `resident`: per device, clusters of 4 and 8 CTAs of this kernel that it holds, plus one (0 = not known yet: not
 // asked, or without an answer).
 using ResidentClusters = std::atomic<int>[kMaxDevices][2];
@@ -365,11 +369,11 @@ int run_rowconv(DeviceState *dev, RowConvParams &p, int kind, bool b_mn, int til
     return rc;
   // Operand rows go through the copy engine (tile::gather4 requests of four rows and 128 bytes), but rows of
   // more than 128 bytes whose column blocks cross 128-byte lines by 16-byte cp.async.  (60 000 scanned rows,
-  // forward, us, gather4 and cp.async: 72 channels 49.7 and 43.9, 88 59.6 and 53.9, 104 61.1 and 55.0, 112 49.0 and
-  // 46.9, 120 57.9 and 52.8, 128 44.4 and 46.8, 136 86.7 and 81.9, 160 75.3 and 75.4, 192 69.6 and 76.8, 200 94.1 and
-  // 85.3, 224 76.1 and 78.5, 248 95.6 and 89.6, 256 72.3 and 78.3, 320 101 and 111, 512 134 and 148; 150 000 uniform rows
-  // 136 41.6 and 38.4, 192 33.3 and 35.0, 256 35.3 and 36.7; of one column block: 40 36.5 and 34.5, 64 -- 100 003
-  // rows -- 34 and 43; int8 128, stride 2, 41 and 70.)  Wide rows that overlap, or are all one (a stride below the width), are no
+  // forward to 128 channels, us, gather4 and cp.async: 72 channels 44.0 and 37.5, 88 53.6 and 46.1, 104 51.4 and 44.9, 112 36.9
+  // and 35.3, 120 44.5 and 40.4, 128 31.6 and 34.8, 136 67.2 and 60.6, 160 54.1 and 55.5, 192 50.9 and 56.7, 200 70.7 and 65.0, 224 56.0
+  // and 57.7, 248 71.3 and 66.9, 256 52.6 and 58.4, 320 72.9 and 82.3, 512 97.7 and 109.1; 150 000 uniform rows 104 20.5 and 22.7, 128
+  // 20.3 and 22.0, 136 30.0 and 26.5, 192 24.9 and 25.4, 256 25.8 and 25.9; of one column block: 40 38.2 and 33.3, uniform 18.3 and
+  // 22.0, 64 21.3 and 25.6, uniform 18.4 and 21.3; int8 128, stride 2, 40 and 44.)  Wide rows that overlap, or are all one (a stride below the width), are no
   // tensor that a map describes: cp.async takes them.  CUMM_B200_GATHER forces one path.
   const bool in_lines = (reinterpret_cast<uintptr_t>(p.a) | static_cast<uintptr_t>(p.lda * es)) % 128 == 0 && p.lda >= p.red;
   const bool tma_gather = (p.mask_words > 1 && pl.natom_k == 1) ||

@@ -95,8 +95,8 @@ template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MA
   static constexpr int KRED = NATOM_K * ATOM_ELEMS;       // reduction elements per stage
   static constexpr int TILE_M = 128;
   // What bounds a step is not the bytes of a stage but how many steps are on their way, so narrow fp16 rows
-  // have seven stages (forward and input gradient of 100 003 scanned rows at 64 channels: six 36.4, seven 34.1,
-  // eight 36.0 us; 125 offsets, 30 011 rows: 61.9, 60.6, 58; 2000 rows: 15.4, 14.5, 14.5) and wide fp16 rows
+  // have seven stages (forward of 100 003 scanned rows at 64 channels: seven 24.1, eight 24.4, nine 24.9 us; 125 offsets,
+  // 30 011 rows: 44.7, 43.5, 43.5; 20 000 uniform rows 8.5, 8.4, 8.4) and wide fp16 rows
   // four, which is what the shared memory holds.  int8 keeps five beside sixteen epilogue warps: its stages
   // hold the weights too.
   static constexpr int SA =
@@ -369,7 +369,7 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // `progress` (shared memory): steps that the MMA issuer has issued, tiles without an offset counted as one.
 // `first`, `dealt`: see below.  SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
 // becomes what that makes of the CTA; it stays kSplitUnknown in one that gives up before its item is known.
-// (Items of up to 0, 3 and 7 offsets kept, forward, us: 1900 and 4000 uniform rows at 64 channels 8.4, 6.9, 6.9 and 9.1, 7.7,
+// (Items of up to 0, 3 and 7 offsets kept, forward, before launches overlapped, us: 1900 and 4000 uniform rows at 64 channels 8.4, 6.9, 6.9 and 9.1, 7.7,
 // 7.7; 8 offsets, 3800 rows at 64 and 128 9.6, 9.6, 9.2 and 10.9, 10.9, 11.4.)
 constexpr int kSplitSoloOffsets = 3;
 enum SplitState {
@@ -640,9 +640,7 @@ __device__ __forceinline__ uint4 rowconv_finish8(const RowConvParams &p, const f
 // SPLIT: a launch with so few items that most SMs would be idle.  What such a launch takes is one tile's offsets,
 // one after the other, so a cluster of `split` CTAs shares an item's offsets: each sums its own in tensor memory and
 // leaves the sums, fp32, in its shared memory; then each makes the output rows of its share of the tile from the
-// sums of all, in the order of the CTAs, through distributed shared memory.  (Forward, us, without, with, and with
-// launches that start under their predecessor's tail: 2000 rows of a crop at 64 channels 14.9, 11.5, 10.3, scanned scenes
-// of 4000 rows, 64 to 32, 12.9, 10.4, 9.3, 1600 at 128 18.5, 12.6, 11.0; 2000 uniform rows 7.2, 7.9, 6.7.  Clusters of
+// sums of all, in the order of the CTAs, through distributed shared memory.  (Figures: cluster_split.  Clusters of
 // two, for up to half as many items as SMs, gained 8 % on 9000 scanned rows and lost 6 % on uniform ones, most of
 // whose tiles have one offset.)
 template <int KIND, int NATOM_K, int BLOCK_N, bool B_MN, bool TMA_GATHER, int MASK_WORDS = 1, bool SPLIT = false>
@@ -1047,7 +1045,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     // ======================= MMA issuer: one thread, from the walk to the commits.  It paces tiles with
     // several offsets.  Elected, so that the compiler keeps descriptors in uniform registers: with lane 0
     // chosen by its number four MMAs took 310 cycles of a step's 1000, elected 100; a thread that walks by itself
-    // needs no votes between them.  (Warp that walks together, lane 0 by number / the same, elected to issue /
+    // needs no votes between them.  A step of 64 channels now takes it 560 cycles: 80 to see its operands there, 95 for four
+    // MMAs, 215 for two commits, 170 to look at the next step's barriers.  (Warp that walks together, lane 0 by number / the same, elected to issue /
     // one thread, before the gathers were sped up: 30 011 rows of 125 offsets 87 / 79 / 77.8 us, 100 003 scanned
     // rows at 64 channels 42.5 / 39.5 / 39.8, after: - / 73 / 60.6 and - / 35.7 / 34.1.)  Whoever is waited for
     // next is looked at as soon as a step is committed.
