@@ -293,3 +293,54 @@ def test_layers_that_read_what_their_predecessor_writes(cuda_lib, n, grid, C):
             H.check_status()
             for k, v in want_b.items():
                 assert torch.equal(v, b[k]), (i, k)
+
+
+@pytest.mark.parametrize("n,grid,C", [(30011, (12, 80, 80), 64), (20000, (12, 64, 64), 72), (9000, (8, 48, 48), 128)])
+def test_layers_directly_behind_new_tables_in_old_places(cuda_lib, n, grid, C):
+    """Calls that do not say their tables are as they were, each directly behind whatever wrote its tables, masks and rows
+    into the buffers that the call before it still reads (gather4, cp.async, one tile a CTA): forward and input gradient
+    of scene after scene are those of calls with everything in between waited for, bit for bit."""
+    import torch
+    from cumm_b200.conv.main import ConvMainUnitTest
+    from cumm_b200.layer import DeviceTables
+    from cumm_b200.tensorview.gemm import ConvOpType, ConvParams
+    rng = np.random.default_rng(751)
+    scenes = [DeviceTables.from_host(W.build_tables(W.sample_coords(n, 750 + i, grid), grid=grid), "cuda") for i in range(3)]
+    half = lambda *shape: H.dev((rng.standard_normal(shape) / 8).astype(np.float16), torch)
+    rows, w = [half(n, C) for _ in scenes], half(C, 27, C)
+    names = ("indices", "mask", "mask_argsort", "indices_bwd", "mask_bwd", "mask_argsort_bwd")
+    here = scenes[0].clone()
+    x = torch.zeros_like(rows[0])
+
+    def call(op, inp, out, stream):
+        p = ConvParams(3, op)
+        p.conv_algo_desp = H.conv_desp(op, C, C)
+        p.input, p.weight, p.output = inp, w, out
+        back = "_bwd" if op == ConvOpType.BackwardInput else ""
+        p.indices, p.mask, p.mask_argsort = (getattr(here, name + back) for name in names[:3])
+        p.stream = stream.cuda_stream
+        ConvMainUnitTest.implicit_gemm2(p)
+
+    def passes(order, wait):
+        made = []
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for i in order:
+                y, din = torch.empty_like(x), torch.empty_like(x)
+                for name in names:
+                    getattr(here, name).copy_(getattr(scenes[i], name))
+                x.copy_(rows[i])
+                wait(stream)
+                call(ConvOpType.Forward, x, y, stream)
+                wait(stream)
+                call(ConvOpType.BackwardInput, din, y, stream)
+                wait(stream)
+                made.append((y, din))
+            stream.synchronize()
+        H.check_status()
+        return made
+
+    want = passes(range(3), lambda s: s.synchronize())
+    order = [0, 1, 2, 1, 0, 2, 0, 1]
+    for i, got in zip(order, passes(order, lambda s: None)):
+        assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), i
