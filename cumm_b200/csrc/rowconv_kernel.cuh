@@ -367,7 +367,8 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 
 // An L2 prefetch of the first tile's words runs while the CTA sets up its barriers and tensor memory.
 // `progress` (shared memory): steps that the MMA issuer has issued, tiles without an offset counted as one.
-// `first`, `dealt`: see below.  SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
+// `first`, `dealt`: see below.  WAIT_FIRST: a convolution's tables are read behind the predecessor's end, unless the caller
+// knows them to be as they were.  SPLIT: the CTA's cluster has one item, and this CTA every split-th of its offsets.  `split_state` (shared memory)
 // becomes what that makes of the CTA; it stays kSplitUnknown in one that gives up before its item is known.
 // (Items of up to 0, 3 and 7 offsets kept, forward, before launches overlapped, us: 1900 and 4000 uniform rows at 64 channels 8.4, 6.9, 6.9 and 9.1, 7.7,
 // 7.7; 8 offsets, 3800 rows at 64 and 128 9.6, 9.6, 9.2 and 10.9, 10.9, 11.4.)
@@ -380,7 +381,8 @@ enum SplitState {
 };
 template <int MW, bool SPLIT, int STEP_BUDGET, bool WAIT_FIRST>
 __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const RingView &rv, int ntiles, int block_n,
-                                              int kpasses, int first, int dealt, volatile int *progress, volatile int *split_state) {
+                                              int kpasses, int first, int dealt, volatile int *progress,
+                                              volatile int *split_state) {
   const int nitems = ntiles * p.n_parts;
   const int lane = (int)lane_id();
   const bool dynamic = !SPLIT && p.tickets != nullptr && gridDim.y == 1;
@@ -1045,11 +1047,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     // ======================= MMA issuer: one thread, from the walk to the commits.  It paces tiles with
     // several offsets.  Elected, so that the compiler keeps descriptors in uniform registers: with lane 0
     // chosen by its number four MMAs took 310 cycles of a step's 1000, elected 100; a thread that walks by itself
-    // needs no votes between them.  A step of 64 channels now takes it 560 cycles: 80 to see its operands there, 95 for four
-    // MMAs, 215 for two commits, 170 to look at the next step's barriers.  (Warp that walks together, lane 0 by number / the same, elected to issue /
-    // one thread, before the gathers were sped up: 30 011 rows of 125 offsets 87 / 79 / 77.8 us, 100 003 scanned
-    // rows at 64 channels 42.5 / 39.5 / 39.8, after: - / 73 / 60.6 and - / 35.7 / 34.1.)  Whoever is waited for
-    // next is looked at as soon as a step is committed.
+    // needs no votes between them.  A step of 64 channels takes it 560 cycles: 80 to see its operands there, 95 for four
+    // MMAs, 215 for two commits, 170 to look at the next step's barriers.  (Warp that walks together, lane 0 by number /
+    // the same, elected to issue / one thread, before the gathers were sped up: 30 011 rows of 125 offsets 87 / 79 / 77.8 us,
+    // 100 003 scanned rows at 64 channels 42.5 / 39.5 / 39.8, after: - / 73 / 60.6 and - / 35.7 / 34.1.)  Whoever is waited
+    // for next is looked at as soon as a step is committed.
     if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(KIND, false, B_MN, 128, BLOCK_N);
       constexpr int KSTEPS_FULL = NATOM_K * 4;
@@ -1225,7 +1227,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
-    scheduler_run<MW, SPLIT, Cfg::STEP_BUDGET, KIND == 0>(p, rv, ntiles, BLOCK_N, kpasses, first_ticket, Cfg::DEALT ? (int)gridDim.x : 0, misc + 15, misc + 2);
+    scheduler_run<MW, SPLIT, Cfg::STEP_BUDGET, KIND == 0>(p, rv, ntiles, BLOCK_N, kpasses, first_ticket,
+                                                          Cfg::DEALT ? (int)gridDim.x : 0, misc + 15, misc + 2);
   } else {
     // ======================= operand-row gather: group g owns stage g
     if constexpr (TMA_GATHER) {
