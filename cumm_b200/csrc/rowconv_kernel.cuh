@@ -436,6 +436,8 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
   // rows, 104 to 72 channels, 48.1, 48.6, 39.4, 150 000 at 128 70.1, 74.1, 64.5, 100 003 at 64 30.5, 31.2, 27.8; 125 offsets,
   // 30 011 rows 59.7, 52.6, 52.4.)
   int issued = 0, accounted = 0, released = 0, drawn_steps = 0;
+  int item_tile = -1;  // SPLIT: the tile whose mask words this CTA reports, and those words
+  uint32_t item_mask[MW] = {};
   int guess = (conv && dynamic) ? STEP_BUDGET + 1 : 1;
   // The scheduler's own instructions are what paces a CTA whose tiles carry one offset each: every
   // poll here is made by all lanes at once (a vote instead of a test by one lane and a shuffle), and releases are only looked at when the
@@ -449,12 +451,10 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
       if constexpr (SPLIT) {
         if (sl[0] >= 0) {
           const int rank = (int)cluster_rank();
-          if (rank == 0 && lane == 0 && p.mask_out && sl[3] == 0) {
+          item_tile = rank == 0 && p.mask_out && sl[3] == 0 ? sl[0] : -1;
 #pragma unroll
-            for (int w = 0; w < MW; ++w)
-              if (w < p.mask_words)
-                p.mask_out[(long long)sl[0] * p.mask_words + w] = km[w];  // forward: not reversed
-          }
+          for (int w = 0; w < MW; ++w)
+            item_mask[w] = km[w];  // forward: not reversed
           const bool alone = offsets <= kSplitSoloOffsets;
           int before = 0, kept = 0;
 #pragma unroll
@@ -594,6 +594,16 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
     if (ended)
       account();
   }
+  // The predecessor may still read or write the tile masks where the tables were read ahead of its end.
+  if constexpr (SPLIT) {
+    if (item_tile >= 0) {
+      grid_dep_wait();
+#pragma unroll
+      for (int w = 0; w < MW; ++w)
+        if (lane == 0 && w < p.mask_words)
+          p.mask_out[(long long)item_tile * p.mask_words + w] = item_mask[w];
+    }
+  }
   // the last CTA to run out of tiles puts the two counters back to zero for the next launch
   if (ended && dynamic && lane == 0) {
     if (next_cnt != 0)  // an outstanding request must have been served before the counters may be reset
@@ -662,8 +672,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
   // (see launch_after).  In an fp16 convolution the scheduler waits before it reads a table, so that it may follow
   // whatever made its tables, at the price of its first lookups' overlap -- but not where the
   // caller has said that an earlier call found the tables as they are.  Every role calls
-  // grid_dep_wait() before it first touches operand rows, weights or the output.  The weight warp lets the next kernel
-  // begin.
+  // grid_dep_wait() before it first touches operand rows, weights, the output or the tile masks.  The weight warp lets the
+  // next kernel begin.
   // 1024-byte alignment: required by the 128-byte swizzle atoms of TMA and tcgen05.
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;

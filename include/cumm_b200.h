@@ -178,7 +178,8 @@ typedef struct cb2_conv_args {
    *   weight gradient's, whose partial sums are cut by the number of CTAs.
    * reuse_plan, forward and backward input: bit 0 says that indice_ptr, mask_ptr and mask_argsort_ptr hold what they
    *   held when an earlier, stream-ordered call read them.  An fp16 launch then reads them while its predecessor on the
-   *   stream still runs; without it it waits first (int8 launches always read ahead).
+   *   stream still runs; without it it waits first (int8 launches always read ahead).  That goes for what is read:
+   *   mask_out_ptr is written behind the predecessor's end like the output.
    *   Backward weight: the workspace still holds the plan of an earlier, stream-ordered
    *   call on the same workspace with the same reduced masks (contents, not just address), row count,
    *   mask_width, mask_filter, tile_n and max_ctas -- skip the planning kernel.  The plan depends on

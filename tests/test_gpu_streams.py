@@ -344,3 +344,42 @@ def test_layers_directly_behind_new_tables_in_old_places(cuda_lib, n, grid, C):
     order = [0, 1, 2, 1, 0, 2, 0, 1]
     for i, got in zip(order, passes(order, lambda s: None)):
         assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), i
+
+
+@pytest.mark.parametrize("max_ctas", [0, 4])
+def test_tile_masks_of_launches_in_a_row_come_in_their_order(cuda_lib, max_ctas):
+    """Two prepared forward calls over the fixed tables of two scenes, which report into one buffer.  The second is one
+    that clusters share and that reads its tables while the first (such a call, too, or one whose four CTAs store their
+    masks tile after tile) still runs: its masks are the ones that stay."""
+    import torch
+    from cumm_b200 import _lib
+    from cumm_b200.layer import make_desp
+    from cumm_b200.tensorview.gemm import ConvOpType, ConvParams, prepare_conv
+    n, C, grid = 2000, 64, (8, 24, 24)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        masks = torch.zeros((n + 127) // 128, dtype=torch.int32, device="cuda")
+        x, w = torch.zeros((n, C), dtype=torch.float16, device="cuda"), torch.zeros((C, 27, C), dtype=torch.float16, device="cuda")
+        calls, wants = [], []
+        for i, ctas in enumerate((max_ctas, 0)):
+            tb = W.build_tables(W.sample_coords(n, 760 + i, grid), grid=grid)
+            p = ConvParams(3, ConvOpType.Forward)
+            p.conv_algo_desp = make_desp(ConvOpType.Forward, False, C, C)
+            p.input, p.weight, p.output, p.mask_output = x, w, torch.zeros_like(x), masks
+            p.indices, p.mask, p.mask_argsort = H.dev(tb.indices, torch), H.mask_to_torch(tb.mask, torch), H.dev(tb.mask_argsort, torch)
+            p.max_ctas, p.stream = ctas, stream.cuda_stream
+            p.mask_filter = 0xffffffff if i else 0x155
+            calls.append(prepare_conv(p, static_tables=True))
+            tile_masks = np.bitwise_or.reduceat(tb.mask & np.uint32(p.mask_filter), np.arange(0, n, 128))
+            wants.append(H.mask_to_torch(tile_masks, torch))
+        first, second = calls
+        for c in calls + calls:
+            c.launch()
+        assert _lib.last_launch_info()["cluster"] == 4 and not torch.equal(*wants)
+        for rounds in range(100):
+            for c in (first, second, first, second) if rounds % 2 else (second, first, first, second):
+                c.launch()
+            assert torch.equal(masks, wants[1]), rounds
+        first.launch()
+        assert torch.equal(masks, wants[0])
+    H.check_status()
