@@ -5,6 +5,7 @@ There is no fallback: if the library is missing or a call fails, an exception is
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from pathlib import Path
@@ -19,6 +20,7 @@ CB2_ERR_RUNTIME = -2
 CB2_ERR_UNSUPPORTED = -3
 CB2_ERR_CUDA = -4
 CB2_PLAN_ROW_LISTS = 2
+CB2_CAPTURE_RELAXED = 2  # cudaStreamCaptureModeRelaxed
 
 EXPORTED_SYMBOLS = (
     "cb2_gemm_run",
@@ -43,6 +45,7 @@ EXPORTED_SYMBOLS = (
     "cb2_last_launch_info",
     "cb2_last_launch_cluster",
     "cb2_dense_tables_run",
+    "cb2_exchange_capture_mode",
     "cb2_gemm_sequence_workspace_size",
     "cb2_gemm_sequence_run",
 )
@@ -238,6 +241,8 @@ def load() -> ctypes.CDLL:
     L.cb2_gemm_sequence_run.argtypes = [ctypes.POINTER(GemmSequenceArgs), ctypes.c_void_p]
     L.cb2_dense_tables_run.restype = ctypes.c_int
     L.cb2_dense_tables_run.argtypes = [ctypes.POINTER(DenseTablesArgs), ctypes.c_void_p]
+    L.cb2_exchange_capture_mode.restype = ctypes.c_int
+    L.cb2_exchange_capture_mode.argtypes = [ctypes.POINTER(ctypes.c_int)]
     L.cb2_last_launch_info.restype = ctypes.c_int
     L.cb2_last_launch_info.argtypes = [ctypes.POINTER(ctypes.c_int)] * 3
     L.cb2_last_launch_cluster.restype = ctypes.c_int
@@ -291,6 +296,17 @@ def device_status() -> int:
     v = ctypes.c_int(0)
     raise_for(load().cb2_device_status(ctypes.byref(v)))
     return v.value
+
+
+@contextlib.contextmanager
+def beside_captures():
+    """Inside, this thread may allocate and wait while some stream is being captured; nothing of it is captured."""
+    mode = ctypes.c_int(CB2_CAPTURE_RELAXED)
+    raise_for(load().cb2_exchange_capture_mode(ctypes.byref(mode)))
+    try:
+        yield
+    finally:
+        raise_for(load().cb2_exchange_capture_mode(ctypes.byref(mode)))
 
 
 def kernel_table(which: str):

@@ -1162,6 +1162,14 @@ int cb2_gemm_sequence_run(const cb2_gemm_sequence_args *a, void *stream_v) {
 }
 
 // ---------------------------------------------------------------- tables of a dense convolution
+int cb2_exchange_capture_mode(int *mode) {
+  CB2_CHECK_ARG(mode != nullptr, "null arguments");
+  cudaStreamCaptureMode m = static_cast<cudaStreamCaptureMode>(*mode);
+  CB2_CUDA(cudaThreadExchangeStreamCaptureMode(&m));
+  *mode = m;
+  return CB2_OK;
+}
+
 int cb2_dense_tables_run(const cb2_dense_tables_args *a, void *stream_v) {
   CB2_CHECK_ARG(a != nullptr, "null arguments");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);

@@ -432,7 +432,7 @@ bool read_dense(PyObject *params, PyObject *tables, cb2_conv_args &g) {
   g.mask_width = wgrad ? 128 : -1;
   g.mask_filter = 0xffffffffu;
   fill_conv(p, d, ds, op, t, g);
-  g.reuse_plan = wgrad ? 0 : 1;  // an earlier call made the grid's tables, and nothing writes them again
+  g.reuse_plan = wgrad ? 0 : 1;  // the grid's tables were whole before the call, and nothing writes them again
   return true;
 }
 

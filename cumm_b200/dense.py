@@ -8,7 +8,8 @@ cumm/conv/input_iters.py:2353; harness cumm/conv/main_real.py:41-231, checked ag
 fill the grid: ``cb2_dense_tables_run`` writes the neighbour table of the geometry on the GPU
 (the reference's coordinate rule, in = out * stride - pad + r * dilation), every row carries every
 filter offset, rows keep their order, and the three operators run through the same sm_100a
-row-gather kernels.  Tables are cached per geometry and device."""
+row-gather kernels.  Tables are cached per geometry and device; they are whole before a call sees them, so that calls
+on any stream, captured ones among them, read them without waiting for anybody."""
 from __future__ import annotations
 
 import ctypes
@@ -55,7 +56,20 @@ def _geometry(params):
     return (batch, ext(in_dims, 1), ext(out_dims, 1), ext(ksize, 1), ext(stride, 1), ext(pad, 0), ext(dil, 1), C, K)
 
 
-def _tables(device: int, geom, stream: int) -> dict:
+def _idle_stream(device: int):
+    """A stream that nothing is being captured on."""
+    import torch
+    while True:
+        s = torch.cuda.Stream(device)
+        with torch.cuda.stream(s):
+            if not torch.cuda.is_current_stream_capturing():
+                return s
+
+
+def _tables(device: int, geom) -> dict:
+    """The tables of a geometry, the first time made on a stream of their own and waited for: they depend on nothing that
+    the call's stream holds, calls on other streams find them in the cache, and a captured call must not be the one that
+    writes them (they would be there only once its graph has run)."""
     import torch
     batch, in_dims, out_dims, ksize, stride, pad, dil, _, _ = geom
     key = (device, batch, tuple(in_dims), tuple(out_dims), tuple(ksize), tuple(stride), tuple(pad), tuple(dil))
@@ -68,28 +82,28 @@ def _tables(device: int, geom, stream: int) -> dict:
     words = (kv + 31) // 32
     dev = f"cuda:{device}"
     i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=dev)
-    t = dict(n_in=n_in, n_out=n_out, kv=kv, words=words,
-             indices_fwd=i32(kv, n_out), indices_bwd=i32(kv, n_in),
-             mask_fwd=i32(n_out, words) if words > 1 else i32(n_out), argsort_fwd=i32(n_out),
-             mask_bwd=i32(n_in, words) if words > 1 else i32(n_in), argsort_bwd=i32(n_in))
-    tiles = (n_out + 127) // 128
-    a = _lib.DenseTablesArgs()
-    a.batch = batch
-    for name, vals in (("in_dims", in_dims), ("out_dims", out_dims), ("ksize", ksize), ("stride", stride),
-                       ("pad", pad), ("dil", dil)):
-        arr = getattr(a, name)
-        for i in range(3):
-            arr[i] = int(vals[i])
-    for name in ("indices_fwd", "indices_bwd", "mask_fwd", "argsort_fwd", "mask_bwd", "argsort_bwd"):
-        setattr(a, name, t[name].data_ptr())
-    with torch.cuda.device(device):
-        _lib.raise_for(_lib.load().cb2_dense_tables_run(ctypes.byref(a), ctypes.c_void_p(int(stream))))
-    # the reduced masks of the weight gradient: every tile carries every offset
-    t["tile_masks"] = t["mask_fwd"][:tiles].clone()
+    stream = _idle_stream(device)
+    with _lib.beside_captures(), torch.cuda.stream(stream):
+        t = dict(n_in=n_in, n_out=n_out, kv=kv, words=words,
+                 indices_fwd=i32(kv, n_out), indices_bwd=i32(kv, n_in),
+                 mask_fwd=i32(n_out, words) if words > 1 else i32(n_out), argsort_fwd=i32(n_out),
+                 mask_bwd=i32(n_in, words) if words > 1 else i32(n_in), argsort_bwd=i32(n_in))
+        a = _lib.DenseTablesArgs()
+        a.batch = batch
+        for name, vals in (("in_dims", in_dims), ("out_dims", out_dims), ("ksize", ksize), ("stride", stride),
+                           ("pad", pad), ("dil", dil)):
+            arr = getattr(a, name)
+            for i in range(3):
+                arr[i] = int(vals[i])
+        for name in ("indices_fwd", "indices_bwd", "mask_fwd", "argsort_fwd", "mask_bwd", "argsort_bwd"):
+            setattr(a, name, t[name].data_ptr())
+        _lib.raise_for(_lib.load().cb2_dense_tables_run(ctypes.byref(a), ctypes.c_void_p(stream.cuda_stream)))
+        # the reduced masks of the weight gradient: every tile carries every offset
+        t["tile_masks"] = t["mask_fwd"][:(n_out + 127) // 128].clone()
+        stream.synchronize()
     t["native"] = tuple(t[name] for name in ("indices_fwd", "indices_bwd", "mask_fwd", "mask_bwd", "argsort_fwd",
                                              "argsort_bwd", "tile_masks"))
-    _TABLES[key] = t
-    return t
+    return _TABLES.setdefault(key, t)  # another thread's, if it was first: calls may be reading those
 
 
 def run_dense_conv(params, host=None) -> None:
@@ -115,7 +129,7 @@ def run_dense_conv(params, host=None) -> None:
     C, K = geom[7], geom[8]
     inp, weight, output = params.input, params.weight, params.output
     device = as_view(output).device
-    t = _tables(device, geom, int(params.stream))
+    t = _tables(device, geom)
     d = desp.copy()
     d.mask_sparse = True
     d.increment_k_first = True

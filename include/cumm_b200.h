@@ -177,7 +177,7 @@ typedef struct cb2_conv_args {
    *   leaves room for them (cb2_last_launch_cluster), on one otherwise; fp32 sums in a fixed order either way, as the
    *   weight gradient's, whose partial sums are cut by the number of CTAs.
    * reuse_plan, forward and backward input: bit 0 says that indice_ptr, mask_ptr and mask_argsort_ptr hold what they
-   *   held when an earlier, stream-ordered call read them.  An fp16 launch then reads them while its predecessor on the
+   *   held when an earlier, stream-ordered call read them, or that whoever wrote them had ended when the call was made.  An fp16 launch then reads them while its predecessor on the
    *   stream still runs; without it it waits first (int8 launches always read ahead).  That goes for what is read:
    *   mask_out_ptr is written behind the predecessor's end like the output.
    *   Backward weight: the workspace still holds the plan of an earlier, stream-ordered
@@ -343,6 +343,13 @@ typedef struct cb2_dense_tables_args {
 } cb2_dense_tables_args;
 
 int cb2_dense_tables_run(const cb2_dense_tables_args *args, void *stream);
+
+/*
+ * Sets the calling thread's cudaStreamCaptureMode to *mode and leaves the one it had there
+ * (cudaThreadExchangeStreamCaptureMode).  Relaxed (2), a host layer may allocate and fill what later calls share
+ * -- the tables above -- on a stream of its own while another stream is being captured.
+ */
+int cb2_exchange_capture_mode(int *mode);
 
 /*
  * Sum of one fp32 array per GPU over NVLink peer memory, for the weight gradient of a

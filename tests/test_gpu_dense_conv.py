@@ -147,3 +147,57 @@ def test_dense_calls_read_in_native_code_are_those_read_in_python(cuda_lib, shap
             run_dense_conv(p, _host())
     torch.cuda.synchronize()
     H.check_status()
+
+
+@pytest.mark.parametrize("first", ["on a busy stream", "captured"])
+def test_the_first_call_over_a_grid_makes_whole_tables(cuda_lib, first):
+    """The first call over a grid on a stream other than torch's, directly followed by calls on another one, while torch's
+    own stream is busy; and captured, with eager calls before the graph has run.  All three operators, against
+    the same calls with everything in between waited for, bit for bit."""
+    import torch
+    from cumm_b200.dense import _TABLES
+    shape, ksize, C, K = (2, 37, 45), (3, 3), 32, 48
+    half = lambda *s: torch.randn(s, device="cuda").half()
+    x, w, dout = half(*shape, C), half(K, *ksize, C), half(*shape, K)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def results():
+        return {ConvOpType.Forward: torch.zeros_like(dout), ConvOpType.BackwardInput: torch.zeros_like(x),
+                ConvOpType.BackwardWeight: torch.zeros_like(w)}
+
+    def call(op, made, stream):
+        p = dense_params(op, 2, C, K, (1, 1), (1, 1), (1, 1))
+        t = {ConvOpType.Forward: dout, ConvOpType.BackwardInput: x, ConvOpType.BackwardWeight: w}
+        t[op] = made[op]
+        p.input, p.weight, p.output = t[ConvOpType.BackwardInput], t[ConvOpType.BackwardWeight], t[ConvOpType.Forward]
+        p.stream, p.mask_width = stream.cuda_stream, 128
+        ConvMainUnitTest.implicit_gemm2(p)
+
+    want, made, eager = results(), results(), results()
+    for i, op in enumerate(want):  # the library's and torch's scratch is there before anything is captured
+        call(op, want, torch.cuda.default_stream())
+        call(op, want, streams[0])
+        torch.cuda.synchronize()
+    want = {op: t.clone() for op, t in want.items()}
+    big = half(4096, 4096)
+    torch.cuda.synchronize()
+    _TABLES.clear()
+    if first == "captured":
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=streams[0]):
+            for op in made:
+                call(op, made, streams[0])
+        for op in eager:
+            call(op, eager, streams[1])
+        streams[1].synchronize()
+        g.replay()
+    else:
+        for _ in range(20):
+            big @ big
+        for op in made:
+            call(op, made, streams[0])
+            call(op, eager, streams[1])
+    torch.cuda.synchronize()
+    H.check_status()
+    for op in want:
+        assert torch.equal(made[op], want[op]) and torch.equal(eager[op], want[op]), op
