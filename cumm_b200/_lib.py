@@ -9,6 +9,7 @@ import contextlib
 import ctypes
 import os
 from pathlib import Path
+from typing import Optional
 
 _HERE = Path(__file__).resolve().parent
 # CUMM_B200_LIBRARY: another build of the same library (e.g. one compiled with -DCB2_TRACE)
@@ -260,15 +261,31 @@ def host_path() -> Path:
     return _HERE / f"_host.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
 
 
+def host_sources() -> Optional[str]:
+    """A digest of what that extension is built from, which it carries: the records' layout and its own functions are
+    agreed with this package by their sources alone.  None where the sources are not there."""
+    import hashlib
+    h = hashlib.sha256()
+    try:
+        for path in (_HERE / "csrc" / "host_args.cpp", _HERE.parent / "include" / "cumm_b200.h"):
+            h.update(path.read_bytes())
+    except OSError:
+        return None
+    return h.hexdigest()[:16]
+
+
 def load_host():
-    """That extension; None, with a warning, where there is none for this torch and this Python: the Python layer
-    reads the records itself, which takes longer and gives the same calls."""
+    """That extension; None, with a warning, where there is none for this torch, this Python and these sources: the Python
+    layer reads the records itself, which takes longer and gives the same calls."""
     import importlib.util
     import warnings
     try:
         spec = importlib.util.spec_from_file_location("cumm_b200._host", host_path())
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
+        sources = host_sources()
+        if sources is not None and getattr(module, "SOURCES", None) != sources:
+            raise ImportError(f"{host_path().name} was built from other sources")
     except ImportError as e:
         warnings.warn(f"the native reader of parameter records does not load ({e}); a call takes 8 to 12 us longer on "
                       "the host (run `python -c 'import cumm_b200.build as b; b.build()'`)", RuntimeWarning, stacklevel=2)

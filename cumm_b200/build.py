@@ -8,7 +8,7 @@ import subprocess
 import warnings
 from pathlib import Path
 
-from ._lib import host_path
+from ._lib import host_path, host_sources
 
 _HERE = Path(__file__).resolve().parent
 CSRC = _HERE / "csrc"
@@ -43,7 +43,8 @@ def _build_host() -> None:
     if cxx is None:
         raise RuntimeError("g++ not found")
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", str(host_path())]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DCB2_HOST_SOURCES="{host_sources()}"', "-o", str(host_path())]
     cmd += ["-I" + p for p in (sysconfig.get_paths()["include"], str(root / "include"),
                                str(root / "include" / "torch" / "csrc" / "api" / "include"))]
     cmd += [str(CSRC / s) for s in HOST_SOURCES]

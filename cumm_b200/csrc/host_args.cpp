@@ -564,5 +564,12 @@ PyMODINIT_FUNC PyInit__host(void) {
     return nullptr;
   CB2_NAMES(X)
 #undef X
-  return PyModule_Create(&module);
+  PyObject *m = PyModule_Create(&module);
+#ifdef CB2_HOST_SOURCES  // a digest of this file and the header, by which the Python layer knows its own reader
+  if (m && PyModule_AddStringConstant(m, "SOURCES", CB2_HOST_SOURCES) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+#endif
+  return m;
 }

@@ -495,3 +495,23 @@ def test_the_native_reader_may_be_missing(monkeypatch, tmp_path):
     with pytest.warns(RuntimeWarning, match="was not built"):
         assert build.build(force=True) == build.OUT
     assert built == [False]
+
+
+def test_a_reader_built_from_other_sources_is_not_used(monkeypatch, tmp_path):
+    """An extension of the right name that an older tree left behind, with fewer functions: a warning, and the Python
+    layer reads every record."""
+    import shutil
+    import subprocess
+    import sysconfig
+    import torch  # noqa: F401
+    if shutil.which("gcc") is None:
+        pytest.skip("no C compiler")
+    source = tmp_path / "old.c"
+    source.write_text('#include <Python.h>\nstatic struct PyModuleDef m = {PyModuleDef_HEAD_INIT, "_host", 0, -1, 0};\n'
+                      'PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&m); }\n')
+    old = tmp_path / _lib.host_path().name
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], str(source), "-o", str(old)], check=True)
+    assert _lib.load_host().SOURCES == _lib.host_sources()
+    monkeypatch.setattr(_lib, "host_path", lambda: old)
+    with pytest.warns(RuntimeWarning, match="built from other sources"):
+        assert _lib.load_host() is None
