@@ -86,6 +86,15 @@ __device__ __forceinline__ bool elect_one() {
   return one != 0;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// A kernel launched with the programmatic-serialisation attribute may start while the kernel
+// before it on the stream still runs; it must not touch that kernel's results before
+// grid_dep_wait(), which returns once the earlier grid has completed and its writes are visible.
+// grid_dep_launch() in the earlier kernel allows the later one to be scheduled from then on.
+// Both are no-ops for a kernel launched the ordinary way.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -131,7 +140,8 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
 
 // Time limit of every wait, in nanoseconds of the global timer.  Far above any legitimate
 // delay on this path (whole kernels run for tens of microseconds), far below anything an
-// operator would notice.
+// operator would notice.  A predecessor on the stream may take longer than that: who waits for something that comes
+// from behind its end has either waited for that end first or counts anew from there (UNDER).
 constexpr unsigned long long kWaitLimitNs = 1000ull * 1000ull * 1000ull;
 
 __device__ __forceinline__ unsigned long long global_timer_ns() {
@@ -140,26 +150,40 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   return t;
 }
 
+// Whether a wait has run out; asked now and then, the first time at its begin.
+template <bool UNDER> struct WaitClock {
+  unsigned long long t0 = 0;  // UNDER: odd from the predecessor's end on
+  __device__ __forceinline__ bool out(unsigned long long now) {
+    if (t0 < 2) {
+      t0 = UNDER ? (now & ~1ull) | t0 : now;
+    } else if (now - t0 > kWaitLimitNs) {
+      if (!UNDER || (t0 & 1))
+        return true;
+      grid_dep_wait();
+      t0 = 1;
+    }
+    return false;
+  }
+};
+
 // Bounded wait.  `abort_flag` (shared memory) is polled so that once any thread of the
 // CTA has given up, everybody else leaves quickly too.  Returns false on give-up.
 // A waiter only asks again: try_wait itself suspends the thread, and whoever sleeps between two of them wakes up late.
 // (Sleeping 20 ns, growing to 160, and not, forward, us: 60 000 scanned rows at 256 channels 94.0 and 90.4, 150 000 at 128
 // 61.3 and 59.1, 9000 17.6 and 16.9, 100 003 at 64 24.9 and 24.4; 20 000 uniform ones 9.0 and 8.5; int8, 150 000 scanned
 // rows 41.5 and 40.1, stride 2 from uniform ones 39.8 and 40.1; 16 tries before the first sleep lie half-way.)
+template <bool UNDER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
   if (mbar_test(bar, parity))
     return true;
-  unsigned long long t0 = 0;
+  WaitClock<UNDER> clock;
   for (uint32_t i = 0;; ++i) {
     if (mbar_test(bar, parity))
       return true;
     if ((i & 63u) == 63u) {
       if (*abort_flag)
         return false;
-      unsigned long long now = global_timer_ns();
-      if (t0 == 0)
-        t0 = now;
-      else if (now - t0 > kWaitLimitNs)
+      if (clock.out(global_timer_ns()))
         break;
     }
   }
@@ -167,18 +191,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
-// The same for a condition that the whole warp looks at together.
+// The same for a condition that the whole warp looks at together, under the predecessor or not.
 template <class Cond> __device__ __forceinline__ bool wait_for(Cond cond, volatile int *abort_flag) {
-  unsigned long long t0 = 0;
+  WaitClock<true> clock;
   for (uint32_t i = 0; !cond(); ++i) {
     __nanosleep(20);
     if ((i & 63u) == 63u) {
       const unsigned long long now = __shfl_sync(0xffffffffu, global_timer_ns(), 0);
       if (__any_sync(0xffffffffu, *abort_flag != 0))
         return false;
-      if (t0 == 0)
-        t0 = now;
-      else if (now - t0 > kWaitLimitNs) {
+      if (clock.out(now)) {
         *abort_flag = 1;
         return false;
       }
@@ -190,10 +212,11 @@ template <class Cond> __device__ __forceinline__ bool wait_for(Cond cond, volati
 // Warp-collective wait: lane 0 polls, the other lanes sleep at the shuffle.  Keeps the
 // number of spinning threads per SM small (one per warp), which matters because pollers
 // compete for issue slots with the warps that do the work.
+template <bool UNDER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
   int ok = 1;
   if (lane_id() == 0)
-    ok = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
+    ok = mbar_wait<UNDER>(bar, parity, abort_flag) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
@@ -226,15 +249,6 @@ __device__ __forceinline__ uint4 ld_shared_16(uint32_t addr) {
 __device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
 }
-
-// ---------------------------------------------------------------- programmatic dependent launch
-// A kernel launched with the programmatic-serialisation attribute may start while the kernel
-// before it on the stream still runs; it must not touch that kernel's results before
-// grid_dep_wait(), which returns once the earlier grid has completed and its writes are visible.
-// grid_dep_launch() in the earlier kernel allows the later one to be scheduled from then on.
-// Both are no-ops for a kernel launched the ordinary way.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- thread-block clusters
 __device__ __forceinline__ uint32_t cluster_rank() {

@@ -281,10 +281,11 @@ template <int MW> struct TileCursor {
   uint32_t m;
   unsigned long long lo, hi;  // four words
   // Returns 1 on a tile, 0 at the end, -1 when the wait gave up.  read(slot) runs before the slot is
-  // given back.  ALONE: one thread walks for its warp (the MMA issuer).
-  template <bool ALONE = false, class ReadFn>
+  // given back.  ALONE: one thread walks for its warp (the MMA issuer).  UNDER: the role walks before the predecessor's
+  // end, and the scheduler may wait for that.
+  template <bool ALONE = false, bool UNDER = false, class ReadFn>
   __device__ __forceinline__ int next(const RowConvParams &p, const RingView &rv, ReadFn read) {
-    const bool ok = mbar_wait(rv.full0 + 8u * slot, phase, rv.abort_flag);
+    const bool ok = mbar_wait<UNDER>(rv.full0 + 8u * slot, phase, rv.abort_flag);
     auto same = [](auto v) {
       if constexpr (ALONE)
         return v;
@@ -517,7 +518,7 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
       if (accounted < issued)
         ok = mbar_wait_warp(rv.landed0 + 8u * (accounted % rv.ring), (accounted / rv.ring) & 1, rv.abort_flag);
       else if (issued - released >= rv.ring)
-        ok = mbar_wait_warp(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1, rv.abort_flag);
+        ok = mbar_wait_warp<true>(rv.empty0 + 8u * (released % rv.ring), (released / rv.ring) & 1, rv.abort_flag);
       else if constexpr (!SPLIT)
         ok = wait_for([&]() { return within_budget(); }, rv.abort_flag);
       if (!ok)
@@ -796,7 +797,6 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     const bool sectors = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(p.ldo * Cfg::OES)) & 31u) == 0;
     int buf = 0;
     uint32_t acc_phase = 0;
-    bool dep_waited = false;
     auto next_acc = [&]() {
       if (++buf == Cfg::NUM_ACC) {
         buf = 0;
@@ -807,6 +807,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     // else that orders its clearing before them.
     if constexpr (SPLIT)
       named_bar_sync(1, Cfg::CLEARED_THREADS);
+    grid_dep_wait();
     CB2_PROF_BEGIN();
     TileCursor<MW> tc;
     int o = -1;  // destination row of this thread's tile row
@@ -825,10 +826,6 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
           }
           const int n0 = Cfg::PARTS ? tc.n0 : static_cast<int>(blockIdx.y) * BLOCK_N;
           CB2_PROF_MARK(0);  // walk
-          if (!dep_waited) {
-            grid_dep_wait();
-            dep_waited = true;
-          }
           if (!SPLIT && erow == 0 && half == 0 && p.mask_out && n0 == 0) {
             if constexpr (MW == 1) {
               p.mask_out[tile] = tc.m;  // forward: not reversed
@@ -1074,6 +1071,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       uint32_t a_phase = 0, b_phase = 1, acc_phase = 1;
       bool ok = true;
       volatile int *const progress = misc + 15;
+      grid_dep_wait();  // no operand comes before
       CB2_PROF_BEGIN();
       for (int more; ok && (more = tc.template next<true>(p, rv, [](const int *) {})) != 0;) {
         CB2_PROF_MARK(0);  // next tile
@@ -1271,7 +1269,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       uint32_t phase = 1;    // of this group's own stage
       TileCursor<MW> tc;
       int4 o = make_int4(-1, -1, -1, -1);
-      for (int more; ok && (more = tc.next(p, rv, [&](const int *sl) {
+      for (int more; ok && (more = tc.template next<false, true>(p, rv, [&](const int *sl) {
                              o = *reinterpret_cast<const int4 *>(sl + 8 + lane * 4);
                            })) != 0;) {
         ok = more > 0;
@@ -1368,7 +1366,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         o[r] = -1;
       const uint8_t *a_bytes = reinterpret_cast<const uint8_t *>(p.a);
       TileCursor<MW> tc;
-      for (int more; ok && (more = tc.next(p, rv, [&](const int *sl) {
+      for (int more; ok && (more = tc.template next<false, true>(p, rv, [&](const int *sl) {
                              // the rows this thread's gathers start from (sort index, or the row itself)
 #pragma unroll
                              for (int r = 0; r < RPT; ++r)

@@ -783,6 +783,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
     int stage = 0, acc_use = 0;
     uint32_t phase = 0;
     bool ok_all = true;
+    grid_dep_wait();  // no operand comes before
     // The lane that issues.  Elected, the descriptors stay in uniform registers and a step costs the issuer a third:
     // 100 003 scanned rows at 64 channels 40.2 -> 35.3 us, 30 011 rows of 125 offsets 31.7 -> 27.4.  At the widest
     // tiles, three stages, it makes no difference but on the largest scenes, which it slows down (128 channels, lane 0

@@ -383,3 +383,63 @@ def test_tile_masks_of_launches_in_a_row_come_in_their_order(cuda_lib, max_ctas)
         first.launch()
         assert torch.equal(masks, wants[0])
     H.check_status()
+
+
+def test_launches_behind_a_kernel_that_takes_longer_than_a_wait_may(cuda_lib):
+    """A forward pass, over fixed tables and over tables that may be new, and a weight gradient with a plan of its own, each
+    launched directly behind a forward pass that one CTA works at for 1.5 to 3 s.  They start beside it, and most of
+    their warps wait for those that wait for its end: no wait has run out, results are those of launches on their own."""
+    import torch
+    from cumm_b200.conv.main import ConvMainUnitTest
+    from cumm_b200.layer import DeviceTables, SparseConvLayer, make_desp
+    from cumm_b200.tensorview.gemm import ConvOpType, ConvParams, prepare_conv
+    half = lambda *s: torch.randn(s, device="cuda").half()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        C, K, kv = 1024, 2048, 27
+        w = half(K, kv, C)
+
+        def long_call(rows):
+            p = ConvParams(3, ConvOpType.Forward)
+            p.conv_algo_desp = make_desp(ConvOpType.Forward, False, C, K)
+            p.input, p.weight, p.output = half(rows, C), w, torch.empty((rows, K), dtype=torch.float16, device="cuda")
+            p.indices = torch.randint(0, rows, (kv, rows), dtype=torch.int32, device="cuda")
+            p.mask = torch.full((rows,), (1 << kv) - 1, dtype=torch.int32, device="cuda")
+            p.mask_argsort = torch.arange(rows, dtype=torch.int32, device="cuda")
+            p.max_ctas, p.stream = 1, stream.cuda_stream
+            return prepare_conv(p, static_tables=True)
+
+        def seconds(call):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            call.launch()
+            end.record()
+            stream.synchronize()
+            return begin.elapsed_time(end) / 1000
+
+        few = 128 * 16
+        trial = long_call(few)
+        seconds(trial)
+        long = long_call(int(few * 2 / seconds(trial)) // 128 * 128)
+        tb = W.build_tables(W.sample_coords(9000, 770, (8, 48, 48)), grid=(8, 48, 48))
+        n, c = tb.n_out, 64
+        t = DeviceTables.from_host(tb, "cuda")
+        x, dout, out, din = half(n, c), half(n, c), half(n, c), half(n, c)
+        dw = half(c, 27, c)
+        layer = SparseConvLayer(t, half(c, 27, c), x, out, dout, din, dw, stream=stream.cuda_stream)
+        for call, result in ((layer.fwd.launch, out), (lambda: ConvMainUnitTest.implicit_gemm2(layer.fwd_params), out),
+                             (layer.wgrad.launch, dw)):
+            for _ in range(2):
+                call()
+            stream.synchronize()
+            want = result.clone()
+            result.zero_()
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            long.launch()
+            call()
+            end.record()
+            stream.synchronize()
+            assert 1.2 < begin.elapsed_time(end) / 1000 < 5
+            H.check_status()
+            assert torch.equal(result, want)
