@@ -150,6 +150,18 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   return t;
 }
 
+// Waits, whatever the abort flag says, for copies or MMAs that are on their way: they must not find the shared or tensor
+// memory of the SM's next CTA.  For who gives up a short limit does, which all that was asked for keeps by far: a phase
+// that lacks somebody's arrival besides does not complete.
+constexpr unsigned long long kDrainLimitNs = kWaitLimitNs / 1000;
+__device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity, unsigned long long limit = kDrainLimitNs) {
+  const unsigned long long t0 = global_timer_ns();
+  while (!mbar_test(bar, parity))
+    if (global_timer_ns() - t0 > limit)
+      return false;
+  return true;
+}
+
 // Whether a wait has run out; asked now and then, the first time at its begin.
 template <bool UNDER> struct WaitClock {
   unsigned long long t0 = 0;  // UNDER: odd from the predecessor's end on

@@ -1173,14 +1173,11 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       }
       CB2_TRACE_CTA(2, (unsigned long long)steps);
       CB2_PROF_END();
-      if (!ok) {
+      if (!ok)
         fail(kStatusWaitTimeout);
-      } else {
-        // make sure every MMA has retired before TMEM is released
-        tc_commit(final_bar);
-        if (!mbar_wait(final_bar, 0, abort_flag))
-          fail(kStatusWaitTimeout);
-      }
+      tc_commit(final_bar);  // every MMA has retired before TMEM is released
+      if (!mbar_drain(final_bar, 0, kWaitLimitNs))
+        fail(kStatusWaitTimeout);
     }
     __syncwarp();
   } else if (warp == Cfg::TMA_WARP) {
@@ -1232,6 +1229,9 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     }
     if (!ok && lane == 0)
       fail(kStatusWaitTimeout);
+    if (*abort_flag)
+      for (int s = 0; s < Cfg::SB; ++s)  // slots before bslot were last filled in this round, the others in the one before
+        mbar_drain(Cfg::JOINT ? full_a(s) : full_b(s), s < bslot ? b_phase ^ 1u : b_phase);
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
@@ -1346,6 +1346,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       }
       if (!ok && lane == 0)
         fail(kStatusWaitTimeout);
+      if (*abort_flag)
+        mbar_drain(full_a(g), phase);  // the group's last copies
     } else {
       constexpr int GT = Cfg::GROUP_THREADS;
       constexpr int RPT = (128 + GT - 1) / GT;                  // tile rows whose index each thread fetches

@@ -843,9 +843,9 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
           }
           return true;
         });
-    if (ok_all && issuer()) {
-      tc_commit(final_bar);
-      if (!mbar_wait(final_bar, 0, abort_flag))
+    if (issuer()) {
+      tc_commit(final_bar);  // every MMA has retired before the stages are used anew and TMEM is released
+      if (!mbar_drain(final_bar, 0, kWaitLimitNs))
         fail(kStatusWaitTimeout);
     }
     __syncwarp();
@@ -935,7 +935,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
       load_order(cur, ca);
       load_order(nxt, na);
       load_rows(cur, ca, cb);
-      for (uint32_t phase = 1; cur.tile >= 0; phase ^= 1u) {
+      uint32_t phase = 1;
+      for (; cur.tile >= 0; phase ^= 1u) {
         const Step after = next_step();
         Rows fa;
         load_rows(nxt, na, nb);
@@ -980,6 +981,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
         cur = nxt, nxt = after;
         ca = na, cb = nb, na = fa;
       }
+      if (*abort_flag)
+        mbar_drain(full_s(g), phase);  // the group's last copies
     }
   } else {
     // ======================= the same with 16-byte cp.async: group g of 128 threads owns stage g

@@ -580,3 +580,50 @@ def test_timer_verbose_and_nvrtc_entry_point(torch, oracle, capsys, monkeypatch)
     torch.cuda.synchronize()
     H.assert_close_f16(p.output.cpu().numpy(), want, "forward through run_nvrtc_conv_kernel, opted in")
     H.check_status()
+
+
+def broken_and_whole(torch, kind, C):
+    """Two prepared calls over one scene of 40 000 rows, of whose second one's row indices one in twenty lies beyond the
+    operand; their results, and the broken call's index table beside the whole one."""
+    from cumm_b200.layer import DeviceTables
+    from cumm_b200.tensorview.gemm import prepare_conv
+    op = ConvOpType.BackwardWeight if kind == "wgrad" else ConvOpType.Forward
+    t = DeviceTables.from_host(W.build_tables(W.sample_coords(40000, 505, (41, 300, 300)), grid=(41, 300, 300)), "cuda")
+    broken = t.indices.clone()
+    broken[(torch.rand(broken.shape, device="cuda") < 0.05) & (broken >= 0)] = t.n_in
+    made = []
+    values = [torch.randint(-9, 10, s, device="cuda").to(torch.int8 if kind == "int8" else torch.float16)
+              for s in ((t.n_in, C), (C, 27, C), (t.n_out, C))]
+    for indices in (t.indices, broken):
+        p = ConvParams(3, op)
+        p.conv_algo_desp = H.conv_desp(op, C, C, int8_inference=kind == "int8")
+        p.input, p.weight, p.output = (v.clone() for v in values)
+        p.indices, p.mask, p.mask_argsort = indices, t.mask, t.mask_argsort
+        if kind == "int8":
+            p.scale, p.bias = torch.full((C,), 0.01, device="cuda"), torch.zeros(C, device="cuda")
+        if kind == "wgrad":
+            p.mask, p.mask_width, p.split_k_slices = t.mask_output, 128, 32
+        made += [prepare_conv(p), p.weight if kind == "wgrad" else p.output]
+    torch.cuda.synchronize()
+    return made, broken, t.indices
+
+
+ABORTED = pytest.mark.parametrize("kind,C", [("fwd", 64), ("fwd", 72), ("fwd", 128), ("int8", 128), ("wgrad", 64), ("wgrad", 128)])
+
+
+@ABORTED
+def test_a_launch_that_gave_up_leaves_nothing_behind(torch, kind, C):
+    """Row indices beyond the operand make roles give up with copies and MMAs on their way; the launches directly behind,
+    whose CTAs take over its shared and tensor memory, are right, bit for bit."""
+    (whole, out, bad, _), _, _ = broken_and_whole(torch, kind, C)
+    whole.launch()
+    torch.cuda.synchronize()
+    want = out.clone()
+    for rounds in range(2 if kind == "wgrad" else 30):
+        out.zero_()
+        torch.cuda.synchronize()
+        bad.launch()
+        whole.launch()
+        assert _lib.device_status() == 2
+        assert torch.equal(out, want), rounds
+    H.check_status()
