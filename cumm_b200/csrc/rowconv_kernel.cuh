@@ -605,8 +605,8 @@ __device__ __forceinline__ void scheduler_run(const RowConvParams &p, const Ring
           p.mask_out[(long long)item_tile * p.mask_words + w] = item_mask[w];
     }
   }
-  // the last CTA to run out of tiles puts the two counters back to zero for the next launch
-  if (ended && dynamic && lane == 0) {
+  // the last CTA to run out of tiles, or to give up, puts the two counters back to zero for the next launch
+  if (dynamic && lane == 0) {
     if (next_cnt != 0)  // an outstanding request must have been served before the counters may be reset
       asm volatile("" ::"r"(next_base) : "memory");
     __threadfence();

@@ -627,3 +627,22 @@ def test_a_launch_that_gave_up_leaves_nothing_behind(torch, kind, C):
         assert _lib.device_status() == 2
         assert torch.equal(out, want), rounds
     H.check_status()
+
+
+@ABORTED
+def test_a_record_whose_launch_gave_up_serves_again(torch, kind, C):
+    """The counters that a launch hands its tiles out by are back at zero when it has given up: the same record, whose
+    table has been put right, leaves no tile out."""
+    (whole, out, bad, bad_out), broken, indices = broken_and_whole(torch, kind, C)
+    whole.launch()
+    for rounds in range(1 if kind == "wgrad" else 5):
+        for _ in range(2):  # both pairs of counters
+            bad.launch()
+        assert _lib.device_status() == 2
+    broken.copy_(indices)
+    for rounds in range(4):
+        bad_out.zero_()
+        bad.launch()
+        torch.cuda.synchronize()
+        H.check_status()
+        assert torch.equal(bad_out, out), rounds
