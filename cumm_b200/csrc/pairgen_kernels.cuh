@@ -735,38 +735,28 @@ __global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const __grid_co
   // where this chunk's rows of digit t go: rows with smaller digits, then those of earlier chunks
   int before = 0, all = 0;
   // All loads in flight together: one after the other they were most of a pass, three times 25 of them still 3 us of a set of
-  // 150 000 rows (78.9 -> 75.9); for few chunks the 74 cost as much as they save (20 000 rows 57.2 -> 60.7).  The loop of
-  // one round, as it is written for chunks of few rows, is faster than its body alone there (72 and 78 us) and slower
-  // where a thread has eight rows (174 and 164, stride 2).
-  auto count = [&](auto many) {
+  // 150 000 rows (78.9 -> 75.9); for few chunks the 74 cost as much as they save (20 000 rows 57.2 -> 60.7).
+  auto count = [&](auto many, int c0) {
     constexpr int N = decltype(many)::value;
     int v[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      v[i] = i < s.n_chunks ? __ldg(s.hist + i * kSortBins + t) : 0;
+      v[i] = c0 + i < s.n_chunks ? __ldg(s.hist + (c0 + i) * kSortBins + t) : 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       all += v[i];
-      before += i < me ? v[i] : 0;
+      before += c0 + i < me ? v[i] : 0;
     }
   };
-  if (s.n_chunks <= 25) {
-    count(std::integral_constant<int, 25>());
-  } else if constexpr (FEW) {
-    for (int c0 = 0; c0 < s.n_chunks; c0 += kSortChunks) {
-      int v[kSortChunks];
-#pragma unroll
-      for (int i = 0; i < kSortChunks; ++i)
-        v[i] = c0 + i < s.n_chunks ? __ldg(s.hist + (c0 + i) * kSortBins + t) : 0;
-#pragma unroll
-      for (int i = 0; i < kSortChunks; ++i) {
-        all += v[i];
-        before += c0 + i < me ? v[i] : 0;
-      }
-    }
-  } else {
-    count(std::integral_constant<int, kSortChunks>());
-  }
+  // Never more chunks than kSortChunks.  Written as a loop of that one round all the same where a thread has four rows
+  // (72 us, straight 78), straight where it has eight (164 us, as a loop 174, stride 2): what the compiler makes of it.
+  if (s.n_chunks <= 25)
+    count(std::integral_constant<int, 25>(), 0);
+  else if constexpr (FEW)
+    for (int c0 = 0; c0 < s.n_chunks; c0 += kSortChunks)
+      count(std::integral_constant<int, kSortChunks>(), c0);
+  else
+    count(std::integral_constant<int, kSortChunks>(), 0);
   int total;
   s_base[t] = block_scan_512(all, s_warp, total) + before;
   const int begin = me * s.chunk, end = min(begin + s.chunk, s.n);
