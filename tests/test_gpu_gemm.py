@@ -286,6 +286,43 @@ def test_layer_sequence_in_one_launch(torch, oracle, n, C, K):
                                rtol=2e-2, atol=2e-2)
 
 
+def test_layer_sequence_launched_back_to_back(torch):
+    """A sequence has one pair of ticket counters and each launch adds to what the one before it left: many in a row,
+    eager and captured, give bit for bit what they give one at a time."""
+    from cumm_b200.sequence import prepare_gemm_sequence
+    grid, launches = (41, 200, 176), 24
+    tb = W.build_tables(W.sample_coords(30000, 83, grid), grid=grid)
+    rng = np.random.default_rng(84)
+    x = rng.standard_normal((tb.n_in, 64)).astype(np.float16)
+    w = (rng.standard_normal((64, 27, 64)) / 64).astype(np.float16)
+    out = torch.zeros((tb.n_out, 64), dtype=torch.float16, device="cuda")
+    stream = torch.cuda.Stream()
+    seq = prepare_gemm_sequence(_layer_as_calls(torch, tb, x, w, out), stream=stream.cuda_stream)
+    torch.cuda.synchronize()
+    for _ in range(launches):
+        seq.launch()
+        torch.cuda.synchronize()
+    want = out.clone()
+    assert int((want != 0).sum()) > want.numel() // 2
+    for rounds in range(10):
+        out.zero_()
+        torch.cuda.synchronize()
+        for _ in range(launches):
+            seq.launch()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want), rounds
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        for _ in range(launches):
+            seq.launch()
+    out.zero_()
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    H.check_status()
+
+
 def test_layer_sequence_refuses_calls_that_are_not_one_layer(torch):
     from cumm_b200.sequence import prepare_gemm_sequence
     grid = (8, 24, 24)

@@ -93,6 +93,7 @@ def test_kernel_volumes_above_32(torch, ksize, subm, stride):
 @pytest.mark.parametrize("n,shift,grid,kw", [
     # rows around the sort's chunk of 2048 and past 74 of them (the chunks grow)
     (2048, 0, (8, 24, 24), {}), (2049, 0, (8, 24, 24), {}), (151553, 0, (41, 200, 176), {}),
+    (151553, 0, (41, 400, 352), dict(ksize=(5, 5, 5))),
     # offsets that are not symmetric: the backward table is inverted, not mirrored
     (3000, 0, (8, 24, 24), dict(ksize=(2, 3, 3))), (3000, 0, (8, 24, 24), dict(pad=(0, 1, 1))),
     # grids of more than 2^32 cells: the hash table's tag is not the voxel itself

@@ -16,8 +16,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("env", [
     {"CUMM_B200_GATHER": "0", "CUMM_B200_PDL": "0", "CUMM_B200_STATIC_TILES": "1"},  # cp.async everywhere, plain launches, static tiles
-    {"CUMM_B200_GATHER": "2", "CUMM_B200_PDL": "2"},                                  # TMA gather everywhere, PDL for every kernel
-], ids=["cp.async+plain-launch+static-tiles", "tma-gather+pdl-everywhere"])
+    {"CUMM_B200_GATHER": "2", "CUMM_B200_PDL": "0"},                                  # TMA gather everywhere, plain launches, tickets
+], ids=["cp.async+plain-launch+static-tiles", "tma-gather+plain-launch"])
 def test_smoke_under_switches(cuda_lib, env):
     r = subprocess.run([sys.executable, "-c", "import __graft_entry__ as g; g.smoke()"], cwd=str(ROOT),
                        env={**os.environ, **env}, capture_output=True, text=True, timeout=600)
