@@ -321,13 +321,9 @@ bool conv_record(PyObject *params, PyObject *desp) {
 
 // The flat record of a convolution call whose tensors are on the current device.
 bool read_conv(PyObject *params, cb2_conv_args &g, bool with_weight_gradient) {
-  if (!g_run_conv || reinterpret_cast<PyObject *>(Py_TYPE(params)) != g_conv_params)
-    return false;
   const Record p{params};
-  if (!p.none(k_timer) || p.flag(k_verbose) || !p.is_tensor(k_output))
-    return false;
   Ref desp(p.get(k__conv_algo_desp));
-  if (reinterpret_cast<PyObject *>(Py_TYPE(desp.p)) != g_conv_desp)
+  if (!conv_record(params, desp.p))
     return false;
   const Record d{desp.p};
   const int op = d.small(k_op_type);
