@@ -15,7 +15,7 @@ from typing import Optional, Sequence
 
 from . import _lib
 from .tensorview import as_view
-from .tensorview.gemm import GemmParams, _gemm_args
+from .tensorview.gemm import GemmParams, _gemm_args, _on
 
 
 class PreparedGemmSequence:
@@ -40,7 +40,8 @@ class PreparedGemmSequence:
         need = L.cb2_gemm_sequence_workspace_size(ctypes.byref(a))
         if need == 0:
             raise ValueError("a sequence holds 1 to 32 calls")
-        self._ws = torch.empty(need, dtype=torch.uint8, device=f"cuda:{self._device}")
+        with _on(self._device, self._stream):
+            self._ws = torch.empty(need, dtype=torch.uint8, device=f"cuda:{self._device}")
         a.workspace, a.workspace_bytes = self._ws.data_ptr(), need
         self._args = a
         self._L = L

@@ -547,17 +547,30 @@ _WORKSPACES = {}
 _NO_ROOM = {}  # (device, stream) -> the fewest bytes that could not be had
 
 
-def _scratch(device: int, nbytes: int, best: int, have=None):
+def _on(device: int, stream: int):
+    """The stream that a record names as torch's current one.  What a call owns is allocated and filled there: elsewhere
+    its memory could still be in use by work of torch's own stream, and be given away while the call's launches run."""
+    import contextlib
+
+    import torch
+    if not torch.cuda.is_initialized() or torch.cuda.current_stream(device).cuda_stream == stream:
+        return contextlib.nullcontext()
+    legacy = stream in (0, 1)  # two names of one stream
+    return torch.cuda.stream(torch.cuda.default_stream(device) if legacy else torch.cuda.ExternalStream(stream, device))
+
+
+def _scratch(device: int, stream: int, nbytes: int, best: int, have=None):
     """A buffer of ``best`` bytes; where the card has no room for those, ``have`` or a new one of ``nbytes``,
     which are enough."""
     import torch
-    if best > nbytes:
-        try:
-            return torch.empty(best, dtype=torch.uint8, device=f"cuda:{device}")
-        except torch.cuda.OutOfMemoryError:
-            if have is not None and have.numel() >= nbytes:
-                return have
-    return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{device}")
+    with _on(device, stream):
+        if best > nbytes:
+            try:
+                return torch.empty(best, dtype=torch.uint8, device=f"cuda:{device}")
+            except torch.cuda.OutOfMemoryError:
+                if have is not None and have.numel() >= nbytes:
+                    return have
+        return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{device}")
 
 
 def _workspace_for(device: int, stream: int, nbytes: int, user_ws, best: int = 0):
@@ -580,7 +593,7 @@ def _workspace_for(device: int, stream: int, nbytes: int, user_ws, best: int = 0
     if best >= _NO_ROOM.get(key, best + 1):
         best = 0
     if buf is None or buf.numel() < max(nbytes, best):
-        buf = _WORKSPACES[key] = _scratch(device, nbytes, best, buf)
+        buf = _WORKSPACES[key] = _scratch(device, stream, nbytes, best, buf)
         if buf.numel() < best:
             _NO_ROOM[key] = best
     return buf.data_ptr(), buf.numel()
@@ -963,7 +976,8 @@ class PreparedCall:
     tile-ticket counters (``sched_scratch``), so a captured launch shares them with nobody --
     two pairs, used in turn: with programmatic dependent launch a launch may start drawing
     tickets while its predecessor on the stream still runs, and that predecessor can be the
-    same call.
+    same call.  What the record owns is made on the stream that its parameters name; ``launch`` on another one is ordered
+    behind that by the caller.
     ``static_tables``: the caller promises that the neighbour tables (for the weight gradient:
     the reduced masks) keep their contents while the call is in use; from the second launch on the
     weight gradient then does without planning its schedule, and the other convolutions read their
@@ -976,7 +990,8 @@ class PreparedCall:
         self._device = device
         self._stream = int(stream)
         self._keep = keep  # tensors whose memory the record points at
-        self._tickets = torch.zeros(8, dtype=torch.int32, device=f"cuda:{device}")
+        with _on(device, self._stream):
+            self._tickets = torch.zeros(8, dtype=torch.int32, device=f"cuda:{device}")
         self._turn = 0
         args.sched_scratch = self._tickets.data_ptr()
         self._fixed = bool(static_tables) and (bool(args.workspace) or
@@ -1000,7 +1015,7 @@ def _attach_workspace(L, args, params, keep, size_fn, best_fn=None) -> None:
     if need:
         t = as_view(params.workspace)
         if t is None or t.nbytes() < need:
-            ws = _scratch(args._device, need, best_fn(ctypes.byref(args)) if best_fn is not None else 0)
+            ws = _scratch(args._device, int(params.stream), need, best_fn(ctypes.byref(args)) if best_fn is not None else 0)
             keep.append(ws)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
         else:

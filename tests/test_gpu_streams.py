@@ -443,3 +443,36 @@ def test_launches_behind_a_kernel_that_takes_longer_than_a_wait_may(cuda_lib):
             assert 1.2 < begin.elapsed_time(end) / 1000 < 5
             H.check_status()
             assert torch.equal(result, want)
+
+
+def test_a_prepared_call_is_ready_on_its_own_stream(cuda_lib):
+    """Prepared while torch's own stream is busy and launched on the call's stream at once: the ticket counters are zero
+    there, and neither they nor the scratch lie where memory of torch's stream was given back."""
+    import torch
+    from cumm_b200.layer import DeviceTables, SparseConvLayer
+    t = DeviceTables.from_host(W.build_tables(W.sample_coords(20000, 780, (41, 100, 100)), grid=(41, 100, 100)), "cuda")
+    half = lambda *s: (torch.randn(s, device="cuda") / 8).half()
+    x, dout, w = half(t.n_in, 64), half(t.n_out, 64), half(64, 27, 64)
+    big = half(8192, 8192)
+
+    def launched(stream, busy):
+        outs = torch.zeros_like(dout), torch.zeros_like(x), torch.zeros_like(w)
+        ones = [torch.ones(n, dtype=torch.int32, device="cuda") for n in [8] * 6 + [1 << 20] * 6]
+        torch.cuda.synchronize()
+        for _ in range(busy):
+            big @ big
+        del ones  # free again, for torch's own stream
+        layer = SparseConvLayer(t, w, x, outs[0], dout, outs[1], outs[2], stream=stream.cuda_stream)
+        for call in (layer.fwd, layer.dgrad, layer.wgrad):
+            call.launch()
+            call.launch()
+        stream.synchronize()
+        assert not busy or not torch.cuda.current_stream().query()
+        torch.cuda.synchronize()
+        H.check_status()
+        return outs
+
+    want = launched(torch.cuda.current_stream(), 0)
+    for rounds in range(3):
+        for a, b in zip(launched(torch.cuda.Stream(), 30), want):
+            assert torch.equal(a, b), rounds
