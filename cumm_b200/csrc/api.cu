@@ -199,9 +199,10 @@ cudaError_t launch_after(int cluster, Kern kern, dim3 grid, dim3 block, size_t s
 // How many CTAs share an item's filter offsets in a launch whose items leave most SMs idle: 4 or 8 where the clusters
 // fit the CTAs the launch may have and are all resident at once (each has one item; 148 SMs hold 33 clusters of four and
 // 15 of eight), else 1, and the ordinary kernel runs.  Four from two offsets a CTA on, eight from
-// eight.  That line was laid before every launch overlapped its predecessor; by the figures now four CTAs pay from 16 offsets on,
-// at 128 channels from 12.  It stays where callers (cb2_last_launch_cluster) and tests know it.  (One forward after the other over
-// fixed tables, us, one CTA and four.  8 offsets: crops of 1000, 1900 and 3800 rows at 64 channels 4.8 and 6.2, 5.0 and 6.3,
+// eight: with ordinary launches both sides were even there (8 offsets, 2000 and 3800 rows at 64 channels, us, one CTA and
+// four: 8.8 and 8.8, 9.6 and 9.6).  Overlap with the predecessor has since done more for one CTA than for four, which pay from 16
+// offsets on now, at 128 channels from 12; the line has not followed.  (One forward after the other over fixed tables, us, one CTA
+// and four.  8 offsets: crops of 1000, 1900 and 3800 rows at 64 channels 4.8 and 6.2, 5.0 and 6.3,
 // 5.6 and 9.2, 1900 at 128 7.8 and 7.7; 12: 5.8 and 6.3, 6.5 and 6.7, 6.8 and 9.4, at 128 10.2 and 8.5; 18: 7.7 and 7.0, 8.3 and 7.3, 8.5
 // and 10.0, 13.4 and 9.4; 27: 10.0 and 7.5, 10.7 and 7.9, 11.1 and 10.8, 18.2 and 10.5, scanned scenes of 2000 rows 9.5 and 7.1, uniform
 // ones, whose tiles stay with one CTA of the cluster, 3.9 and 4.5.  125 offsets at 32 channels, one CTA, four and eight: crops of 1900
