@@ -151,8 +151,9 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 }
 
 // Waits, whatever the abort flag says, for copies or MMAs that are on their way: they must not find the shared or tensor
-// memory of the SM's next CTA.  For who gives up a short limit does, which all that was asked for keeps by far: a phase
-// that lacks somebody's arrival besides does not complete.
+// memory of the SM's next CTA.  Every role does so for its last ones before it leaves, as it cannot know who gives up after
+// it.  For copies a short limit does, which all that was asked for keeps by far: a phase that lacks the arrival of somebody
+// who gave up does not complete.
 constexpr unsigned long long kDrainLimitNs = kWaitLimitNs / 1000;
 __device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity, unsigned long long limit = kDrainLimitNs) {
   const unsigned long long t0 = global_timer_ns();

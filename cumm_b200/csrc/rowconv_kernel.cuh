@@ -1229,9 +1229,8 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
     }
     if (!ok && lane == 0)
       fail(kStatusWaitTimeout);
-    if (*abort_flag)
-      for (int s = 0; s < Cfg::SB; ++s)  // slots before bslot were last filled in this round, the others in the one before
-        mbar_drain(Cfg::JOINT ? full_a(s) : full_b(s), s < bslot ? b_phase ^ 1u : b_phase);
+    for (int s = 0; s < Cfg::SB; ++s)  // slots before bslot were last filled in this round, the others in the one before
+      mbar_drain(Cfg::JOINT ? full_a(s) : full_b(s), s < bslot ? b_phase ^ 1u : b_phase);
     __syncwarp();
   } else if (warp == Cfg::SCHED_WARP) {
     // ======================= scheduler: draws tiles, publishes their masks and row numbers
@@ -1346,8 +1345,7 @@ rowconv_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
       }
       if (!ok && lane == 0)
         fail(kStatusWaitTimeout);
-      if (*abort_flag)
-        mbar_drain(full_a(g), phase);  // the group's last copies
+      mbar_drain(full_a(g), phase);  // the group's last copies
     } else {
       constexpr int GT = Cfg::GROUP_THREADS;
       constexpr int RPT = (128 + GT - 1) / GT;                  // tile rows whose index each thread fetches

@@ -981,8 +981,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dout, const __grid_constan
         cur = nxt, nxt = after;
         ca = na, cb = nb, na = fa;
       }
-      if (*abort_flag)
-        mbar_drain(full_s(g), phase);  // the group's last copies
+      mbar_drain(full_s(g), phase);  // the group's last copies
     }
   } else {
     // ======================= the same with 16-byte cp.async: group g of 128 threads owns stage g
